@@ -1,12 +1,11 @@
-// A decaying matrix state walked in chunks of CS_CHUNK tokens: the kernels that scalar_scan.cu and decay_scan.cu share
-// for steps of many tokens.  Per head, with S0 the state before a chunk,
+// A decaying matrix state walked in chunks of CS_CHUNK tokens: the kernels of decay_scan.cu for steps of many tokens.  Per head, with S0 the state before a chunk,
 //
 //     S_end[j, i] = d_i S0[j, i] + sum_s v_s[j] (w_s k_s[i]),
-//     o_t[j]      = f_t sum_i q_t[i] S0[j, i] + sum_{s <= t} P[t, s] v_s[j]   (+ skip v_t[j]).
+//     o_t[j]      = f_t sum_i q_t[i] S0[j, i] + sum_{s <= t} P[t, s] v_s[j].
 //
-// "By token" (CHANNEL false): one decay a token and head; d_i = e^(c_last), w_s = e^(c_last - c_s) b_s, f_t = e^(c_t) q_scale
-// with c the running sum of log a over the chunk, and P[t, s] = (q_t . k_s) e^(c_t - c_s) b_s q_scale from the products
-// q_t . k_s, which the heads of a group share.  "By channel": q, k, d and P come prepared, w = f = 1.
+// "By head" (CHANNEL false): one decay a head; d_i = e^(c_last), w_s = e^(c_last - c_s), f_t = e^(c_t) q_scale
+// with c the running sum of log a over the chunk, and P[t, s] = (q_t . k_s) e^(c_t - c_s) q_scale from the products
+// q_t . k_s.  "By channel": q, k, d and P come prepared, w = f = 1.
 // cs_walk_kernel has a tile of a head's state in registers, walks the sequence's chunks and leaves the state before every
 // chunk; that is all that is sequential.  cs_output_kernel then works on all chunks at once.  Everything is float32 on the CUDA
 // cores: both are bound by the multiply-adds and the shared-memory loads that feed them.
@@ -20,21 +19,18 @@
 #define CS_THREADS 128
 
 struct CsArgs {
-    const float *q, *k, *v;             // rows of the step's tokens; head h reads the columns (h / heads_per_group) dk, the same, h dv
+    const float *q, *k, *v;             // rows of the step's tokens; head h reads the columns h dk, h dk, h dv
     int ldq, ldk, ldv;
-    const float *log_a, *b;             // by token: [N, n_heads] with row strides; b null: 1
-    int ld_a, ld_b;
-    const float* head_decay;            // [n_heads], with log_a null: the decay itself
+    const float* head_decay;            // by head: [n_heads]
     const float* ed;                    // by channel: the chunks' decays [chunk][n_heads * dk]
-    const double* c;                    // by token: the running sums of log a [chunk][head][CS_CHUNK]
-    const float *w, *d;                 // by token: w_s [chunk][head][CS_CHUNK] and d [chunk][head]
-    const float* P;                     // by token: q . k [chunk][group][CS_CHUNK][CS_CHUNK]; by channel: P [chunk][head][..][..]
-    const float *skip, *m_tok;          // [n_heads] or null; [N, n_heads]: the state has a normalizer column, o is divided
+    const double* c;                    // by head: the running sums of log a [chunk][head][CS_CHUNK]
+    const float *w, *d;                 // by head: w_s [chunk][head][CS_CHUNK] and d [chunk][head]
+    const float* P;                     // by head: q . k [chunk][head][CS_CHUNK][CS_CHUNK]; by channel: P [chunk][head][..][..]
     float q_scale;
-    float *state, *before;              // [slot][head][cols][dk]; [chunk][head][cols][lds]: the state before every chunk
+    float *state, *before;              // [slot][head][dv][dk]; [chunk][head][dv][lds]: the state before every chunk
     const int *slots, *cu;
     float* o;                           // [N, n_heads * dv]
-    int n_heads, heads_per_group, dk, dv, lds, wide;
+    int n_heads, dk, dv, lds, wide;
 };
 
 namespace {
@@ -87,11 +83,6 @@ __device__ __forceinline__ double2 cs_running(float l0, float l1) {
     return make_double2(before + l0, run);
 }
 
-__device__ __forceinline__ float cs_log_a(const CsArgs& a, size_t row, int h) {
-    // a decay of exactly 0 has no logarithm; e^-80 stands in for it (what is left of the state then lies 35 decimal places down)
-    return a.log_a ? a.log_a[row * a.ld_a + h] : fmaxf(logf(a.head_decay[h]), -80.f);
-}
-
 // What follows from the decays alone, a warp a chunk and head: the running sums, w and d.
 __global__ void __launch_bounds__(CS_THREADS)
 cs_factors_kernel(const CsArgs a, double* __restrict__ c_out, float* __restrict__ w_out, float* __restrict__ d_out) {
@@ -100,14 +91,15 @@ cs_factors_kernel(const CsArgs a, double* __restrict__ c_out, float* __restrict_
     const int row0 = a.cu[b], len = a.cu[b + 1] - row0;
     if (c * CS_CHUNK >= len || h >= a.n_heads) return;
     const int nt = min(CS_CHUNK, len - c * CS_CHUNK);
-    const size_t row = (size_t)row0 + c * CS_CHUNK + 2 * lane, at = (size_t)(row0 / CS_CHUNK + b + c) * a.n_heads + h;
+    const size_t at = (size_t)(row0 / CS_CHUNK + b + c) * a.n_heads + h;
     const bool in0 = 2 * lane < nt, in1 = 2 * lane + 1 < nt;
-    const float b0 = in0 ? (a.b ? a.b[row * a.ld_b + h] : 1.f) : 0.f, b1 = in1 ? (a.b ? a.b[(row + 1) * a.ld_b + h] : 1.f) : 0.f;
-    const double2 run = cs_running(in0 ? cs_log_a(a, row, h) : 0.f, in1 ? cs_log_a(a, row + 1, h) : 0.f);
+    // a decay of exactly 0 has no logarithm; e^-80 stands in for it (what is left of the state then lies 35 decimal places down)
+    const float log_a = fmaxf(logf(a.head_decay[h]), -80.f);
+    const double2 run = cs_running(in0 ? log_a : 0.f, in1 ? log_a : 0.f);
     const double last = __shfl_sync(0xffffffffu, run.y, 31);
     *reinterpret_cast<double2*>(c_out + at * CS_CHUNK + 2 * lane) = run;
     *reinterpret_cast<float2*>(w_out + at * CS_CHUNK + 2 * lane) =
-        make_float2(in0 ? expf((float)(last - run.x)) * b0 : 0.f, in1 ? expf((float)(last - run.y)) * b1 : 0.f);
+        make_float2(in0 ? expf((float)(last - run.x)) : 0.f, in1 ? expf((float)(last - run.y)) : 0.f);
     if (lane == 0) d_out[at] = expf((float)last);
 }
 
@@ -124,18 +116,17 @@ cs_walk_kernel(const CsArgs a) {
     float* ks = cw_smem;                                // [STAGES][SUB][64]
     float* vs = ks + STAGES * SUB * 64;                 // [STAGES][SUB][JT]
     float* ws = vs + STAGES * SUB * JT;                 // [STAGES][SUB]
-    float4* meet = reinterpret_cast<float4*>(ws + STAGES * SUB);    // [GROUPS - 1][TJ + 1][CS_THREADS]
+    float4* meet = reinterpret_cast<float4*>(ws + STAGES * SUB);    // [GROUPS - 1][TJ][CS_THREADS]
     mv_pdl_begin();
     const int tiles_i = (a.dk + 63) / 64, i0 = (blockIdx.x % tiles_i) * 64, j0 = (blockIdx.x / tiles_i) * JT;
     const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, grp = tid / CS_THREADS, lt = tid % CS_THREADS, ti = lt & 15, tj = lt >> 4;
     const int row0 = a.cu[b], len = a.cu[b + 1] - row0;
     if (len <= 0) return;
-    const bool norm = a.m_tok != nullptr, with_n = norm && j0 == 0;
-    const int cols = a.dv + (norm ? 1 : 0), slot = mv_read_slot(a.slots[b]);
+    const int slot = mv_read_slot(a.slots[b]);
     const int i = i0 + ti * 4, j = j0 + tj * TJ;
-    float* st = a.state + ((size_t)slot * a.n_heads + h) * cols * a.dk;
+    float* st = a.state + ((size_t)slot * a.n_heads + h) * a.dv * a.dk;
     const bool vec = a.dk % 4 == 0;                     // the state's rows start on 16 bytes
-    float S[TJ][4], n[4] = {0.f, 0.f, 0.f, 0.f};
+    float S[TJ][4];
     auto read4 = [&](const float* p, float* out) {
         float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
         if (vec && i < a.dk) r = *reinterpret_cast<const float4*>(p + i);
@@ -154,8 +145,7 @@ cs_walk_kernel(const CsArgs a) {
 #pragma unroll
             for (int x = 0; x < 4; ++x) S[y][x] = 0.f;
     }
-    if (with_n && grp == 0) read4(st + (size_t)a.dv * a.dk, n);
-    const float* kp = a.k + (size_t)row0 * a.ldk + (size_t)(h / a.heads_per_group) * a.dk + i0;
+    const float* kp = a.k + (size_t)row0 * a.ldk + (size_t)h * a.dk + i0;
     const float* vp = a.v + (size_t)row0 * a.ldv + (size_t)h * a.dv + j0;
     const int n_sub = (len + SUB - 1) / SUB, chunk0 = row0 / CS_CHUNK + b;
     auto load = [&](int sub) {
@@ -182,25 +172,23 @@ cs_walk_kernel(const CsArgs a) {
     // the other groups' sums go into the first group's
     auto join = [&]() {
         if (grp > 0) {
-            float4* m = meet + (size_t)(grp - 1) * (TJ + 1) * CS_THREADS + lt;
+            float4* m = meet + (size_t)(grp - 1) * TJ * CS_THREADS + lt;
 #pragma unroll
             for (int y = 0; y < TJ; ++y) {
                 m[y * CS_THREADS] = make_float4(S[y][0], S[y][1], S[y][2], S[y][3]);
                 S[y][0] = S[y][1] = S[y][2] = S[y][3] = 0.f;
             }
-            if (with_n) { m[TJ * CS_THREADS] = make_float4(n[0], n[1], n[2], n[3]); n[0] = n[1] = n[2] = n[3] = 0.f; }
         }
         __syncthreads();
         if (grp == 0) {
 #pragma unroll
             for (int q = 0; q < GROUPS - 1; ++q) {
-                const float4* m = meet + (size_t)q * (TJ + 1) * CS_THREADS + lt;
+                const float4* m = meet + (size_t)q * TJ * CS_THREADS + lt;
 #pragma unroll
                 for (int y = 0; y < TJ; ++y) {
                     const float4 r = m[y * CS_THREADS];
                     S[y][0] += r.x; S[y][1] += r.y; S[y][2] += r.z; S[y][3] += r.w;
                 }
-                if (with_n) { const float4 r = m[TJ * CS_THREADS]; n[0] += r.x; n[1] += r.y; n[2] += r.z; n[3] += r.w; }
             }
         }
     };
@@ -209,20 +197,17 @@ cs_walk_kernel(const CsArgs a) {
             const int c = sub;
             if (GROUPS > 1 && c > 0) join();
             // the state as it is before this chunk
-            float* to = a.before + ((size_t)(chunk0 + c) * a.n_heads + h) * cols * a.lds;
+            float* to = a.before + ((size_t)(chunk0 + c) * a.n_heads + h) * a.dv * a.lds;
             if (grp == 0 && i < a.lds) {
 #pragma unroll
                 for (int y = 0; y < TJ; ++y)
                     if (j + y < a.dv)
                         *reinterpret_cast<float4*>(to + (size_t)(j + y) * a.lds + i) = make_float4(S[y][0], S[y][1], S[y][2], S[y][3]);
-                if (with_n && tj == 0) *reinterpret_cast<float4*>(to + (size_t)a.dv * a.lds + i) = make_float4(n[0], n[1], n[2], n[3]);
             }
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
+            for (int x = 0; x < 4; ++x)
 #pragma unroll
                 for (int y = 0; y < TJ; ++y) S[y][x] *= d_next[x];
-                n[x] *= d_next[x];
-            }
             if ((c + 1) * CS_CHUNK < len) decay(c + 1);
         }
         cs_wait<STAGES - 2>();
@@ -256,7 +241,6 @@ cs_walk_kernel(const CsArgs a) {
                     S[y][0] = fmaf(k[s].x, vy, S[y][0]); S[y][1] = fmaf(k[s].y, vy, S[y][1]);
                     S[y][2] = fmaf(k[s].z, vy, S[y][2]); S[y][3] = fmaf(k[s].w, vy, S[y][3]);
                 }
-                if (with_n) { n[0] += k[s].x; n[1] += k[s].y; n[2] += k[s].z; n[3] += k[s].w; }
             }
         }
     }
@@ -272,7 +256,6 @@ cs_walk_kernel(const CsArgs a) {
 #pragma unroll
         for (int y = 0; y < TJ; ++y)
             if (j + y < a.dv) write4(st + (size_t)(j + y) * a.dk, S[y]);
-        if (with_n && tj == 0) write4(st + (size_t)a.dv * a.dk, n);
     }
 }
 
@@ -281,7 +264,7 @@ cs_walk_kernel(const CsArgs a) {
 // come in slices of 32 key channels, the next slice on its way; rows of 36 floats keep the 16-byte reads of neighbouring rows
 // apart in the banks, and the state's rows are laid down so that a thread's four columns lie together in the result.
 constexpr int CO_LD = 36, CO_PLD = CS_CHUNK + 4;
-constexpr size_t CO_SMEM = sizeof(float) * (2 * 2 * 64 * CO_LD + CS_CHUNK * 64 + 4 * CS_CHUNK);
+constexpr size_t CO_SMEM = sizeof(float) * (2 * 2 * 64 * CO_LD + CS_CHUNK * 64 + 2 * CS_CHUNK);
 static_assert(CS_CHUNK * CO_PLD <= 2 * 64 * CO_LD, "P takes one stage's place");
 
 template <bool CHANNEL>
@@ -291,8 +274,6 @@ cs_output_kernel(const CsArgs a) {
     constexpr int STAGE = 2 * 64 * CO_LD;               // [64][CO_LD] of q, then of the state
     float* vs = co_smem + 2 * STAGE;                    // [64][64]
     double* cs = reinterpret_cast<double*>(vs + CS_CHUNK * 64);     // [64] running sums of the log decays
-    float* bs = reinterpret_cast<float*>(cs + CS_CHUNK);            // [64] input factors
-    float* dn = bs + CS_CHUNK;                          // [64] denominators
     mv_pdl_begin();
     const int tiles_j = (a.dv + 63) / 64, c = blockIdx.x / tiles_j, j0 = (blockIdx.x % tiles_j) * 64;
     const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, tj = tid & 15, tt = tid >> 4;
@@ -300,10 +281,8 @@ cs_output_kernel(const CsArgs a) {
     if (c * CS_CHUNK >= len) return;
     const int nt = min(CS_CHUNK, len - c * CS_CHUNK), chunk = row0 / CS_CHUNK + b + c;
     const size_t first = (size_t)row0 + c * CS_CHUNK;
-    const bool norm = a.m_tok != nullptr;
-    const int cols = a.dv + (norm ? 1 : 0), g = h / a.heads_per_group, n_groups = a.n_heads / a.heads_per_group;
-    const float* S0 = a.before + ((size_t)chunk * a.n_heads + h) * cols * a.lds;
-    const float* qp = a.q + first * a.ldq + (size_t)g * a.dk;
+    const float* S0 = a.before + ((size_t)chunk * a.n_heads + h) * a.dv * a.lds;
+    const float* qp = a.q + first * a.ldq + (size_t)h * a.dk;
     const int slices = (a.dk + 31) / 32;
     auto load = [&](int s) {
         cs_load<64, 32, CO_LD>(co_smem + (s & 1) * STAGE, qp + s * 32, a.ldq, nt, a.dk - s * 32, a.wide);
@@ -314,18 +293,14 @@ cs_output_kernel(const CsArgs a) {
     load(0);
     cs_load<CS_CHUNK, 64, 64>(vs, a.v + first * a.ldv + (size_t)h * a.dv + j0, a.ldv, nt, a.dv - j0, a.wide);
     cs_commit();
-    if (!CHANNEL && tid < CS_CHUNK) {                   // read after the loop's barriers
-        cs[tid] = a.c[((size_t)chunk * a.n_heads + h) * CS_CHUNK + tid];
-        bs[tid] = tid < nt ? (a.b ? a.b[(first + tid) * a.ld_b + h] : 1.f) : 0.f;
-    }
-    const float* Pc = a.P + ((size_t)chunk * (CHANNEL ? a.n_heads : n_groups) + (CHANNEL ? h : g)) * CS_CHUNK * CS_CHUNK;
+    if (!CHANNEL && tid < CS_CHUNK) cs[tid] = a.c[((size_t)chunk * a.n_heads + h) * CS_CHUNK + tid];    // read after the loop's barriers
+    const float* Pc = a.P + ((size_t)chunk * a.n_heads + h) * CS_CHUNK * CS_CHUNK;
     float* ps = co_smem + (slices & 1) * STAGE;         // [64][CO_PLD]: comes behind the last slice, into the stage that is free
     float acc[8][4];
 #pragma unroll
     for (int y = 0; y < 8; ++y)
 #pragma unroll
         for (int x = 0; x < 4; ++x) acc[y][x] = 0.f;
-    float dot = 0.f;                                    // with a normalizer: half of token tid / 2's q . n
     for (int s = 0; s < slices; ++s) {
         if (s + 1 < slices) load(s + 1);
         else {
@@ -350,47 +325,32 @@ cs_output_kernel(const CsArgs a) {
                 }
             }
         }
-        if (norm) {
-            const float* n0 = S0 + (size_t)a.dv * a.lds + s * 32 + (tid & 1) * 16;
-            const float* qt = co_smem + (s & 1) * STAGE + (tid >> 1) * CO_LD + (tid & 1) * 16;
-#pragma unroll 4
-            for (int x = 0; x < 16; ++x)
-                if (s * 32 + (tid & 1) * 16 + x < a.dk) dot = fmaf(qt[x], n0[x], dot);
-        }
         __syncthreads();
     }
     cs_wait<0>();                                       // P is there
     __syncthreads();
     if (!CHANNEL) {
-        // this head's factors on the group's products (what lies above the diagonal is not read)
+        // the decays on the products (what lies above the diagonal is not read)
 #pragma unroll 4
         for (int idx = tid; idx < CS_CHUNK * CS_CHUNK / 4; idx += CS_THREADS) {
             const int t = idx / (CS_CHUNK / 4), s = idx % (CS_CHUNK / 4) * 4;
             if (s > t || t >= nt) continue;
             float4 p = *reinterpret_cast<const float4*>(ps + t * CO_PLD + s);
             const double ct = cs[t];
-            p.x *= expf((float)(ct - cs[s])) * bs[s] * a.q_scale;
-            p.y *= s + 1 <= t ? expf((float)(ct - cs[s + 1])) * bs[s + 1] * a.q_scale : 0.f;
-            p.z *= s + 2 <= t ? expf((float)(ct - cs[s + 2])) * bs[s + 2] * a.q_scale : 0.f;
-            p.w *= s + 3 <= t ? expf((float)(ct - cs[s + 3])) * bs[s + 3] * a.q_scale : 0.f;
+            p.x *= expf((float)(ct - cs[s])) * a.q_scale;
+            p.y *= s + 1 <= t ? expf((float)(ct - cs[s + 1])) * a.q_scale : 0.f;
+            p.z *= s + 2 <= t ? expf((float)(ct - cs[s + 2])) * a.q_scale : 0.f;
+            p.w *= s + 3 <= t ? expf((float)(ct - cs[s + 3])) * a.q_scale : 0.f;
             *reinterpret_cast<float4*>(ps + t * CO_PLD + s) = p;
         }
 #pragma unroll
         for (int y = 0; y < 8; ++y) {
-            const float f = expf((float)cs[tt + 8 * y]) * a.q_scale, sk = a.skip ? a.skip[h] : 0.f;
+            const float f = expf((float)cs[tt + 8 * y]) * a.q_scale;
 #pragma unroll
-            for (int x = 0; x < 4; ++x) acc[y][x] = acc[y][x] * f + (a.skip && tt + 8 * y < nt ? sk * vs[(tt + 8 * y) * 64 + tj * 4 + x] : 0.f);
+            for (int x = 0; x < 4; ++x) acc[y][x] *= f;
         }
     }
     if (!CHANNEL) __syncthreads();
-    if (norm) {
-        const int t = tid >> 1;
-        dot *= expf((float)cs[t]) * a.q_scale;
-        for (int s = tid & 1; s <= t; s += 2) dot += ps[t * CO_PLD + s];
-        dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-        if ((tid & 1) == 0 && t < nt) dn[t] = fmaxf(fabsf(dot), expf(-a.m_tok[(first + t) * a.n_heads + h])) + 1e-6f;
-        __syncthreads();
-    }
     // what the chunk's tokens read from one another
     // (tokens 8 sb .. 8 sb + 7 for the rows from 8 sb on; a later token's value, which may not be finite, never meets an earlier row)
     // (short loops: unrolled whole, a third of the time went to fetching instructions)
@@ -429,11 +389,6 @@ cs_output_kernel(const CsArgs a) {
         const int t = tt + 8 * y;
         if (t >= nt) continue;
         float* to = a.o + (first + t) * a.n_heads * a.dv + (size_t)h * a.dv + j;
-        if (norm) {
-            const float d = dn[t];
-#pragma unroll
-            for (int x = 0; x < 4; ++x) acc[y][x] /= d;
-        }
         if (vec) *reinterpret_cast<float4*>(to) = make_float4(acc[y][0], acc[y][1], acc[y][2], acc[y][3]);
         else
 #pragma unroll
@@ -442,7 +397,7 @@ cs_output_kernel(const CsArgs a) {
     }
 }
 
-// G[chunk][group][t][s] = q_t . k_s of every chunk (all 64 x 64; what lies beyond a chunk's tokens is zero).
+// G[chunk][head][t][s] = q_t . k_s of every chunk (all 64 x 64; what lies beyond a chunk's tokens is zero).
 __global__ void __launch_bounds__(CS_THREADS)
 cs_products_kernel(const CsArgs a, float* __restrict__ G) {
     __shared__ __align__(16) float qs[2][64 * CO_LD], ks[2][64 * CO_LD];
@@ -485,7 +440,7 @@ cs_products_kernel(const CsArgs a, float* __restrict__ G) {
         }
         __syncthreads();
     }
-    float* to = G + ((size_t)(row0 / CS_CHUNK + b + c) * (a.n_heads / a.heads_per_group) + g) * CS_CHUNK * CS_CHUNK + tj * 4;
+    float* to = G + ((size_t)(row0 / CS_CHUNK + b + c) * a.n_heads + g) * CS_CHUNK * CS_CHUNK + tj * 4;
 #pragma unroll
     for (int y = 0; y < 8; ++y)
         *reinterpret_cast<float4*>(to + (tt + 8 * y) * CS_CHUNK) = make_float4(acc[y][0], acc[y][1], acc[y][2], acc[y][3]);
@@ -498,7 +453,7 @@ inline bool cs_aligned(const float* p, int ld, int cols) { return ((uintptr_t)p 
 // tiles; 59 us with 128 half tiles of four groups, 104 with one group).
 template <int TJ, int GROUPS, bool CHANNEL>
 int cs_walk_launch(const CsArgs& a, int tiles, int n_seqs, cudaStream_t stream) {
-    constexpr size_t smem = sizeof(float) * (2 * CS_CHUNK * (64 + 8 * TJ + 1) + (GROUPS - 1) * (TJ + 1) * CS_THREADS * 4);
+    constexpr size_t smem = sizeof(float) * (2 * CS_CHUNK * (64 + 8 * TJ + 1) + (GROUPS - 1) * TJ * CS_THREADS * 4);
     static const cudaError_t attr = cudaFuncSetAttribute(cs_walk_kernel<TJ, GROUPS, CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                          (int)smem);
     if (attr != cudaSuccess) return (int)attr;
@@ -506,8 +461,8 @@ int cs_walk_launch(const CsArgs& a, int tiles, int n_seqs, cudaStream_t stream) 
     return mv_launch_status();
 }
 
-// All kernels; a.wide, a.lds and by token a.P, a.c, a.w and a.d are filled in here.  By token G is scratch for the products
-// [chunks][groups][CS_CHUNK][CS_CHUNK] and `factors` (16-byte aligned) for cs_factor_floats(n_heads) floats a chunk.
+// All kernels; a.wide, a.lds and by head a.P, a.c, a.w and a.d are filled in here.  By head G is scratch for the products
+// [chunks][heads][CS_CHUNK][CS_CHUNK] and `factors` (16-byte aligned) for cs_factor_floats(n_heads) floats a chunk.
 inline int cs_factor_floats(int n_heads) { return n_heads * (3 * CS_CHUNK + 1); }
 
 template <bool CHANNEL>
@@ -523,7 +478,7 @@ int cs_launch(CsArgs a, float* G, float* factors, int chunks, int n_seqs, int ma
                   CS_THREADS, 0, stream, a, c, w, d);
         int code = mv_launch_status();
         if (code) return code;
-        mv_launch(cs_products_kernel, dim3((max_len + CS_CHUNK - 1) / CS_CHUNK, a.n_heads / a.heads_per_group, n_seqs), CS_THREADS, 0,
+        mv_launch(cs_products_kernel, dim3((max_len + CS_CHUNK - 1) / CS_CHUNK, a.n_heads, n_seqs), CS_THREADS, 0,
                   stream, a, G);
         code = mv_launch_status();
         if (code) return code;

@@ -138,7 +138,7 @@ MV_API int mv_decay_scan(const float* q, int ldq, const float* k, int ldk, const
 //
 // Every exponent is a difference of cumulative logarithms taken the right way round, so every factor
 // lies in (0, 1]: nothing overflows however small a decay is.  All of it is float32 on the CUDA cores.
-// With one constant decay a head the chunks take the path with one decay a token; with a decay a channel
+// With one constant decay a head the chunks take the path with one decay for all channels; with a decay a channel
 // the kernel below prepares, per (sequence, head, chunk), the decayed q and k, the chunk's total decay and P.  The factors
 // e^(c_t - c_s) of P are products of the tokens' own decays: a warp takes eight s and walks t, multiplying the eight
 // rows k_s e^(c_t - c_s) that its lanes hold by the next token's decay; the eight sums over the lanes are folded.
@@ -299,11 +299,13 @@ static int decay_prepare_launch(const float* q, int ldq, const float* k, int ldk
 
 // How many chunks the scratch of a step of N tokens in n_seqs sequences must hold.
 MV_API int mv_decay_chunks(int N, int n_seqs) { return N / CS_CHUNK + n_seqs + 1; }
+// And how many floats a chunk its factors take.
+MV_API int mv_decay_factor_floats(int n_heads) { return cs_factor_floats(n_heads); }
 
 // Arguments as mv_decay_scan, plus the step's tokens N, the longest sequence's (max_len) and scratch with chunks =
 // mv_decay_chunks(N, n_seqs): copies [N, n_heads * (2 dk + dv)] (with act), qd, kd [N, n_heads * dk] and ed
 // [chunks, n_heads * dk] (with z), P [chunks, n_heads, CS_CHUNK, CS_CHUNK], before [chunks, n_heads, dv, dk rounded up to 4],
-// factors [chunks, mv_scalar_factor_floats(n_heads)] (without z).
+// factors [chunks, mv_decay_factor_floats(n_heads)] (without z).
 MV_API int mv_decay_scan_chunked(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
                                  const float* z, int ldz, const float* head_decay, float inv_tau, float q_scale, int act,
                                  float* state, const int* slots, const int* cu, float* o, float* copies, float* qd, float* kd,
@@ -316,7 +318,7 @@ MV_API int mv_decay_scan_chunked(const float* q, int ldq, const float* k, int ld
     a.q = q; a.ldq = ldq; a.k = k; a.ldk = ldk; a.v = v; a.ldv = ldv;
     a.q_scale = q_scale; a.head_decay = head_decay;
     a.state = state; a.before = before; a.slots = slots; a.cu = cu; a.o = o;
-    a.n_heads = n_heads; a.heads_per_group = 1; a.dk = dk; a.dv = dv;
+    a.n_heads = n_heads; a.dk = dk; a.dv = dv;
     if (act) {
         float *qa = copies, *ka = qa + (size_t)N * wk, *va = ka + (size_t)N * wk;
         mv_launch(decay_activate_kernel, dim3(N, 3), 256, 0, stream, q, ldq, k, ldk, v, ldv, qa, ka, va, wk, wv);

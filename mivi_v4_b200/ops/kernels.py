@@ -72,9 +72,9 @@ _SIGNATURES = {
         "mv_scalar_scan": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
                            _P],
         "mv_scalar_chunks": [_I, _I],
-        "mv_scalar_scan_chunked": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I,
+        "mv_scalar_scan_chunked": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _I, _I,
                                    _I, _I, _I, _I, _I, _P],
-        "mv_scalar_factor_floats": [_I],
+        "mv_decay_factor_floats": [_I],
         "mv_memory_gates": [_P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _I, _P],
         "mv_causal_conv": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
         "mv_ssm_decode_prepare": [_P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _P, _I, _P, _P, _P, _P, _I, _P],
@@ -327,7 +327,7 @@ def _need(t: Optional[torch.Tensor], name: str, dtype=None, shape=None, optional
 
 _launches = 0
 # kernels launched by one call of each entry point
-_KERNELS_PER_CALL = {"mv_shortconv": 2, "mv_decay_scan_chunked": 3, "mv_causal_conv": 2, "mv_scalar_scan_chunked": 4}
+_KERNELS_PER_CALL = {"mv_shortconv": 2, "mv_decay_scan_chunked": 3, "mv_causal_conv": 2, "mv_scalar_scan_chunked": 2}
 
 
 def launch_count() -> int:
@@ -647,7 +647,7 @@ def scalar_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_a: torch.
     o_t <- o_t / (max(|n . q_t|, exp(-m_tok)) + 1e-6).  Everything is computed in float32; the order of every
     sum depends on dk alone, so any cut of a prompt gives the same numbers.  ``max_len``: the most tokens that a
     sequence brings; with ``ws`` (a Workspace, for scratch) steps of ``SCAN_CHUNKED_FROM`` tokens a sequence and
-    more take the kernels that work in chunks of 64 tokens, whose sums come in another order (the
+    more take the kernels that walk a sequence in chunks of 32 tokens, whose sums come in another order (the
     results differ from the token-by-token kernel's by rounding)."""
     N = out.shape[0]
     if not 1 <= dk <= MAX_SCAN_KEY_DIM:
@@ -666,17 +666,17 @@ def scalar_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_a: torch.
     if ws is not None and max_len >= SCAN_CHUNKED_FROM:
         chunks = int(_fn("core", "mv_scalar_chunks")(N, int(n_seqs)))
         G = ws.get("scalar_scan_products", (chunks, groups, SCAN_CHUNK, SCAN_CHUNK), torch.float32)
-        before = ws.get("scan_before", (chunks, n_heads, dv + (1 if norm else 0), (dk + 3) & ~3), torch.float32)
-        factors = ws.get("scan_factors", (chunks, int(_fn("core", "mv_scalar_factor_floats")(n_heads))), torch.float32)
+        o_aug = ws.get("scalar_scan_o_aug", (N, n_heads * (dv + 1)), torch.float32) if norm else None
         _check(_fn("core", "mv_scalar_scan_chunked")(
             qp, ldq, kp, ldk, vp, ldv, ap, lda, bp, ldb, _need(skip, "scalar_scan skip", torch.float32, (n_heads,), True),
             _need(m_tok, "scalar_scan m", torch.float32, (N, n_heads), True), float(q_scale), state.data_ptr(),
             _need(slots, "slots", torch.int32), _need(cu, "cu", torch.int32),
             _need(out, "scalar_scan out", torch.float32, (N, n_heads * dv)), G.data_ptr(),
-            before.data_ptr(), factors.data_ptr(), chunks, int(n_seqs), int(max_len), n_heads, int(heads_per_group), dk, dv,
+            o_aug.data_ptr() if norm else None, N, int(n_seqs), int(max_len), n_heads, int(heads_per_group), dk, dv,
             int(norm), _stream()), "mv_scalar_scan_chunked")
+        add_launches(1 if norm else 0)
         account(N * n_heads * (2 * dk // heads_per_group + 2 * dv) * 4 + 2 * n_seqs * n_heads * dk * dv * 4
-                + 2 * chunks * (groups * SCAN_CHUNK * SCAN_CHUNK + n_heads * dk * dv) * 4,
+                + 2 * chunks * groups * SCAN_CHUNK * SCAN_CHUNK * 4,
                 4 * N * n_heads * dk * dv + N * n_heads * SCAN_CHUNK * dv + N * groups * SCAN_CHUNK * dk)
         return out
     _check(_fn("core", "mv_scalar_scan")(
@@ -970,7 +970,8 @@ def expert_combine(ys: torch.Tensor, place: torch.Tensor, pick_w: Optional[torch
 MAX_SCAN_KEY_DIM = 256
 SCAN_ACT_NONE, SCAN_ACT_SILU = 0, 1
 SCAN_CHUNKED_FROM = 16          # a step whose longest sequence brings this many tokens walks them in chunks
-SCAN_CHUNK = 64
+SCAN_CHUNK = 32                 # of scalar_scan
+DECAY_CHUNK = 64                # of decay_scan
 
 
 def _cols(t: torch.Tensor, name: str, n_rows: int, width: int):
@@ -1015,9 +1016,9 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
         kd = ws.get("scan_kd", (N, n_heads * dk), torch.float32) if by_channel else None
         ed = ws.get("scan_ed", (chunks, n_heads * dk), torch.float32) if by_channel else None
         before = ws.get("scan_before", (chunks, n_heads, dv, (dk + 3) & ~3), torch.float32)
-        factors = None if by_channel else ws.get("scan_factors", (chunks, int(_fn("core", "mv_scalar_factor_floats")(n_heads))),
+        factors = None if by_channel else ws.get("scan_factors", (chunks, int(_fn("core", "mv_decay_factor_floats")(n_heads))),
                                                  torch.float32)
-        pm = ws.get("scan_p", (chunks, n_heads, SCAN_CHUNK, SCAN_CHUNK), torch.float32)
+        pm = ws.get("scan_p", (chunks, n_heads, DECAY_CHUNK, DECAY_CHUNK), torch.float32)
         _check(_fn("core", "mv_decay_scan_chunked")(
             qp, ldq, kp, ldk, vp, ldv, zp, ldz, _need(head_decay, "head decay", torch.float32, (n_heads,), True),
             float(inv_tau), float(q_scale), int(act), state.data_ptr(), _need(slots, "slots", torch.int32),
