@@ -162,23 +162,29 @@ MV_API int mv_delta_scan(const float* q, int ldq, const float* k, int ldk, const
 // ------------------------------------------------------------------------------------------- steps of many tokens
 // Two kernels.  delta_prepare does, once per token, what does not depend on the state: q and k as unit vectors
 // (q also times q_scale), k . q of each q/k head, the decays g, and beta; one row of `prep` a token:
-//     [q: kv_heads dk | k: kv_heads dk | g: heads dk | beta: heads | k.q: kv_heads]      (row stride ldp, 32-bit)
+//     [q: kv_heads W | k: kv_heads W | g: heads W | beta: heads | k.q: kv_heads]      (row stride ldp, 32-bit)
+// W is dk, or from 64 key channels on dk rounded up to 64, 128 or 256 (zeros beyond dk), a head's channels then in the order in
+// which delta_scan_wide_kernel's lanes own them.
 // delta_scan_long then walks a sequence with nothing but the recurrence in its loop.  The tokens come through
 // shared memory sixteen at a time, the next sixteen on their way (cp.async) while these are worked on.  In the
 // loop  S' = diag(g) S  is read twice at once, a = S'^T k and b = S'^T q, so that one round of shuffles serves
 // both; u = beta (v - a); o = b + u (k . q), which is (S' + k u^T)^T q; S = S' + k u^T.
 #define DL_CHUNK 16
 
+// Channel i of a head's W = 32 R in prep: lane i % 8 owns the channels i, i + 8, .., 4 R of them, and finds them side by side,
+// first those that are 32 apart.
+__device__ __forceinline__ int dl_place(int i, int R) { return R ? (i & 7) * (4 * R) + ((i >> 3) & 3) * R + (i >> 5) : i; }
+
 __global__ void __launch_bounds__(256)
 delta_prepare_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
                      const float* __restrict__ b, int ldb, const float* __restrict__ a, int lda,
                      const float* __restrict__ dt_bias, const float* __restrict__ a_log, float q_scale, float norm_eps,
-                     float* __restrict__ prep, int ldp, int n_heads, int kv_heads, int dk, int head_decay) {
+                     float* __restrict__ prep, int ldp, int n_heads, int kv_heads, int dk, int W, int R, int head_decay) {
     mv_pdl_begin();
     const int n = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     float* row = prep + (size_t)n * ldp;
-    const int qk = kv_heads * dk, hk = n_heads * dk;
+    const int qk = kv_heads * W, hk = n_heads * W;
     for (int h = warp; h < kv_heads; h += nwarps) {
         const float* qh = q + (size_t)n * ldq + (size_t)h * dk;
         const float* kh = k + (size_t)n * ldk + (size_t)h * dk;
@@ -193,16 +199,18 @@ delta_prepare_kernel(const float* __restrict__ q, int ldq, const float* __restri
         sk = mv_warp_sum(sk);
         dot = mv_warp_sum(dot);
         const float fq = q_scale / sqrtf(sq + norm_eps), fk = 1.0f / sqrtf(sk + norm_eps);
-        for (int i = lane; i < dk; i += 32) {
-            row[(size_t)h * dk + i] = qh[i] * fq;
-            row[qk + (size_t)h * dk + i] = kh[i] * fk;
+        for (int i = lane; i < W; i += 32) {
+            const int at = h * W + dl_place(i, R);
+            row[at] = i < dk ? qh[i] * fq : 0.f;
+            row[qk + at] = i < dk ? kh[i] * fk : 0.f;
         }
         if (lane == 0) row[2 * qk + hk + n_heads + h] = dot * fq * fk;
     }
     for (int e = threadIdx.x; e < hk; e += blockDim.x) {
-        const int h = e / dk;
-        const int ai = head_decay ? h : e;
-        row[2 * qk + e] = expf(-expf(a_log[h]) * dr_softplus(a[(size_t)n * lda + ai] + dt_bias[ai]));
+        const int h = e / W, i = e - h * W;
+        const int ai = head_decay ? h : h * dk + i;
+        row[2 * qk + h * W + dl_place(i, R)] =
+            i < dk ? expf(-expf(a_log[h]) * dr_softplus(a[(size_t)n * lda + ai] + dt_bias[ai])) : 0.f;
     }
     for (int h = threadIdx.x; h < n_heads; h += blockDim.x)
         row[2 * qk + hk + h] = 1.0f / (1.0f + expf(-b[(size_t)n * ldb + h]));
@@ -262,8 +270,7 @@ __device__ __forceinline__ void dl_stage(float* buf, const float* __restrict__ p
 
 // One buffer of shared memory: [q: CHUNK dk | k: CHUNK dk | g: CHUNK dk | v: CHUNK DR_COLS | beta: CHUNK | k.q: CHUNK]
 // PART lanes share a column of the state (element i of it with lane i % PART).  Keys under 64 channels run here with 8
-// lanes a column; from 64 channels on delta_scan_warp_kernel below takes over.  (A whole warp a column, 16 warps a
-// block, was measured issue-bound: 740 us for 2,048 tokens of 128 x 128 against 696 for the kernel below.)
+// lanes a column; from 64 channels on delta_scan_wide_kernel below takes over.
 template <int R, int PART>
 __global__ void __launch_bounds__(DR_COLS * PART)
 delta_scan_long_kernel(const float* __restrict__ prep, int ldp, const float* __restrict__ v, int ldv,
@@ -358,46 +365,82 @@ delta_scan_long_kernel(const float* __restrict__ prep, int ldp, const float* __r
     }
 }
 
-// From 64 key channels on: a warp carries TWO columns of the state, lane l the channels l, l + 32, ...  A token's q, k and
-// g are read once for both columns, and the four sums of a token (what the state says for k and what it reads out
-// for q, in each column) are folded while they are added up: lanes exchange the half they do not keep, so 4 + 2 + 1
-// values go round instead of 4 x 5, and lanes 0, 8, 16 and 24 end up with one whole sum each.
+// From 64 key channels on: 8 lanes share a column of the state, lane l the channels l, l + 8, l + 16, .. (4 R of dk <= 32 R), four
+// columns a warp, 16 a block.  What bounds it is the chain from one token to the next: decay, dot product with k, its sum
+// over the lanes, u, the state's update.  A lane adds its channels in four chains (those 32 apart) and joins them two and two, so that
+// three exchanges remain, after which all eight lanes have the sum and no broadcast follows; the next token's rows are
+// requested from shared memory before the exchanges.  (With a whole warp on two columns the chain had six exchanges and 690 us for
+// 2,048 tokens of 16 heads of 128 x 128; the order in which a sum's parts are added is the same, and so is every bit.)  @MEASURED@
+constexpr int DW_THREADS = DR_COLS * 8;
+
 template <int R>
-__global__ void __launch_bounds__(DR_COLS * 16)
-delta_scan_warp_kernel(const float* __restrict__ prep, int ldp, const float* __restrict__ v, int ldv,
+__global__ void __launch_bounds__(DW_THREADS)
+delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __restrict__ v, int ldv,
                        float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ cu,
-                       float* __restrict__ o, int n_heads, int kv_heads, int dk, int dv, int wide) {
+                       float* __restrict__ o, int n_heads, int kv_heads, int dk, int dv) {
+    constexpr int E = 4 * R, W = 32 * R, LANE = E + 4, ROW = 8 * LANE;      // a lane's channels, 16 bytes of padding between lanes
+    constexpr int BUF = DL_CHUNK * (3 * ROW + DR_COLS + 2);
     mv_pdl_wait();                          // the successor is let go when the last token is done
     extern __shared__ __align__(16) float dl_smem[];
-    const int per = DL_CHUNK * (3 * dk + DR_COLS + 2);
     const int tile = blockIdx.x, h = blockIdx.y, sq = blockIdx.z;
-    const int tid = threadIdx.x, lane = tid & 31, jl = (tid >> 5) * 2;
-    const int col0 = tile * DR_COLS;
-    const int j0 = col0 + jl, j1 = j0 + 1;
+    const int tid = threadIdx.x, l = tid & 7, jl = tid >> 3;
+    const int col0 = tile * DR_COLS, j = col0 + jl;
     const int row0 = cu[sq], len = cu[sq + 1] - row0;
     if (len <= 0) return;
-    const int hk = h / (n_heads / kv_heads);
-    const int qk = kv_heads * dk;
+    const int hk = h / (n_heads / kv_heads), qk = kv_heads * W;
     const int slot = mv_read_slot(slots[sq]);
-    float* srow0 = state + (((size_t)slot * n_heads + h) * dv + (j0 < dv ? j0 : 0)) * dk;
-    float* srow1 = state + (((size_t)slot * n_heads + h) * dv + (j1 < dv ? j1 : 0)) * dk;
-    float S0[R], S1[R];
+    float* srow = state + (((size_t)slot * n_heads + h) * dv + (j < dv ? j : 0)) * dk;
+    // S[c][r]: channel l + 8 c + 32 r
+    float S[4][R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int i = lane + 32 * r;
-        S0[r] = (j0 < dv && i < dk) ? srow0[i] : 0.f;
-        S1[r] = (j1 < dv && i < dk) ? srow1[i] : 0.f;
-    }
-    const bool hi16 = lane & 16, hi8 = lane & 8;
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = l + 8 * c + 32 * r;
+            S[c][r] = (j < dv && i < dk) ? srow[i] : 0.f;
+        }
+    // 16 tokens' rows of q, k and g, DR_COLS columns of v, beta and k.q on their way into one buffer
+    auto stage = [&](int c0, float* buf) {
+        const int nt = min(DL_CHUNK, len - c0);
+        for (int idx = tid; idx < nt * (W / 4); idx += DW_THREADS) {
+            const int t = idx / (W / 4), i = (idx % (W / 4)) * 4;
+            const float* src = prep + (size_t)(row0 + c0 + t) * ldp;
+            float* to = buf + t * ROW + i / E * LANE + i % E;
+            dl_copy16(to, src + (size_t)hk * W + i);
+            dl_copy16(to + DL_CHUNK * ROW, src + qk + (size_t)hk * W + i);
+            dl_copy16(to + 2 * DL_CHUNK * ROW, src + 2 * qk + (size_t)h * W + i);
+        }
+        float* vs = buf + 3 * DL_CHUNK * ROW;
+        for (int idx = tid; idx < nt * DR_COLS; idx += DW_THREADS) {
+            const int t = idx / DR_COLS, c = idx - t * DR_COLS;
+            if (col0 + c < dv) dl_copy4(vs + idx, v + (size_t)(row0 + c0 + t) * ldv + (size_t)h * dv + col0 + c);
+        }
+        if (tid < nt) {
+            const float* src = prep + (size_t)(row0 + c0 + tid) * ldp + 2 * qk + (size_t)n_heads * W;
+            dl_copy4(vs + DL_CHUNK * DR_COLS + tid, src + h);
+            dl_copy4(vs + DL_CHUNK * DR_COLS + DL_CHUNK + tid, src + n_heads + hk);
+        }
+    };
+    auto read = [&](const float* from, float (&x)[4][R]) {
+        float flat[E];
+#pragma unroll
+        for (int e = 0; e < E; e += 4) {
+            const float4 y = *reinterpret_cast<const float4*>(from + e);
+            flat[e] = y.x; flat[e + 1] = y.y; flat[e + 2] = y.z; flat[e + 3] = y.w;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int r = 0; r < R; ++r) x[c][r] = flat[c * R + r];
+    };
 
-    dl_stage(dl_smem, prep, ldp, v, ldv, row0, 0, len, h, hk, qk, n_heads, dk, dv, col0, wide, tid, DR_COLS * 16);
+    stage(0, dl_smem);
     dl_commit();
     int which = 0;
     for (int c0 = 0; c0 < len; c0 += DL_CHUNK, which ^= 1) {
-        float* buf = dl_smem + which * per;
+        float* buf = dl_smem + which * BUF;
         if (c0 + DL_CHUNK < len) {
-            dl_stage(dl_smem + (which ^ 1) * per, prep, ldp, v, ldv, row0, c0 + DL_CHUNK, len, h, hk, qk, n_heads, dk, dv,
-                     col0, wide, tid, DR_COLS * 16);
+            stage(c0 + DL_CHUNK, dl_smem + (which ^ 1) * BUF);
             dl_commit();
             dl_wait<1>();
         } else {
@@ -405,72 +448,73 @@ delta_scan_warp_kernel(const float* __restrict__ prep, int ldp, const float* __r
         }
         __syncthreads();
         const int nt = min(DL_CHUNK, len - c0);
-        const float* qs = buf;
-        const float* ks = qs + DL_CHUNK * dk;
-        const float* gs = ks + DL_CHUNK * dk;
-        const float* vs = gs + DL_CHUNK * dk;
+        const float* qs = buf + l * LANE;
+        const float* ks = qs + DL_CHUNK * ROW;
+        const float* gs = ks + DL_CHUNK * ROW;
+        const float* vs = buf + 3 * DL_CHUNK * ROW;
         const float* bs = vs + DL_CHUNK * DR_COLS;
         const float* ds = bs + DL_CHUNK;
-        for (int t = 0; t < nt; ++t) {
-            const float* qt = qs + t * dk;
-            const float* kt = ks + t * dk;
-            const float* gt = gs + t * dk;
-            float kr[R];
-            float a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
+        float* orow = o + (size_t)(row0 + c0) * n_heads * dv + (size_t)h * dv + j;
+        float q[4][R], g[4][R], k0[4][R], k1[4][R], vt = vs[jl], beta = bs[0], kq = ds[0];
+        read(qs, q);
+        read(gs, g);
+        read(ks, k0);
+        auto token = [&](int t, const float (&k)[4][R], float (&k_next)[4][R]) {
+            float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const int i = lane + 32 * r;
-                kr[r] = 0.f;
-                if (i < dk) {
-                    const float g = gt[i], q = qt[i];
-                    kr[r] = kt[i];
-                    S0[r] *= g;
-                    S1[r] *= g;
-                    a0 = fmaf(S0[r], kr[r], a0);
-                    a1 = fmaf(S1[r], kr[r], a1);
-                    b0 = fmaf(S0[r], q, b0);
-                    b1 = fmaf(S1[r], q, b1);
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    S[c][r] *= g[c][r];
+                    a[c] = fmaf(S[c][r], k[c][r], a[c]);
+                    b[c] = fmaf(S[c][r], q[c][r], b[c]);
                 }
+            const float v_now = vt, beta_now = beta, kq_now = kq;
+            if (t + 1 < nt) {
+                read(qs + (t + 1) * ROW, q);
+                read(gs + (t + 1) * ROW, g);
+                read(ks + (t + 1) * ROW, k_next);
+                vt = vs[(t + 1) * DR_COLS + jl];
+                beta = bs[t + 1];
+                kq = ds[t + 1];
             }
-            // lanes 0..15 keep what the state says for k, lanes 16..31 what it reads for q; then lanes with bit 3 clear
-            // keep the first column and the others the second
-            const float x0 = (hi16 ? b0 : a0) + __shfl_xor_sync(0xffffffffu, hi16 ? a0 : b0, 16);
-            const float x1 = (hi16 ? b1 : a1) + __shfl_xor_sync(0xffffffffu, hi16 ? a1 : b1, 16);
-            float y = (hi8 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, hi8 ? x0 : x1, 8);
-            y += __shfl_xor_sync(0xffffffffu, y, 4);
-            y += __shfl_xor_sync(0xffffffffu, y, 2);
-            y += __shfl_xor_sync(0xffffffffu, y, 1);
-            const float said0 = __shfl_sync(0xffffffffu, y, 0), said1 = __shfl_sync(0xffffffffu, y, 8);
-            const float beta = bs[t];
-            const float u0 = beta * ((j0 < dv ? vs[t * DR_COLS + jl] : 0.f) - said0);
-            const float u1 = beta * ((j1 < dv ? vs[t * DR_COLS + jl + 1] : 0.f) - said1);
+            float said = (a[0] + a[2]) + (a[1] + a[3]), out = (b[0] + b[2]) + (b[1] + b[3]);
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                S0[r] = fmaf(kr[r], u0, S0[r]);
-                S1[r] = fmaf(kr[r], u1, S1[r]);
+            for (int d = 4; d >= 1; d >>= 1) {
+                said += __shfl_xor_sync(0xffffffffu, said, d);
+                out += __shfl_xor_sync(0xffffffffu, out, d);
             }
-            float* orow = o + (size_t)(row0 + c0 + t) * n_heads * dv + (size_t)h * dv;
-            if (lane == 16 && j0 < dv) orow[j0] = fmaf(u0, ds[t], y);
-            if (lane == 24 && j1 < dv) orow[j1] = fmaf(u1, ds[t], y);
+            const float u = beta_now * ((j < dv ? v_now : 0.f) - said);
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int r = 0; r < R; ++r) S[c][r] = fmaf(k[c][r], u, S[c][r]);
+            if (l == 0 && j < dv) orow[(size_t)t * n_heads * dv] = fmaf(u, kq_now, out);
+        };
+        int t = 0;
+        for (; t + 1 < nt; t += 2) {
+            token(t, k0, k1);
+            token(t + 1, k1, k0);
         }
+        if (t < nt) token(t, k0, k1);
         __syncthreads();
     }
     mv_pdl_launch_dependents();
-    if (mv_slot_ok(slots[sq])) {
+    if (j < dv && mv_slot_ok(slots[sq])) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int i = lane + 32 * r;
-            if (i < dk) {
-                if (j0 < dv) srow0[i] = S0[r];
-                if (j1 < dv) srow1[i] = S1[r];
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int i = l + 8 * c + 32 * r;
+                if (i < dk) srow[i] = S[c][r];
             }
-        }
     }
 }
 
 // Row width of `prep` for these sizes (a multiple of 4 floats, so that rows start on 16 bytes).
-static inline int mv_delta_prep_width(int n_heads, int kv_heads, int dk) {
-    const int w = 2 * kv_heads * dk + n_heads * dk + n_heads + kv_heads;
+static inline int dl_width(int dk) { return dk < 64 ? dk : dk == 64 ? 64 : dk <= 128 ? 128 : 256; }
+MV_API int mv_delta_prep_width(int n_heads, int kv_heads, int dk) {
+    const int w = (2 * kv_heads + n_heads) * dl_width(dk) + n_heads + kv_heads;
     return (w + 3) & ~3;
 }
 
@@ -481,15 +525,16 @@ MV_API int mv_delta_scan_long(const float* q, int ldq, const float* k, int ldk, 
                               int n_seqs, int n_heads, int kv_heads, int dk, int dv, int head_decay, cudaStream_t stream) {
     if (n_seqs <= 0 || N <= 0) return 0;
     if (dk < 1 || dk > 256 || dv < 1 || kv_heads < 1 || n_heads % kv_heads) return (int)cudaErrorInvalidValue;
-    const int ldp = mv_delta_prep_width(n_heads, kv_heads, dk);
+    const int ldp = mv_delta_prep_width(n_heads, kv_heads, dk), W = dl_width(dk), R = dk < 64 ? 0 : W / 32;
     mv_launch(delta_prepare_kernel, N, 256, 0, stream, q, ldq, k, ldk, b, ldb, a, lda, dt_bias, a_log, q_scale, norm_eps, prep,
-              ldp, n_heads, kv_heads, dk, head_decay);
+              ldp, n_heads, kv_heads, dk, W, R, head_decay);
     // The walk is launched as an ordinary successor, not a programmatic one.  Started while the preparing kernel's blocks
     // still hold the multiprocessors, its few blocks (one sequence of 16 heads x 128 values: 128) went where room came
     // up first, several to a multiprocessor, and the walk, bound by what ONE multiprocessor issues, took 1.75 times as
     // long as when they are dealt out over an idle device (measured: 1.26 ms against 0.72 for 2,048 tokens).
     const dim3 grid((dv + DR_COLS - 1) / DR_COLS, n_heads, n_seqs);
-    const size_t smem = 2 * (size_t)DL_CHUNK * (3 * dk + DR_COLS + 2) * sizeof(float);
+    if (R && ((uintptr_t)prep & 15)) return (int)cudaErrorInvalidValue;
+    const size_t smem = 2 * (size_t)DL_CHUNK * (3 * (R ? 8 * (4 * R + 4) : dk) + DR_COLS + 2) * sizeof(float);
     // 16-byte copies: every row of q, k and g of a head starts on 16 bytes (ldp is a multiple of 4 floats)
     const int wide = dk % 4 == 0 && (((uintptr_t)prep) & 15) == 0;
 #define DL_LAUNCH(R, PART)                                                                                                   \
@@ -506,12 +551,12 @@ MV_API int mv_delta_scan_long(const float* q, int ldq, const float* k, int ldk, 
 #define DW_LAUNCH(R)                                                                                                     \
     do {                                                                                                                 \
         if (smem > 48 * 1024) {                                                                                          \
-            const cudaError_t e = cudaFuncSetAttribute(delta_scan_warp_kernel<R>,                                        \
+            const cudaError_t e = cudaFuncSetAttribute(delta_scan_wide_kernel<R>,                                        \
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
             if (e != cudaSuccess) return (int)e;                                                                         \
         }                                                                                                                \
-        delta_scan_warp_kernel<R><<<grid, DR_COLS * 16, smem, stream>>>((const float*)prep, ldp, v, ldv, state, slots,  \
-                                                                        cu, o, n_heads, kv_heads, dk, dv, wide);         \
+        delta_scan_wide_kernel<R><<<grid, DW_THREADS, smem, stream>>>((const float*)prep, ldp, v, ldv, state, slots,  \
+                                                                        cu, o, n_heads, kv_heads, dk, dv);               \
     } while (0)
     if (dk <= 32) DL_LAUNCH(4, 8);
     else if (dk < 64) DL_LAUNCH(8, 8);

@@ -2,8 +2,8 @@
 // tensor cores.  Where a few query tokens fold W_uk into the query and read the cached rows as they are, many query
 // tokens pay for building every head's keys and values once: the cached rows a step can see are copied out of their
 // pages side by side, one product with [W_uk; W_uv] turns them into keys and values for all heads, and the attention
-// itself is attention_sink_prefill.cu's plan: a block is 64 consecutive query tokens of one sequence for one head, 4
-// warps of 16 queries; keys and values stream through shared memory in blocks of 64 (cp.async, double-buffered); both
+// itself is attention_sink_prefill.cu's plan: a block is 64 or 128 consecutive query tokens of one sequence for one head, 4
+// warps of 16 or 32 queries; keys and values stream through shared memory in blocks of 64 (cp.async, three buffers); both
 // products are mma.sync m16n8k16 with float32 accumulation and the running-maximum softmax in float32 registers
 // between them.  A head's key is [its unrotated part | the rotated part that all heads share]; the sink starts every
 // row's maximum and denominator; the output is multiplied element by element by the sigmoid of a gate.
@@ -17,7 +17,6 @@
 
 namespace {
 
-constexpr int QT = 64;          // queries per block
 constexpr int KB = 64;          // keys per block of the stream
 constexpr int NWARPS = 4;
 constexpr float LOG2E = 1.4426950408889634f;
@@ -40,6 +39,20 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], unsigned a0, unsigned a1
 __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const unsigned*>(&v);
+}
+__device__ __forceinline__ void ldmatrix_x4(unsigned (&r)[4], const void* smem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(s));
+}
+__device__ __forceinline__ void ldmatrix_x2(unsigned (&r)[4], const void* smem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(s));
+}
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 __device__ __forceinline__ void ldmatrix_x4_trans(unsigned (&r)[4], const void* smem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -113,21 +126,28 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, long long page_stri
 // gate: 32-bit logits [N, >= nh dv] with row stride ld_gate (with gate_heads [N, >= nh], one a head), or null; o [N, nh dv].  The softmax weights enter the
 // second product as two bfloat16 numbers each (the rounded weight and what the rounding left), so the sum over the
 // values carries the weights to 16 bits of mantissa although the tensor cores read bfloat16.
-template <int DKM, int DVM>
+//
+// A warp has MT tiles of 16 queries.  Bound by mma.sync (8 cycles an instruction and scheduler): with MT 2 a key or value
+// fragment that is read from shared memory serves two of them, the reads are ldmatrix, and the softmax of one warp runs under the
+// products of the scheduler's other one.  A row's sums are added in the same order whatever MT is: blocks of 64 keys from multiples
+// of 64, 16 channels and 16 keys at a time, and key blocks that a warp's queries cannot see change nothing and are passed over.
+// Longest blocks first, so that no long one is left for the end.  @MEASURED@
+template <int DKM, int DVM, int MT>
 __global__ void __launch_bounds__(NWARPS * 32)
 latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kx, int ld_kx,
                                 int v0, const __nv_bfloat16* __restrict__ rk, const int* __restrict__ cu,
                                 const int* __restrict__ starts, const float* __restrict__ sinks,
                                 const float* __restrict__ gate, int ld_gate, int gate_heads, __nv_bfloat16* __restrict__ o, int B, int nh,
                                 int dim, int rot, int dv, float scale, int window) {
+    constexpr int QT = NWARPS * 16 * MT, STAGES = 3;
     mv_pdl_begin();
     const int dk = dim + rot;
     const int ldk = dk + 8, ldv = dv + 8;             // padded rows: conflict-free fragment loads
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __nv_bfloat16* ks = reinterpret_cast<__nv_bfloat16*>(smem_raw);     // [2][KB][ldk]
-    __nv_bfloat16* vs = ks + 2 * KB * ldk;                              // [2][KB][ldv]
+    __nv_bfloat16* ks = reinterpret_cast<__nv_bfloat16*>(smem_raw);     // [STAGES][KB][ldk]
+    __nv_bfloat16* vs = ks + STAGES * KB * ldk;                         // [STAGES][KB][ldv]
 
-    int b = 0, tile = blockIdx.x, base = 0;           // base: the gathered row of this sequence's first seen position
+    int b = 0, tile = (int)(gridDim.x - 1 - blockIdx.x), base = 0;      // base: the gathered row of this sequence's first seen position
     for (; b < B; ++b) {
         const int len = cu[b + 1] - cu[b];
         const int tiles = (len + QT - 1) / QT;
@@ -143,42 +163,50 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
     const int pos0 = starts[b] + tile * QT;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gq = lane >> 2, t4 = lane & 3;
+    const int w0 = warp * 16 * MT;                    // the warp's first query
 
-    const int qi0 = warp * 16 + gq, qi1 = qi0 + 8;
-    const int p0 = pos0 + qi0, p1 = pos0 + qi1;
-    unsigned qf[DKM / 16][4];
-    {
-        const __nv_bfloat16* r0 = q + ((size_t)(row0 + min(qi0, nq - 1)) * nh + h) * dk;
-        const __nv_bfloat16* r1 = q + ((size_t)(row0 + min(qi1, nq - 1)) * nh + h) * dk;
+    unsigned qf[MT][DKM / 16][4];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+        const int qi = w0 + mt * 16 + gq;
+        const __nv_bfloat16* r0 = q + ((size_t)(row0 + min(qi, nq - 1)) * nh + h) * dk;
+        const __nv_bfloat16* r1 = q + ((size_t)(row0 + min(qi + 8, nq - 1)) * nh + h) * dk;
 #pragma unroll
         for (int kk = 0; kk < DKM / 16; ++kk) {
             if (kk * 16 < dk) {
-                qf[kk][0] = *reinterpret_cast<const unsigned*>(r0 + kk * 16 + 2 * t4);
-                qf[kk][1] = *reinterpret_cast<const unsigned*>(r1 + kk * 16 + 2 * t4);
-                qf[kk][2] = *reinterpret_cast<const unsigned*>(r0 + kk * 16 + 2 * t4 + 8);
-                qf[kk][3] = *reinterpret_cast<const unsigned*>(r1 + kk * 16 + 2 * t4 + 8);
+                qf[mt][kk][0] = *reinterpret_cast<const unsigned*>(r0 + kk * 16 + 2 * t4);
+                qf[mt][kk][1] = *reinterpret_cast<const unsigned*>(r1 + kk * 16 + 2 * t4);
+                qf[mt][kk][2] = *reinterpret_cast<const unsigned*>(r0 + kk * 16 + 2 * t4 + 8);
+                qf[mt][kk][3] = *reinterpret_cast<const unsigned*>(r1 + kk * 16 + 2 * t4 + 8);
             }
         }
     }
 
-    float oacc[DVM / 8][4];
-#pragma unroll
-    for (int j = 0; j < DVM / 8; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) oacc[j][e] = 0.f;
+    float oacc[MT][DVM / 8][4];
     // the sink starts the running maximum and the denominator (its own term, exp(sink - max), is 1 now); a row's
     // denominator is summed over the four lanes of its quad at the end, so one of them holds the sink's 1
-    float m0 = sinks ? sinks[h] : -INFINITY, m1 = m0;
-    float l0 = (sinks && t4 == 0) ? 1.f : 0.f, l1 = l0;
+    float m[MT][2], l[MT][2];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+#pragma unroll
+        for (int j = 0; j < DVM / 8; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) oacc[mt][j][e] = 0.f;
+        m[mt][0] = m[mt][1] = sinks ? sinks[h] : -INFINITY;
+        l[mt][0] = l[mt][1] = (sinks && t4 == 0) ? 1.f : 0.f;
+    }
 
     const int last_pos = pos0 + nq - 1;
     const int first_key = window > 0 ? max(0, pos0 - window + 1) : 0;
     const int kb_begin = first_key / KB, n_iter = last_pos / KB + 1 - kb_begin;
+    // the key blocks that the warp's queries see
+    const int w_last = min(pos0 + w0 + 16 * MT - 1, last_pos), w_first = window > 0 ? max(0, pos0 + w0 - window + 1) : 0;
+    const bool live = w0 < nq;
 
+    const int kc = dim >> 3, rc = rot >> 3, all = kc + rc + (dv >> 3);
+    const int step_r = NWARPS * 32 / all, step_c = NWARPS * 32 % all, r_of = threadIdx.x / all, c_of = threadIdx.x % all;
     auto load_block = [&](int kb, int buf) {
-        const int kc = dim >> 3, rc = rot >> 3, vc = dv >> 3, all = kc + rc + vc;
-        for (int idx = threadIdx.x; idx < KB * all; idx += NWARPS * 32) {
-            const int r = idx / all, c = idx - r * all;
+        for (int r = r_of, c = c_of; r < KB;) {
             const int t = min(max(kb * KB + r, lo), last_pos);           // rows outside repeat a row that is there
             const size_t row = (size_t)(base + t - lo);
             if (c < kc)
@@ -188,147 +216,180 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
             else
                 cp_async16(vs + ((size_t)buf * KB + r) * ldv + (c - kc - rc) * 8,
                            kx + row * ld_kx + v0 + (size_t)h * dv + (c - kc - rc) * 8);
+            r += step_r;
+            c += step_c;
+            if (c >= all) { c -= all; ++r; }
         }
     };
 
-    load_block(kb_begin, 0);
-    cp_async_commit();
-    for (int it = 0; it < n_iter; ++it) {
-        const int kb = kb_begin + it, buf = it & 1;
-        if (it + 1 < n_iter) load_block(kb + 1, buf ^ 1);
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; ++i) {
+        if (i < n_iter) load_block(kb_begin + i, i);
         cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
+    }
+    int buf = 0;
+    for (int it = 0; it < n_iter; ++it, buf = buf + 1 == STAGES ? 0 : buf + 1) {
+        const int kb = kb_begin + it;
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();                              // this block's keys are there, the ones before are done with
+        if (it + STAGES - 1 < n_iter) load_block(kb + STAGES - 1, buf == 0 ? STAGES - 1 : buf - 1);
+        cp_async_commit();
+        const int key0 = kb * KB;
+        if (!live || key0 > w_last || key0 + KB <= w_first) continue;
 
         const __nv_bfloat16* kt = ks + (size_t)buf * KB * ldk;
         const __nv_bfloat16* vt = vs + (size_t)buf * KB * ldv;
-        float s[KB / 8][4];
+        float s[MT][KB / 8][4];
+        const int mi = lane >> 3, r8 = lane & 7;
 #pragma unroll
         for (int j = 0; j < KB / 8; ++j) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
-            const __nv_bfloat16* krow = kt + (size_t)(j * 8 + gq) * ldk + 2 * t4;
+            for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-            for (int kk = 0; kk < DKM / 16; ++kk) {
+                for (int e = 0; e < 4; ++e) s[mt][j][e] = 0.f;
+            const __nv_bfloat16* krow = kt + (size_t)(j * 8 + r8) * ldk + mi * 8;
+#pragma unroll
+            for (int kk = 0; kk < DKM / 16; kk += 2) {
                 if (kk * 16 < dk) {
-                    const unsigned b0 = *reinterpret_cast<const unsigned*>(krow + kk * 16);
-                    const unsigned b1 = *reinterpret_cast<const unsigned*>(krow + kk * 16 + 8);
-                    mma_bf16(s[j], qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3], b0, b1);
+                    unsigned kf[4];
+                    const bool two = kk * 16 + 16 < dk;
+                    if (two) ldmatrix_x4(kf, krow + kk * 16);
+                    else ldmatrix_x2(kf, krow + kk * 16 - (mi >> 1) * 16);
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt) mma_bf16(s[mt][j], qf[mt][kk][0], qf[mt][kk][1], qf[mt][kk][2], qf[mt][kk][3], kf[0], kf[1]);
+                    if (two && kk + 1 < DKM / 16) {
+                        const int k1 = kk + 1 < DKM / 16 ? kk + 1 : kk;
+#pragma unroll
+                        for (int mt = 0; mt < MT; ++mt)
+                            mma_bf16(s[mt][j], qf[mt][k1][0], qf[mt][k1][1], qf[mt][k1][2], qf[mt][k1][3], kf[2], kf[3]);
+                    }
                 }
             }
         }
-        const int key0 = kb * KB;
-        const bool need_mask = key0 + KB - 1 > pos0 + warp * 16 || (window > 0 && key0 <= pos0 + warp * 16 + 15 - window);
-        float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
-        for (int j = 0; j < KB / 8; ++j) {
+        for (int mt = 0; mt < MT; ++mt) {
+            const int q0 = pos0 + w0 + mt * 16, p0 = q0 + gq, p1 = p0 + 8;
+            const bool need_mask = key0 + KB - 1 > q0 || (window > 0 && key0 <= q0 + 15 - window);
+            float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                float sc = s[j][e] * scale;
-                if (need_mask) {
-                    const int t = key0 + j * 8 + 2 * t4 + (e & 1);
-                    const int p = (e < 2) ? p0 : p1;
-                    if (t > p || (window > 0 && t <= p - window)) sc = -INFINITY;
+            for (int j = 0; j < KB / 8; ++j) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float sc = s[mt][j][e] * scale;
+                    if (need_mask) {
+                        const int t = key0 + j * 8 + 2 * t4 + (e & 1);
+                        const int p = (e < 2) ? p0 : p1;
+                        if (t > p || (window > 0 && t <= p - window)) sc = -INFINITY;
+                    }
+                    s[mt][j][e] = sc;
                 }
-                s[j][e] = sc;
+                mx0 = fmaxf(mx0, fmaxf(s[mt][j][0], s[mt][j][1]));
+                mx1 = fmaxf(mx1, fmaxf(s[mt][j][2], s[mt][j][3]));
             }
-            mx0 = fmaxf(mx0, fmaxf(s[j][0], s[j][1]));
-            mx1 = fmaxf(mx1, fmaxf(s[j][2], s[j][3]));
-        }
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-        const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
-        // a row whose keys are all masked so far (and that has no sink) keeps m = -inf; use 0 as its reference
-        const float ref0 = mn0 == -INFINITY ? 0.f : mn0, ref1 = mn1 == -INFINITY ? 0.f : mn1;
-        const float c0 = m0 == -INFINITY ? 0.f : exp2f((m0 - ref0) * LOG2E);
-        const float c1 = m1 == -INFINITY ? 0.f : exp2f((m1 - ref1) * LOG2E);
-        m0 = mn0; m1 = mn1;
-        float sum0 = 0.f, sum1 = 0.f;
+            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+            const float mn0 = fmaxf(m[mt][0], mx0), mn1 = fmaxf(m[mt][1], mx1);
+            // a row whose keys are all masked so far (and that has no sink) keeps m = -inf; use 0 as its reference
+            const float ref0 = mn0 == -INFINITY ? 0.f : mn0, ref1 = mn1 == -INFINITY ? 0.f : mn1;
+            const float c0 = m[mt][0] == -INFINITY ? 0.f : ex2((m[mt][0] - ref0) * LOG2E);
+            const float c1 = m[mt][1] == -INFINITY ? 0.f : ex2((m[mt][1] - ref1) * LOG2E);
+            m[mt][0] = mn0; m[mt][1] = mn1;
+            float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
-        for (int j = 0; j < KB / 8; ++j) {
-            s[j][0] = exp2f((s[j][0] - ref0) * LOG2E);
-            s[j][1] = exp2f((s[j][1] - ref0) * LOG2E);
-            s[j][2] = exp2f((s[j][2] - ref1) * LOG2E);
-            s[j][3] = exp2f((s[j][3] - ref1) * LOG2E);
-            sum0 += s[j][0] + s[j][1];
-            sum1 += s[j][2] + s[j][3];
-        }
-        l0 = l0 * c0 + sum0;
-        l1 = l1 * c1 + sum1;
+            for (int j = 0; j < KB / 8; ++j) {
+                s[mt][j][0] = ex2((s[mt][j][0] - ref0) * LOG2E);
+                s[mt][j][1] = ex2((s[mt][j][1] - ref0) * LOG2E);
+                s[mt][j][2] = ex2((s[mt][j][2] - ref1) * LOG2E);
+                s[mt][j][3] = ex2((s[mt][j][3] - ref1) * LOG2E);
+                sum0 += s[mt][j][0] + s[mt][j][1];
+                sum1 += s[mt][j][2] + s[mt][j][3];
+            }
+            l[mt][0] = l[mt][0] * c0 + sum0;
+            l[mt][1] = l[mt][1] * c1 + sum1;
+            if (__any_sync(0xffffffffu, c0 != 1.f || c1 != 1.f)) {
 #pragma unroll
-        for (int j = 0; j < DVM / 8; ++j) {
-            oacc[j][0] *= c0; oacc[j][1] *= c0;
-            oacc[j][2] *= c1; oacc[j][3] *= c1;
+                for (int j = 0; j < DVM / 8; ++j) {
+                    oacc[mt][j][0] *= c0; oacc[mt][j][1] *= c0;
+                    oacc[mt][j][2] *= c1; oacc[mt][j][3] *= c1;
+                }
+            }
         }
         // O += P V, 16 keys at a time; P = hi + lo
 #pragma unroll
         for (int kk = 0; kk < KB / 16; ++kk) {
-            unsigned hi[4], lw[4];
+            unsigned hi[MT][4], lw[MT][4];
 #pragma unroll
-            for (int f = 0; f < 4; ++f) {
-                const float x = s[2 * kk + (f >> 1)][(f & 1) * 2], y = s[2 * kk + (f >> 1)][(f & 1) * 2 + 1];
-                const __nv_bfloat162 hv = __floats2bfloat162_rn(x, y);
-                hi[f] = *reinterpret_cast<const unsigned*>(&hv);
-                lw[f] = pack_bf16(x - __low2float(hv), y - __high2float(hv));
-            }
+            for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                for (int f = 0; f < 4; ++f) {
+                    const float x = s[mt][2 * kk + (f >> 1)][(f & 1) * 2], y = s[mt][2 * kk + (f >> 1)][(f & 1) * 2 + 1];
+                    const __nv_bfloat162 hv = __floats2bfloat162_rn(x, y);
+                    hi[mt][f] = *reinterpret_cast<const unsigned*>(&hv);
+                    lw[mt][f] = pack_bf16(x - __uint_as_float(hi[mt][f] << 16), y - __uint_as_float(hi[mt][f] & 0xffff0000u));
+                }
 #pragma unroll
             for (int dj = 0; dj < DVM / 16; ++dj) {
                 if (dj * 16 < dv) {
                     unsigned vb[4];
-                    const int mi = lane >> 3, r = lane & 7;
-                    ldmatrix_x4_trans(vb, vt + (size_t)(kk * 16 + (mi & 1) * 8 + r) * ldv + dj * 16 + (mi >> 1) * 8);
-                    mma_bf16(oacc[2 * dj], hi[0], hi[1], hi[2], hi[3], vb[0], vb[1]);
-                    mma_bf16(oacc[2 * dj + 1], hi[0], hi[1], hi[2], hi[3], vb[2], vb[3]);
-                    mma_bf16(oacc[2 * dj], lw[0], lw[1], lw[2], lw[3], vb[0], vb[1]);
-                    mma_bf16(oacc[2 * dj + 1], lw[0], lw[1], lw[2], lw[3], vb[2], vb[3]);
+                    ldmatrix_x4_trans(vb, vt + (size_t)(kk * 16 + (mi & 1) * 8 + r8) * ldv + dj * 16 + (mi >> 1) * 8);
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt) {
+                        mma_bf16(oacc[mt][2 * dj], hi[mt][0], hi[mt][1], hi[mt][2], hi[mt][3], vb[0], vb[1]);
+                        mma_bf16(oacc[mt][2 * dj + 1], hi[mt][0], hi[mt][1], hi[mt][2], hi[mt][3], vb[2], vb[3]);
+                    }
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt) {
+                        mma_bf16(oacc[mt][2 * dj], lw[mt][0], lw[mt][1], lw[mt][2], lw[mt][3], vb[0], vb[1]);
+                        mma_bf16(oacc[mt][2 * dj + 1], lw[mt][0], lw[mt][1], lw[mt][2], lw[mt][3], vb[2], vb[3]);
+                    }
                 }
             }
         }
-        __syncthreads();
     }
+    if (!live) return;
 
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-    const float inv[2] = {l0 > 0.f ? 1.f / l0 : 0.f, l1 > 0.f ? 1.f / l1 : 0.f};
-    const int qi[2] = {qi0, qi1};
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        if (qi[half] >= nq) continue;
-        const size_t n = (size_t)(row0 + qi[half]);
-        const float* g = gate && !gate_heads ? gate + n * ld_gate + (size_t)h * dv + 2 * t4 : nullptr;
-        const float gh = (gate && gate_heads ? 1.0f / (1.0f + expf(-gate[n * ld_gate + h])) : 1.f) * inv[half];
-        __nv_bfloat16* dst = o + (n * nh + h) * dv + 2 * t4;
+    for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
-        for (int j = 0; j < DVM / 8; ++j) {
-            if (j * 8 < dv) {
-                float x = oacc[j][2 * half] * gh, y = oacc[j][2 * half + 1] * gh;
-                if (g) {
-                    x *= 1.0f / (1.0f + expf(-g[j * 8]));
-                    y *= 1.0f / (1.0f + expf(-g[j * 8 + 1]));
+        for (int half = 0; half < 2; ++half) {
+            float den = l[mt][half];
+            den += __shfl_xor_sync(0xffffffffu, den, 1);
+            den += __shfl_xor_sync(0xffffffffu, den, 2);
+            const float inv = den > 0.f ? 1.f / den : 0.f;
+            const int qi = w0 + mt * 16 + gq + 8 * half;
+            if (qi >= nq) continue;
+            const size_t n = (size_t)(row0 + qi);
+            const float* g = gate && !gate_heads ? gate + n * ld_gate + (size_t)h * dv + 2 * t4 : nullptr;
+            const float gh = (gate && gate_heads ? 1.0f / (1.0f + expf(-gate[n * ld_gate + h])) : 1.f) * inv;
+            __nv_bfloat16* dst = o + (n * nh + h) * dv + 2 * t4;
+#pragma unroll
+            for (int j = 0; j < DVM / 8; ++j) {
+                if (j * 8 < dv) {
+                    float x = oacc[mt][j][2 * half] * gh, y = oacc[mt][j][2 * half + 1] * gh;
+                    if (g) {
+                        x *= 1.0f / (1.0f + expf(-g[j * 8]));
+                        y *= 1.0f / (1.0f + expf(-g[j * 8 + 1]));
+                    }
+                    *reinterpret_cast<unsigned*>(dst + j * 8) = pack_bf16(x, y);
                 }
-                *reinterpret_cast<unsigned*>(dst + j * 8) = pack_bf16(x, y);
             }
         }
     }
 }
 
-template <int DKM, int DVM>
+template <int DKM, int DVM, int MT>
 int launch(const void* q, const void* kx, int ld_kx, int v0, const void* rk, const int* cu, const int* starts,
            const float* sinks, const float* gate, int ld_gate, int gate_heads, void* o, int N, int B, int nh, int dim, int rot, int dv,
            float scale, int window, cudaStream_t stream) {
-    const size_t smem = (size_t)2 * KB * (dim + rot + 8 + dv + 8) * sizeof(__nv_bfloat16);
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaFuncSetAttribute(latent_attention_prefill_kernel<DKM, DVM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)((size_t)2 * KB * (DKM + 8 + DVM + 8) * sizeof(__nv_bfloat16)));
-        attr_set = true;
-    }
+    constexpr int QT = NWARPS * 16 * MT;
+    const size_t smem = (size_t)3 * KB * (dim + rot + 8 + dv + 8) * sizeof(__nv_bfloat16);
+    static const cudaError_t attr = cudaFuncSetAttribute(latent_attention_prefill_kernel<DKM, DVM, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)((size_t)3 * KB * (DKM + 8 + DVM + 8) * sizeof(__nv_bfloat16)));
+    if (attr != cudaSuccess) return (int)attr;
     const dim3 grid((N + QT - 1) / QT + B, nh);       // an upper bound of the tiles; spare blocks return at once
-    mv_launch(latent_attention_prefill_kernel<DKM, DVM>, grid, NWARPS * 32, smem, stream, (const __nv_bfloat16*)q,
+    mv_launch(latent_attention_prefill_kernel<DKM, DVM, MT>, grid, NWARPS * 32, smem, stream, (const __nv_bfloat16*)q,
               (const __nv_bfloat16*)kx, ld_kx, v0, (const __nv_bfloat16*)rk, cu, starts, sinks, gate, ld_gate,
               gate_heads, (__nv_bfloat16*)o, B, nh, dim, rot, dv, scale, window);
     return mv_launch_status();
@@ -374,12 +435,14 @@ MV_API int mv_latent_attention_prefill(const void* q, const void* kx, int ld_kx,
     if (dim % 8 || rot % 8 || dk % 16 || dv % 16 || dk < 16 || dv < 16 || dk > 192 || dv > 128 || ld_kx % 8 || v0 % 8 ||
         window < 0)
         return (int)cudaErrorInvalidValue;
-#define LP_GO(A, C)                                                                                                        \
-    return launch<A, C>(q, kx, ld_kx, v0, r, cu, starts, sinks, gate, ld_gate, gate_heads, o, N, B, nh, dim, rot, dv, scale, window, \
-                        stream)
-    if (dk <= 128 && dv <= 64) LP_GO(128, 64);
-    if (dk <= 128) LP_GO(128, 128);
-    if (dv <= 64) LP_GO(192, 64);
-    LP_GO(192, 128);
+#define LP_GO(A, C, M)                                                                                                     \
+    return launch<A, C, M>(q, kx, ld_kx, v0, r, cu, starts, sinks, gate, ld_gate, gate_heads, o, N, B, nh, dim, rot, dv, scale, window, \
+                           stream)
+    // two tiles of queries a warp where their fragments fit the registers and the blocks of 128 queries still go round
+    if (dk <= 96 && dv <= 64 && (long long)N * nh >= 148 * 2 * 64) LP_GO(96, 64, 2);
+    if (dk <= 128 && dv <= 64) LP_GO(128, 64, 1);
+    if (dk <= 128) LP_GO(128, 128, 1);
+    if (dv <= 64) LP_GO(192, 64, 1);
+    LP_GO(192, 128, 1);
 #undef LP_GO
 }

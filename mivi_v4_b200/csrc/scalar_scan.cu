@@ -18,7 +18,7 @@
 // column in registers.  With a normalizer every block carries that column too (as a 17th group of lanes),
 // so that it can divide without waiting for another block; the block of the first tile stores it.  The
 // order of every sum depends on nothing but dk, so a prompt gives the same numbers however it is cut.
-#include "common.cuh"
+#include "chunked_state.cuh"
 
 #define SS_COLS 16
 #define SS_PART 8
@@ -218,274 +218,447 @@ MV_API int mv_memory_gates(const float* zi, int ld_i, const float* zf, int ld_f,
 //
 // Every exponent is a difference of cumulative logarithms taken the right way round, so every factor lies in
 // (0, 1] (times b): nothing overflows however small a decay is.  Because the decay is one number a head, q and k
-// need no decayed copies: the products q_t . k_s are worked out once per GROUP of heads that share q and k (the
-// first kernel), and each head puts its own factors on them.  The second kernel walks a sequence's chunks with
-// the state in registers: a block is 16 value columns of one head of one sequence, its 32 half-warps each hold
-// RH key channels of every column.  With a normalizer the state's last column is fed ones instead of values and
-// comes out as n . q; a third kernel divides.  All of it is float32 on the CUDA cores.
+// need no decayed copies: the products q_t . k_s are worked out once per GROUP of heads that share q and k
+// (ss_products_kernel), and each head puts its own factors on them (ss_factors_kernel).  ss_walk_kernel walks a sequence's chunks
+// with nothing but the state, a tile of which lies in a block's registers, and leaves the state before every chunk;
+// ss_output_kernel then has a block for every chunk, head and 64 value columns.  With a normalizer the state's last column is fed
+// ones instead of values and comes out as n . q, by which the outputs are divided.  All of it is float32 on the CUDA cores.
+//
+// Every sum is added up in a fixed order: a state's element token by token; an output as the sums over 4 key channels (8 from
+// dk 129 on), these one after the other, times the decay, then the chunk's tokens in order.  A layer behind a matrix memory
+// divides by sums that may nearly cancel and routers compare what comes out, so another order moves whole outputs by percents.
+// @MEASURED@
 //
 // Chunks are numbered floor(cu[b] / SC_CHUNK) + b + c for chunk c of the step's sequence b: distinct numbers
 // below N / SC_CHUNK + n_seqs + 1 that need nothing from the host.
 #define SC_CHUNK 32
-#define SC_COLS 16
-#define SC_THREADS 256
-#define SC_SCAN_THREADS 512
-#define SC_GROUPS (SC_SCAN_THREADS / 16)
-#define SC_RED_STRIDE (SC_CHUNK * SC_COLS + 16)
+#define SC_WALK_THREADS 256
 
-__global__ void __launch_bounds__(SC_THREADS)
-scalar_chunk_products_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
-                             const int* __restrict__ cu, float* __restrict__ G, int n_groups, int dk) {
+struct ScArgs {
+    const float *q, *k, *v;             // rows of the step's tokens; head h reads the columns (h / heads_per_group) dk, the same, h dv
+    int ldq, ldk, ldv;
+    const float *log_a, *b, *skip, *m_tok;
+    int ld_a, ld_b;
+    float q_scale;
+    float *state, *before;              // [slot][head][cols][dk]; [chunk][head][cols][lds]: the state before every chunk
+    float *G;                           // q_t . k_s [chunk][group][SC_CHUNK][SC_CHUNK]
+    float *run, *e1, *e2, *el;          // [chunk][head][SC_CHUNK]: running log decay, e^(c_t) q_scale, e^(c_last - c_t) b_t; [chunk][head]: e^(c_last)
+    const int *slots, *cu;
+    float* o;
+    int n_heads, heads_per_group, dk, dv, lds, wide, normalizer;
+};
+
+namespace {
+
+// a warp a chunk and head
+__global__ void __launch_bounds__(128)
+ss_factors_kernel(const ScArgs a) {
     mv_pdl_begin();
-    extern __shared__ float smem[];
-    const int lds = dk + 1;                         // odd row stride: rows of different tokens fall into different banks
-    float* qa = smem;                               // [SC_CHUNK][lds]
-    float* ka = qa + SC_CHUNK * lds;
-    const int c = blockIdx.x, g = blockIdx.y, b = blockIdx.z;
-    const int row0 = cu[b], len = cu[b + 1] - row0;
-    if (c * SC_CHUNK >= len) return;
+    const int c = blockIdx.x, h = blockIdx.y * 4 + (threadIdx.x >> 5), b = blockIdx.z, t = threadIdx.x & 31;
+    const int row0 = a.cu[b], len = a.cu[b + 1] - row0;
+    if (c * SC_CHUNK >= len || h >= a.n_heads) return;
     const int nt = min(SC_CHUNK, len - c * SC_CHUNK);
-    const int first = row0 + c * SC_CHUNK;
-    const int chunk = row0 / SC_CHUNK + b + c;
-    for (int idx = threadIdx.x; idx < nt * dk; idx += SC_THREADS) {
-        const int t = idx / dk, i = idx - t * dk;
-        qa[t * lds + i] = q[(size_t)(first + t) * ldq + (size_t)g * dk + i];
-        ka[t * lds + i] = k[(size_t)(first + t) * ldk + (size_t)g * dk + i];
+    const size_t row = (size_t)row0 + c * SC_CHUNK + t, at = (size_t)(row0 / SC_CHUNK + b + c) * a.n_heads + h;
+    float run = t < nt ? a.log_a[row * a.ld_a + h] : 0.f;
+    const float bt = t < nt ? a.b[row * a.ld_b + h] : 0.f;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const float up = __shfl_up_sync(0xffffffffu, run, d);
+        if (t >= d) run += up;
     }
-    __syncthreads();
-    float* Gc = G + ((size_t)chunk * n_groups + g) * SC_CHUNK * SC_CHUNK;
-    for (int p = threadIdx.x; p < SC_CHUNK * SC_CHUNK; p += SC_THREADS) {
-        const int t = p / SC_CHUNK, s = p - t * SC_CHUNK;
-        float sum = 0.f;
-        if (s <= t && t < nt) {
-            const float* qt = qa + t * lds;
-            const float* kt = ka + s * lds;
-            for (int i = 0; i < dk; ++i) sum = fmaf(qt[i], kt[i], sum);
-        }
-        Gc[p] = sum;
-    }
+    const float last = __shfl_sync(0xffffffffu, run, nt - 1);
+    a.run[at * SC_CHUNK + t] = run;
+    a.e1[at * SC_CHUNK + t] = expf(run) * a.q_scale;
+    a.e2[at * SC_CHUNK + t] = t < nt ? expf(last - run) * bt : 0.f;
+    if (t == 0) a.el[at] = expf(last);
 }
 
-template <int RH>
-__global__ void __launch_bounds__(SC_SCAN_THREADS)
-scalar_chunk_scan_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
-                         const float* __restrict__ v, int ldv, const float* __restrict__ log_a, int ld_a,
-                         const float* __restrict__ b_in, int ld_b, const float* __restrict__ skip, float q_scale,
-                         const float* __restrict__ G, float* __restrict__ state, const int* __restrict__ slots,
-                         const int* __restrict__ cu, float* __restrict__ o, int n_heads, int heads_per_group, int dk,
-                         int dv, int ones_col) {
+constexpr int SP_LD = 36;
+
+// 64 threads, 4 x 4 products each; channels in order
+__global__ void __launch_bounds__(64)
+ss_products_kernel(const ScArgs a) {
+    __shared__ __align__(16) float qs[2][SC_CHUNK * SP_LD], ks[2][SC_CHUNK * SP_LD];
     mv_pdl_begin();
-    constexpr int DKP = SC_GROUPS * RH;
-    extern __shared__ __align__(16) float smem[];
-    float* qt = smem;                               // [SC_CHUNK][DKP], zero beyond dk
-    float* kt = qt + SC_CHUNK * DKP;
-    float* vt = kt + SC_CHUNK * DKP;                // [SC_CHUNK][SC_COLS]
-    float* pt = vt + SC_CHUNK * SC_COLS;            // [SC_CHUNK][SC_CHUNK]
-    float* la = pt + SC_CHUNK * SC_CHUNK;           // [SC_CHUNK] log decays, then their running sum
-    float* bs = la + SC_CHUNK;                      // [SC_CHUNK] input factors
-    float* e1 = bs + SC_CHUNK;                      // [SC_CHUNK] e^(c_t) q_scale
-    float* e2 = e1 + SC_CHUNK;                      // [SC_CHUNK] e^(c_last - c_t) b_t
-    float* el = e2 + SC_CHUNK;                      // [1] e^(c_last) (padded to 16 floats)
-    float* red = el + 16;                           // [SC_GROUPS][SC_RED_STRIDE]: [SC_CHUNK][SC_COLS] a group
-    const int tile = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
-    const int tid = threadIdx.x, col = tid & 15, grp = tid >> 4;
-    const int cols = dv + (ones_col >= 0 ? 1 : 0);  // the state's and the output's columns
-    const int j = tile * SC_COLS + col;
-    const int row0 = cu[b], len = cu[b + 1] - row0;
-    if (len <= 0) return;
-    const int slot = mv_read_slot(slots[b]);
-    const int n_groups = n_heads / heads_per_group, g = h / heads_per_group;
-    const size_t goff = (size_t)g * dk;
-    float* srow = state + (((size_t)slot * n_heads + h) * cols + (j < cols ? j : 0)) * dk;
-    float S[RH];
-#pragma unroll
-    for (int r = 0; r < RH; ++r) {
-        const int i = grp * RH + r;
-        S[r] = (j < cols && i < dk) ? srow[i] : 0.f;
-    }
-    const float sk = skip ? skip[h] : 0.f;
-    const int n_chunks = (len + SC_CHUNK - 1) / SC_CHUNK;
-    constexpr int IT = SC_CHUNK * DKP / SC_SCAN_THREADS;
-    static_assert(SC_CHUNK * SC_COLS == SC_SCAN_THREADS && SC_CHUNK * SC_CHUNK % SC_SCAN_THREADS == 0,
-                  "a thread requests one value of v and whole rounds of the products");
-    float rq[IT], rk[IT], rv, rp[SC_CHUNK * SC_CHUNK / SC_SCAN_THREADS], rla = 0.f, rb = 0.f;
-    auto request = [&](int c) {
-        const int nt = min(SC_CHUNK, len - c * SC_CHUNK);
-        const int first = row0 + c * SC_CHUNK;
-        const int chunk = row0 / SC_CHUNK + b + c;
-#pragma unroll
-        for (int it = 0; it < IT; ++it) {
-            const int idx = tid + it * SC_SCAN_THREADS, t = idx / DKP, i = idx - t * DKP;
-            const bool in = t < nt && i < dk;
-            rq[it] = in ? q[(size_t)(first + t) * ldq + goff + i] : 0.f;
-            rk[it] = in ? k[(size_t)(first + t) * ldk + goff + i] : 0.f;
-        }
-        {
-            const int t = tid / SC_COLS, cc = tile * SC_COLS + (tid - t * SC_COLS);
-            rv = t < nt ? (cc < dv ? v[(size_t)(first + t) * ldv + (size_t)h * dv + cc] : (cc == ones_col ? 1.f : 0.f)) : 0.f;
-        }
-        const float* Gc = G + ((size_t)chunk * n_groups + g) * SC_CHUNK * SC_CHUNK;
-#pragma unroll
-        for (int it = 0; it < SC_CHUNK * SC_CHUNK / SC_SCAN_THREADS; ++it) rp[it] = Gc[tid + it * SC_SCAN_THREADS];
-        if (tid < SC_CHUNK) {
-            rla = tid < nt ? log_a[(size_t)(first + tid) * ld_a + h] : 0.f;
-            rb = tid < nt ? b_in[(size_t)(first + tid) * ld_b + h] : 0.f;
-        }
+    const int c = blockIdx.x, g = blockIdx.y, b = blockIdx.z, ts = threadIdx.x & 7, tt = threadIdx.x >> 3;
+    const int row0 = a.cu[b], len = a.cu[b + 1] - row0;
+    if (c * SC_CHUNK >= len) return;
+    const int nt = min(SC_CHUNK, len - c * SC_CHUNK), slices = (a.dk + 31) / 32;
+    const size_t first = (size_t)row0 + c * SC_CHUNK;
+    auto load = [&](int s) {
+        cs_load<SC_CHUNK, 32, SP_LD, false, 64>(qs[s & 1], a.q + first * a.ldq + (size_t)g * a.dk + s * 32, a.ldq, nt, a.dk - s * 32, a.wide);
+        cs_load<SC_CHUNK, 32, SP_LD, false, 64>(ks[s & 1], a.k + first * a.ldk + (size_t)g * a.dk + s * 32, a.ldk, nt, a.dk - s * 32, a.wide);
+        cs_commit();
     };
-    request(0);
+    float acc[4][4];
+#pragma unroll
+    for (int y = 0; y < 4; ++y)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) acc[y][x] = 0.f;
+    load(0);
+    for (int s = 0; s < slices; ++s) {
+        if (s + 1 < slices) { load(s + 1); cs_wait<1>(); }
+        else cs_wait<0>();
+        __syncthreads();
+#pragma unroll 4
+        for (int kk = 0; kk < 32; kk += 4) {
+            float4 w[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) w[x] = *reinterpret_cast<const float4*>(ks[s & 1] + (ts + 8 * x) * SP_LD + kk);
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+                const float4 u = *reinterpret_cast<const float4*>(qs[s & 1] + (tt + 8 * y) * SP_LD + kk);
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    acc[y][x] = fmaf(u.x, w[x].x, acc[y][x]); acc[y][x] = fmaf(u.y, w[x].y, acc[y][x]);
+                    acc[y][x] = fmaf(u.z, w[x].z, acc[y][x]); acc[y][x] = fmaf(u.w, w[x].w, acc[y][x]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    float* to = a.G + ((size_t)(row0 / SC_CHUNK + b + c) * (a.n_heads / a.heads_per_group) + g) * SC_CHUNK * SC_CHUNK;
+#pragma unroll
+    for (int y = 0; y < 4; ++y)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) to[(tt + 8 * y) * SC_CHUNK + ts + 8 * x] = acc[y][x];
+}
+
+// A block has 64 value columns x 64 key channels of a head's state, a thread 4 x 4; two chunks' rows are on their way
+// while one is worked on, whose values are first multiplied by their factors in place.
+constexpr int SW_STAGES = 3;
+constexpr size_t SW_SMEM = sizeof(float) * SW_STAGES * (2 * SC_CHUNK * 64 + SC_CHUNK);
+
+__global__ void __launch_bounds__(SC_WALK_THREADS)
+ss_walk_kernel(const ScArgs a) {
+    extern __shared__ __align__(16) float sw_smem[];
+    float* ks = sw_smem;                                // [STAGES][SC_CHUNK][64]
+    float* vs = ks + SW_STAGES * SC_CHUNK * 64;         // [STAGES][SC_CHUNK][64]
+    float* ws = vs + SW_STAGES * SC_CHUNK * 64;         // [STAGES][SC_CHUNK]
+    mv_pdl_begin();
+    const int tiles_i = (a.dk + 63) / 64, i0 = (blockIdx.x % tiles_i) * 64, j0 = (blockIdx.x / tiles_i) * 64;
+    const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, ti = tid & 15, tj = tid >> 4;
+    const int row0 = a.cu[b], len = a.cu[b + 1] - row0;
+    if (len <= 0) return;
+    const int cols = a.dv + a.normalizer, slot = mv_read_slot(a.slots[b]);
+    const bool with_n = a.normalizer && j0 == 0;
+    const int i = i0 + ti * 4, j = j0 + tj * 4;
+    float* st = a.state + ((size_t)slot * a.n_heads + h) * cols * a.dk;
+    const bool vec = a.dk % 4 == 0;                     // the state's rows start on 16 bytes
+    float S[4][4], n[4];
+    auto read4 = [&](const float* p, float* out) {
+        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (vec && i < a.dk) r = *reinterpret_cast<const float4*>(p + i);
+        else {
+            if (i < a.dk) r.x = p[i];
+            if (i + 1 < a.dk) r.y = p[i + 1];
+            if (i + 2 < a.dk) r.z = p[i + 2];
+            if (i + 3 < a.dk) r.w = p[i + 3];
+        }
+        out[0] = r.x; out[1] = r.y; out[2] = r.z; out[3] = r.w;
+    };
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+        if (j + y < a.dv) read4(st + (size_t)(j + y) * a.dk, S[y]);
+        else S[y][0] = S[y][1] = S[y][2] = S[y][3] = 0.f;
+    }
+    n[0] = n[1] = n[2] = n[3] = 0.f;
+    if (with_n) read4(st + (size_t)a.dv * a.dk, n);
+    const float* kp = a.k + (size_t)row0 * a.ldk + (size_t)(h / a.heads_per_group) * a.dk + i0;
+    const float* vp = a.v + (size_t)row0 * a.ldv + (size_t)h * a.dv + j0;
+    const int n_chunks = (len + SC_CHUNK - 1) / SC_CHUNK, chunk0 = row0 / SC_CHUNK + b;
+    auto load = [&](int c) {
+        if (c < n_chunks) {
+            const int st_ = c % SW_STAGES;
+            const size_t t = (size_t)c * SC_CHUNK;
+            cs_load<SC_CHUNK, 64, 64, false, SC_WALK_THREADS>(ks + st_ * SC_CHUNK * 64, kp + t * a.ldk, a.ldk, len - (int)t, a.dk - i0, a.wide);
+            cs_load<SC_CHUNK, 64, 64, false, SC_WALK_THREADS>(vs + st_ * SC_CHUNK * 64, vp + t * a.ldv, a.ldv, len - (int)t, a.dv - j0, a.wide);
+            if (tid < SC_CHUNK / 4)
+                cs_copy(ws + st_ * SC_CHUNK + tid * 4, a.e2 + ((size_t)(chunk0 + c) * a.n_heads + h) * SC_CHUNK + tid * 4, true, true);
+        }
+        cs_commit();
+    };
+#pragma unroll
+    for (int c = 0; c < SW_STAGES - 1; ++c) load(c);
+    float d_next = a.el[(size_t)chunk0 * a.n_heads + h];        // the chunk's decay, requested a chunk ahead
     for (int c = 0; c < n_chunks; ++c) {
-        const int nt = min(SC_CHUNK, len - c * SC_CHUNK);
-        const int first = row0 + c * SC_CHUNK;
-        __syncthreads();                            // the chunk before is done with shared memory
+        // the state as it is before this chunk
+        float* to = a.before + ((size_t)(chunk0 + c) * a.n_heads + h) * cols * a.lds;
+        if (i < a.lds) {
 #pragma unroll
-        for (int it = 0; it < IT; ++it) {
-            qt[tid + it * SC_SCAN_THREADS] = rq[it];
-            kt[tid + it * SC_SCAN_THREADS] = rk[it];
+            for (int y = 0; y < 4; ++y)
+                if (j + y < a.dv)
+                    *reinterpret_cast<float4*>(to + (size_t)(j + y) * a.lds + i) = make_float4(S[y][0], S[y][1], S[y][2], S[y][3]);
+            if (with_n && tj == 0) *reinterpret_cast<float4*>(to + (size_t)a.dv * a.lds + i) = make_float4(n[0], n[1], n[2], n[3]);
         }
-        vt[tid] = rv;
 #pragma unroll
-        for (int it = 0; it < SC_CHUNK * SC_CHUNK / SC_SCAN_THREADS; ++it) pt[tid + it * SC_SCAN_THREADS] = rp[it];
-        if (tid < SC_CHUNK) {
-            // the running sum of the log decays over the chunk (one warp), and the factors that follow from it
-            float run = rla;
+        for (int x = 0; x < 4; ++x) {
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const float up = __shfl_up_sync(0xffffffffu, run, d);
-                if (tid >= d) run += up;
-            }
-            const float last = __shfl_sync(0xffffffffu, run, nt - 1);
-            la[tid] = run;
-            bs[tid] = rb;
-            e1[tid] = expf(run) * q_scale;
-            e2[tid] = tid < nt ? expf(last - run) * rb : 0.f;
-            if (tid == 0) el[0] = expf(last);
+            for (int y = 0; y < 4; ++y) S[y][x] *= d_next;
+            n[x] *= d_next;
         }
-        __syncthreads();
-        if (c + 1 < n_chunks) request(c + 1);
-        // this head's factors on the group's products: e^(c_t - c_s) b_s q_scale (own entries only: no one else reads them yet)
+        if (c + 1 < n_chunks) d_next = a.el[(size_t)(chunk0 + c + 1) * a.n_heads + h];
+        cs_wait<SW_STAGES - 2>();
+        __syncthreads();                                // this chunk's rows are there, the ones before are done with
+        load(c + SW_STAGES - 1);
+        const float* kt = ks + c % SW_STAGES * SC_CHUNK * 64 + ti * 4;
+        float* vt = vs + c % SW_STAGES * SC_CHUNK * 64;
+        const float* wt = ws + c % SW_STAGES * SC_CHUNK;
 #pragma unroll
-        for (int it = 0; it < SC_CHUNK * SC_CHUNK / SC_SCAN_THREADS; ++it) {
-            const int p = tid + it * SC_SCAN_THREADS, t = p / SC_CHUNK, s = p - t * SC_CHUNK;
-            pt[p] = (s <= t && t < nt) ? pt[p] * expf(la[t] - la[s]) * bs[s] * q_scale : 0.f;
-        }
-        // what the chunk's tokens read from the state before the chunk: this half-warp's key channels
-#pragma unroll 4
-        for (int t = 0; t < SC_CHUNK; ++t) {
-            const float4* q4 = reinterpret_cast<const float4*>(qt + t * DKP + grp * RH);
-            float acc = 0.f;
-#pragma unroll
-            for (int r = 0; r < RH; r += 4) {
-                const float4 x = q4[r >> 2];
-                acc = fmaf(x.x, S[r], acc); acc = fmaf(x.y, S[r + 1], acc);
-                acc = fmaf(x.z, S[r + 2], acc); acc = fmaf(x.w, S[r + 3], acc);
-            }
-            red[grp * SC_RED_STRIDE + t * SC_COLS + col] = acc;
-        }
-        // the state after the chunk
-        const float decay = el[0];
-#pragma unroll
-        for (int r = 0; r < RH; ++r) S[r] *= decay;
-#pragma unroll 4
-        for (int s = 0; s < SC_CHUNK; ++s) {
-            const float vj = vt[s * SC_COLS + col] * e2[s];
-            const float4* k4 = reinterpret_cast<const float4*>(kt + s * DKP + grp * RH);
-#pragma unroll
-            for (int r = 0; r < RH; r += 4) {
-                const float4 x = k4[r >> 2];
-                S[r] = fmaf(x.x, vj, S[r]); S[r + 1] = fmaf(x.y, vj, S[r + 1]);
-                S[r + 2] = fmaf(x.z, vj, S[r + 2]); S[r + 3] = fmaf(x.w, vj, S[r + 3]);
-            }
+        for (int e = 0; e < SC_CHUNK * 16 / SC_WALK_THREADS; ++e) {
+            const int at = tid + e * SC_WALK_THREADS;
+            const float w = wt[at >> 4];
+            float4 x = reinterpret_cast<float4*>(vt)[at];
+            x.x *= w; x.y *= w; x.z *= w; x.w *= w;
+            reinterpret_cast<float4*>(vt)[at] = x;
         }
         __syncthreads();
-        // outputs: the groups' shares in a fixed order, then the chunk's own tokens
-        for (int idx = tid; idx < nt * SC_COLS; idx += SC_SCAN_THREADS) {
-            const int t = idx / SC_COLS, cc = idx - t * SC_COLS;
-            float sum = 0.f;
+#pragma unroll 2
+        for (int s0 = 0; s0 < SC_CHUNK; s0 += 4) {
+            float4 k[4], v[4];
 #pragma unroll
-            for (int gg = 0; gg < SC_GROUPS; ++gg) sum += red[gg * SC_RED_STRIDE + t * SC_COLS + cc];
-            sum *= e1[t];
-            for (int s = 0; s <= t; ++s) sum = fmaf(pt[t * SC_CHUNK + s], vt[s * SC_COLS + cc], sum);
-            const int oc = tile * SC_COLS + cc;
-            if (oc < dv) sum = fmaf(sk, vt[t * SC_COLS + cc], sum);
-            if (oc < cols) o[(size_t)(first + t) * n_heads * cols + (size_t)h * cols + oc] = sum;
+            for (int s = 0; s < 4; ++s) {
+                k[s] = *reinterpret_cast<const float4*>(kt + (s0 + s) * 64);
+                v[s] = *reinterpret_cast<const float4*>(vt + (s0 + s) * 64 + tj * 4);
+            }
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                const float vy[4] = {v[s].x, v[s].y, v[s].z, v[s].w};
+#pragma unroll
+                for (int y = 0; y < 4; ++y) {
+                    S[y][0] = fmaf(k[s].x, vy[y], S[y][0]); S[y][1] = fmaf(k[s].y, vy[y], S[y][1]);
+                    S[y][2] = fmaf(k[s].z, vy[y], S[y][2]); S[y][3] = fmaf(k[s].w, vy[y], S[y][3]);
+                }
+            }
+            if (with_n) {
+                const float4 w = *reinterpret_cast<const float4*>(wt + s0);
+                const float wy[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    n[0] = fmaf(k[s].x, wy[s], n[0]); n[1] = fmaf(k[s].y, wy[s], n[1]);
+                    n[2] = fmaf(k[s].z, wy[s], n[2]); n[3] = fmaf(k[s].w, wy[s], n[3]);
+                }
+            }
         }
     }
-    if (j < cols && mv_slot_ok(slots[b])) {
+    if (mv_slot_ok(a.slots[b])) {
+        auto write4 = [&](float* p, const float* from) {
+            if (vec && i < a.dk) *reinterpret_cast<float4*>(p + i) = make_float4(from[0], from[1], from[2], from[3]);
+            else
 #pragma unroll
-        for (int r = 0; r < RH; ++r) {
-            const int i = grp * RH + r;
-            if (i < dk) srow[i] = S[r];
-        }
+                for (int x = 0; x < 4; ++x)
+                    if (i + x < a.dk) p[i + x] = from[x];
+        };
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+            if (j + y < a.dv) write4(st + (size_t)(j + y) * a.dk, S[y]);
+        if (with_n && tj == 0) write4(st + (size_t)a.dv * a.dk, n);
     }
 }
+
+// A block has one chunk's outputs in 64 value columns of one head, a thread 4 x 4 of them.  q and the state come in slices of
+// 32 key channels, the next slice on its way (the state's row of the normalizer behind its 64 rows).  RH: key channels a group.
+constexpr int SO_LD = 36, SO_THREADS = 128, SO_STAGE = (SC_CHUNK + 64 + 1) * SO_LD;
+constexpr size_t SO_SMEM = sizeof(float) * (2 * SO_STAGE + SC_CHUNK * SO_LD + SC_CHUNK * 64 + 2 * SC_CHUNK);
 
 template <int RH>
-static int scalar_chunk_scan_launch(dim3 grid, cudaStream_t stream, const float* q, int ldq, const float* k, int ldk,
-                                    const float* v, int ldv, const float* log_a, int ld_a, const float* b, int ld_b,
-                                    const float* skip, float q_scale, const float* G, float* state, const int* slots,
-                                    const int* cu, float* o, int n_heads, int hpg, int dk, int dv, int ones_col) {
-    const size_t smem = sizeof(float) * ((size_t)2 * SC_CHUNK * SC_GROUPS * RH + SC_CHUNK * SC_COLS + SC_CHUNK * SC_CHUNK +
-                                         4 * SC_CHUNK + 16 + SC_GROUPS * SC_RED_STRIDE);
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaFuncSetAttribute(scalar_chunk_scan_kernel<RH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr_set = true;
+__global__ void __launch_bounds__(SO_THREADS)
+ss_output_kernel(const ScArgs a) {
+    extern __shared__ __align__(16) float so_smem[];    // 2 x [q: 32 rows | state: 64 rows | n: 1 row][SO_LD]
+    float* ps = so_smem + 2 * SO_STAGE;                 // [32][SO_LD]
+    float* vs = ps + SC_CHUNK * SO_LD;                  // [32][64]
+    float* e1 = vs + SC_CHUNK * 64;                     // [32]
+    float* dn = e1 + SC_CHUNK;                          // [32] denominators
+    mv_pdl_begin();
+    const int tiles_j = (a.dv + 63) / 64, c = blockIdx.x / tiles_j, j0 = (blockIdx.x % tiles_j) * 64;
+    const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, tj = tid & 15, tt = tid >> 4;
+    const int row0 = a.cu[b], len = a.cu[b + 1] - row0;
+    if (c * SC_CHUNK >= len) return;
+    const int nt = min(SC_CHUNK, len - c * SC_CHUNK), chunk = row0 / SC_CHUNK + b + c;
+    const size_t first = (size_t)row0 + c * SC_CHUNK, at = (size_t)chunk * a.n_heads + h;
+    const int cols = a.dv + a.normalizer, g = h / a.heads_per_group, n_groups = a.n_heads / a.heads_per_group;
+    const float* S0 = a.before + at * cols * a.lds;
+    const float* qp = a.q + first * a.ldq + (size_t)g * a.dk;
+    const int slices = (a.dk + 31) / 32;
+    auto load = [&](int s) {
+        float* to = so_smem + (s & 1) * SO_STAGE;
+        cs_load<SC_CHUNK, 32, SO_LD, false, SO_THREADS>(to, qp + s * 32, a.ldq, nt, a.dk - s * 32, a.wide);
+        cs_load<64, 32, SO_LD, true, SO_THREADS>(to + SC_CHUNK * SO_LD, S0 + (size_t)j0 * a.lds + s * 32, a.lds, a.dv - j0, a.lds - s * 32, 1);
+        if (a.normalizer && tid < 8) {
+            const bool in = s * 32 + tid * 4 < a.lds;
+            cs_copy(to + (SC_CHUNK + 64) * SO_LD + tid * 4, S0 + (size_t)a.dv * a.lds + (in ? s * 32 + tid * 4 : 0), in, true);
+        }
+        cs_commit();
+    };
+    load(0);
+    cs_load<SC_CHUNK, 64, 64, false, SO_THREADS>(vs, a.v + first * a.ldv + (size_t)h * a.dv + j0, a.ldv, nt, a.dv - j0, a.wide);
+    cs_commit();
+    {
+        // this head's factors on the group's products
+        const float* Gc = a.G + ((size_t)chunk * n_groups + g) * SC_CHUNK * SC_CHUNK;
+        const float *run = a.run + at * SC_CHUNK, *bp = a.b + first * a.ld_b + h;
+        if (tid < SC_CHUNK) e1[tid] = a.e1[at * SC_CHUNK + tid];
+        const int s = tid & 31;
+        const float cs = run[s], bs = s < nt ? bp[(size_t)s * a.ld_b] : 0.f;
+#pragma unroll
+        for (int e = 0; e < SC_CHUNK * SC_CHUNK / SO_THREADS; ++e) {
+            const int t = (tid >> 5) + e * (SO_THREADS / 32);
+            ps[t * SO_LD + s] = (s <= t && t < nt) ? Gc[t * SC_CHUNK + s] * expf(run[t] - cs) * bs * a.q_scale : 0.f;
+        }
     }
-    mv_launch(scalar_chunk_scan_kernel<RH>, grid, SC_SCAN_THREADS, smem, stream, q, ldq, k, ldk, v, ldv, log_a, ld_a, b, ld_b,
-              skip, q_scale, G, state, slots, cu, o, n_heads, hpg, dk, dv, ones_col);
-    return mv_launch_status();
+    float acc[4][4];
+#pragma unroll
+    for (int y = 0; y < 4; ++y)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) acc[y][x] = 0.f;
+    float dot = 0.f;                                    // with a normalizer, warp 0: token tid's q . n
+    for (int s = 0; s < slices; ++s) {
+        if (s + 1 < slices) { load(s + 1); cs_wait<1>(); }
+        else cs_wait<0>();
+        __syncthreads();
+        const float* stage = so_smem + (s & 1) * SO_STAGE;
+        const float *q = stage + tt * SO_LD, *st = stage + (SC_CHUNK + tj) * SO_LD;
+#pragma unroll 2
+        for (int kk = 0; kk < 32; kk += RH) {
+            float part[4][4];
+#pragma unroll
+            for (int f = 0; f < RH; f += 4) {
+                float4 w[4];
+#pragma unroll
+                for (int x = 0; x < 4; ++x) w[x] = *reinterpret_cast<const float4*>(st + x * 16 * SO_LD + kk + f);
+#pragma unroll
+                for (int y = 0; y < 4; ++y) {
+                    const float4 u = *reinterpret_cast<const float4*>(q + y * 8 * SO_LD + kk + f);
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        float p = f == 0 ? u.x * w[x].x : fmaf(u.x, w[x].x, part[y][x]);
+                        p = fmaf(u.y, w[x].y, p); p = fmaf(u.z, w[x].z, p);
+                        part[y][x] = fmaf(u.w, w[x].w, p);
+                    }
+                }
+            }
+#pragma unroll
+            for (int y = 0; y < 4; ++y)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) acc[y][x] += part[y][x];
+        }
+        if (a.normalizer && tid < 32) {
+            const float *qt = stage + tid * SO_LD, *n0 = stage + (SC_CHUNK + 64) * SO_LD;
+#pragma unroll 2
+            for (int kk = 0; kk < 32; kk += RH) {
+                float p = 0.f;
+#pragma unroll
+                for (int f = 0; f < RH; f += 4) {
+                    const float4 u = *reinterpret_cast<const float4*>(qt + kk + f), w = *reinterpret_cast<const float4*>(n0 + kk + f);
+                    p = fmaf(u.x, w.x, p); p = fmaf(u.y, w.y, p); p = fmaf(u.z, w.z, p); p = fmaf(u.w, w.w, p);
+                }
+                dot += p;
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+        const float f = e1[tt + 8 * y];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) acc[y][x] *= f;
+    }
+    if (a.normalizer) {
+        if (tid < nt) {
+            dot = __fmul_rn(dot, e1[tid]);              // (rounded before the sum goes on, as the outputs are)
+            for (int s = 0; s <= tid; ++s) dot = __fadd_rn(dot, ps[tid * SO_LD + s]);
+            dn[tid] = fmaxf(fabsf(dot), expf(-a.m_tok[(first + tid) * a.n_heads + h])) + 1e-6f;
+        }
+        __syncthreads();
+    }
+    // what the chunk's tokens read from one another, in order (tokens 8 sb .. 8 sb + 7 for the rows from 8 sb on; a later token's
+    // value, which may not be finite, never meets an earlier row)
+    const int n_sb = (nt + 7) / 8;
+#pragma unroll 1
+    for (int s = 0; s < n_sb * 8; s += 4) {
+        const int sb = s >> 3, ds = s & 7;
+        float4 w[4];
+#pragma unroll
+        for (int z = 0; z < 4; ++z) w[z] = *reinterpret_cast<const float4*>(vs + (s + z) * 64 + tj * 4);
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+            if (y < sb) continue;
+            const float4 u = *reinterpret_cast<const float4*>(ps + (tt + 8 * y) * SO_LD + s);
+            const float uz[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int z = 0; z < 4; ++z)
+                if (y > sb || ds + z <= tt) {
+                    acc[y][0] = fmaf(uz[z], w[z].x, acc[y][0]); acc[y][1] = fmaf(uz[z], w[z].y, acc[y][1]);
+                    acc[y][2] = fmaf(uz[z], w[z].z, acc[y][2]); acc[y][3] = fmaf(uz[z], w[z].w, acc[y][3]);
+                }
+        }
+    }
+    const float sk = a.skip ? a.skip[h] : 0.f;
+    const int j = j0 + tj * 4;
+    const bool vec = a.dv % 4 == 0 && j + 3 < a.dv;
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+        const int t = tt + 8 * y;
+        if (t >= nt) continue;
+        float* to = a.o + (first + t) * a.n_heads * a.dv + (size_t)h * a.dv + j;
+        if (a.skip)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) acc[y][x] = fmaf(sk, vs[t * 64 + tj * 4 + x], acc[y][x]);
+        if (a.normalizer) {
+            const float d = dn[t];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) acc[y][x] = acc[y][x] / d;
+        }
+        if (vec) *reinterpret_cast<float4*>(to) = make_float4(acc[y][0], acc[y][1], acc[y][2], acc[y][3]);
+        else
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+                if (j + x < a.dv) to[x] = acc[y][x];
+    }
 }
 
-// o[n, h, :] = o_aug[n, h, :dv] / (max(|o_aug[n, h, dv]|, e^(-m[n, h])) + 1e-6)
-__global__ void __launch_bounds__(256)
-memory_normalize_kernel(const float* __restrict__ o_aug, const float* __restrict__ m_tok, float* __restrict__ o,
-                        long long total, int dv) {
-    mv_pdl_begin();
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= total) return;
-    const long long nh = idx / dv;
-    const int d = (int)(idx - nh * dv);
-    const float den = fmaxf(fabsf(o_aug[nh * (dv + 1) + dv]), expf(-m_tok[nh])) + 1e-6f;
-    o[idx] = o_aug[nh * (dv + 1) + d] / den;
-}
+}  // namespace
 
 // How many chunks the scratch of a step of N tokens in n_seqs sequences must hold.
 MV_API int mv_scalar_chunks(int N, int n_seqs) { return N / SC_CHUNK + n_seqs + 1; }
 
-// Arguments as mv_scalar_scan, plus the longest sequence's tokens (max_len) and scratch: G [chunks, groups,
-// SC_CHUNK, SC_CHUNK] with chunks = mv_scalar_chunks(N, n_seqs), and with a normalizer o_aug [N, n_heads * (dv + 1)].
+// Arguments as mv_scalar_scan, plus the longest sequence's tokens (max_len) and scratch with chunks =
+// mv_scalar_chunks(N, n_seqs): G [chunks, groups, SC_CHUNK, SC_CHUNK], before [chunks, n_heads, dv (+ 1), dk rounded up to 4]
+// and factors [chunks, n_heads, 3 SC_CHUNK + 4], both 16-byte aligned.
 MV_API int mv_scalar_scan_chunked(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
                                   const float* log_a, int ld_a, const float* b, int ld_b, const float* skip,
                                   const float* m_tok, float q_scale, float* state, const int* slots, const int* cu,
-                                  float* o, float* G, float* o_aug, int N, int n_seqs, int max_len, int n_heads,
-                                  int heads_per_group, int dk, int dv, int normalizer, cudaStream_t stream) {
+                                  float* o, float* G, float* before, float* factors, int chunks, int n_seqs, int max_len,
+                                  int n_heads, int heads_per_group, int dk, int dv, int normalizer, cudaStream_t stream) {
     if (n_seqs <= 0 || max_len <= 0) return 0;
-    if (dk < 1 || dk > 256 || dv < 1 || heads_per_group < 1 || n_heads % heads_per_group ||
-        (normalizer && (!m_tok || !o_aug)))
+    if (dk < 1 || dk > 256 || dv < 1 || heads_per_group < 1 || n_heads % heads_per_group || (normalizer && !m_tok) ||
+        ((uintptr_t)before | (uintptr_t)factors) % 16)
         return (int)cudaErrorInvalidValue;
-    const int n_groups = n_heads / heads_per_group;
-    const size_t smem_a = sizeof(float) * (size_t)2 * SC_CHUNK * (dk + 1);
-    static size_t attr_a = 0;
-    if (smem_a > attr_a) {
-        cudaFuncSetAttribute(scalar_chunk_products_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a);
-        attr_a = smem_a;
-    }
-    mv_launch(scalar_chunk_products_kernel, dim3((max_len + SC_CHUNK - 1) / SC_CHUNK, n_groups, n_seqs), SC_THREADS, smem_a,
-              stream, q, ldq, k, ldk, cu, G, n_groups, dk);
+    ScArgs a = {};
+    a.q = q; a.ldq = ldq; a.k = k; a.ldk = ldk; a.v = v; a.ldv = ldv;
+    a.log_a = log_a; a.ld_a = ld_a; a.b = b; a.ld_b = ld_b; a.skip = skip; a.m_tok = m_tok; a.q_scale = q_scale;
+    a.state = state; a.before = before; a.G = G; a.slots = slots; a.cu = cu; a.o = o;
+    const size_t rows = (size_t)chunks * n_heads;
+    a.run = factors; a.e1 = a.run + rows * SC_CHUNK; a.e2 = a.e1 + rows * SC_CHUNK; a.el = a.e2 + rows * SC_CHUNK;
+    a.n_heads = n_heads; a.heads_per_group = heads_per_group; a.dk = dk; a.dv = dv; a.lds = (dk + 3) & ~3;
+    a.normalizer = normalizer ? 1 : 0;
+    a.wide = cs_aligned(q, ldq, dk) && cs_aligned(k, ldk, dk) && cs_aligned(v, ldv, dv);
+    static const cudaError_t attr[3] = {
+        cudaFuncSetAttribute(ss_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SW_SMEM),
+        cudaFuncSetAttribute(ss_output_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SO_SMEM),
+        cudaFuncSetAttribute(ss_output_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SO_SMEM)};
+    for (const cudaError_t e : attr)
+        if (e != cudaSuccess) return (int)e;
+    const int n_chunks = (max_len + SC_CHUNK - 1) / SC_CHUNK;
+    mv_launch(ss_factors_kernel, dim3(n_chunks, (n_heads + 3) / 4, n_seqs), 128, 0, stream, a);
     int code = mv_launch_status();
     if (code) return code;
-    const int cols = dv + (normalizer ? 1 : 0);
-    const dim3 grid((cols + SC_COLS - 1) / SC_COLS, n_heads, n_seqs);
-    float* out = normalizer ? o_aug : o;
-    const int ones_col = normalizer ? dv : -1;
-    if (dk <= 128)
-        code = scalar_chunk_scan_launch<4>(grid, stream, q, ldq, k, ldk, v, ldv, log_a, ld_a, b, ld_b, skip, q_scale, G, state,
-                                           slots, cu, out, n_heads, heads_per_group, dk, dv, ones_col);
-    else
-        code = scalar_chunk_scan_launch<8>(grid, stream, q, ldq, k, ldk, v, ldv, log_a, ld_a, b, ld_b, skip, q_scale, G, state,
-                                           slots, cu, out, n_heads, heads_per_group, dk, dv, ones_col);
-    if (code || !normalizer) return code;
-    const long long total = (long long)N * n_heads * dv;
-    mv_launch(memory_normalize_kernel, (unsigned)((total + 255) / 256), 256, 0, stream, (const float*)o_aug, m_tok, o, total, dv);
+    mv_launch(ss_products_kernel, dim3(n_chunks, n_heads / heads_per_group, n_seqs), 64, 0, stream, a);
+    if ((code = mv_launch_status())) return code;
+    mv_launch(ss_walk_kernel, dim3((dv + 63) / 64 * ((dk + 63) / 64), n_heads, n_seqs), SC_WALK_THREADS, SW_SMEM, stream, a);
+    if ((code = mv_launch_status())) return code;
+    const dim3 grid(n_chunks * ((dv + 63) / 64), n_heads, n_seqs);
+    if (dk <= 128) mv_launch(ss_output_kernel<4>, grid, SO_THREADS, SO_SMEM, stream, a);
+    else mv_launch(ss_output_kernel<8>, grid, SO_THREADS, SO_SMEM, stream, a);
     return mv_launch_status();
 }

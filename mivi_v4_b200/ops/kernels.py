@@ -72,7 +72,7 @@ _SIGNATURES = {
         "mv_scalar_scan": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
                            _P],
         "mv_scalar_chunks": [_I, _I],
-        "mv_scalar_scan_chunked": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _I, _I,
+        "mv_scalar_scan_chunked": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I,
                                    _I, _I, _I, _I, _I, _P],
         "mv_decay_factor_floats": [_I],
         "mv_memory_gates": [_P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _I, _P],
@@ -89,6 +89,7 @@ _SIGNATURES = {
                               _P, _P, _P],
         "mv_head_product": [_P, _Q, _I, _P, _I, _I, _P, _Q, _I, _P, _I, _Q, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P, _P],
         "mv_latent_attention": [_P, _P, _Q, _I, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _P, _P, _P],
+        "mv_delta_prep_width": [_I, _I, _I],
         "mv_delta_scan_long": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _F, _F, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
         "mv_delta_scan": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _F, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
         "mv_expert_rank": [_P, _I, _I, _P, _P, _P],
@@ -327,7 +328,7 @@ def _need(t: Optional[torch.Tensor], name: str, dtype=None, shape=None, optional
 
 _launches = 0
 # kernels launched by one call of each entry point
-_KERNELS_PER_CALL = {"mv_shortconv": 2, "mv_decay_scan_chunked": 3, "mv_causal_conv": 2, "mv_scalar_scan_chunked": 2}
+_KERNELS_PER_CALL = {"mv_shortconv": 2, "mv_decay_scan_chunked": 3, "mv_causal_conv": 2, "mv_scalar_scan_chunked": 4}
 
 
 def launch_count() -> int:
@@ -666,17 +667,17 @@ def scalar_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_a: torch.
     if ws is not None and max_len >= SCAN_CHUNKED_FROM:
         chunks = int(_fn("core", "mv_scalar_chunks")(N, int(n_seqs)))
         G = ws.get("scalar_scan_products", (chunks, groups, SCAN_CHUNK, SCAN_CHUNK), torch.float32)
-        o_aug = ws.get("scalar_scan_o_aug", (N, n_heads * (dv + 1)), torch.float32) if norm else None
+        before = ws.get("scan_before", (chunks, n_heads, dv + (1 if norm else 0), (dk + 3) & ~3), torch.float32)
+        factors = ws.get("scan_factors", (chunks, n_heads, 3 * SCAN_CHUNK + 4), torch.float32)
         _check(_fn("core", "mv_scalar_scan_chunked")(
             qp, ldq, kp, ldk, vp, ldv, ap, lda, bp, ldb, _need(skip, "scalar_scan skip", torch.float32, (n_heads,), True),
             _need(m_tok, "scalar_scan m", torch.float32, (N, n_heads), True), float(q_scale), state.data_ptr(),
             _need(slots, "slots", torch.int32), _need(cu, "cu", torch.int32),
             _need(out, "scalar_scan out", torch.float32, (N, n_heads * dv)), G.data_ptr(),
-            o_aug.data_ptr() if norm else None, N, int(n_seqs), int(max_len), n_heads, int(heads_per_group), dk, dv,
+            before.data_ptr(), factors.data_ptr(), chunks, int(n_seqs), int(max_len), n_heads, int(heads_per_group), dk, dv,
             int(norm), _stream()), "mv_scalar_scan_chunked")
-        add_launches(1 if norm else 0)
         account(N * n_heads * (2 * dk // heads_per_group + 2 * dv) * 4 + 2 * n_seqs * n_heads * dk * dv * 4
-                + 2 * chunks * groups * SCAN_CHUNK * SCAN_CHUNK * 4,
+                + 2 * chunks * (groups * SCAN_CHUNK * SCAN_CHUNK + n_heads * dk * dv) * 4,
                 4 * N * n_heads * dk * dv + N * n_heads * SCAN_CHUNK * dv + N * groups * SCAN_CHUNK * dk)
         return out
     _check(_fn("core", "mv_scalar_scan")(
@@ -1561,7 +1562,7 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
     _guard("core", "delta_rule", out.device, n_slots=state.shape[0])
     if long_step:
         # a row: q and k of the q/k heads, the decays, beta, k . q; padded to 16 bytes (as the kernel lays it out)
-        width = (2 * kv_heads * dk + n_heads * dk + n_heads + kv_heads + 3) & ~3
+        width = int(_fn("core", "mv_delta_prep_width")(n_heads, kv_heads, dk))
         prep = ws.get("delta_scan.prep", (N, width), torch.float32)
         _check(_fn("core", "mv_delta_scan_long")(
             qp, ldq, kp, ldk, vp, ldv, bp, ldb, ap, lda, _need(dt_bias, "dt_bias", torch.float32, (n_decays,)),
