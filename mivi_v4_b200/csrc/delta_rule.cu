@@ -171,9 +171,30 @@ MV_API int mv_delta_scan(const float* q, int ldq, const float* k, int ldk, const
 // both; u = beta (v - a); o = b + u (k . q), which is (S' + k u^T)^T q; S = S' + k u^T.
 #define DL_CHUNK 16
 
-// Channel i of a head's W = 32 R in prep: lane i % 8 owns the channels i, i + 8, .., 4 R of them, and finds them side by side,
-// first those that are 32 apart.
-__device__ __forceinline__ int dl_place(int i, int R) { return R ? (i & 7) * (4 * R) + ((i >> 3) & 3) * R + (i >> 5) : i; }
+// Channel i of a head's W = 32 R in prep: lane i % 8 owns the channels i, i + 8, .., 4 R of them, and finds them side by side.
+__device__ __forceinline__ int dl_place(int i, int R) { return R ? (i & 7) * (4 * R) + (i >> 3) : i; }
+
+// two products or multiply-adds in one instruction, each rounded as the single one is
+__device__ __forceinline__ unsigned long long dl_pair(float x, float y) {
+    unsigned long long p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(x), "f"(y));
+    return p;
+}
+__device__ __forceinline__ float2 dl_split(unsigned long long p) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ unsigned long long dl_mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long dl_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
 
 __global__ void __launch_bounds__(256)
 delta_prepare_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
@@ -390,15 +411,12 @@ delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __r
     const int hk = h / (n_heads / kv_heads), qk = kv_heads * W;
     const int slot = mv_read_slot(slots[sq]);
     float* srow = state + (((size_t)slot * n_heads + h) * dv + (j < dv ? j : 0)) * dk;
-    // S[c][r]: channel l + 8 c + 32 r
-    float S[4][R];
+    // S[2 r + c / 2]: the channels l + 8 c + 32 r for c and c + 1
+    using pair = unsigned long long;
+    pair S[2 * R];
+    auto kept = [&](int i) { return (j < dv && i < dk) ? srow[i] : 0.f; };
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int i = l + 8 * c + 32 * r;
-            S[c][r] = (j < dv && i < dk) ? srow[i] : 0.f;
-        }
+    for (int e = 0; e < 2 * R; ++e) S[e] = dl_pair(kept(l + 16 * e), kept(l + 16 * e + 8));
     // 16 tokens' rows of q, k and g, DR_COLS columns of v, beta and k.q on their way into one buffer
     auto stage = [&](int c0, float* buf) {
         const int nt = min(DL_CHUNK, len - c0);
@@ -421,18 +439,7 @@ delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __r
             dl_copy4(vs + DL_CHUNK * DR_COLS + DL_CHUNK + tid, src + n_heads + hk);
         }
     };
-    auto read = [&](const float* from, float (&x)[4][R]) {
-        float flat[E];
-#pragma unroll
-        for (int e = 0; e < E; e += 4) {
-            const float4 y = *reinterpret_cast<const float4*>(from + e);
-            flat[e] = y.x; flat[e + 1] = y.y; flat[e + 2] = y.z; flat[e + 3] = y.w;
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int r = 0; r < R; ++r) x[c][r] = flat[c * R + r];
-    };
+    struct Token { pair q[2 * R], g[2 * R], k[2 * R]; float v, beta, kq; };
 
     stage(0, dl_smem);
     dl_commit();
@@ -455,59 +462,61 @@ delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __r
         const float* bs = vs + DL_CHUNK * DR_COLS;
         const float* ds = bs + DL_CHUNK;
         float* orow = o + (size_t)(row0 + c0) * n_heads * dv + (size_t)h * dv + j;
-        float q[4][R], g[4][R], k0[4][R], k1[4][R], vt = vs[jl], beta = bs[0], kq = ds[0];
-        read(qs, q);
-        read(gs, g);
-        read(ks, k0);
-        auto token = [&](int t, const float (&k)[4][R], float (&k_next)[4][R]) {
-            float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};
+        auto read = [&](int t, Token& x) {
 #pragma unroll
-            for (int r = 0; r < R; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    S[c][r] *= g[c][r];
-                    a[c] = fmaf(S[c][r], k[c][r], a[c]);
-                    b[c] = fmaf(S[c][r], q[c][r], b[c]);
-                }
-            const float v_now = vt, beta_now = beta, kq_now = kq;
-            if (t + 1 < nt) {
-                read(qs + (t + 1) * ROW, q);
-                read(gs + (t + 1) * ROW, g);
-                read(ks + (t + 1) * ROW, k_next);
-                vt = vs[(t + 1) * DR_COLS + jl];
-                beta = bs[t + 1];
-                kq = ds[t + 1];
+            for (int e = 0; e < R; ++e) {
+                const ulonglong2 q2 = *reinterpret_cast<const ulonglong2*>(qs + t * ROW + 4 * e);
+                const ulonglong2 g2 = *reinterpret_cast<const ulonglong2*>(gs + t * ROW + 4 * e);
+                const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(ks + t * ROW + 4 * e);
+                x.q[2 * e] = q2.x; x.q[2 * e + 1] = q2.y;
+                x.g[2 * e] = g2.x; x.g[2 * e + 1] = g2.y;
+                x.k[2 * e] = k2.x; x.k[2 * e + 1] = k2.y;
             }
-            float said = (a[0] + a[2]) + (a[1] + a[3]), out = (b[0] + b[2]) + (b[1] + b[3]);
+            x.v = vs[t * DR_COLS + jl];
+            x.beta = bs[t];
+            x.kq = ds[t];
+        };
+        Token x0, x1;
+        read(0, x0);
+        auto token = [&](int t, const Token& x, Token& next) {
+            // (requested first: behind the exchanges' own requests they would hold those up)
+            if (t + 1 < nt) read(t + 1, next);
+            pair a[2] = {0ull, 0ull}, b[2] = {0ull, 0ull};      // four chains: c = 0, 1 and 2, 3
+#pragma unroll
+            for (int e = 0; e < 2 * R; ++e) {
+                S[e] = dl_mul2(S[e], x.g[e]);
+                a[e & 1] = dl_fma2(S[e], x.k[e], a[e & 1]);
+                b[e & 1] = dl_fma2(S[e], x.q[e], b[e & 1]);
+            }
+            const float2 a01 = dl_split(a[0]), a23 = dl_split(a[1]), b01 = dl_split(b[0]), b23 = dl_split(b[1]);
+            float said = (a01.x + a23.x) + (a01.y + a23.y), out = (b01.x + b23.x) + (b01.y + b23.y);
 #pragma unroll
             for (int d = 4; d >= 1; d >>= 1) {
                 said += __shfl_xor_sync(0xffffffffu, said, d);
                 out += __shfl_xor_sync(0xffffffffu, out, d);
             }
-            const float u = beta_now * ((j < dv ? v_now : 0.f) - said);
+            const float u = x.beta * ((j < dv ? x.v : 0.f) - said);
+            const pair uu = dl_pair(u, u);
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-#pragma unroll
-                for (int r = 0; r < R; ++r) S[c][r] = fmaf(k[c][r], u, S[c][r]);
-            if (l == 0 && j < dv) orow[(size_t)t * n_heads * dv] = fmaf(u, kq_now, out);
+            for (int e = 0; e < 2 * R; ++e) S[e] = dl_fma2(x.k[e], uu, S[e]);
+            if (l == 0 && j < dv) orow[(size_t)t * n_heads * dv] = fmaf(u, x.kq, out);
         };
         int t = 0;
         for (; t + 1 < nt; t += 2) {
-            token(t, k0, k1);
-            token(t + 1, k1, k0);
+            token(t, x0, x1);
+            token(t + 1, x1, x0);
         }
-        if (t < nt) token(t, k0, k1);
+        if (t < nt) token(t, x0, x1);
         __syncthreads();
     }
     mv_pdl_launch_dependents();
     if (j < dv && mv_slot_ok(slots[sq])) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const int i = l + 8 * c + 32 * r;
-                if (i < dk) srow[i] = S[c][r];
-            }
+        for (int e = 0; e < 2 * R; ++e) {
+            const float2 y = dl_split(S[e]);
+            if (l + 16 * e < dk) srow[l + 16 * e] = y.x;
+            if (l + 16 * e + 8 < dk) srow[l + 16 * e + 8] = y.y;
+        }
     }
 }
 

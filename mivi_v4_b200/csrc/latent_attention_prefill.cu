@@ -31,7 +31,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
 }
 __device__ __forceinline__ void mma_bf16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
                                          unsigned b0, unsigned b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
                  "{%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -44,10 +44,6 @@ __device__ __forceinline__ void ldmatrix_x4(unsigned (&r)[4], const void* smem) 
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(s));
-}
-__device__ __forceinline__ void ldmatrix_x2(unsigned (&r)[4], const void* smem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(s));
 }
 __device__ __forceinline__ float ex2(float x) {
     float y;
@@ -203,22 +199,21 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
     const int w_last = min(pos0 + w0 + 16 * MT - 1, last_pos), w_first = window > 0 ? max(0, pos0 + w0 - window + 1) : 0;
     const bool live = w0 < nq;
 
-    const int kc = dim >> 3, rc = rot >> 3, all = kc + rc + (dv >> 3);
-    const int step_r = NWARPS * 32 / all, step_c = NWARPS * 32 % all, r_of = threadIdx.x / all, c_of = threadIdx.x % all;
+    // eight lanes a row, 16 rows a round: no lane takes another branch than its neighbours (dealt out chunk by chunk, a third of
+    // the kernel's instructions were these copies)
+    const int lr = threadIdx.x >> 3, lc = (threadIdx.x & 7) * 8;
+    const __nv_bfloat16 *kx_k = kx + (size_t)h * dim + lc, *kx_v = kx + v0 + (size_t)h * dv + lc, *rk_c = rk + lc;
+    __nv_bfloat16 *ks_at = ks + lr * ldk + lc, *vs_at = vs + lr * ldv + lc;
     auto load_block = [&](int kb, int buf) {
-        for (int r = r_of, c = c_of; r < KB;) {
-            const int t = min(max(kb * KB + r, lo), last_pos);           // rows outside repeat a row that is there
+#pragma unroll
+        for (int r = 0; r < KB; r += NWARPS * 4) {
+            const int t = min(max(kb * KB + r + lr, lo), last_pos);      // rows outside repeat a row that is there
             const size_t row = (size_t)(base + t - lo);
-            if (c < kc)
-                cp_async16(ks + ((size_t)buf * KB + r) * ldk + c * 8, kx + row * ld_kx + (size_t)h * dim + c * 8);
-            else if (c < kc + rc)
-                cp_async16(ks + ((size_t)buf * KB + r) * ldk + dim + (c - kc) * 8, rk + row * rot + (c - kc) * 8);
-            else
-                cp_async16(vs + ((size_t)buf * KB + r) * ldv + (c - kc - rc) * 8,
-                           kx + row * ld_kx + v0 + (size_t)h * dv + (c - kc - rc) * 8);
-            r += step_r;
-            c += step_c;
-            if (c >= all) { c -= all; ++r; }
+            const __nv_bfloat16 *kr = kx_k + row * ld_kx, *vr = kx_v + row * ld_kx, *rr = rk_c + row * rot;
+            __nv_bfloat16 *kd = ks_at + (buf * KB + r) * ldk, *vd = vs_at + (buf * KB + r) * ldv;
+            for (int c = 0; c + lc < dim; c += 64) cp_async16(kd + c, kr + c);
+            for (int c = 0; c + lc < rot; c += 64) cp_async16(kd + dim + c, rr + c);
+            for (int c = 0; c + lc < dv; c += 64) cp_async16(vd + c, vr + c);
         }
     };
 
@@ -242,26 +237,23 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
         float s[MT][KB / 8][4];
         const int mi = lane >> 3, r8 = lane & 7;
 #pragma unroll
-        for (int j = 0; j < KB / 8; ++j) {
+        for (int j = 0; j < KB / 8; ++j)
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) s[mt][j][e] = 0.f;
-            const __nv_bfloat16* krow = kt + (size_t)(j * 8 + r8) * ldk + mi * 8;
+        // channels outside, keys inside: 8 MT sums take turns, no product waits for the one before it
 #pragma unroll
-            for (int kk = 0; kk < DKM / 16; kk += 2) {
-                if (kk * 16 < dk) {
-                    unsigned kf[4];
-                    const bool two = kk * 16 + 16 < dk;
-                    if (two) ldmatrix_x4(kf, krow + kk * 16);
-                    else ldmatrix_x2(kf, krow + kk * 16 - (mi >> 1) * 16);
+        for (int kk = 0; kk < DKM / 16; ++kk) {
+            if (kk * 16 < dk) {
 #pragma unroll
-                    for (int mt = 0; mt < MT; ++mt) mma_bf16(s[mt][j], qf[mt][kk][0], qf[mt][kk][1], qf[mt][kk][2], qf[mt][kk][3], kf[0], kf[1]);
-                    if (two && kk + 1 < DKM / 16) {
-                        const int k1 = kk + 1 < DKM / 16 ? kk + 1 : kk;
+                for (int j = 0; j < KB / 8; j += 2) {
+                    unsigned kf[4];                                      // 16 keys x 16 elements
+                    ldmatrix_x4(kf, kt + (size_t)(j * 8 + (mi >> 1) * 8 + r8) * ldk + kk * 16 + (mi & 1) * 8);
 #pragma unroll
-                        for (int mt = 0; mt < MT; ++mt)
-                            mma_bf16(s[mt][j], qf[mt][k1][0], qf[mt][k1][1], qf[mt][k1][2], qf[mt][k1][3], kf[2], kf[3]);
+                    for (int mt = 0; mt < MT; ++mt) {
+                        mma_bf16(s[mt][j], qf[mt][kk][0], qf[mt][kk][1], qf[mt][kk][2], qf[mt][kk][3], kf[0], kf[1]);
+                        mma_bf16(s[mt][j + 1], qf[mt][kk][0], qf[mt][kk][1], qf[mt][kk][2], qf[mt][kk][3], kf[2], kf[3]);
                     }
                 }
             }
