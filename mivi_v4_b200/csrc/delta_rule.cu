@@ -171,30 +171,10 @@ MV_API int mv_delta_scan(const float* q, int ldq, const float* k, int ldk, const
 // both; u = beta (v - a); o = b + u (k . q), which is (S' + k u^T)^T q; S = S' + k u^T.
 #define DL_CHUNK 16
 
-// Channel i of a head's W = 32 R in prep: lane i % 8 owns the channels i, i + 8, .., 4 R of them, and finds them side by side.
-__device__ __forceinline__ int dl_place(int i, int R) { return R ? (i & 7) * (4 * R) + (i >> 3) : i; }
-
-// two products or multiply-adds in one instruction, each rounded as the single one is
-__device__ __forceinline__ unsigned long long dl_pair(float x, float y) {
-    unsigned long long p;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(x), "f"(y));
-    return p;
-}
-__device__ __forceinline__ float2 dl_split(unsigned long long p) {
-    float2 v;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ unsigned long long dl_mul2(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned long long dl_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
+// A column of the state is shared by DW_LANES lanes.  Channel i of a head's W = 32 R in prep: lane i % DW_LANES owns the channels
+// i, i + DW_LANES, .. and finds them side by side.
+constexpr int DW_LANES = 16, DW_C = 32 / DW_LANES;
+__device__ __forceinline__ int dl_place(int i, int R) { return R ? i % DW_LANES * (DW_C * R) + i / DW_LANES : i; }
 
 __global__ void __launch_bounds__(256)
 delta_prepare_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
@@ -392,31 +372,35 @@ delta_scan_long_kernel(const float* __restrict__ prep, int ldp, const float* __r
 // three exchanges remain, after which all eight lanes have the sum and no broadcast follows; the next token's rows are
 // requested from shared memory before the exchanges.  (With a whole warp on two columns the chain had six exchanges and 690 us for
 // 2,048 tokens of 16 heads of 128 x 128; the order in which a sum's parts are added is the same, and so is every bit.)  @MEASURED@
-constexpr int DW_THREADS = DR_COLS * 8;
+constexpr int DW_THREADS = DR_COLS * DW_LANES;
+// floats a lane has in a row of shared memory: its channels, and 16 bytes more where neighbours would share banks
+__host__ __device__ constexpr int dw_lane(int R) { return DW_C * R + (DW_C * R % 8 ? 0 : 4); }
 
 template <int R>
 __global__ void __launch_bounds__(DW_THREADS)
 delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __restrict__ v, int ldv,
                        float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ cu,
                        float* __restrict__ o, int n_heads, int kv_heads, int dk, int dv) {
-    constexpr int E = 4 * R, W = 32 * R, LANE = E + 4, ROW = 8 * LANE;      // a lane's channels, 16 bytes of padding between lanes
+    constexpr int C = DW_C, E = C * R, W = 32 * R, LANE = dw_lane(R), ROW = DW_LANES * LANE;
     constexpr int BUF = DL_CHUNK * (3 * ROW + DR_COLS + 2);
     mv_pdl_wait();                          // the successor is let go when the last token is done
     extern __shared__ __align__(16) float dl_smem[];
     const int tile = blockIdx.x, h = blockIdx.y, sq = blockIdx.z;
-    const int tid = threadIdx.x, l = tid & 7, jl = tid >> 3;
+    const int tid = threadIdx.x, l = tid % DW_LANES, jl = tid / DW_LANES;
     const int col0 = tile * DR_COLS, j = col0 + jl;
     const int row0 = cu[sq], len = cu[sq + 1] - row0;
     if (len <= 0) return;
     const int hk = h / (n_heads / kv_heads), qk = kv_heads * W;
     const int slot = mv_read_slot(slots[sq]);
     float* srow = state + (((size_t)slot * n_heads + h) * dv + (j < dv ? j : 0)) * dk;
-    // S[2 r + c / 2]: the channels l + 8 c + 32 r for c and c + 1
-    using pair = unsigned long long;
-    pair S[2 * R];
-    auto kept = [&](int i) { return (j < dv && i < dk) ? srow[i] : 0.f; };
+    float S[R][C];                          // channel l + DW_LANES c + 32 r
 #pragma unroll
-    for (int e = 0; e < 2 * R; ++e) S[e] = dl_pair(kept(l + 16 * e), kept(l + 16 * e + 8));
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const int i = l + DW_LANES * c + 32 * r;
+            S[r][c] = (j < dv && i < dk) ? srow[i] : 0.f;
+        }
     // 16 tokens' rows of q, k and g, DR_COLS columns of v, beta and k.q on their way into one buffer
     auto stage = [&](int c0, float* buf) {
         const int nt = min(DL_CHUNK, len - c0);
@@ -439,7 +423,19 @@ delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __r
             dl_copy4(vs + DL_CHUNK * DR_COLS + DL_CHUNK + tid, src + n_heads + hk);
         }
     };
-    struct Token { pair q[2 * R], g[2 * R], k[2 * R]; float v, beta, kq; };
+    struct Token { float q[R][C], g[R][C], k[R][C], v, beta, kq; };
+    auto read = [&](const float* from, float (&x)[R][C]) {
+        float flat[E];
+#pragma unroll
+        for (int e = 0; e < E; e += 4) {
+            const float4 y = *reinterpret_cast<const float4*>(from + e);
+            flat[e] = y.x; flat[e + 1] = y.y; flat[e + 2] = y.z; flat[e + 3] = y.w;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int c = 0; c < C; ++c) x[r][c] = flat[r * C + c];
+    };
 
     stage(0, dl_smem);
     dl_commit();
@@ -462,43 +458,43 @@ delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __r
         const float* bs = vs + DL_CHUNK * DR_COLS;
         const float* ds = bs + DL_CHUNK;
         float* orow = o + (size_t)(row0 + c0) * n_heads * dv + (size_t)h * dv + j;
-        auto read = [&](int t, Token& x) {
-#pragma unroll
-            for (int e = 0; e < R; ++e) {
-                const ulonglong2 q2 = *reinterpret_cast<const ulonglong2*>(qs + t * ROW + 4 * e);
-                const ulonglong2 g2 = *reinterpret_cast<const ulonglong2*>(gs + t * ROW + 4 * e);
-                const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(ks + t * ROW + 4 * e);
-                x.q[2 * e] = q2.x; x.q[2 * e + 1] = q2.y;
-                x.g[2 * e] = g2.x; x.g[2 * e + 1] = g2.y;
-                x.k[2 * e] = k2.x; x.k[2 * e + 1] = k2.y;
-            }
+        auto fetch = [&](int t, Token& x) {
+            read(gs + t * ROW, x.g);
+            read(ks + t * ROW, x.k);
+            read(qs + t * ROW, x.q);
             x.v = vs[t * DR_COLS + jl];
             x.beta = bs[t];
             x.kq = ds[t];
         };
         Token x0, x1;
-        read(0, x0);
+        fetch(0, x0);
         auto token = [&](int t, const Token& x, Token& next) {
             // (requested first: behind the exchanges' own requests they would hold those up)
-            if (t + 1 < nt) read(t + 1, next);
-            pair a[2] = {0ull, 0ull}, b[2] = {0ull, 0ull};      // four chains: c = 0, 1 and 2, 3
+            if (t + 1 < nt) fetch(t + 1, next);
+            float a[C], b[C];
 #pragma unroll
-            for (int e = 0; e < 2 * R; ++e) {
-                S[e] = dl_mul2(S[e], x.g[e]);
-                a[e & 1] = dl_fma2(S[e], x.k[e], a[e & 1]);
-                b[e & 1] = dl_fma2(S[e], x.q[e], b[e & 1]);
-            }
-            const float2 a01 = dl_split(a[0]), a23 = dl_split(a[1]), b01 = dl_split(b[0]), b23 = dl_split(b[1]);
-            float said = (a01.x + a23.x) + (a01.y + a23.y), out = (b01.x + b23.x) + (b01.y + b23.y);
+            for (int c = 0; c < C; ++c) a[c] = b[c] = 0.f;
 #pragma unroll
-            for (int d = 4; d >= 1; d >>= 1) {
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    S[r][c] *= x.g[r][c];
+                    a[c] = fmaf(S[r][c], x.k[r][c], a[c]);
+                    b[c] = fmaf(S[r][c], x.q[r][c], b[c]);
+                }
+            // the chains 16 apart first, then 8 apart: the order of an exchange over 32 lanes
+            float said = C == 4 ? (a[0] + a[C / 2]) + (a[1] + a[C - 1]) : a[0] + a[1];
+            float out = C == 4 ? (b[0] + b[C / 2]) + (b[1] + b[C - 1]) : b[0] + b[1];
+#pragma unroll
+            for (int d = DW_LANES / 2; d >= 1; d >>= 1) {
                 said += __shfl_xor_sync(0xffffffffu, said, d);
                 out += __shfl_xor_sync(0xffffffffu, out, d);
             }
             const float u = x.beta * ((j < dv ? x.v : 0.f) - said);
-            const pair uu = dl_pair(u, u);
 #pragma unroll
-            for (int e = 0; e < 2 * R; ++e) S[e] = dl_fma2(x.k[e], uu, S[e]);
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int c = 0; c < C; ++c) S[r][c] = fmaf(x.k[r][c], u, S[r][c]);
             if (l == 0 && j < dv) orow[(size_t)t * n_heads * dv] = fmaf(u, x.kq, out);
         };
         int t = 0;
@@ -512,11 +508,12 @@ delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __r
     mv_pdl_launch_dependents();
     if (j < dv && mv_slot_ok(slots[sq])) {
 #pragma unroll
-        for (int e = 0; e < 2 * R; ++e) {
-            const float2 y = dl_split(S[e]);
-            if (l + 16 * e < dk) srow[l + 16 * e] = y.x;
-            if (l + 16 * e + 8 < dk) srow[l + 16 * e + 8] = y.y;
-        }
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const int i = l + DW_LANES * c + 32 * r;
+                if (i < dk) srow[i] = S[r][c];
+            }
     }
 }
 
@@ -543,7 +540,7 @@ MV_API int mv_delta_scan_long(const float* q, int ldq, const float* k, int ldk, 
     // long as when they are dealt out over an idle device (measured: 1.26 ms against 0.72 for 2,048 tokens).
     const dim3 grid((dv + DR_COLS - 1) / DR_COLS, n_heads, n_seqs);
     if (R && ((uintptr_t)prep & 15)) return (int)cudaErrorInvalidValue;
-    const size_t smem = 2 * (size_t)DL_CHUNK * (3 * (R ? 8 * (4 * R + 4) : dk) + DR_COLS + 2) * sizeof(float);
+    const size_t smem = 2 * (size_t)DL_CHUNK * (3 * (R ? DW_LANES * dw_lane(R) : dk) + DR_COLS + 2) * sizeof(float);
     // 16-byte copies: every row of q, k and g of a head starts on 16 bytes (ldp is a multiple of 4 floats)
     const int wide = dk % 4 == 0 && (((uintptr_t)prep) & 15) == 0;
 #define DL_LAUNCH(R, PART)                                                                                                   \
