@@ -36,7 +36,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
 }
 __device__ __forceinline__ void mma_bf16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
                                          unsigned b0, unsigned b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
                  "{%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -208,25 +208,52 @@ attention_sink_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bf
         // the smallest distance between this warp's queries and the block's keys: from the table's last column on it is one number
         const bool near = dist != nullptr && pos0 + warp * 16 - (key0 + KB - 1) < dist_len - 1;
         const float add = dist != nullptr && !near ? beyond : 0.f;
-        const bool need_mask = r1 != nullptr || near || it < n_kept || key0 + KB - 1 > pos0 + warp * 16 ||
+        const bool need_mask = it < n_kept || key0 + KB - 1 > pos0 + warp * 16 ||
                                (chunk > 0 ? key0 < cs1 : (window > 0 && key0 <= pos0 + warp * 16 + 15 - window));
         float mx0 = -INFINITY, mx1 = -INFINITY;
+        // (scale and cap, then the mask, each behind one branch a tile: inside the loop they were one a score)
+        if (cap > 0.f) {
+#pragma unroll
+            for (int j = 0; j < KB / 8; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[j][e] = fmaf(-2.0f * cap_l, rcp(1.0f + ex2(s[j][e] * scale_l)), cap_l + add);
+        } else {
+#pragma unroll
+            for (int j = 0; j < KB / 8; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[j][e] = fmaf(s[j][e], scale_l, add);
+        }
+        if (near) {
+#pragma unroll
+            for (int j = 0; j < KB / 8; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int n = ((e < 2) ? p0 : p1) - (key0 + j * 8 + 2 * t4 + (e & 1));
+                    if (n >= 0) s[j][e] = fmaf(by_dist[min(n, dist_len - 1)], dist_unit, s[j][e]);
+                }
+        } else if (r1) {
+#pragma unroll
+            for (int j = 0; j < KB / 8; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int n = ((e < 2) ? p0 : p1) - (key0 + j * 8 + 2 * t4 + (e & 1));
+                    s[j][e] -= db1 * __logf(1.0f + db2 * (float)n);         // (a later key's is struck out below)
+                }
+        }
+        if (need_mask) {
+            // seen: t <= p, and either from `from` on or before `keep`
+            const int from0 = chunk > 0 ? cs0 : window > 0 ? p0 - window + 1 : 0, from1 = chunk > 0 ? cs1 : window > 0 ? p1 - window + 1 : 0;
+            const int keep = chunk == 0 && window > 0 ? keep_first : 0;
+#pragma unroll
+            for (int j = 0; j < KB / 8; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int t = key0 + j * 8 + 2 * t4 + (e & 1);
+                    if (t > ((e < 2) ? p0 : p1) || (t < ((e < 2) ? from0 : from1) && t >= keep)) s[j][e] = -INFINITY;
+                }
+        }
 #pragma unroll
         for (int j = 0; j < KB / 8; ++j) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                float sc = cap > 0.f ? fmaf(-2.0f * cap_l, rcp(1.0f + ex2(s[j][e] * scale_l)), cap_l + add)
-                                     : fmaf(s[j][e], scale_l, add);
-                if (need_mask) {
-                    const int t = key0 + j * 8 + 2 * t4 + (e & 1);
-                    const int p = (e < 2) ? p0 : p1;
-                    if (t > p || (chunk > 0 ? t < ((e < 2) ? cs0 : cs1)
-                                            : (window > 0 && t <= p - window && t >= keep_first))) sc = -INFINITY;
-                    else if (r1) sc -= db1 * __logf(1.0f + db2 * (float)(p - t));
-                    else if (near) sc = fmaf(by_dist[min(p - t, dist_len - 1)], dist_unit, sc);
-                }
-                s[j][e] = sc;
-            }
             mx0 = fmaxf(mx0, fmaxf(s[j][0], s[j][1]));
             mx1 = fmaxf(mx1, fmaxf(s[j][2], s[j][3]));
         }

@@ -163,18 +163,17 @@ MV_API int mv_delta_scan(const float* q, int ldq, const float* k, int ldk, const
 // Two kernels.  delta_prepare does, once per token, what does not depend on the state: q and k as unit vectors
 // (q also times q_scale), k . q of each q/k head, the decays g, and beta; one row of `prep` a token:
 //     [q: kv_heads W | k: kv_heads W | g: heads W | beta: heads | k.q: kv_heads]      (row stride ldp, 32-bit)
-// W is dk, or from 64 key channels on dk rounded up to 64, 128 or 256 (zeros beyond dk), a head's channels then in the order in
-// which delta_scan_wide_kernel's lanes own them.
+// W is dk, or from 64 key channels on what delta_scan_wide_kernel reads: dk rounded up to 32 R = 64, 128 or 256 (zeros beyond dk)
+// in the order in which its lanes own them.
 // delta_scan_long then walks a sequence with nothing but the recurrence in its loop.  The tokens come through
 // shared memory sixteen at a time, the next sixteen on their way (cp.async) while these are worked on.  In the
 // loop  S' = diag(g) S  is read twice at once, a = S'^T k and b = S'^T q, so that one round of shuffles serves
 // both; u = beta (v - a); o = b + u (k . q), which is (S' + k u^T)^T q; S = S' + k u^T.
 #define DL_CHUNK 16
 
-// A column of the state is shared by DW_LANES lanes.  Channel i of a head's W = 32 R in prep: lane i % DW_LANES owns the channels
-// i, i + DW_LANES, .. and finds them side by side.
-constexpr int DW_LANES = 16, DW_C = 32 / DW_LANES;
-__device__ __forceinline__ int dl_place(int i, int R) { return R ? i % DW_LANES * (DW_C * R) + i / DW_LANES : i; }
+// Where channel i of a head's 32 R lies in its W = 8 (4 R + 4) floats of prep: lane i % 8 owns the channels i, i + 8, .. and finds
+// them side by side, 16 bytes of padding behind them keep the lanes' reads from shared memory in different banks.
+__device__ __forceinline__ int dl_place(int i, int R) { return R ? (i & 7) * (4 * R + 4) + (i >> 3) : i; }
 
 __global__ void __launch_bounds__(256)
 delta_prepare_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
@@ -200,15 +199,16 @@ delta_prepare_kernel(const float* __restrict__ q, int ldq, const float* __restri
         sk = mv_warp_sum(sk);
         dot = mv_warp_sum(dot);
         const float fq = q_scale / sqrtf(sq + norm_eps), fk = 1.0f / sqrtf(sk + norm_eps);
-        for (int i = lane; i < W; i += 32) {
+        for (int i = lane; i < (R ? 32 * R : dk); i += 32) {
             const int at = h * W + dl_place(i, R);
             row[at] = i < dk ? qh[i] * fq : 0.f;
             row[qk + at] = i < dk ? kh[i] * fk : 0.f;
         }
         if (lane == 0) row[2 * qk + hk + n_heads + h] = dot * fq * fk;
     }
-    for (int e = threadIdx.x; e < hk; e += blockDim.x) {
-        const int h = e / W, i = e - h * W;
+    const int n_ch = R ? 32 * R : dk;
+    for (int e = threadIdx.x; e < n_heads * n_ch; e += blockDim.x) {
+        const int h = e / n_ch, i = e - h * n_ch;
         const int ai = head_decay ? h : h * dk + i;
         row[2 * qk + h * W + dl_place(i, R)] =
             i < dk ? expf(-expf(a_log[h]) * dr_softplus(a[(size_t)n * lda + ai] + dt_bias[ai])) : 0.f;
@@ -366,137 +366,165 @@ delta_scan_long_kernel(const float* __restrict__ prep, int ldp, const float* __r
     }
 }
 
-// From 64 key channels on: 8 lanes share a column of the state, lane l the channels l, l + 8, l + 16, .. (4 R of dk <= 32 R), four
-// columns a warp, 16 a block.  What bounds it is the chain from one token to the next: decay, dot product with k, its sum
-// over the lanes, u, the state's update.  A lane adds its channels in four chains (those 32 apart) and joins them two and two, so that
-// three exchanges remain, after which all eight lanes have the sum and no broadcast follows; the next token's rows are
-// requested from shared memory before the exchanges.  (With a whole warp on two columns the chain had six exchanges and 690 us for
-// 2,048 tokens of 16 heads of 128 x 128; the order in which a sum's parts are added is the same, and so is every bit.)  @MEASURED@
-constexpr int DW_THREADS = DR_COLS * DW_LANES;
-// floats a lane has in a row of shared memory: its channels, and 16 bytes more where neighbours would share banks
-__host__ __device__ constexpr int dw_lane(int R) { return DW_C * R + (DW_C * R % 8 ? 0 : 4); }
+// From 64 key channels on: four warps carry 16 columns of the state, 8 lanes a column, lane l the channels l, l + 8, .. (4 R of
+// dk <= 32 R).  What bounds it is the chain from one token to the next - decay, dot product with k, its sum over the lanes,
+// u, the state's update - and what the warps issue beside it.  So a lane adds its channels in four chains (those 32 apart) and
+// joins them two and two, which leaves three exchanges, after which all eight lanes have the sum; the next token's rows are
+// requested between the exchanges; a fifth warp does all copying; and the lanes only leave their parts of q's read-out (and
+// u) behind, which a sixth warp adds up and writes out a chunk later.  (Two columns a warp of 32 lanes: six exchanges in the chain,
+// 690 us for 2,048 tokens of 16 heads of 128 x 128; without the two further warps 540.  The order in which a sum's parts are
+// added is the same in all of them, and so is every bit.)  2,048 tokens of 16 heads of
+// 128 x 128: 690 -> 395 us (four sequences of 130 to 1,500 tokens, 8 heads: 572 -> 345).
+constexpr int DW_THREADS = DR_COLS * 8, DW_ALL = DW_THREADS + 64;
+constexpr size_t dw_smem(int R) {
+    return sizeof(float) * 2 * (DL_CHUNK * (3 * 8 * (4 * R + 4) + DR_COLS + 1 + 3) + DL_CHUNK * (DW_THREADS + DR_COLS));
+}
 
 template <int R>
-__global__ void __launch_bounds__(DW_THREADS)
+__global__ void __launch_bounds__(DW_ALL)
 delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __restrict__ v, int ldv,
                        float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ cu,
                        float* __restrict__ o, int n_heads, int kv_heads, int dk, int dv) {
-    constexpr int C = DW_C, E = C * R, W = 32 * R, LANE = dw_lane(R), ROW = DW_LANES * LANE;
-    constexpr int BUF = DL_CHUNK * (3 * ROW + DR_COLS + 2);
+    constexpr int E = 4 * R, LANE = E + 4, ROW = 8 * LANE;
+    constexpr int BUF = DL_CHUNK * (3 * ROW + DR_COLS + 4), PART = DL_CHUNK * DW_THREADS;
     mv_pdl_wait();                          // the successor is let go when the last token is done
-    extern __shared__ __align__(16) float dl_smem[];
+    extern __shared__ __align__(16) float dl_smem[];    // 2 x [q | k | g: 16 x ROW; v: 16 x 16; beta: 16 (64)], 2 x parts, 2 x u
+    float* parts = dl_smem + 2 * BUF;       // [16 tokens][16 columns][8 lanes]
+    float* us = parts + 2 * PART;           // [16 tokens][16 columns]
     const int tile = blockIdx.x, h = blockIdx.y, sq = blockIdx.z;
-    const int tid = threadIdx.x, l = tid % DW_LANES, jl = tid / DW_LANES;
-    const int col0 = tile * DR_COLS, j = col0 + jl;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int col0 = tile * DR_COLS;
     const int row0 = cu[sq], len = cu[sq + 1] - row0;
     if (len <= 0) return;
-    const int hk = h / (n_heads / kv_heads), qk = kv_heads * W;
+    const int hk = h / (n_heads / kv_heads), qk = kv_heads * ROW, hw = n_heads * ROW;
+    const int n_chunks = (len + DL_CHUNK - 1) / DL_CHUNK;
+
+    if (warp == DW_THREADS / 32) {          // copies: the rows of q, k and g, DR_COLS columns of v, and beta of 16 tokens
+        const float* qp = prep + (size_t)row0 * ldp + (size_t)hk * ROW + lane * 4;
+        const size_t to_g = 2 * (size_t)qk + (size_t)(h - hk) * ROW;
+        auto load = [&](int c) {
+            const int nt = min(DL_CHUNK, len - c * DL_CHUNK);
+            float* buf = dl_smem + (c & 1) * BUF;
+            for (int t = 0; t < nt; ++t) {
+                const float* src = qp + (size_t)(c * DL_CHUNK + t) * ldp;
+                float* to = buf + t * ROW + lane * 4;
+#pragma unroll
+                for (int i = 0; i < ROW; i += 128)
+                    if (i + 128 <= ROW || i + lane * 4 < ROW) {
+                        dl_copy16(to + i, src + i);
+                        dl_copy16(to + DL_CHUNK * ROW + i, src + qk + i);
+                        dl_copy16(to + 2 * DL_CHUNK * ROW + i, src + to_g + i);
+                    }
+            }
+            float* vs = buf + 3 * DL_CHUNK * ROW;
+            for (int idx = lane; idx < nt * DR_COLS; idx += 32) {
+                const int t = idx / DR_COLS, x = idx % DR_COLS;
+                if (col0 + x < dv) dl_copy4(vs + idx, v + (size_t)(row0 + c * DL_CHUNK + t) * ldv + (size_t)h * dv + col0 + x);
+            }
+            if (lane < nt) dl_copy4(vs + DL_CHUNK * DR_COLS + lane, prep + (size_t)(row0 + c * DL_CHUNK + lane) * ldp + 2 * qk + hw + h);
+            dl_commit();
+        };
+        load(0);
+        dl_wait<0>();
+        __syncthreads();
+        for (int c = 0; c < n_chunks; ++c) {
+            if (c + 1 < n_chunks) load(c + 1);
+            dl_wait<0>();
+            __syncthreads();
+        }
+        return;
+    }
+    if (warp > DW_THREADS / 32) {           // outputs of the chunk before
+        auto write = [&](int c) {
+            const int nt = min(DL_CHUNK, len - c * DL_CHUNK);
+            const float *p = parts + (c & 1) * PART, *u = us + (c & 1) * DL_CHUNK * DR_COLS;
+#pragma unroll 4
+            for (int e = 0; e < DL_CHUNK * DR_COLS / 32; ++e) {
+                const int idx = lane + 32 * e, t = idx / DR_COLS, x = idx % DR_COLS;
+                if (t >= nt || col0 + x >= dv) continue;
+                const size_t row = (size_t)(row0 + c * DL_CHUNK + t);
+                const float kq = prep[row * ldp + 2 * qk + hw + n_heads + hk];
+                const float4 y = *reinterpret_cast<const float4*>(p + idx * 8), z = *reinterpret_cast<const float4*>(p + idx * 8 + 4);
+                const float out = ((y.x + z.x) + (y.z + z.z)) + ((y.y + z.y) + (y.w + z.w));     // as exchanges 4, 2 and 1 lanes apart
+                o[row * n_heads * dv + (size_t)h * dv + col0 + x] = fmaf(u[idx], kq, out);
+            }
+        };
+        __syncthreads();
+        for (int c = 0; c < n_chunks; ++c) {
+            if (c > 0) write(c - 1);
+            __syncthreads();
+        }
+        write(n_chunks - 1);
+        return;
+    }
+
+    const int l = tid & 7, jl = tid >> 3, j = col0 + jl;
     const int slot = mv_read_slot(slots[sq]);
     float* srow = state + (((size_t)slot * n_heads + h) * dv + (j < dv ? j : 0)) * dk;
-    float S[R][C];                          // channel l + DW_LANES c + 32 r
+    float S[R][4];                          // channel l + 8 c + 32 r
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int c = 0; c < C; ++c) {
-            const int i = l + DW_LANES * c + 32 * r;
+        for (int c = 0; c < 4; ++c) {
+            const int i = l + 8 * c + 32 * r;
             S[r][c] = (j < dv && i < dk) ? srow[i] : 0.f;
         }
-    // 16 tokens' rows of q, k and g, DR_COLS columns of v, beta and k.q on their way into one buffer
-    auto stage = [&](int c0, float* buf) {
-        const int nt = min(DL_CHUNK, len - c0);
-        for (int idx = tid; idx < nt * (W / 4); idx += DW_THREADS) {
-            const int t = idx / (W / 4), i = (idx % (W / 4)) * 4;
-            const float* src = prep + (size_t)(row0 + c0 + t) * ldp;
-            float* to = buf + t * ROW + i / E * LANE + i % E;
-            dl_copy16(to, src + (size_t)hk * W + i);
-            dl_copy16(to + DL_CHUNK * ROW, src + qk + (size_t)hk * W + i);
-            dl_copy16(to + 2 * DL_CHUNK * ROW, src + 2 * qk + (size_t)h * W + i);
-        }
-        float* vs = buf + 3 * DL_CHUNK * ROW;
-        for (int idx = tid; idx < nt * DR_COLS; idx += DW_THREADS) {
-            const int t = idx / DR_COLS, c = idx - t * DR_COLS;
-            if (col0 + c < dv) dl_copy4(vs + idx, v + (size_t)(row0 + c0 + t) * ldv + (size_t)h * dv + col0 + c);
-        }
-        if (tid < nt) {
-            const float* src = prep + (size_t)(row0 + c0 + tid) * ldp + 2 * qk + (size_t)n_heads * W;
-            dl_copy4(vs + DL_CHUNK * DR_COLS + tid, src + h);
-            dl_copy4(vs + DL_CHUNK * DR_COLS + DL_CHUNK + tid, src + n_heads + hk);
+    struct Token { float q[R][4], g[R][4], k[R][4], v, beta; };
+    auto read = [&](const float* from, float (&x)[R][4]) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float4 y = *reinterpret_cast<const float4*>(from + 4 * r);
+            x[r][0] = y.x; x[r][1] = y.y; x[r][2] = y.z; x[r][3] = y.w;
         }
     };
-    struct Token { float q[R][C], g[R][C], k[R][C], v, beta, kq; };
-    auto read = [&](const float* from, float (&x)[R][C]) {
-        float flat[E];
-#pragma unroll
-        for (int e = 0; e < E; e += 4) {
-            const float4 y = *reinterpret_cast<const float4*>(from + e);
-            flat[e] = y.x; flat[e + 1] = y.y; flat[e + 2] = y.z; flat[e + 3] = y.w;
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int c = 0; c < C; ++c) x[r][c] = flat[r * C + c];
-    };
-
-    stage(0, dl_smem);
-    dl_commit();
-    int which = 0;
-    for (int c0 = 0; c0 < len; c0 += DL_CHUNK, which ^= 1) {
-        float* buf = dl_smem + which * BUF;
-        if (c0 + DL_CHUNK < len) {
-            stage(c0 + DL_CHUNK, dl_smem + (which ^ 1) * BUF);
-            dl_commit();
-            dl_wait<1>();
-        } else {
-            dl_wait<0>();
-        }
-        __syncthreads();
-        const int nt = min(DL_CHUNK, len - c0);
+    __syncthreads();
+    for (int chunk = 0; chunk < n_chunks; ++chunk) {
+        const int nt = min(DL_CHUNK, len - chunk * DL_CHUNK);
+        const float* buf = dl_smem + (chunk & 1) * BUF;
         const float* qs = buf + l * LANE;
         const float* ks = qs + DL_CHUNK * ROW;
         const float* gs = ks + DL_CHUNK * ROW;
-        const float* vs = buf + 3 * DL_CHUNK * ROW;
-        const float* bs = vs + DL_CHUNK * DR_COLS;
-        const float* ds = bs + DL_CHUNK;
-        float* orow = o + (size_t)(row0 + c0) * n_heads * dv + (size_t)h * dv + j;
-        auto fetch = [&](int t, Token& x) {
-            read(gs + t * ROW, x.g);
-            read(ks + t * ROW, x.k);
-            read(qs + t * ROW, x.q);
-            x.v = vs[t * DR_COLS + jl];
-            x.beta = bs[t];
-            x.kq = ds[t];
-        };
-        Token x0, x1;
-        fetch(0, x0);
+        const float* vs = buf + 3 * DL_CHUNK * ROW + jl;
+        const float* bs = buf + 3 * DL_CHUNK * ROW + DL_CHUNK * DR_COLS;
+        float* p = parts + (chunk & 1) * PART + tid;
+        float* up = us + (chunk & 1) * DL_CHUNK * DR_COLS + jl;
         auto token = [&](int t, const Token& x, Token& next) {
-            // (requested first: behind the exchanges' own requests they would hold those up)
-            if (t + 1 < nt) fetch(t + 1, next);
-            float a[C], b[C];
-#pragma unroll
-            for (int c = 0; c < C; ++c) a[c] = b[c] = 0.f;
+            float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int r = 0; r < R; ++r)
 #pragma unroll
-                for (int c = 0; c < C; ++c) {
+                for (int c = 0; c < 4; ++c) {
                     S[r][c] *= x.g[r][c];
                     a[c] = fmaf(S[r][c], x.k[r][c], a[c]);
-                    b[c] = fmaf(S[r][c], x.q[r][c], b[c]);
                 }
-            // the chains 16 apart first, then 8 apart: the order of an exchange over 32 lanes
-            float said = C == 4 ? (a[0] + a[C / 2]) + (a[1] + a[C - 1]) : a[0] + a[1];
-            float out = C == 4 ? (b[0] + b[C / 2]) + (b[1] + b[C - 1]) : b[0] + b[1];
+            const int n = t + 1 < nt ? t + 1 : t;           // (behind the last token: its own rows again)
+            float said = (a[0] + a[2]) + (a[1] + a[3]);
+            said += __shfl_xor_sync(0xffffffffu, said, 4);
+            read(gs + n * ROW, next.g);
 #pragma unroll
-            for (int d = DW_LANES / 2; d >= 1; d >>= 1) {
-                said += __shfl_xor_sync(0xffffffffu, said, d);
-                out += __shfl_xor_sync(0xffffffffu, out, d);
-            }
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) b[c] = fmaf(S[r][c], x.q[r][c], b[c]);
+            said += __shfl_xor_sync(0xffffffffu, said, 2);
+            read(ks + n * ROW, next.k);
+            p[t * DW_THREADS] = (b[0] + b[2]) + (b[1] + b[3]);
+            said += __shfl_xor_sync(0xffffffffu, said, 1);
+            read(qs + n * ROW, next.q);
+            next.v = vs[n * DR_COLS];
+            next.beta = bs[n];
             const float u = x.beta * ((j < dv ? x.v : 0.f) - said);
 #pragma unroll
             for (int r = 0; r < R; ++r)
 #pragma unroll
-                for (int c = 0; c < C; ++c) S[r][c] = fmaf(x.k[r][c], u, S[r][c]);
-            if (l == 0 && j < dv) orow[(size_t)t * n_heads * dv] = fmaf(u, x.kq, out);
+                for (int c = 0; c < 4; ++c) S[r][c] = fmaf(x.k[r][c], u, S[r][c]);
+            if (l == 0) up[t * DR_COLS] = u;
         };
+        Token x0, x1;
+        read(gs, x0.g);
+        read(ks, x0.k);
+        read(qs, x0.q);
+        x0.v = vs[0];
+        x0.beta = bs[0];
         int t = 0;
         for (; t + 1 < nt; t += 2) {
             token(t, x0, x1);
@@ -510,15 +538,16 @@ delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __r
 #pragma unroll
         for (int r = 0; r < R; ++r)
 #pragma unroll
-            for (int c = 0; c < C; ++c) {
-                const int i = l + DW_LANES * c + 32 * r;
+            for (int c = 0; c < 4; ++c) {
+                const int i = l + 8 * c + 32 * r;
                 if (i < dk) srow[i] = S[r][c];
             }
     }
 }
 
 // Row width of `prep` for these sizes (a multiple of 4 floats, so that rows start on 16 bytes).
-static inline int dl_width(int dk) { return dk < 64 ? dk : dk == 64 ? 64 : dk <= 128 ? 128 : 256; }
+static inline int dl_rounds(int dk) { return dk < 64 ? 0 : dk == 64 ? 2 : dk <= 128 ? 4 : 8; }
+static inline int dl_width(int dk) { return dk < 64 ? dk : 8 * (4 * dl_rounds(dk) + 4); }
 MV_API int mv_delta_prep_width(int n_heads, int kv_heads, int dk) {
     const int w = (2 * kv_heads + n_heads) * dl_width(dk) + n_heads + kv_heads;
     return (w + 3) & ~3;
@@ -531,7 +560,7 @@ MV_API int mv_delta_scan_long(const float* q, int ldq, const float* k, int ldk, 
                               int n_seqs, int n_heads, int kv_heads, int dk, int dv, int head_decay, cudaStream_t stream) {
     if (n_seqs <= 0 || N <= 0) return 0;
     if (dk < 1 || dk > 256 || dv < 1 || kv_heads < 1 || n_heads % kv_heads) return (int)cudaErrorInvalidValue;
-    const int ldp = mv_delta_prep_width(n_heads, kv_heads, dk), W = dl_width(dk), R = dk < 64 ? 0 : W / 32;
+    const int ldp = mv_delta_prep_width(n_heads, kv_heads, dk), W = dl_width(dk), R = dl_rounds(dk);
     mv_launch(delta_prepare_kernel, N, 256, 0, stream, q, ldq, k, ldk, b, ldb, a, lda, dt_bias, a_log, q_scale, norm_eps, prep,
               ldp, n_heads, kv_heads, dk, W, R, head_decay);
     // The walk is launched as an ordinary successor, not a programmatic one.  Started while the preparing kernel's blocks
@@ -540,7 +569,7 @@ MV_API int mv_delta_scan_long(const float* q, int ldq, const float* k, int ldk, 
     // long as when they are dealt out over an idle device (measured: 1.26 ms against 0.72 for 2,048 tokens).
     const dim3 grid((dv + DR_COLS - 1) / DR_COLS, n_heads, n_seqs);
     if (R && ((uintptr_t)prep & 15)) return (int)cudaErrorInvalidValue;
-    const size_t smem = 2 * (size_t)DL_CHUNK * (3 * (R ? DW_LANES * dw_lane(R) : dk) + DR_COLS + 2) * sizeof(float);
+    const size_t smem = R ? dw_smem(R) : 2 * (size_t)DL_CHUNK * (3 * dk + DR_COLS + 2) * sizeof(float);
     // 16-byte copies: every row of q, k and g of a head starts on 16 bytes (ldp is a multiple of 4 floats)
     const int wide = dk % 4 == 0 && (((uintptr_t)prep) & 15) == 0;
 #define DL_LAUNCH(R, PART)                                                                                                   \
@@ -561,7 +590,7 @@ MV_API int mv_delta_scan_long(const float* q, int ldq, const float* k, int ldk, 
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
             if (e != cudaSuccess) return (int)e;                                                                         \
         }                                                                                                                \
-        delta_scan_wide_kernel<R><<<grid, DW_THREADS, smem, stream>>>((const float*)prep, ldp, v, ldv, state, slots,  \
+        delta_scan_wide_kernel<R><<<grid, DW_ALL, smem, stream>>>((const float*)prep, ldp, v, ldv, state, slots,  \
                                                                         cu, o, n_heads, kv_heads, dk, dv);               \
     } while (0)
     if (dk <= 32) DL_LAUNCH(4, 8);

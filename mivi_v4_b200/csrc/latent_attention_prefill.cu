@@ -264,17 +264,21 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
             const bool need_mask = key0 + KB - 1 > q0 || (window > 0 && key0 <= q0 + 15 - window);
             float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
-            for (int j = 0; j < KB / 8; ++j) {
+            for (int j = 0; j < KB / 8; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    float sc = s[mt][j][e] * scale;
-                    if (need_mask) {
+                for (int e = 0; e < 4; ++e) s[mt][j][e] *= scale;
+            if (need_mask) {                          // (one branch a tile; inside the loop it was one a score)
+                const int from0 = window > 0 ? p0 - window : -1, from1 = window > 0 ? p1 - window : -1;
+#pragma unroll
+                for (int j = 0; j < KB / 8; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
                         const int t = key0 + j * 8 + 2 * t4 + (e & 1);
-                        const int p = (e < 2) ? p0 : p1;
-                        if (t > p || (window > 0 && t <= p - window)) sc = -INFINITY;
+                        if (t > (e < 2 ? p0 : p1) || t <= (e < 2 ? from0 : from1)) s[mt][j][e] = -INFINITY;
                     }
-                    s[mt][j][e] = sc;
-                }
+            }
+#pragma unroll
+            for (int j = 0; j < KB / 8; ++j) {
                 mx0 = fmaxf(mx0, fmaxf(s[mt][j][0], s[mt][j][1]));
                 mx1 = fmaxf(mx1, fmaxf(s[mt][j][2], s[mt][j][3]));
             }
