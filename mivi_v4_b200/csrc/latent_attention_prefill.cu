@@ -127,7 +127,9 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, long long page_stri
 // fragment that is read from shared memory serves two of them, the reads are ldmatrix, and the softmax of one warp runs under the
 // products of the scheduler's other one.  A row's sums are added in the same order whatever MT is: blocks of 64 keys from multiples
 // of 64, 16 channels and 16 keys at a time, and key blocks that a warp's queries cannot see change nothing and are passed over.
-// Longest blocks first, so that no long one is left for the end.  @MEASURED@
+// Longest blocks first, so that no long one is left for the end.  A third of what was issued used to be the copies' addresses and
+// branches, and every score had a branch for the mask.  32 heads of 64 + 32 / 64: 6,000 tokens 2,050 -> 1,205 us (0.37 of what
+// mma.sync gives), three prompts of 333 to 2,048 tokens 355 -> 235 us.
 template <int DKM, int DVM, int MT>
 __global__ void __launch_bounds__(NWARPS * 32)
 latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kx, int ld_kx,
