@@ -349,6 +349,174 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ pool, lo
     }
 }
 
+// The same in float32 for steps of many tokens: a block is 32 packed query rows of one head; keys and values come in blocks of 64
+// into shared memory, once for all of the rows that read their sequence, where a warp a row reads every key for itself.  The
+// rows' sequences are taken one after the other (most tiles have one); scores, weights and sums are float32 throughout.  A
+// thread has 4 x 4 scores and 4 x (4 NB) of the output, four threads a row do the softmax.  Bound by the latency of its few
+// steps a tile: 1,165 rows of four prompts, 16 heads of 64: 680 us with a warp a row, @T@ so.
+constexpr int FT_Q = 32, FT_K = 64, FT_SLD = FT_K + 4;
+
+template <int NB>
+__global__ void __launch_bounds__(128)
+attention_f32_tile_kernel(const float* __restrict__ q, const float* __restrict__ pool, long long page_stride,
+                          const int* __restrict__ page_table, int table_stride, int page_shift,
+                          const int* __restrict__ positions, const int* __restrict__ seq_of, float* __restrict__ o, int N,
+                          int nh, int nkv, int hd, float scale, int window) {
+    constexpr int W = 64 * NB, LD = W + 4;
+    extern __shared__ __align__(16) float ft_smem[];
+    float* qs = ft_smem;                        // [FT_Q][LD]
+    float* ks = qs + FT_Q * LD;                 // [FT_K][LD]
+    float* vs = ks + FT_K * LD;                 // [FT_K][W]
+    float* ps = vs + FT_K * W;                  // [FT_Q][FT_SLD]
+    float* cs = ps + FT_Q * FT_SLD;             // [FT_Q]: what the sums so far are multiplied by, at the end 1 / the denominator
+    mv_pdl_begin();
+    const int n0 = blockIdx.x * FT_Q, rows = min(FT_Q, N - n0), h = blockIdx.y, g = h / (nh / nkv);
+    const int tid = threadIdx.x, tk = tid & 15, tq = tid >> 4, row = tid >> 2, part = tid & 3;
+    const int page_size = 1 << page_shift;
+    const size_t v_off = (size_t)nkv * page_size * hd;
+    for (int idx = tid; idx < FT_Q * W; idx += 128) {
+        const int r = idx / W, d = idx % W;
+        qs[r * LD + d] = r < rows && d < hd ? q[(size_t)(n0 + r) * nh * hd + (size_t)h * hd + d] * scale : 0.f;
+    }
+    float acc[4][4 * NB], m = -INFINITY, l = 0.f;       // m, l: of row `row`, in each of its four threads
+#pragma unroll
+    for (int y = 0; y < 4; ++y)
+#pragma unroll
+        for (int x = 0; x < 4 * NB; ++x) acc[y][x] = 0.f;
+    const int my_pos = row < rows ? positions[n0 + row] : -1;
+    for (int r0 = 0; r0 < rows;) {
+        // the rows r0 .. r1 - 1 read one sequence; the keys that any of them sees
+        const int b = seq_of[n0 + r0];
+        int r1 = r0, last = -1, first = 0x7fffffff;
+        for (; r1 < rows && seq_of[n0 + r1] == b; ++r1) {
+            const int p = positions[n0 + r1];
+            last = max(last, p);
+            first = min(first, window > 0 ? max(0, p - window + 1) : 0);
+        }
+        const int* table = page_table + (size_t)b * table_stride;
+        const bool mine = row >= r0 && row < r1;
+        for (int t0 = first; t0 <= last; t0 += FT_K) {
+            __syncthreads();                            // the block before is done with; the queries are there
+            for (int idx = tid; idx < FT_K * (W / 4); idx += 128) {
+                const int r = idx / (W / 4), d = idx % (W / 4) * 4, t = t0 + r;
+                float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f), v4 = k4;
+                if (t <= last && d < hd) {
+                    const float* kr = pool + (size_t)mv_read_page(table[t >> page_shift]) * page_stride +
+                                      ((size_t)g * page_size + (t & (page_size - 1))) * hd + d;
+                    k4 = *reinterpret_cast<const float4*>(kr);
+                    v4 = *reinterpret_cast<const float4*>(kr + v_off);
+                }
+                *reinterpret_cast<float4*>(ks + r * LD + d) = k4;
+                *reinterpret_cast<float4*>(vs + r * W + d) = v4;
+            }
+            __syncthreads();
+            float sc[4][4];
+#pragma unroll
+            for (int y = 0; y < 4; ++y)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) sc[y][x] = 0.f;
+#pragma unroll 4
+            for (int d = 0; d < W; d += 4) {
+                float4 w[4];
+#pragma unroll
+                for (int x = 0; x < 4; ++x) w[x] = *reinterpret_cast<const float4*>(ks + (tk + 16 * x) * LD + d);
+#pragma unroll
+                for (int y = 0; y < 4; ++y) {
+                    const float4 u = *reinterpret_cast<const float4*>(qs + (tq + 8 * y) * LD + d);
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        sc[y][x] = fmaf(u.x, w[x].x, sc[y][x]); sc[y][x] = fmaf(u.y, w[x].y, sc[y][x]);
+                        sc[y][x] = fmaf(u.z, w[x].z, sc[y][x]); sc[y][x] = fmaf(u.w, w[x].w, sc[y][x]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int y = 0; y < 4; ++y)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) ps[(tq + 8 * y) * FT_SLD + tk + 16 * x] = sc[y][x];
+            __syncthreads();
+            {
+                // key part + 4 i of the row; a row of another sequence sees none of them
+                float s[FT_K / 4], mx = -INFINITY, sum = 0.f;
+#pragma unroll
+                for (int i = 0; i < FT_K / 4; ++i) {
+                    const int t = t0 + part + 4 * i;
+                    const bool seen = mine && t <= my_pos && (window <= 0 || t > my_pos - window);
+                    s[i] = seen ? ps[row * FT_SLD + part + 4 * i] : -INFINITY;
+                    mx = fmaxf(mx, s[i]);
+                }
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+                const float m_new = fmaxf(m, mx), ref = m_new == -INFINITY ? 0.f : m_new;
+                const float corr = m == -INFINITY ? (m_new == -INFINITY ? 1.f : 0.f) : expf(m - ref);
+#pragma unroll
+                for (int i = 0; i < FT_K / 4; ++i) {
+                    const float w = s[i] == -INFINITY ? 0.f : expf(s[i] - ref);
+                    sum += w;
+                    ps[row * FT_SLD + part + 4 * i] = w;
+                }
+                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                l = l * corr + sum;
+                m = m_new;
+                if (part == 0) cs[row] = corr;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+                const float c = cs[tq + 8 * y];
+#pragma unroll
+                for (int x = 0; x < 4 * NB; ++x) acc[y][x] *= c;
+            }
+            const int n_keys = min(FT_K, last - t0 + 1);
+#pragma unroll 2
+            for (int t = 0; t < n_keys; ++t) {
+                float4 w[NB];
+#pragma unroll
+                for (int x = 0; x < NB; ++x) w[x] = *reinterpret_cast<const float4*>(vs + t * W + 64 * x + tk * 4);
+#pragma unroll
+                for (int y = 0; y < 4; ++y) {
+                    const float pt = ps[(tq + 8 * y) * FT_SLD + t];
+                    if (pt != 0.f)                      // (a value that the row does not see may be anything)
+#pragma unroll
+                        for (int x = 0; x < NB; ++x) {
+                            acc[y][4 * x] = fmaf(pt, w[x].x, acc[y][4 * x]); acc[y][4 * x + 1] = fmaf(pt, w[x].y, acc[y][4 * x + 1]);
+                            acc[y][4 * x + 2] = fmaf(pt, w[x].z, acc[y][4 * x + 2]); acc[y][4 * x + 3] = fmaf(pt, w[x].w, acc[y][4 * x + 3]);
+                        }
+                }
+            }
+        }
+        r0 = r1;
+    }
+    __syncthreads();
+    if (part == 0) cs[row] = 1.0f / l;
+    __syncthreads();
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+        const int r = tq + 8 * y;
+        if (r >= rows) continue;
+        const float inv = cs[r];
+        float* to = o + (size_t)(n0 + r) * nh * hd + (size_t)h * hd;
+#pragma unroll
+        for (int x = 0; x < 4 * NB; ++x) {
+            const int d = 64 * (x / 4) + tk * 4 + x % 4;
+            if (d < hd) to[d] = acc[y][x] * inv;
+        }
+    }
+}
+
+template <int NB>
+static int attention_f32_tile_launch(const float* q, const float* pool, long long page_stride, const int* page_table, int table_stride,
+                                     int page_shift, const int* positions, const int* seq_of, float* o, int N, int nh, int nkv, int hd,
+                                     float scale, int window, cudaStream_t stream) {
+    constexpr size_t smem = sizeof(float) * ((FT_Q + FT_K) * (64 * NB + 4) + FT_K * 64 * NB + FT_Q * FT_SLD + FT_Q);
+    static const cudaError_t attr = cudaFuncSetAttribute(attention_f32_tile_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (attr != cudaSuccess) return (int)attr;
+    mv_launch(attention_f32_tile_kernel<NB>, dim3((N + FT_Q - 1) / FT_Q, nh), 128, smem, stream, q, pool, page_stride, page_table,
+              table_stride, page_shift, positions, seq_of, o, N, nh, nkv, hd, scale, window);
+    return mv_launch_status();
+}
+
 MV_API int mv_attention_generic(const void* q, const void* pool, long long page_stride,
                                 const int* page_table, int table_stride, int page_size,
                                 const int* positions, const int* seq_of, void* o, int dtype, int N,
@@ -363,6 +531,12 @@ MV_API int mv_attention_generic(const void* q, const void* pool, long long page_
         mv_launch(attention_generic_kernel<__nv_bfloat16>, blocks, 128, 0, stream, 
             (const __nv_bfloat16*)q, (const __nv_bfloat16*)pool, page_stride, page_table, table_stride,
             page_shift, positions, seq_of, (__nv_bfloat16*)o, N, nh, nkv, hd, scale, window);
+    else if (N >= FT_Q && hd <= 128 && hd % 4 == 0 && page_stride % 4 == 0 && ((uintptr_t)pool & 15) == 0)
+        // (a tile of one or two rows repays nothing)
+        return hd <= 64 ? attention_f32_tile_launch<1>((const float*)q, (const float*)pool, page_stride, page_table, table_stride, page_shift,
+                                                       positions, seq_of, (float*)o, N, nh, nkv, hd, scale, window, stream)
+                        : attention_f32_tile_launch<2>((const float*)q, (const float*)pool, page_stride, page_table, table_stride, page_shift,
+                                                       positions, seq_of, (float*)o, N, nh, nkv, hd, scale, window, stream);
     else
         mv_launch(attention_generic_kernel<float>, blocks, 128, 0, stream, 
             (const float*)q, (const float*)pool, page_stride, page_table, table_stride, page_shift,
