@@ -21,36 +21,32 @@ __device__ __forceinline__ float gr_softplus(float z) { return z > 20.f ? z : lo
 // block read consecutive outputs; ba, bi, lam [C].  a_out, x_out [N, C]: the decay and the gated input
 // sqrt(1 - a^2) i u.  A block is (16 tokens, 128 outputs of one part): the tokens' inputs of that part lie in
 // shared memory as [in][token], a thread keeps one output of all 16 tokens in registers.
-// TOK 32 where that still leaves two blocks a multiprocessor: every block reads its outputs' columns of both matrices from
-// L2, which is what bounds it with 16 (2,588 tokens of 4 parts of 256: @A@ us, @B@ with 32).  A row of the inputs is padded by 16
-// bytes so that storing them turned meets fewer bank conflicts.
-template <int TOK>
 __global__ void __launch_bounds__(128)
 block_gates_kernel(const float* __restrict__ u, const float* __restrict__ wa_t, const float* __restrict__ wi_t,
                    const float* __restrict__ ba, const float* __restrict__ bi, const float* __restrict__ lam, float c,
                    float* __restrict__ a_out, float* __restrict__ x_out, int N, int C, int bs) {
     mv_pdl_begin();
-    extern __shared__ __align__(16) float gr_us[];           // [bs][TOK + 4]
-    const int n0 = blockIdx.x * TOK, b = blockIdx.y;
+    extern __shared__ __align__(16) float gr_us[];           // [bs][GR_TOK]
+    const int n0 = blockIdx.x * GR_TOK, b = blockIdx.y;
     const int o = blockIdx.z * blockDim.x + threadIdx.x;
-    const int nt = min(TOK, N - n0);
-    for (int idx = threadIdx.x; idx < bs * TOK; idx += blockDim.x) {
+    const int nt = min(GR_TOK, N - n0);
+    for (int idx = threadIdx.x; idx < bs * GR_TOK; idx += blockDim.x) {
         const int t = idx / bs, in = idx - t * bs;           // consecutive threads read consecutive inputs
-        gr_us[in * (TOK + 4) + t] = t < nt ? u[(size_t)(n0 + t) * C + (size_t)b * bs + in] : 0.f;
+        gr_us[in * GR_TOK + t] = t < nt ? u[(size_t)(n0 + t) * C + (size_t)b * bs + in] : 0.f;
     }
     __syncthreads();
     if (o >= bs) return;
-    float ar[TOK], ai[TOK];
+    float ar[GR_TOK], ai[GR_TOK];
 #pragma unroll
-    for (int t = 0; t < TOK; ++t) ar[t] = ai[t] = 0.f;
+    for (int t = 0; t < GR_TOK; ++t) ar[t] = ai[t] = 0.f;
     const float* wa = wa_t + (size_t)b * bs * bs + o;
     const float* wi = wi_t + (size_t)b * bs * bs + o;
 #pragma unroll 8
     for (int in = 0; in < bs; ++in) {
         const float x = wa[(size_t)in * bs], y = wi[(size_t)in * bs];
-        const float4* row = reinterpret_cast<const float4*>(gr_us + in * (TOK + 4));
+        const float4* row = reinterpret_cast<const float4*>(gr_us + in * GR_TOK);
 #pragma unroll
-        for (int q = 0; q < TOK / 4; ++q) {
+        for (int q = 0; q < GR_TOK / 4; ++q) {
             const float4 v = row[q];
             ar[4 * q] = fmaf(x, v.x, ar[4 * q]);         ai[4 * q] = fmaf(y, v.x, ai[4 * q]);
             ar[4 * q + 1] = fmaf(x, v.y, ar[4 * q + 1]); ai[4 * q + 1] = fmaf(y, v.y, ai[4 * q + 1]);
@@ -61,7 +57,7 @@ block_gates_kernel(const float* __restrict__ u, const float* __restrict__ wa_t, 
     const int ch = b * bs + o;
     const float rate = c * gr_softplus(lam[ch]), bra = ba[ch], bri = bi[ch];
 #pragma unroll
-    for (int t = 0; t < TOK; ++t) {
+    for (int t = 0; t < GR_TOK; ++t) {
         if (t < nt) {
             const float r = 1.0f / (1.0f + expf(-(ar[t] + bra)));
             const float ig = 1.0f / (1.0f + expf(-(ai[t] + bri)));
@@ -69,7 +65,7 @@ block_gates_kernel(const float* __restrict__ u, const float* __restrict__ wa_t, 
             const size_t at = (size_t)(n0 + t) * C + ch;
             a_out[at] = expf(log_a);
             // 1 - a^2 = -expm1(2 log a): exact also where a is close to 1
-            x_out[at] = sqrtf(-expm1f(2.0f * log_a)) * ig * gr_us[o * (TOK + 4) + t];
+            x_out[at] = sqrtf(-expm1f(2.0f * log_a)) * ig * gr_us[o * GR_TOK + t];
         }
     }
 }
@@ -163,18 +159,13 @@ MV_API int mv_block_gates(const float* u, const float* wa_t, const float* wi_t, 
                   x_out, N, C, bs);
         return mv_launch_status();
     }
-    const int threads = bs >= 128 ? 128 : ((bs + 31) / 32) * 32, parts = n_blocks * ((bs + threads - 1) / threads);
-    const size_t wide = (size_t)bs * (32 + 4) * sizeof(float), narrow = (size_t)bs * (GR_TOK + 4) * sizeof(float);
-    const bool many = (long long)((N + 31) / 32) * parts >= 296 && wide <= 64 * 1024;
-    const size_t bytes = many ? wide : narrow;
-    if (bytes > 48 * 1024) {
-        const cudaError_t e = many ? cudaFuncSetAttribute(block_gates_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
-                                   : cudaFuncSetAttribute(block_gates_kernel<GR_TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(block_gates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    const dim3 grid((N + (many ? 32 : GR_TOK) - 1) / (many ? 32 : GR_TOK), n_blocks, (bs + threads - 1) / threads);
-    if (many) mv_launch(block_gates_kernel<32>, grid, threads, bytes, stream, u, wa_t, wi_t, ba, bi, lam, c, a_out, x_out, N, C, bs);
-    else mv_launch(block_gates_kernel<GR_TOK>, grid, threads, bytes, stream, u, wa_t, wi_t, ba, bi, lam, c, a_out, x_out, N, C, bs);
+    const int threads = bs >= 128 ? 128 : ((bs + 31) / 32) * 32;
+    const dim3 grid((N + GR_TOK - 1) / GR_TOK, n_blocks, (bs + threads - 1) / threads);
+    mv_launch(block_gates_kernel, grid, threads, smem, stream, u, wa_t, wi_t, ba, bi, lam, c, a_out, x_out, N, C, bs);
     return mv_launch_status();
 }
 

@@ -146,6 +146,20 @@ gemm_f32_tile_kernel(const float* __restrict__ X, const float* __restrict__ W, c
     cluster.sync();                                                 // nobody leaves while its tile is read
 }
 
+// Two blocks a multiprocessor run at once.  K is cut over 1, 2, 4 or 8 blocks so that the rounds of such blocks, each as long as a
+// share of K and about four steps of filling and (cut) adding up, end soonest; a tile of 32 rows takes 0.63 of the time of one of
+// 64 (half the products, fewer of them a read).  In 64ths of a step; `ranks` gets the cut.
+inline long gemm_f32_tile_cost(int bm, int M, int N, int K, int* ranks) {
+    const long tiles = (long)((N + FT_BN - 1) / FT_BN) * ((M + bm - 1) / bm);
+    const int kb = (K + FT_BK - 1) / FT_BK;
+    long best = 0;
+    for (int r = 1; r <= 8; r *= 2) {
+        const long cost = (tiles * r + 295) / 296 * ((kb + r - 1) / r + 4 + (r > 1 ? 2 : 0)) * (bm == 64 ? 64 : 40);
+        if (r == 1 || cost < best) { best = cost; *ranks = r; }
+    }
+    return best;
+}
+
 template <int TM>
 int gemm_f32_tile_launch(const float* X, const float* W, const float* bias, void* out, int mode, int M, int N, int K, int ldo,
                          cudaStream_t stream) {
@@ -156,14 +170,8 @@ int gemm_f32_tile_launch(const float* X, const float* W, const float* bias, void
                                                          (int)smem);
     if (attr != cudaSuccess) return (int)attr;
     const int gx = (N + FT_BN - 1) / FT_BN, gy = (M + BM - 1) / BM, kb = (K + FT_BK - 1) / FT_BK;
-    // Two blocks a multiprocessor run at once.  K is cut over 1, 2, 4 or 8 blocks so that the rounds of such blocks, each as
-    // long as a share of K and about four steps of filling and adding up, end soonest.
     int ranks = 1;
-    long best = 0;
-    for (int r = 1; r <= 8; r *= 2) {
-        const long rounds = ((long)gx * gy * r + 295) / 296, cost = rounds * ((kb + r - 1) / r + 4 + (r > 1 ? 2 : 0));
-        if (r == 1 || cost < best) { best = cost; ranks = r; }
-    }
+    gemm_f32_tile_cost(BM, M, N, K, &ranks);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(gx, gy, ranks);
     cfg.blockDim = dim3(FT_THREADS);
@@ -342,7 +350,11 @@ MV_API int mv_gemm_simt(const void* X, const void* W, int in_dtype, const float*
         if (M == 2) return gemm_f32_stream_launch<2, 4>(x, w, bias, out, mode, M, N, K, ldo, stream);
         if (M <= 4) return gemm_f32_stream_launch<4, 4>(x, w, bias, out, mode, M, N, K, ldo, stream);
         if (M <= 8) return gemm_f32_stream_launch<8, 4>(x, w, bias, out, mode, M, N, K, ldo, stream);
-        if (M <= 32) return gemm_f32_tile_launch<4>(x, w, bias, out, mode, M, N, K, ldo, stream);
+        // 1,165 rows against 1,024 x 4,608: 152 tiles of 64 rows leave one block on a multiprocessor (305 us with K cut in four), 296
+        // of 32 rows fill them (@G@)
+        int r;
+        if (gemm_f32_tile_cost(32, M, N, K, &r) < gemm_f32_tile_cost(64, M, N, K, &r))
+            return gemm_f32_tile_launch<4>(x, w, bias, out, mode, M, N, K, ldo, stream);
         return gemm_f32_tile_launch<8>(x, w, bias, out, mode, M, N, K, ldo, stream);
     }
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
