@@ -353,7 +353,7 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ pool, lo
 // into shared memory, once for all of the rows that read their sequence, where a warp a row reads every key for itself.  The
 // rows' sequences are taken one after the other (most tiles have one); scores, weights and sums are float32 throughout.  A
 // thread has 4 x 4 scores and 4 x (4 NB) of the output, four threads a row do the softmax.  Bound by the latency of its few
-// steps a tile: 1,165 rows of four prompts, 16 heads of 64: 680 us with a warp a row, @T@ so.
+// steps a tile: 1,165 rows of four prompts, 16 heads of 64: 680 us with a warp a row, 129 so.
 constexpr int FT_Q = 32, FT_K = 64, FT_SLD = FT_K + 4;
 
 template <int NB>

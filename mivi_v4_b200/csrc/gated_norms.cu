@@ -679,7 +679,7 @@ __global__ void round_rows_kernel(const float* __restrict__ x, TO* __restrict__ 
 }
 
 // Eight values a thread and 16 bytes a store, for arrays that start on 16 bytes: bound by memory (2,048 x 2,048: 18 us with a
-// value a thread, @R@ so).
+// value a thread, 6 so).
 __global__ void __launch_bounds__(256)
 round_rows_vec_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ out, long long eighths) {
     mv_pdl_begin();

@@ -351,7 +351,7 @@ MV_API int mv_gemm_simt(const void* X, const void* W, int in_dtype, const float*
         if (M <= 4) return gemm_f32_stream_launch<4, 4>(x, w, bias, out, mode, M, N, K, ldo, stream);
         if (M <= 8) return gemm_f32_stream_launch<8, 4>(x, w, bias, out, mode, M, N, K, ldo, stream);
         // 1,165 rows against 1,024 x 4,608: 152 tiles of 64 rows leave one block on a multiprocessor (305 us with K cut in four), 296
-        // of 32 rows fill them (@G@)
+        // of 32 rows fill them (273; against 1,024 x 1,024: 109 and 63)
         int r;
         if (gemm_f32_tile_cost(32, M, N, K, &r) < gemm_f32_tile_cost(64, M, N, K, &r))
             return gemm_f32_tile_launch<4>(x, w, bias, out, mode, M, N, K, ldo, stream);
