@@ -1,4 +1,5 @@
-// A decaying matrix state walked in chunks of CS_CHUNK tokens: the kernels of decay_scan.cu for steps of many tokens.  Per head, with S0 the state before a chunk,
+// A decaying matrix state walked in chunks of CS_CHUNK tokens: the kernels of decay_scan.cu for steps of many tokens (scalar_scan.cu uses
+// the copies into shared memory).  Per head, with S0 the state before a chunk,
 //
 //     S_end[j, i] = d_i S0[j, i] + sum_s v_s[j] (w_s k_s[i]),
 //     o_t[j]      = f_t sum_i q_t[i] S0[j, i] + sum_{s <= t} P[t, s] v_s[j].
