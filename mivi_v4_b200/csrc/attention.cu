@@ -451,8 +451,10 @@ attention_f32_tile_kernel(const float* __restrict__ q, const float* __restrict__
                 const float corr = m == -INFINITY ? (m_new == -INFINITY ? 1.f : 0.f) : expf(m - ref);
 #pragma unroll
                 for (int i = 0; i < FT_K / 4; ++i) {
-                    const float w = s[i] == -INFINITY ? 0.f : expf(s[i] - ref);
-                    sum += w;
+                    const int t = t0 + part + 4 * i;
+                    const bool seen = mine && t <= my_pos && (window <= 0 || t > my_pos - window);
+                    const float w = seen ? expf(s[i] - ref) : -1.f;         // (-1: not to be added)
+                    sum += seen ? w : 0.f;
                     ps[row * FT_SLD + part + 4 * i] = w;
                 }
                 sum += __shfl_xor_sync(0xffffffffu, sum, 1);
@@ -477,7 +479,7 @@ attention_f32_tile_kernel(const float* __restrict__ q, const float* __restrict__
 #pragma unroll
                 for (int y = 0; y < 4; ++y) {
                     const float pt = ps[(tq + 8 * y) * FT_SLD + t];
-                    if (pt != 0.f)                      // (a value that the row does not see may be anything)
+                    if (!(pt < 0.f))                    // (a value that the row does not see may be anything)
 #pragma unroll
                         for (int x = 0; x < NB; ++x) {
                             acc[y][4 * x] = fmaf(pt, w[x].x, acc[y][4 * x]); acc[y][4 * x + 1] = fmaf(pt, w[x].y, acc[y][4 * x + 1]);
