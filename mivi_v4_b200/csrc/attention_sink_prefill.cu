@@ -215,10 +215,11 @@ attention_sink_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bf
         // the code too long for the instruction cache: 2,048 tokens of 32 heads of 80 / 64 with a cap and a window of 1,024 took
         // 202 us and take 118, three prompts of 333 to 2,048 tokens with a bias by distance 314 and 186)
         if (cap > 0.f) {
+            const float top = fmaf(cap, LOG2E, add);    // (rounded once)
 #pragma unroll
             for (int j = 0; j < KB / 8; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) s[j][e] = fmaf(-2.0f * cap_l, rcp(1.0f + ex2(s[j][e] * scale_l)), cap_l + add);
+                for (int e = 0; e < 4; ++e) s[j][e] = fmaf(-2.0f * cap_l, rcp(1.0f + ex2(s[j][e] * scale_l)), top);
         } else {
 #pragma unroll
             for (int j = 0; j < KB / 8; ++j)
