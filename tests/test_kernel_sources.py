@@ -1,0 +1,20 @@
+"""Rules for the kernels' sources that no run on one device can show broken."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mivi_v4_b200", "csrc")
+
+
+def sources():
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, name)) as f:
+                yield name, f.read()
+
+
+def test_instructions_of_a_whole_warp_are_volatile():
+    """An instruction that all lanes of a warp must reach together may not be moved behind a branch that some of them skip, which the
+    compiler is free to do with an asm statement that is not volatile."""
+    found = [f"{name}: {m.group(1)[:60]}" for name, text in sources()
+             for m in re.finditer(r'asm\s*\(\s*"([^"]*)"', text) if ".sync" in m.group(1) or ".aligned" in m.group(1)]
+    assert not found, found
