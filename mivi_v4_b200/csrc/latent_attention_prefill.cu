@@ -56,6 +56,8 @@ __device__ __forceinline__ void ldmatrix_x4_trans(unsigned (&r)[4], const void* 
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(s));
 }
 
+template <bool B> struct Flag { static constexpr bool value = B; };
+
 // first position a step's tokens of a sequence that starts the step at `start` can see
 __device__ __forceinline__ int first_seen(int start, int window) { return window > 0 ? max(0, start - window + 1) : 0; }
 
@@ -180,20 +182,7 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
         }
     }
 
-    float oacc[MT][DVM / 8][4];
-    // the sink starts the running maximum and the denominator (its own term, exp(sink - max), is 1 now); a row's
-    // denominator is summed over the four lanes of its quad at the end, so one of them holds the sink's 1
-    float m[MT][2], l[MT][2];
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-#pragma unroll
-        for (int j = 0; j < DVM / 8; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) oacc[mt][j][e] = 0.f;
-        m[mt][0] = m[mt][1] = sinks ? sinks[h] : -INFINITY;
-        l[mt][0] = l[mt][1] = (sinks && t4 == 0) ? 1.f : 0.f;
-    }
-
+    float oacc[MT][DVM / 8][4], m[MT][2], l[MT][2];
     const int last_pos = pos0 + nq - 1;
     const int first_key = window > 0 ? max(0, pos0 - window + 1) : 0;
     const int kb_begin = first_key / KB, n_iter = last_pos / KB + 1 - kb_begin;
@@ -219,6 +208,23 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
         }
     };
 
+    // One walk over the keys.  ex2 gives 0 for a weight below 2^-126, which is nothing beside the row's other weights as long as its
+    // largest is a key's; where that is the sink, far above them all, the block walks once more with an exponential that keeps them
+    // (with exp2f in every walk 6,000 tokens of 32 heads of 64 + 32 / 64 take 1,280 us and not 1,190; 800 of 16 heads of 128 + 64 / 128,
+    // where it is in the only walk, 45 and with two walks 69).
+    auto walk = [&](auto keep_small) {
+    auto weight = [&](float x) { return decltype(keep_small)::value ? exp2f(x) : ex2(x); };
+    // the sink starts the running maximum and the denominator (its own term, exp(sink - max), is 1 now); a row's
+    // denominator is summed over the four lanes of its quad at the end, so one of them holds the sink's 1
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+#pragma unroll
+        for (int j = 0; j < DVM / 8; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) oacc[mt][j][e] = 0.f;
+        m[mt][0] = m[mt][1] = sinks ? sinks[h] : -INFINITY;
+        l[mt][0] = l[mt][1] = (sinks && t4 == 0) ? 1.f : 0.f;
+    }
 #pragma unroll
     for (int i = 0; i < STAGES - 1; ++i) {
         if (i < n_iter) load_block(kb_begin + i, i);
@@ -291,16 +297,16 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
             const float mn0 = fmaxf(m[mt][0], mx0), mn1 = fmaxf(m[mt][1], mx1);
             // a row whose keys are all masked so far (and that has no sink) keeps m = -inf; use 0 as its reference
             const float ref0 = mn0 == -INFINITY ? 0.f : mn0, ref1 = mn1 == -INFINITY ? 0.f : mn1;
-            const float c0 = m[mt][0] == -INFINITY ? 0.f : ex2((m[mt][0] - ref0) * LOG2E);
-            const float c1 = m[mt][1] == -INFINITY ? 0.f : ex2((m[mt][1] - ref1) * LOG2E);
+            const float c0 = m[mt][0] == -INFINITY ? 0.f : weight((m[mt][0] - ref0) * LOG2E);
+            const float c1 = m[mt][1] == -INFINITY ? 0.f : weight((m[mt][1] - ref1) * LOG2E);
             m[mt][0] = mn0; m[mt][1] = mn1;
             float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
             for (int j = 0; j < KB / 8; ++j) {
-                s[mt][j][0] = ex2((s[mt][j][0] - ref0) * LOG2E);
-                s[mt][j][1] = ex2((s[mt][j][1] - ref0) * LOG2E);
-                s[mt][j][2] = ex2((s[mt][j][2] - ref1) * LOG2E);
-                s[mt][j][3] = ex2((s[mt][j][3] - ref1) * LOG2E);
+                s[mt][j][0] = weight((s[mt][j][0] - ref0) * LOG2E);
+                s[mt][j][1] = weight((s[mt][j][1] - ref0) * LOG2E);
+                s[mt][j][2] = weight((s[mt][j][2] - ref1) * LOG2E);
+                s[mt][j][3] = weight((s[mt][j][3] - ref1) * LOG2E);
                 sum0 += s[mt][j][0] + s[mt][j][1];
                 sum1 += s[mt][j][2] + s[mt][j][3];
             }
@@ -346,15 +352,33 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
             }
         }
     }
+    // a row's denominator, in all four lanes of its quad
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            l[mt][half] += __shfl_xor_sync(0xffffffffu, l[mt][half], 1);
+            l[mt][half] += __shfl_xor_sync(0xffffffffu, l[mt][half], 2);
+        }
+    };  // walk
+
+    constexpr bool TWICE = DKM <= 128 && DVM <= 64;   // (with more sums a second walk's code costs the first its registers)
+    walk(Flag<!TWICE>());
+    if (TWICE && sinks) {
+        bool alone = false;                           // the sink is a row's maximum and all that its denominator shows
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) alone = alone || (live && m[mt][half] == sinks[h] && l[mt][half] == 1.f);
+        if (__syncthreads_or(alone)) walk(Flag<true>());
+    }
     if (!live) return;
 
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-            float den = l[mt][half];
-            den += __shfl_xor_sync(0xffffffffu, den, 1);
-            den += __shfl_xor_sync(0xffffffffu, den, 2);
+            const float den = l[mt][half];
             const float inv = den > 0.f ? 1.f / den : 0.f;
             const int qi = w0 + mt * 16 + gq + 8 * half;
             if (qi >= nq) continue;
