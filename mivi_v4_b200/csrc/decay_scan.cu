@@ -141,7 +141,11 @@ MV_API int mv_decay_scan(const float* q, int ldq, const float* k, int ldk, const
 // With one constant decay a head the chunks take the path with one decay for all channels; with a decay a channel
 // the kernel below prepares, per (sequence, head, chunk), the decayed q and k, the chunk's total decay and P.  The factors
 // e^(c_t - c_s) of P are products of the tokens' own decays: a warp takes eight s and walks t, multiplying the eight
-// rows k_s e^(c_t - c_s) that its lanes hold by the next token's decay; the eight sums over the lanes are folded.
+// rows k_s e^(c_t - c_s) that its lanes hold by the next token's decay; the eight sums over the lanes are folded.  A row meets up
+// to 63 decays, and a decay near 1 in 32 bits is off by up to 2^-25 of what it takes away from a row that hardly decays: from 1/2
+// on it is held as a - 1 to full relative precision and the row becomes fma(p, a - 1, p), rounded once a step and nowhere else
+// (64 tokens with decays about 1 - 2^-13: 4.2e-7 off the 64-bit outputs with plain factors, 1.9e-7 so; with an exponential for every
+// difference of sums, as in the kernels for few tokens, 2.1e-7).
 // 2,048 tokens of 8 heads of 128 x 256 with a decay a channel: 43 us this kernel, 59 the walk, 48 the outputs, where preparing
 // with an exponential for every t, s and channel and walking 32 tokens and 16 columns at a time took 64 and 243; of 16 heads
 // of 128 x 128 with a constant decay and the activation: 20 + 3 + 23 + 65 + 55 us against 64 and 243.
@@ -177,7 +181,7 @@ decay_chunk_prepare_kernel(const float* __restrict__ q, int ldq, const float* __
     constexpr int W = 32 * NC;
     extern __shared__ __align__(16) float smem[];
     float* qs = smem;                               // [CS_CHUNK][W] scaled q, zero beyond the tokens and channels
-    float* as = qs + CS_CHUNK * W;                  // the decays, and (until then) their logarithms
+    float* as = qs + CS_CHUNK * W;                  // the decays' logarithms, then the decays: a - 1 (its sign set) from 1/2 on, else a
     float* cs = as + CS_CHUNK * W;                  // running sums of the logarithms
     mv_pdl_begin();
     const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -224,7 +228,8 @@ decay_chunk_prepare_kernel(const float* __restrict__ q, int ldq, const float* __
 #pragma unroll 8
     for (int e = 0; e < CS_CHUNK * W / DC_THREADS; ++e) {
         const int idx = tid + e * DC_THREADS, t = idx / W, i = idx % W;
-        as[idx] = expf(as[idx]);
+        const float l = as[idx];
+        as[idx] = l >= -0.6931f ? -fabsf(expm1f(l)) : expf(l);
         if (i < dk && t < nt) kd[(first + t) * width + (size_t)h * dk + i] = k[(first + t) * ldk + (size_t)h * dk + i] * expf(cs[idx]);
     }
     __syncthreads();
@@ -250,10 +255,22 @@ decay_chunk_prepare_kernel(const float* __restrict__ q, int ldq, const float* __
             qt[x] = q4.x; qt[x + 1] = q4.y; qt[x + 2] = q4.z; qt[x + 3] = q4.w;
             at[x] = a4.x; at[x + 1] = a4.y; at[x + 2] = a4.z; at[x + 3] = a4.w;
         }
+        int weak = -1;
 #pragma unroll
-        for (int s = 0; s < 8; ++s)
+        for (int x = 0; x < NC; ++x) weak &= __float_as_int(at[x]);
+        if (__all_sync(0xffffffffu, weak < 0)) {
 #pragma unroll
-            for (int x = 0; x < NC; ++x) p[s][x] *= at[x];
+            for (int s = 0; s < 8; ++s)
+#pragma unroll
+                for (int x = 0; x < NC; ++x) p[s][x] = fmaf(p[s][x], at[x], p[s][x]);
+        } else {
+#pragma unroll
+            for (int x = 0; x < NC; ++x) {
+                const int keep = __float_as_int(at[x]) >> 31;
+#pragma unroll
+                for (int s = 0; s < 8; ++s) p[s][x] = fmaf(p[s][x], at[x], __int_as_float(__float_as_int(p[s][x]) & keep));
+            }
+        }
         if (t - s0 < 8) {                           // token t's own row begins
 #pragma unroll
             for (int s = 0; s < 8; ++s)

@@ -81,3 +81,27 @@ def test_a_later_token_that_is_not_finite():
                  head_decay=torch.full((heads,), 0.9, device=DEV), max_len=N, ws=Scratch())
     assert bool(torch.isfinite(out[:37]).all()) and not bool(torch.isfinite(out[37:, 5]).any())
     assert bool(torch.isfinite(out[:, 6:]).all())
+
+
+@pytest.mark.parametrize("tokens", [33, 64, 100])
+@pytest.mark.parametrize("shift,inv_tau", [(6.0, 1 / 16), (3.0, 1 / 8), (0.0, 1.0), (-2.0, 1.0)])
+def test_decay_near_one(tokens, shift, inv_tau):
+    """Decays near 1 lose nothing by being multiplied up over a chunk.  Of an output's 2-norm: a product of up to 63 factors is rounded
+    63 times (uniform in half a place either way, 0.29 * 2^-23 of a number halfway between two powers of two, so 2^-23 * 0.29 / 1.4 *
+    sqrt(63) = 2.0e-7 for the oldest token of a chunk, 1.4e-7 over all), the sum over the key channels averages that down, and the
+    sums' own rounding is 1.2e-7 (seen where there are few tokens): below 2.2e-7 together."""
+    from mivi_v4_b200.ops import kernels as K
+    heads, dk, dv = 4, 128, 128
+    g = torch.Generator().manual_seed(tokens)
+    q, k, z = (torch.randn(tokens, heads * dk, generator=g) for _ in "qkz")
+    v, z = torch.randn(tokens, heads * dv, generator=g), z + shift
+    state = torch.randn(1, heads, dv, dk, generator=g)
+    want = torch.zeros(tokens, heads * dv, dtype=F64)
+    for h in range(heads):
+        c, d = slice(h * dk, (h + 1) * dk), slice(h * dv, (h + 1) * dv)
+        a = torch.exp(torch.nn.functional.logsigmoid(z[:, c].double()) * inv_tau)
+        want[:, d] = scan(q[:, c].double() * 0.5, k[:, c].double(), v[:, d].double(), a, state[0, h].double().T)[0]
+    out = torch.full((tokens, heads * dv), float("nan"), device=DEV)
+    K.decay_scan(q.to(DEV), k.to(DEV), v.to(DEV), state.to(DEV), i32([0]), i32([0, tokens]), out, 1, heads, dk, dv, q_scale=0.5,
+                 decay_logits=z.to(DEV), inv_tau=inv_tau, max_len=tokens, ws=Scratch())
+    assert (out.double().cpu() - want).norm() / want.norm() <= 2.2e-7
