@@ -149,6 +149,7 @@ MV_API int mv_decay_scan(const float* q, int ldq, const float* k, int ldk, const
 // 2,048 tokens of 8 heads of 128 x 256 with a decay a channel: 43 us this kernel, 59 the walk, 48 the outputs, where preparing
 // with an exponential for every t, s and channel and walking 32 tokens and 16 columns at a time took 64 and 243; of 16 heads
 // of 128 x 128 with a constant decay and the activation: 20 + 3 + 23 + 65 + 55 us against 64 and 243.
+
 #define DC_THREADS 256
 
 // The activation before anything else: rows of q, k and v into dense copies.
@@ -353,4 +354,253 @@ MV_API int mv_decay_scan_chunked(const float* q, int ldq, const float* k, int ld
     a.q = qd; a.k = kd; a.ed = ed; a.P = P;
     a.ldq = a.ldk = wk;
     return cs_launch<true>(a, nullptr, nullptr, chunks, n_seqs, max_len, stream);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Chunks for steps of few tokens (below 400, the wrapper's DECAY_CHUNKS_FROM): the same sums with 32 tokens a chunk in two launches.
+// The first kernel prepares, per (sequence, head, chunk), the decayed q and k, the chunk's total decay and P; the second walks a
+// sequence's chunks with the state in registers and works the outputs out on the way.  Such a step is bound by its launches and by
+// a handful of chunks one after the other: one sequence of 16 tokens 41 us (8 heads of 128 x 256, a decay a channel) and 35 (16 heads
+// of 128 x 128, one a head, with the activation) against 57 and 58 with the three to five kernels below; 256 tokens 74 and 67 against 84 and
+// 74; four sequences of 96 84 and 81 against 86 and 87, of 128 96 and 93 against 86 and 80.
+//
+// Chunks are numbered floor(cu[b] / DF_CHUNK) + b + c for chunk c of the step's sequence b: distinct
+// numbers below N / DF_CHUNK + n_seqs + 1 that need nothing from the host.
+#define DF_CHUNK 32
+#define DF_COLS 16
+#define DF_THREADS 256            // the preparing kernel
+#define DF_SCAN_THREADS 512       // the scanning kernel: 32 half-warps
+#define DF_GROUPS (DF_SCAN_THREADS / 16)
+// a group's shares of a chunk's outputs, padded by half a row of banks: the two groups of a warp then store into
+// different banks
+#define DF_RED_STRIDE (DF_CHUNK * DF_COLS + 16)
+
+__global__ void __launch_bounds__(DF_THREADS)
+decay_few_prepare_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
+                           const float* __restrict__ z, int ldz, const float* __restrict__ head_decay, float inv_tau,
+                           float q_scale, int act, const int* __restrict__ cu, float* __restrict__ qd,
+                           float* __restrict__ kd, float* __restrict__ ed, float* __restrict__ P, int n_heads, int dk) {
+    mv_pdl_begin();
+    extern __shared__ float smem[];
+    const int lds = dk + 1;                         // odd row stride: rows of different tokens fall into different banks
+    float* cs = smem;                               // [DF_CHUNK][lds] cumulative log decay
+    float* qa = cs + DF_CHUNK * lds;                // activated, scaled q
+    float* ka = qa + DF_CHUNK * lds;                // activated k
+    const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+    const int row0 = cu[b], len = cu[b + 1] - row0;
+    if (c * DF_CHUNK >= len) return;
+    const int nt = min(DF_CHUNK, len - c * DF_CHUNK);
+    const int first = row0 + c * DF_CHUNK;
+    const int chunk = row0 / DF_CHUNK + b + c;
+    const int tid = threadIdx.x;
+    // a decay of exactly 0 has no logarithm; e^-80 stands in for it (what is left of the state then lies 35
+    // decimal places down)
+    const float log_hd = head_decay ? fmaxf(logf(head_decay[h]), -80.f) : 0.f;
+    for (int idx = tid; idx < nt * dk; idx += DF_THREADS) {
+        const int t = idx / dk, i = idx - t * dk;
+        const size_t row = (size_t)(first + t);
+        float qv = q[row * ldq + (size_t)h * dk + i], kv = k[row * ldk + (size_t)h * dk + i];
+        if (act) { qv = ds_silu(qv); kv = ds_silu(kv); }
+        qa[t * lds + i] = qv * q_scale;
+        ka[t * lds + i] = kv;
+        cs[t * lds + i] = z ? ds_log_sigmoid(z[row * ldz + (size_t)h * dk + i]) * inv_tau : log_hd;
+    }
+    __syncthreads();
+    for (int i = tid; i < dk; i += DF_THREADS) {
+        float run = 0.f;
+        for (int t = 0; t < nt; ++t) {
+            run += cs[t * lds + i];
+            cs[t * lds + i] = run;
+        }
+    }
+    __syncthreads();
+    const int width = n_heads * dk;
+    for (int idx = tid; idx < nt * dk; idx += DF_THREADS) {
+        const int t = idx / dk, i = idx - t * dk;
+        const size_t at = (size_t)(first + t) * width + (size_t)h * dk + i;
+        qd[at] = qa[t * lds + i] * expf(cs[t * lds + i]);
+        kd[at] = ka[t * lds + i] * expf(cs[(nt - 1) * lds + i] - cs[t * lds + i]);
+    }
+    for (int i = tid; i < dk; i += DF_THREADS) ed[(size_t)chunk * width + (size_t)h * dk + i] = expf(cs[(nt - 1) * lds + i]);
+    float* Pc = P + ((size_t)chunk * n_heads + h) * DF_CHUNK * DF_CHUNK;
+    for (int p = tid; p < DF_CHUNK * DF_CHUNK; p += DF_THREADS) {
+        const int t = p / DF_CHUNK, s = p - t * DF_CHUNK;
+        float sum = 0.f;
+        if (s <= t && t < nt) {
+            const float* ct = cs + t * lds;
+            const float* cq = cs + s * lds;
+            const float* qt = qa + t * lds;
+            const float* kt = ka + s * lds;
+            if (z) {
+                for (int i = 0; i < dk; ++i) sum = fmaf(qt[i] * kt[i], expf(ct[i] - cq[i]), sum);
+            } else {
+                // one decay for all of the head's channels: its power is a factor of the whole sum
+                for (int i = 0; i < dk; ++i) sum = fmaf(qt[i], kt[i], sum);
+                sum *= expf(ct[0] - cq[0]);
+            }
+        }
+        Pc[p] = sum;
+    }
+}
+
+// A block is 16 value columns of one head of one sequence; its 16 warps are 32 half-warps, each holding RH key
+// channels of every column in registers (dk <= 32 * RH): lane & 15 is the column, the half-warp the channel group.
+template <int RH>
+__global__ void __launch_bounds__(DF_SCAN_THREADS)
+decay_few_scan_kernel(const float* __restrict__ qd, const float* __restrict__ kd, const float* __restrict__ ed,
+                        const float* __restrict__ P, const float* __restrict__ v, int ldv, int act,
+                        float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ cu,
+                        float* __restrict__ o, int n_heads, int dk, int dv) {
+    mv_pdl_begin();
+    constexpr int DKP = DF_GROUPS * RH;
+    extern __shared__ __align__(16) float smem[];
+    float* qt = smem;                               // [DF_CHUNK][DKP], zero beyond dk
+    float* kt = qt + DF_CHUNK * DKP;
+    float* vt = kt + DF_CHUNK * DKP;                // [DF_CHUNK][DF_COLS]
+    float* pt = vt + DF_CHUNK * DF_COLS;            // [DF_CHUNK][DF_CHUNK]
+    float* et = pt + DF_CHUNK * DF_CHUNK;           // [DKP]
+    float* red = et + DKP;                          // [DF_GROUPS][DF_RED_STRIDE]: [DF_CHUNK][DF_COLS] a group
+    const int tile = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+    const int tid = threadIdx.x, col = tid & 15, grp = tid >> 4;
+    const int j = tile * DF_COLS + col;
+    const int row0 = cu[b], len = cu[b + 1] - row0;
+    if (len <= 0) return;
+    const int slot = mv_read_slot(slots[b]);
+    const int width = n_heads * dk;
+    float* srow = state + (((size_t)slot * n_heads + h) * dv + (j < dv ? j : 0)) * dk;
+    float S[RH];
+#pragma unroll
+    for (int r = 0; r < RH; ++r) {
+        const int i = grp * RH + r;
+        S[r] = (j < dv && i < dk) ? srow[i] : 0.f;
+    }
+    const int n_chunks = (len + DF_CHUNK - 1) / DF_CHUNK;
+    // A chunk's rows are requested into registers while the chunk before is worked on, and go to shared
+    // memory when that one is done: per thread IT values of the decayed q and of the decayed k, 2 of v, 4 of P
+    // and at most one of the chunk's total decay.
+    constexpr int IT = DF_CHUNK * DKP / DF_SCAN_THREADS;
+    static_assert(DF_CHUNK * DF_COLS == DF_SCAN_THREADS && DF_CHUNK * DF_CHUNK % DF_SCAN_THREADS == 0 && DKP <= DF_SCAN_THREADS,
+                  "a thread requests one value of v, whole rounds of P and at most one of the total decay");
+    float rq[IT], rk[IT], rv[DF_CHUNK * DF_COLS / DF_SCAN_THREADS], rp[DF_CHUNK * DF_CHUNK / DF_SCAN_THREADS], re = 0.f;
+    auto request = [&](int c) {
+        const int nt = min(DF_CHUNK, len - c * DF_CHUNK);
+        const int first = row0 + c * DF_CHUNK;
+        const int chunk = row0 / DF_CHUNK + b + c;
+#pragma unroll
+        for (int it = 0; it < IT; ++it) {
+            const int idx = tid + it * DF_SCAN_THREADS, t = idx / DKP, i = idx - t * DKP;
+            const bool in = t < nt && i < dk;
+            const size_t at = in ? (size_t)(first + t) * width + (size_t)h * dk + i : 0;
+            rq[it] = in ? qd[at] : 0.f;
+            rk[it] = in ? kd[at] : 0.f;
+        }
+#pragma unroll
+        for (int it = 0; it < DF_CHUNK * DF_COLS / DF_SCAN_THREADS; ++it) {
+            const int idx = tid + it * DF_SCAN_THREADS, t = idx / DF_COLS, cc = tile * DF_COLS + (idx - t * DF_COLS);
+            const float vv = (t < nt && cc < dv) ? v[(size_t)(first + t) * ldv + (size_t)h * dv + cc] : 0.f;
+            rv[it] = act ? ds_silu(vv) : vv;
+        }
+        const float* Pc = P + ((size_t)chunk * n_heads + h) * DF_CHUNK * DF_CHUNK;
+#pragma unroll
+        for (int it = 0; it < DF_CHUNK * DF_CHUNK / DF_SCAN_THREADS; ++it) rp[it] = Pc[tid + it * DF_SCAN_THREADS];
+        if (tid < DKP) re = tid < dk ? ed[(size_t)chunk * width + (size_t)h * dk + tid] : 0.f;
+    };
+    request(0);
+    for (int c = 0; c < n_chunks; ++c) {
+        const int nt = min(DF_CHUNK, len - c * DF_CHUNK);
+        const int first = row0 + c * DF_CHUNK;
+        __syncthreads();                            // the chunk before is done with shared memory
+#pragma unroll
+        for (int it = 0; it < IT; ++it) {
+            qt[tid + it * DF_SCAN_THREADS] = rq[it];
+            kt[tid + it * DF_SCAN_THREADS] = rk[it];
+        }
+#pragma unroll
+        for (int it = 0; it < DF_CHUNK * DF_COLS / DF_SCAN_THREADS; ++it) vt[tid + it * DF_SCAN_THREADS] = rv[it];
+#pragma unroll
+        for (int it = 0; it < DF_CHUNK * DF_CHUNK / DF_SCAN_THREADS; ++it) pt[tid + it * DF_SCAN_THREADS] = rp[it];
+        if (tid < DKP) et[tid] = re;
+        __syncthreads();
+        if (c + 1 < n_chunks) request(c + 1);
+        // what the chunk's tokens read from the state before the chunk: this half-warp's key channels
+#pragma unroll 4
+        for (int t = 0; t < DF_CHUNK; ++t) {
+            const float4* q4 = reinterpret_cast<const float4*>(qt + t * DKP + grp * RH);
+            float acc = 0.f;
+#pragma unroll
+            for (int r = 0; r < RH; r += 4) {
+                const float4 x = q4[r >> 2];
+                acc = fmaf(x.x, S[r], acc); acc = fmaf(x.y, S[r + 1], acc);
+                acc = fmaf(x.z, S[r + 2], acc); acc = fmaf(x.w, S[r + 3], acc);
+            }
+            red[grp * DF_RED_STRIDE + t * DF_COLS + col] = acc;
+        }
+        // the state after the chunk
+#pragma unroll
+        for (int r = 0; r < RH; ++r) S[r] *= et[grp * RH + r];
+#pragma unroll 4
+        for (int s = 0; s < DF_CHUNK; ++s) {
+            const float vj = vt[s * DF_COLS + col];
+            const float4* k4 = reinterpret_cast<const float4*>(kt + s * DKP + grp * RH);
+#pragma unroll
+            for (int r = 0; r < RH; r += 4) {
+                const float4 x = k4[r >> 2];
+                S[r] = fmaf(x.x, vj, S[r]); S[r + 1] = fmaf(x.y, vj, S[r + 1]);
+                S[r + 2] = fmaf(x.z, vj, S[r + 2]); S[r + 3] = fmaf(x.w, vj, S[r + 3]);
+            }
+        }
+        __syncthreads();
+        // outputs: the groups' shares in a fixed order, then the chunk's own tokens
+        for (int idx = tid; idx < nt * DF_COLS; idx += DF_SCAN_THREADS) {
+            const int t = idx / DF_COLS, cc = idx - t * DF_COLS;
+            float sum = 0.f;
+#pragma unroll
+            for (int g = 0; g < DF_GROUPS; ++g) sum += red[g * DF_RED_STRIDE + t * DF_COLS + cc];
+            for (int s = 0; s <= t; ++s) sum = fmaf(pt[t * DF_CHUNK + s], vt[s * DF_COLS + cc], sum);
+            if (tile * DF_COLS + cc < dv) o[(size_t)(first + t) * n_heads * dv + (size_t)h * dv + tile * DF_COLS + cc] = sum;
+        }
+    }
+    if (j < dv && mv_slot_ok(slots[b])) {
+#pragma unroll
+        for (int r = 0; r < RH; ++r) {
+            const int i = grp * RH + r;
+            if (i < dk) srow[i] = S[r];
+        }
+    }
+}
+
+template <int RH>
+static int decay_few_scan_launch(dim3 grid, cudaStream_t stream, const float* qd, const float* kd, const float* ed,
+                                   const float* P, const float* v, int ldv, int act, float* state, const int* slots,
+                                   const int* cu, float* o, int n_heads, int dk, int dv) {
+    const size_t smem = sizeof(float) * ((size_t)2 * DF_CHUNK * DF_GROUPS * RH + DF_CHUNK * DF_COLS + DF_CHUNK * DF_CHUNK +
+                                         DF_GROUPS * RH + DF_GROUPS * DF_RED_STRIDE);
+    const cudaError_t attr = cudaFuncSetAttribute(decay_few_scan_kernel<RH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (attr != cudaSuccess) return (int)attr;
+    mv_launch(decay_few_scan_kernel<RH>, grid, DF_SCAN_THREADS, smem, stream, qd, kd, ed, P, v, ldv, act, state, slots, cu, o,
+              n_heads, dk, dv);
+    return mv_launch_status();
+}
+
+// Arguments as mv_decay_scan, plus the longest sequence's tokens (max_len) and scratch: qd, kd [N, n_heads * dk],
+// ed [chunks, n_heads * dk], P [chunks, n_heads, DF_CHUNK, DF_CHUNK] with chunks = mv_decay_few_chunks(N, n_seqs).
+MV_API int mv_decay_few_chunks(int N, int n_seqs) { return N / DF_CHUNK + n_seqs + 1; }
+
+MV_API int mv_decay_scan_few(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
+                                 const float* z, int ldz, const float* head_decay, float inv_tau, float q_scale, int act,
+                                 float* state, const int* slots, const int* cu, float* o, float* qd, float* kd, float* ed,
+                                 float* P, int n_seqs, int max_len, int n_heads, int dk, int dv, cudaStream_t stream) {
+    if (n_seqs <= 0 || max_len <= 0) return 0;
+    if (dk < 1 || dk > 256 || dv < 1 || (!z && !head_decay)) return (int)cudaErrorInvalidValue;
+    const size_t smem_a = sizeof(float) * (size_t)3 * DF_CHUNK * (dk + 1);
+    const cudaError_t attr = cudaFuncSetAttribute(decay_few_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)sizeof(float) * 3 * DF_CHUNK * 257);      // what the largest dk needs
+    if (attr != cudaSuccess) return (int)attr;
+    mv_launch(decay_few_prepare_kernel, dim3((max_len + DF_CHUNK - 1) / DF_CHUNK, n_heads, n_seqs), DF_THREADS, smem_a,
+              stream, q, ldq, k, ldk, z, ldz, head_decay, inv_tau, q_scale, act, cu, qd, kd, ed, P, n_heads, dk);
+    int code = mv_launch_status();
+    if (code) return code;
+    const dim3 grid((dv + DF_COLS - 1) / DF_COLS, n_heads, n_seqs);
+    if (dk <= 128) return decay_few_scan_launch<4>(grid, stream, qd, kd, ed, P, v, ldv, act, state, slots, cu, o, n_heads, dk, dv);
+    return decay_few_scan_launch<8>(grid, stream, qd, kd, ed, P, v, ldv, act, state, slots, cu, o, n_heads, dk, dv);
 }

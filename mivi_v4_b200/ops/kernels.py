@@ -75,6 +75,11 @@ _SIGNATURES = {
         "mv_scalar_scan_chunked": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I,
                                    _I, _I, _I, _I, _I, _P],
         "mv_decay_factor_floats": [_I],
+        "mv_decay_few_chunks": [_I, _I],
+        "mv_decay_scan_few": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _F, _F, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I,
+                              _I, _I, _I, _P],
+        "mv_scalar_scan_few": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _I, _I,
+                               _I, _I, _I, _I, _I, _P],
         "mv_memory_gates": [_P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _I, _P],
         "mv_causal_conv": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
         "mv_ssm_decode_prepare": [_P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _P, _I, _P, _P, _P, _P, _I, _P],
@@ -328,7 +333,7 @@ def _need(t: Optional[torch.Tensor], name: str, dtype=None, shape=None, optional
 
 _launches = 0
 # kernels launched by one call of each entry point
-_KERNELS_PER_CALL = {"mv_shortconv": 2, "mv_decay_scan_chunked": 3, "mv_causal_conv": 2, "mv_scalar_scan_chunked": 4}
+_KERNELS_PER_CALL = {"mv_shortconv": 2, "mv_decay_scan_chunked": 3, "mv_causal_conv": 2, "mv_scalar_scan_chunked": 4, "mv_decay_scan_few": 2, "mv_scalar_scan_few": 2}
 
 
 def launch_count() -> int:
@@ -664,6 +669,22 @@ def scalar_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_a: torch.
     norm = m_tok is not None
     _need(state, "scalar_scan state", torch.float32, (None, n_heads, dv + (1 if norm else 0), dk))
     _guard("core", "scalar_scan", out.device, n_slots=state.shape[0])
+    if ws is not None and max_len >= SCAN_CHUNKED_FROM and N < SCALAR_CHUNKS_FROM:
+        chunks = int(_fn("core", "mv_scalar_chunks")(N, int(n_seqs)))
+        G = ws.get("scalar_scan_products", (chunks, groups, SCAN_CHUNK, SCAN_CHUNK), torch.float32)
+        o_aug = ws.get("scalar_scan_o_aug", (N, n_heads * (dv + 1)), torch.float32) if norm else None
+        _check(_fn("core", "mv_scalar_scan_few")(
+            qp, ldq, kp, ldk, vp, ldv, ap, lda, bp, ldb, _need(skip, "scalar_scan skip", torch.float32, (n_heads,), True),
+            _need(m_tok, "scalar_scan m", torch.float32, (N, n_heads), True), float(q_scale), state.data_ptr(),
+            _need(slots, "slots", torch.int32), _need(cu, "cu", torch.int32),
+            _need(out, "scalar_scan out", torch.float32, (N, n_heads * dv)), G.data_ptr(),
+            o_aug.data_ptr() if norm else None, N, int(n_seqs), int(max_len), n_heads, int(heads_per_group), dk, dv,
+            int(norm), _stream()), "mv_scalar_scan_few")
+        add_launches(1 if norm else 0)
+        account(N * n_heads * (2 * dk // heads_per_group + 2 * dv) * 4 + 2 * n_seqs * n_heads * dk * dv * 4
+                + 2 * chunks * groups * SCAN_CHUNK * SCAN_CHUNK * 4,
+                4 * N * n_heads * dk * dv + N * n_heads * SCAN_CHUNK * dv + N * groups * SCAN_CHUNK * dk)
+        return out
     if ws is not None and max_len >= SCAN_CHUNKED_FROM:
         chunks = int(_fn("core", "mv_scalar_chunks")(N, int(n_seqs)))
         G = ws.get("scalar_scan_products", (chunks, groups, SCAN_CHUNK, SCAN_CHUNK), torch.float32)
@@ -971,8 +992,12 @@ def expert_combine(ys: torch.Tensor, place: torch.Tensor, pick_w: Optional[torch
 MAX_SCAN_KEY_DIM = 256
 SCAN_ACT_NONE, SCAN_ACT_SILU = 0, 1
 SCAN_CHUNKED_FROM = 16          # a step whose longest sequence brings this many tokens walks them in chunks
-SCAN_CHUNK = 32                 # of scalar_scan
+SCAN_CHUNK = 32                 # of scalar_scan, and of decay_scan's steps of few tokens
 DECAY_CHUNK = 64                # of decay_scan
+# Chunked steps of fewer tokens in all are bound by launches and take kernels that do more in each (the figures where both are equal
+# stand beside those kernels in decay_scan.cu and scalar_scan.cu)
+DECAY_CHUNKS_FROM = 400
+SCALAR_CHUNKS_FROM = 128
 
 
 def _cols(t: torch.Tensor, name: str, n_rows: int, width: int):
@@ -996,8 +1021,8 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
     float32 and may be column slices of one wider matrix; ``act`` is applied to all three as they are read
     and ``q_scale`` multiplies q.  Everything is computed in float32.  ``max_len``: the most tokens that a
     sequence brings; with ``ws`` (a Workspace, for scratch) steps of ``SCAN_CHUNKED_FROM`` tokens a sequence and
-    more take the kernels that work in chunks of 64 tokens, whose sums come in another order (the
-    results differ from the token-by-token kernel's by rounding)."""
+    more take kernels that work in chunks of 32 or, from ``DECAY_CHUNKS_FROM`` tokens in the step on, of 64 tokens, whose sums
+    come in another order (the results differ from the token-by-token kernel's, and from each other, by rounding)."""
     N = out.shape[0]
     if not 1 <= dk <= MAX_SCAN_KEY_DIM:
         raise KernelError(f"decay_scan: key size {dk} is outside 1..{MAX_SCAN_KEY_DIM}")
@@ -1009,6 +1034,20 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
     zp, ldz = _cols(decay_logits, "decay_scan decay logits", N, n_heads * dk) if decay_logits is not None else (None, 0)
     _need(state, "decay_scan state", torch.float32, (None, n_heads, dv, dk))
     _guard("core", "decay_scan", out.device, n_slots=state.shape[0])
+    if ws is not None and max_len >= SCAN_CHUNKED_FROM and N < DECAY_CHUNKS_FROM:
+        chunks = int(_fn("core", "mv_decay_few_chunks")(N, int(n_seqs)))
+        qd = ws.get("scan_qd", (N, n_heads * dk), torch.float32)
+        kd = ws.get("scan_kd", (N, n_heads * dk), torch.float32)
+        ed = ws.get("scan_ed", (chunks, n_heads * dk), torch.float32)
+        pm = ws.get("scan_p", (chunks, n_heads, SCAN_CHUNK, SCAN_CHUNK), torch.float32)
+        _check(_fn("core", "mv_decay_scan_few")(
+            qp, ldq, kp, ldk, vp, ldv, zp, ldz, _need(head_decay, "head decay", torch.float32, (n_heads,), True),
+            float(inv_tau), float(q_scale), int(act), state.data_ptr(), _need(slots, "slots", torch.int32),
+            _need(cu, "cu", torch.int32), _need(out, "decay_scan out", torch.float32, (N, n_heads * dv)),
+            qd.data_ptr(), kd.data_ptr(), ed.data_ptr(), pm.data_ptr(), int(n_seqs), int(max_len), n_heads, dk, dv,
+            _stream()), "mv_decay_scan_few")
+        account(N * n_heads * (6 * dk + 2 * dv) * 4 + 2 * n_seqs * n_heads * dk * dv * 4, 5 * N * n_heads * dk * dv)
+        return out
     if ws is not None and max_len >= SCAN_CHUNKED_FROM:
         chunks = int(_fn("core", "mv_decay_chunks")(N, int(n_seqs)))
         by_channel = decay_logits is not None

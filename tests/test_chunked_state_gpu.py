@@ -12,6 +12,14 @@ DEV = "cuda:0"
 F64 = torch.float64
 
 
+@pytest.fixture(autouse=True, params=["few", "many"])
+def kernels_for(request, monkeypatch):
+    """Every case with the kernels for steps of few tokens and with those for many, whatever the step's size would choose."""
+    from mivi_v4_b200.ops import kernels as K
+    monkeypatch.setattr(K, "DECAY_CHUNKS_FROM", 0 if request.param == "many" else 1 << 30)
+    return request.param
+
+
 class Scratch:
     def get(self, name, shape, dtype):
         return torch.full(tuple(shape), float("nan"), dtype=dtype, device=DEV)
@@ -85,11 +93,14 @@ def test_a_later_token_that_is_not_finite():
 
 @pytest.mark.parametrize("tokens", [33, 64, 100])
 @pytest.mark.parametrize("shift,inv_tau", [(6.0, 1 / 16), (3.0, 1 / 8), (0.0, 1.0), (-2.0, 1.0)])
-def test_decay_near_one(tokens, shift, inv_tau):
+def test_decay_near_one(kernels_for, tokens, shift, inv_tau):
     """Decays near 1 lose nothing by being multiplied up over a chunk.  Of an output's 2-norm: a product of up to 63 factors is rounded
     63 times (uniform in half a place either way, 0.29 * 2^-23 of a number halfway between two powers of two, so 2^-23 * 0.29 / 1.4 *
     sqrt(63) = 2.0e-7 for the oldest token of a chunk, 1.4e-7 over all), the sum over the key channels averages that down, and the
-    sums' own rounding is 1.2e-7 (seen where there are few tokens): below 2.2e-7 together."""
+    sums' own rounding is 1.2e-7 (seen where there are few tokens): below 2.2e-7 together.  The kernels for few tokens multiply
+    nothing up."""
+    if kernels_for == "few":
+        pytest.skip("no products of decays")
     from mivi_v4_b200.ops import kernels as K
     heads, dk, dv = 4, 128, 128
     g = torch.Generator().manual_seed(tokens)
@@ -105,3 +116,14 @@ def test_decay_near_one(tokens, shift, inv_tau):
     K.decay_scan(q.to(DEV), k.to(DEV), v.to(DEV), state.to(DEV), i32([0]), i32([0, tokens]), out, 1, heads, dk, dv, q_scale=0.5,
                  decay_logits=z.to(DEV), inv_tau=inv_tau, max_len=tokens, ws=Scratch())
     assert (out.double().cpu() - want).norm() / want.norm() <= 2.2e-7
+
+
+@pytest.mark.parametrize("tokens,few", [(16, True), (399, True), (400, False)])
+def test_which_kernels(monkeypatch, tokens, few):
+    """A step's tokens in all choose: below DECAY_CHUNKS_FROM the two launches that suit a short prompt."""
+    from mivi_v4_b200.ops import kernels as K
+    monkeypatch.undo()
+    x, before = torch.randn(tokens, 32, device=DEV), K.launch_count()
+    K.decay_scan(x, x, x, torch.zeros(1, 1, 32, 32, device=DEV), i32([0]), i32([0, tokens]), torch.empty_like(x), 1, 1, 32, 32,
+                 decay_logits=x, max_len=tokens, ws=Scratch())
+    assert K.launch_count() - before == (2 if few else 3)

@@ -36,8 +36,10 @@ def close(got, want, tol, what):
 @pytest.mark.parametrize("heads,group,dk,dv,pad", [(1, 1, 128, 64, 0), (2, 2, 33, 65, 0), (3, 1, 4, 7, 1), (6, 3, 64, 64, 3), (2, 1, 200, 66, 0)])
 @pytest.mark.parametrize("lens", [[32], [16, 1, 33], [95, 64]])
 @pytest.mark.parametrize("normalizer", [False, True])
-def test_scalar_scan(heads, group, dk, dv, pad, lens, normalizer):
+@pytest.mark.parametrize("chunks_from", [0, 1 << 30])        # the kernels for many tokens, and those for few
+def test_scalar_scan(monkeypatch, heads, group, dk, dv, pad, lens, normalizer, chunks_from):
     from mivi_v4_b200.ops import kernels as K
+    monkeypatch.setattr(K, "SCALAR_CHUNKS_FROM", chunks_from)
     g = torch.Generator().manual_seed(heads * 1000 + dk + sum(lens))
     N, groups, B, cu = sum(lens), heads // group, len(lens), starts_of(lens)
     q, k = (torch.randn(N, groups * dk, generator=g) for _ in "qk")
@@ -104,3 +106,31 @@ def test_delta_scan(heads, kv, dk, dv, lens, head_decay):
     close(out, want_o, 4e-6, "outputs")
     close(got, want_s, 4e-6, "state")
     assert torch.equal(got[0].cpu(), state[0])
+
+
+def test_scalar_scan_few_and_many_agree(monkeypatch):
+    """Which kernels a step takes depends on its tokens; the bits do not."""
+    from mivi_v4_b200.ops import kernels as K
+    g = torch.Generator(device=DEV).manual_seed(5)
+    for heads, group, dk, dv, norm, lens in ((4, 4, 128, 64, 0, [127]), (2, 1, 128, 66, 1, [50, 33]), (2, 1, 200, 40, 1, [64, 1, 40])):
+        N, B = sum(lens), len(lens)
+        r = lambda *s: torch.randn(*s, generator=g, device=DEV)
+        q, k, v, m = r(N, heads // group * dk), r(N, heads // group * dk), r(N, heads * dv), r(N, heads)
+        log_a, b, state = -r(N, heads).abs(), r(N, heads).abs(), r(B, heads, dv + norm, dk)
+        got = []
+        for chunks_from in (0, 1 << 30):
+            monkeypatch.setattr(K, "SCALAR_CHUNKS_FROM", chunks_from)
+            s, out = state.clone(), torch.full((N, heads * dv), float("nan"), device=DEV)
+            K.scalar_scan(q, k, v, log_a, b, s, i32(list(range(B))), i32(starts_of(lens)), out, B, heads, dk, dv, heads_per_group=group,
+                          m_tok=m if norm else None, q_scale=0.1, max_len=max(lens), ws=Scratch())
+            got.append((out, s))
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("tokens,few", [(16, True), (127, True), (128, False)])
+def test_which_kernels(tokens, few):
+    from mivi_v4_b200.ops import kernels as K
+    x, ones, before = torch.randn(tokens, 32, device=DEV), torch.ones(tokens, 1, device=DEV), K.launch_count()
+    K.scalar_scan(x, x, x, -ones, ones, torch.zeros(1, 1, 32, 32, device=DEV), i32([0]), i32([0, tokens]), torch.empty_like(x), 1, 1, 32, 32,
+                  max_len=tokens, ws=Scratch())
+    assert K.launch_count() - before == (2 if few else 4)
