@@ -12,7 +12,11 @@
 // cores: both are bound by the multiply-adds and the shared-memory loads that feed them.
 //
 // Chunks are numbered floor(cu[b] / CS_CHUNK) + b + c for chunk c of the step's sequence b: distinct numbers below
-// N / CS_CHUNK + n_seqs + 1 that need nothing from the host.
+// N / CS_CHUNK + n_seqs + 1, ascending, that need nothing from the host.
+//
+// The states before all chunks would be as large as the step is long (2 MB for every 32 tokens of 64 heads of 128 x 64), so walk and outputs go
+// over the numbers in windows of as many chunks as the caller has room for.  At a window's end at most one sequence is cut: its state
+// goes into one of two places behind the window's (in turn: the next window reads it while another sequence's may be left).
 #pragma once
 #include "common.cuh"
 
@@ -28,10 +32,11 @@ struct CsArgs {
     const float *w, *d;                 // by head: w_s [chunk][head][CS_CHUNK] and d [chunk][head]
     const float* P;                     // by head: q . k [chunk][head][CS_CHUNK][CS_CHUNK]; by channel: P [chunk][head][..][..]
     float q_scale;
-    float *state, *before;              // [slot][head][dv][dk]; [chunk][head][dv][lds]: the state before every chunk
+    float *state, *before;              // [slot][head][dv][dk]; [chunk - w0][head][dv][lds]: the state before every chunk
     const int *slots, *cu;
     float* o;                           // [N, n_heads * dv]
     int n_heads, dk, dv, lds, wide;
+    int w0, w1, room;                   // this window's chunk numbers; the chunks that `before` holds (and, with more than one window, two states)
 };
 
 namespace {
@@ -41,6 +46,13 @@ __device__ __forceinline__ void cs_copy(float* to, const float* from, bool in, b
     if (wide) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(from), "r"(in ? 16 : 0) : "memory");
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(s), "l"(from), "r"(in ? 4 : 0) : "memory");
 }
+// The chunks of a sequence that lie in the window: from .first up to .second.
+__device__ __forceinline__ int2 cs_window(int chunk0, int n_chunks, int w0, int w1) {
+    return make_int2(max(0, w0 - chunk0), min(n_chunks, w1 - chunk0));
+}
+// Where a sequence that a window's end cuts leaves its state: behind the window's chunks.
+__device__ __forceinline__ int cs_carry(int w1, int room) { return room + (w1 / room & 1); }
+
 __device__ __forceinline__ void cs_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cs_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
@@ -122,7 +134,9 @@ cs_walk_kernel(const CsArgs a) {
     const int tiles_i = (a.dk + 63) / 64, i0 = (blockIdx.x % tiles_i) * 64, j0 = (blockIdx.x / tiles_i) * JT;
     const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, grp = tid / CS_THREADS, lt = tid % CS_THREADS, ti = lt & 15, tj = lt >> 4;
     const int row0 = a.cu[b], len = a.cu[b + 1] - row0;
-    if (len <= 0) return;
+    const int n_sub = (len + SUB - 1) / SUB, chunk0 = row0 / CS_CHUNK + b;
+    const int2 win = cs_window(chunk0, n_sub, a.w0, a.w1);
+    if (win.x >= win.y) return;
     const int slot = mv_read_slot(a.slots[b]);
     const int i = i0 + ti * 4, j = j0 + tj * TJ;
     float* st = a.state + ((size_t)slot * a.n_heads + h) * a.dv * a.dk;
@@ -141,17 +155,17 @@ cs_walk_kernel(const CsArgs a) {
     };
 #pragma unroll
     for (int y = 0; y < TJ; ++y) {
-        if (grp == 0 && j + y < a.dv) read4(st + (size_t)(j + y) * a.dk, S[y]);
+        if (grp == 0 && j + y < a.dv)
+            read4(win.x ? a.before + (((size_t)cs_carry(a.w0, a.room) * a.n_heads + h) * a.dv + j + y) * a.lds : st + (size_t)(j + y) * a.dk, S[y]);
         else
 #pragma unroll
             for (int x = 0; x < 4; ++x) S[y][x] = 0.f;
     }
     const float* kp = a.k + (size_t)row0 * a.ldk + (size_t)h * a.dk + i0;
     const float* vp = a.v + (size_t)row0 * a.ldv + (size_t)h * a.dv + j0;
-    const int n_sub = (len + SUB - 1) / SUB, chunk0 = row0 / CS_CHUNK + b;
     auto load = [&](int sub) {
         const size_t t = (size_t)sub * SUB;
-        if (sub < n_sub) {
+        if (sub < win.y) {
             const int st = sub % STAGES;
             cs_load<SUB, 64, 64, false, THREADS>(ks + st * SUB * 64, kp + t * a.ldk, a.ldk, len - (int)t, a.dk - i0, a.wide);
             cs_load<SUB, JT, JT, false, THREADS>(vs + st * SUB * JT, vp + t * a.ldv, a.ldv, len - (int)t, a.dv - j0, a.wide);
@@ -161,7 +175,7 @@ cs_walk_kernel(const CsArgs a) {
         cs_commit();
     };
 #pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) load(s);
+    for (int s = 0; s < STAGES - 1; ++s) load(win.x + s);
     float d_next[4];                                    // the chunk's decay, requested a chunk ahead
     auto decay = [&](int c) {
 #pragma unroll
@@ -169,7 +183,7 @@ cs_walk_kernel(const CsArgs a) {
             d_next[x] = CHANNEL ? (i + x < a.dk ? a.ed[(size_t)(chunk0 + c) * a.n_heads * a.dk + (size_t)h * a.dk + i + x] : 0.f)
                                 : a.d[(size_t)(chunk0 + c) * a.n_heads + h];
     };
-    decay(0);
+    decay(win.x);
     // the other groups' sums go into the first group's
     auto join = [&]() {
         if (grp > 0) {
@@ -193,23 +207,25 @@ cs_walk_kernel(const CsArgs a) {
             }
         }
     };
-    for (int sub = 0; sub < n_sub; ++sub) {
+    auto leave = [&](int place) {
+        float* to = a.before + ((size_t)place * a.n_heads + h) * a.dv * a.lds;
+        if (grp == 0 && i < a.lds) {
+#pragma unroll
+            for (int y = 0; y < TJ; ++y)
+                if (j + y < a.dv)
+                    *reinterpret_cast<float4*>(to + (size_t)(j + y) * a.lds + i) = make_float4(S[y][0], S[y][1], S[y][2], S[y][3]);
+        }
+    };
+    for (int sub = win.x; sub < win.y; ++sub) {
         {
             const int c = sub;
-            if (GROUPS > 1 && c > 0) join();
-            // the state as it is before this chunk
-            float* to = a.before + ((size_t)(chunk0 + c) * a.n_heads + h) * a.dv * a.lds;
-            if (grp == 0 && i < a.lds) {
-#pragma unroll
-                for (int y = 0; y < TJ; ++y)
-                    if (j + y < a.dv)
-                        *reinterpret_cast<float4*>(to + (size_t)(j + y) * a.lds + i) = make_float4(S[y][0], S[y][1], S[y][2], S[y][3]);
-            }
+            if (GROUPS > 1 && c > win.x) join();
+            leave(chunk0 + c - a.w0);                   // the state as it is before this chunk
 #pragma unroll
             for (int x = 0; x < 4; ++x)
 #pragma unroll
                 for (int y = 0; y < TJ; ++y) S[y][x] *= d_next[x];
-            if ((c + 1) * CS_CHUNK < len) decay(c + 1);
+            if (c + 1 < win.y) decay(c + 1);
         }
         cs_wait<STAGES - 2>();
         __syncthreads();                                // these tokens are there, the ones before are done with
@@ -246,7 +262,8 @@ cs_walk_kernel(const CsArgs a) {
         }
     }
     if (GROUPS > 1) join();
-    if (grp == 0 && mv_slot_ok(a.slots[b])) {
+    if (win.y < n_sub) leave(cs_carry(a.w1, a.room));
+    else if (grp == 0 && mv_slot_ok(a.slots[b])) {
         auto write4 = [&](float* p, const float* from) {
             if (vec && i < a.dk) *reinterpret_cast<float4*>(p + i) = make_float4(from[0], from[1], from[2], from[3]);
             else
@@ -276,13 +293,15 @@ cs_output_kernel(const CsArgs a) {
     float* vs = co_smem + 2 * STAGE;                    // [64][64]
     double* cs = reinterpret_cast<double*>(vs + CS_CHUNK * 64);     // [64] running sums of the log decays
     mv_pdl_begin();
-    const int tiles_j = (a.dv + 63) / 64, c = blockIdx.x / tiles_j, j0 = (blockIdx.x % tiles_j) * 64;
+    const int tiles_j = (a.dv + 63) / 64, j0 = (blockIdx.x % tiles_j) * 64;
     const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, tj = tid & 15, tt = tid >> 4;
-    const int row0 = a.cu[b], len = a.cu[b + 1] - row0;
-    if (c * CS_CHUNK >= len) return;
-    const int nt = min(CS_CHUNK, len - c * CS_CHUNK), chunk = row0 / CS_CHUNK + b + c;
+    const int row0 = a.cu[b], len = a.cu[b + 1] - row0, chunk0 = row0 / CS_CHUNK + b;
+    const int2 win = cs_window(chunk0, (len + CS_CHUNK - 1) / CS_CHUNK, a.w0, a.w1);
+    const int c = win.x + blockIdx.x / tiles_j, chunk = chunk0 + c;
+    if (c >= win.y) return;
+    const int nt = min(CS_CHUNK, len - c * CS_CHUNK);
     const size_t first = (size_t)row0 + c * CS_CHUNK;
-    const float* S0 = a.before + ((size_t)chunk * a.n_heads + h) * a.dv * a.lds;
+    const float* S0 = a.before + ((size_t)(chunk - a.w0) * a.n_heads + h) * a.dv * a.lds;
     const float* qp = a.q + first * a.ldq + (size_t)h * a.dk;
     const int slices = (a.dk + 31) / 32;
     auto load = [&](int s) {
@@ -468,6 +487,7 @@ inline int cs_factor_floats(int n_heads) { return n_heads * (3 * CS_CHUNK + 1); 
 
 template <bool CHANNEL>
 int cs_launch(CsArgs a, float* G, float* factors, int chunks, int n_seqs, int max_len, cudaStream_t stream) {
+    if (a.room < 1) return (int)cudaErrorInvalidValue;
     a.lds = (a.dk + 3) & ~3;
     a.wide = cs_aligned(a.q, a.ldq, a.dk) && cs_aligned(a.k, a.ldk, a.dk) && cs_aligned(a.v, a.ldv, a.dv);
     if (!CHANNEL) {
@@ -486,16 +506,21 @@ int cs_launch(CsArgs a, float* G, float* factors, int chunks, int n_seqs, int ma
     }
     const int tiles_i = (a.dk + 63) / 64;
     const long tiles = (long)((a.dv + 63) / 64) * tiles_i * a.n_heads * n_seqs;
-    int code;
-    if (tiles > 148) code = cs_walk_launch<8, 2, CHANNEL>(a, (a.dv + 63) / 64 * tiles_i, n_seqs, stream);
-    else if (tiles > 74) code = cs_walk_launch<8, 4, CHANNEL>(a, (a.dv + 63) / 64 * tiles_i, n_seqs, stream);
-    else code = cs_walk_launch<4, 4, CHANNEL>(a, (a.dv + 31) / 32 * tiles_i, n_seqs, stream);
-    if (code) return code;
     static const cudaError_t attr = cudaFuncSetAttribute(cs_output_kernel<CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CO_SMEM);
     if (attr != cudaSuccess) return (int)attr;
-    mv_launch(cs_output_kernel<CHANNEL>, dim3((max_len + CS_CHUNK - 1) / CS_CHUNK * ((a.dv + 63) / 64), a.n_heads, n_seqs), CS_THREADS,
-              CO_SMEM, stream, a);
-    return mv_launch_status();
+    const int per_seq = min((max_len + CS_CHUNK - 1) / CS_CHUNK, a.room);       // the most chunks a sequence has in a window
+    for (a.w0 = 0; a.w0 < chunks; a.w0 += a.room) {
+        a.w1 = a.w0 + a.room;
+        int code;
+        if (tiles > 148) code = cs_walk_launch<8, 2, CHANNEL>(a, (a.dv + 63) / 64 * tiles_i, n_seqs, stream);
+        else if (tiles > 74) code = cs_walk_launch<8, 4, CHANNEL>(a, (a.dv + 63) / 64 * tiles_i, n_seqs, stream);
+        else code = cs_walk_launch<4, 4, CHANNEL>(a, (a.dv + 31) / 32 * tiles_i, n_seqs, stream);
+        if (code) return code;
+        mv_launch(cs_output_kernel<CHANNEL>, dim3(per_seq * ((a.dv + 63) / 64), a.n_heads, n_seqs), CS_THREADS, CO_SMEM, stream, a);
+        code = mv_launch_status();
+        if (code) return code;
+    }
+    return 0;
 }
 
 }  // namespace

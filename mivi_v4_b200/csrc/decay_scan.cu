@@ -322,12 +322,12 @@ MV_API int mv_decay_factor_floats(int n_heads) { return cs_factor_floats(n_heads
 
 // Arguments as mv_decay_scan, plus the step's tokens N, the longest sequence's (max_len) and scratch with chunks =
 // mv_decay_chunks(N, n_seqs): copies [N, n_heads * (2 dk + dv)] (with act), qd, kd [N, n_heads * dk] and ed
-// [chunks, n_heads * dk] (with z), P [chunks, n_heads, CS_CHUNK, CS_CHUNK], before [chunks, n_heads, dv, dk rounded up to 4],
-// factors [chunks, mv_decay_factor_floats(n_heads)] (without z).
+// [chunks, n_heads * dk] (with z), P [chunks, n_heads, CS_CHUNK, CS_CHUNK], before [room (+ 2 where room < chunks), n_heads, dv, dk rounded up to 4]
+// for windows of `room` chunks, factors [chunks, mv_decay_factor_floats(n_heads)] (without z).
 MV_API int mv_decay_scan_chunked(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
                                  const float* z, int ldz, const float* head_decay, float inv_tau, float q_scale, int act,
                                  float* state, const int* slots, const int* cu, float* o, float* copies, float* qd, float* kd,
-                                 float* ed, float* P, float* before, float* factors, int chunks, int N, int n_seqs, int max_len, int n_heads, int dk, int dv,
+                                 float* ed, float* P, float* before, float* factors, int room, int chunks, int N, int n_seqs, int max_len, int n_heads, int dk, int dv,
                                  cudaStream_t stream) {
     if (n_seqs <= 0 || max_len <= 0) return 0;
     if (dk < 1 || dk > 256 || dv < 1 || (!z && !head_decay) || (act && !copies) || (!z && !factors)) return (int)cudaErrorInvalidValue;
@@ -336,7 +336,7 @@ MV_API int mv_decay_scan_chunked(const float* q, int ldq, const float* k, int ld
     a.q = q; a.ldq = ldq; a.k = k; a.ldk = ldk; a.v = v; a.ldv = ldv;
     a.q_scale = q_scale; a.head_decay = head_decay;
     a.state = state; a.before = before; a.slots = slots; a.cu = cu; a.o = o;
-    a.n_heads = n_heads; a.dk = dk; a.dv = dv;
+    a.n_heads = n_heads; a.dk = dk; a.dv = dv; a.room = room;
     if (act) {
         float *qa = copies, *ka = qa + (size_t)N * wk, *va = ka + (size_t)N * wk;
         mv_launch(decay_activate_kernel, dim3(N, 3), 256, 0, stream, q, ldq, k, ldk, v, ldv, qa, ka, va, wk, wv);
@@ -361,7 +361,7 @@ MV_API int mv_decay_scan_chunked(const float* q, int ldq, const float* k, int ld
 // The first kernel prepares, per (sequence, head, chunk), the decayed q and k, the chunk's total decay and P; the second walks a
 // sequence's chunks with the state in registers and works the outputs out on the way.  Such a step is bound by its launches and by
 // a handful of chunks one after the other: one sequence of 16 tokens 41 us (8 heads of 128 x 256, a decay a channel) and 35 (16 heads
-// of 128 x 128, one a head, with the activation) against 57 and 58 with the three to five kernels below; 256 tokens 74 and 67 against 84 and
+// of 128 x 128, one a head, with the activation) against 57 and 58 with the three to five kernels above; 256 tokens 74 and 67 against 84 and
 // 74; four sequences of 96 84 and 81 against 86 and 87, of 128 96 and 93 against 86 and 80.
 //
 // Chunks are numbered floor(cu[b] / DF_CHUNK) + b + c for chunk c of the step's sequence b: distinct

@@ -242,12 +242,13 @@ struct ScArgs {
     const float *log_a, *b, *skip, *m_tok;
     int ld_a, ld_b;
     float q_scale;
-    float *state, *before;              // [slot][head][cols][dk]; [chunk][head][cols][lds]: the state before every chunk
+    float *state, *before;              // [slot][head][cols][dk]; [chunk - w0][head][cols][lds]: the state before every chunk
     float *G;                           // q_t . k_s [chunk][group][SC_CHUNK][SC_CHUNK]
     float *run, *e1, *e2, *el;          // [chunk][head][SC_CHUNK]: running log decay, e^(c_t) q_scale, e^(c_last - c_t) b_t; [chunk][head]: e^(c_last)
     const int *slots, *cu;
     float* o;
     int n_heads, heads_per_group, dk, dv, lds, wide, normalizer;
+    int w0, w1, room;                   // as in CsArgs
 };
 
 namespace {
@@ -341,12 +342,15 @@ ss_walk_kernel(const ScArgs a) {
     const int tiles_i = (a.dk + 63) / 64, i0 = (blockIdx.x % tiles_i) * 64, j0 = (blockIdx.x / tiles_i) * 64;
     const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, ti = tid & 15, tj = tid >> 4;
     const int row0 = a.cu[b], len = a.cu[b + 1] - row0;
-    if (len <= 0) return;
+    const int n_chunks = (len + SC_CHUNK - 1) / SC_CHUNK, chunk0 = row0 / SC_CHUNK + b;
+    const int2 win = cs_window(chunk0, n_chunks, a.w0, a.w1);       // (as in chunked_state.cuh)
+    if (win.x >= win.y) return;
     const int cols = a.dv + a.normalizer, slot = mv_read_slot(a.slots[b]);
     const bool with_n = a.normalizer && j0 == 0;
     const int i = i0 + ti * 4, j = j0 + tj * 4;
     float* st = a.state + ((size_t)slot * a.n_heads + h) * cols * a.dk;
     const bool vec = a.dk % 4 == 0;                     // the state's rows start on 16 bytes
+    const float* carried = a.before + ((size_t)cs_carry(a.w0, a.room) * a.n_heads + h) * cols * a.lds;
     float S[4][4], n[4];
     auto read4 = [&](const float* p, float* out) {
         float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -361,16 +365,15 @@ ss_walk_kernel(const ScArgs a) {
     };
 #pragma unroll
     for (int y = 0; y < 4; ++y) {
-        if (j + y < a.dv) read4(st + (size_t)(j + y) * a.dk, S[y]);
+        if (j + y < a.dv) read4(win.x ? carried + (size_t)(j + y) * a.lds : st + (size_t)(j + y) * a.dk, S[y]);
         else S[y][0] = S[y][1] = S[y][2] = S[y][3] = 0.f;
     }
     n[0] = n[1] = n[2] = n[3] = 0.f;
-    if (with_n) read4(st + (size_t)a.dv * a.dk, n);
+    if (with_n) read4(win.x ? carried + (size_t)a.dv * a.lds : st + (size_t)a.dv * a.dk, n);
     const float* kp = a.k + (size_t)row0 * a.ldk + (size_t)(h / a.heads_per_group) * a.dk + i0;
     const float* vp = a.v + (size_t)row0 * a.ldv + (size_t)h * a.dv + j0;
-    const int n_chunks = (len + SC_CHUNK - 1) / SC_CHUNK, chunk0 = row0 / SC_CHUNK + b;
     auto load = [&](int c) {
-        if (c < n_chunks) {
+        if (c < win.y) {
             const int st_ = c % SW_STAGES;
             const size_t t = (size_t)c * SC_CHUNK;
             cs_load<SC_CHUNK, 64, 64, false, SC_WALK_THREADS>(ks + st_ * SC_CHUNK * 64, kp + t * a.ldk, a.ldk, len - (int)t, a.dk - i0, a.wide);
@@ -381,11 +384,10 @@ ss_walk_kernel(const ScArgs a) {
         cs_commit();
     };
 #pragma unroll
-    for (int c = 0; c < SW_STAGES - 1; ++c) load(c);
-    float d_next = a.el[(size_t)chunk0 * a.n_heads + h];        // the chunk's decay, requested a chunk ahead
-    for (int c = 0; c < n_chunks; ++c) {
-        // the state as it is before this chunk
-        float* to = a.before + ((size_t)(chunk0 + c) * a.n_heads + h) * cols * a.lds;
+    for (int c = 0; c < SW_STAGES - 1; ++c) load(win.x + c);
+    float d_next = a.el[(size_t)(chunk0 + win.x) * a.n_heads + h];        // the chunk's decay, requested a chunk ahead
+    auto leave = [&](int place) {
+        float* to = a.before + ((size_t)place * a.n_heads + h) * cols * a.lds;
         if (i < a.lds) {
 #pragma unroll
             for (int y = 0; y < 4; ++y)
@@ -393,13 +395,16 @@ ss_walk_kernel(const ScArgs a) {
                     *reinterpret_cast<float4*>(to + (size_t)(j + y) * a.lds + i) = make_float4(S[y][0], S[y][1], S[y][2], S[y][3]);
             if (with_n && tj == 0) *reinterpret_cast<float4*>(to + (size_t)a.dv * a.lds + i) = make_float4(n[0], n[1], n[2], n[3]);
         }
+    };
+    for (int c = win.x; c < win.y; ++c) {
+        leave(chunk0 + c - a.w0);                       // the state as it is before this chunk
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
 #pragma unroll
             for (int y = 0; y < 4; ++y) S[y][x] *= d_next;
             n[x] *= d_next;
         }
-        if (c + 1 < n_chunks) d_next = a.el[(size_t)(chunk0 + c + 1) * a.n_heads + h];
+        if (c + 1 < win.y) d_next = a.el[(size_t)(chunk0 + c + 1) * a.n_heads + h];
         cs_wait<SW_STAGES - 2>();
         __syncthreads();                                // this chunk's rows are there, the ones before are done with
         load(c + SW_STAGES - 1);
@@ -443,7 +448,8 @@ ss_walk_kernel(const ScArgs a) {
             }
         }
     }
-    if (mv_slot_ok(a.slots[b])) {
+    if (win.y < n_chunks) leave(cs_carry(a.w1, a.room));
+    else if (mv_slot_ok(a.slots[b])) {
         auto write4 = [&](float* p, const float* from) {
             if (vec && i < a.dk) *reinterpret_cast<float4*>(p + i) = make_float4(from[0], from[1], from[2], from[3]);
             else
@@ -472,14 +478,16 @@ ss_output_kernel(const ScArgs a) {
     float* e1 = vs + SC_CHUNK * 64;                     // [32]
     float* dn = e1 + SC_CHUNK;                          // [32] denominators
     mv_pdl_begin();
-    const int tiles_j = (a.dv + 63) / 64, c = blockIdx.x / tiles_j, j0 = (blockIdx.x % tiles_j) * 64;
+    const int tiles_j = (a.dv + 63) / 64, j0 = (blockIdx.x % tiles_j) * 64;
     const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, tj = tid & 15, tt = tid >> 4;
-    const int row0 = a.cu[b], len = a.cu[b + 1] - row0;
-    if (c * SC_CHUNK >= len) return;
-    const int nt = min(SC_CHUNK, len - c * SC_CHUNK), chunk = row0 / SC_CHUNK + b + c;
+    const int row0 = a.cu[b], len = a.cu[b + 1] - row0, chunk0 = row0 / SC_CHUNK + b;
+    const int2 win = cs_window(chunk0, (len + SC_CHUNK - 1) / SC_CHUNK, a.w0, a.w1);
+    const int c = win.x + blockIdx.x / tiles_j, chunk = chunk0 + c;
+    if (c >= win.y) return;
+    const int nt = min(SC_CHUNK, len - c * SC_CHUNK);
     const size_t first = (size_t)row0 + c * SC_CHUNK, at = (size_t)chunk * a.n_heads + h;
     const int cols = a.dv + a.normalizer, g = h / a.heads_per_group, n_groups = a.n_heads / a.heads_per_group;
-    const float* S0 = a.before + at * cols * a.lds;
+    const float* S0 = a.before + ((size_t)(chunk - a.w0) * a.n_heads + h) * cols * a.lds;
     const float* qp = a.q + first * a.ldq + (size_t)g * a.dk;
     const int slices = (a.dk + 31) / 32;
     auto load = [&](int s) {
@@ -625,15 +633,15 @@ ss_output_kernel(const ScArgs a) {
 MV_API int mv_scalar_chunks(int N, int n_seqs) { return N / SC_CHUNK + n_seqs + 1; }
 
 // Arguments as mv_scalar_scan, plus the longest sequence's tokens (max_len) and scratch with chunks =
-// mv_scalar_chunks(N, n_seqs): G [chunks, groups, SC_CHUNK, SC_CHUNK], before [chunks, n_heads, dv (+ 1), dk rounded up to 4]
+// mv_scalar_chunks(N, n_seqs): G [chunks, groups, SC_CHUNK, SC_CHUNK], before [room (+ 2 where room < chunks), n_heads, dv (+ 1), dk rounded up to 4] for windows of `room` chunks
 // and factors [chunks, n_heads, 3 SC_CHUNK + 4], both 16-byte aligned.
 MV_API int mv_scalar_scan_chunked(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
                                   const float* log_a, int ld_a, const float* b, int ld_b, const float* skip,
                                   const float* m_tok, float q_scale, float* state, const int* slots, const int* cu,
-                                  float* o, float* G, float* before, float* factors, int chunks, int n_seqs, int max_len,
+                                  float* o, float* G, float* before, float* factors, int room, int chunks, int n_seqs, int max_len,
                                   int n_heads, int heads_per_group, int dk, int dv, int normalizer, cudaStream_t stream) {
     if (n_seqs <= 0 || max_len <= 0) return 0;
-    if (dk < 1 || dk > 256 || dv < 1 || heads_per_group < 1 || n_heads % heads_per_group || (normalizer && !m_tok) ||
+    if (dk < 1 || dk > 256 || dv < 1 || heads_per_group < 1 || n_heads % heads_per_group || (normalizer && !m_tok) || room < 1 ||
         ((uintptr_t)before | (uintptr_t)factors) % 16)
         return (int)cudaErrorInvalidValue;
     ScArgs a = {};
@@ -643,7 +651,7 @@ MV_API int mv_scalar_scan_chunked(const float* q, int ldq, const float* k, int l
     const size_t rows = (size_t)chunks * n_heads;
     a.run = factors; a.e1 = a.run + rows * SC_CHUNK; a.e2 = a.e1 + rows * SC_CHUNK; a.el = a.e2 + rows * SC_CHUNK;
     a.n_heads = n_heads; a.heads_per_group = heads_per_group; a.dk = dk; a.dv = dv; a.lds = (dk + 3) & ~3;
-    a.normalizer = normalizer ? 1 : 0;
+    a.normalizer = normalizer ? 1 : 0; a.room = room;
     a.wide = cs_aligned(q, ldq, dk) && cs_aligned(k, ldk, dk) && cs_aligned(v, ldv, dv);
     static const cudaError_t attr[3] = {
         cudaFuncSetAttribute(ss_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SW_SMEM),
@@ -657,12 +665,16 @@ MV_API int mv_scalar_scan_chunked(const float* q, int ldq, const float* k, int l
     if (code) return code;
     mv_launch(ss_products_kernel, dim3(n_chunks, n_heads / heads_per_group, n_seqs), 64, 0, stream, a);
     if ((code = mv_launch_status())) return code;
-    mv_launch(ss_walk_kernel, dim3((dv + 63) / 64 * ((dk + 63) / 64), n_heads, n_seqs), SC_WALK_THREADS, SW_SMEM, stream, a);
-    if ((code = mv_launch_status())) return code;
-    const dim3 grid(n_chunks * ((dv + 63) / 64), n_heads, n_seqs);
-    if (dk <= 128) mv_launch(ss_output_kernel<4>, grid, SO_THREADS, SO_SMEM, stream, a);
-    else mv_launch(ss_output_kernel<8>, grid, SO_THREADS, SO_SMEM, stream, a);
-    return mv_launch_status();
+    const dim3 grid(min(n_chunks, room) * ((dv + 63) / 64), n_heads, n_seqs);
+    for (a.w0 = 0; a.w0 < chunks; a.w0 += room) {
+        a.w1 = a.w0 + room;
+        mv_launch(ss_walk_kernel, dim3((dv + 63) / 64 * ((dk + 63) / 64), n_heads, n_seqs), SC_WALK_THREADS, SW_SMEM, stream, a);
+        if ((code = mv_launch_status())) return code;
+        if (dk <= 128) mv_launch(ss_output_kernel<4>, grid, SO_THREADS, SO_SMEM, stream, a);
+        else mv_launch(ss_output_kernel<8>, grid, SO_THREADS, SO_SMEM, stream, a);
+        if ((code = mv_launch_status())) return code;
+    }
+    return 0;
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -57,7 +57,7 @@ _SIGNATURES = {
         "mv_decay_scan": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _F, _F, _I, _P, _P, _P, _P, _I, _I, _I, _I, _P],
         "mv_decay_chunks": [_I, _I],
         "mv_decay_scan_chunked": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _F, _F, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,
-                                  _P, _I, _I, _I, _I, _I, _I, _I, _P],
+                                  _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
         "mv_qkv_prepare_wide": [_P, _I, _P, _P, _F, _I, _P, _P, _P, _P, _I, _I, _P, _Q, _P, _I, _I, _I, _I, _I, _I, _I,
                                 _F, _F, _F, _P],
         "mv_attention_sink": [_P, _P, _Q, _P, _I, _I, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _F, _I, _I,
@@ -73,7 +73,7 @@ _SIGNATURES = {
                            _P],
         "mv_scalar_chunks": [_I, _I],
         "mv_scalar_scan_chunked": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I,
-                                   _I, _I, _I, _I, _I, _P],
+                                   _I, _I, _I, _I, _I, _I, _P],
         "mv_decay_factor_floats": [_I],
         "mv_decay_few_chunks": [_I, _I],
         "mv_decay_scan_few": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _F, _F, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I,
@@ -688,15 +688,17 @@ def scalar_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_a: torch.
     if ws is not None and max_len >= SCAN_CHUNKED_FROM:
         chunks = int(_fn("core", "mv_scalar_chunks")(N, int(n_seqs)))
         G = ws.get("scalar_scan_products", (chunks, groups, SCAN_CHUNK, SCAN_CHUNK), torch.float32)
-        before = ws.get("scan_before", (chunks, n_heads, dv + (1 if norm else 0), (dk + 3) & ~3), torch.float32)
+        room = scan_room(chunks, n_heads * (dv + (1 if norm else 0)) * ((dk + 3) & ~3) * 4)
+        before = ws.get("scan_before", (room + 2 * (room < chunks), n_heads, dv + (1 if norm else 0), (dk + 3) & ~3), torch.float32)
         factors = ws.get("scan_factors", (chunks, n_heads, 3 * SCAN_CHUNK + 4), torch.float32)
         _check(_fn("core", "mv_scalar_scan_chunked")(
             qp, ldq, kp, ldk, vp, ldv, ap, lda, bp, ldb, _need(skip, "scalar_scan skip", torch.float32, (n_heads,), True),
             _need(m_tok, "scalar_scan m", torch.float32, (N, n_heads), True), float(q_scale), state.data_ptr(),
             _need(slots, "slots", torch.int32), _need(cu, "cu", torch.int32),
             _need(out, "scalar_scan out", torch.float32, (N, n_heads * dv)), G.data_ptr(),
-            before.data_ptr(), factors.data_ptr(), chunks, int(n_seqs), int(max_len), n_heads, int(heads_per_group), dk, dv,
+            before.data_ptr(), factors.data_ptr(), room, chunks, int(n_seqs), int(max_len), n_heads, int(heads_per_group), dk, dv,
             int(norm), _stream()), "mv_scalar_scan_chunked")
+        add_launches(2 * (-(-chunks // room) - 1))
         account(N * n_heads * (2 * dk // heads_per_group + 2 * dv) * 4 + 2 * n_seqs * n_heads * dk * dv * 4
                 + 2 * chunks * (groups * SCAN_CHUNK * SCAN_CHUNK + n_heads * dk * dv) * 4,
                 4 * N * n_heads * dk * dv + N * n_heads * SCAN_CHUNK * dv + N * groups * SCAN_CHUNK * dk)
@@ -998,6 +1000,16 @@ DECAY_CHUNK = 64                # of decay_scan
 # stand beside those kernels in decay_scan.cu and scalar_scan.cu)
 DECAY_CHUNKS_FROM = 400
 SCALAR_CHUNKS_FROM = 128
+# The states before a step's chunks are scratch that an engine keeps: so many bytes of them at a time.  64 heads of 128 x 64 with one decay a
+# token, at 64 / 128 / 256 MB / all at once: one sequence of 2,048 tokens (134 MB) 254 / 251 / 233 / 235 us, of 8,192 890 / 961 / 940 / 1,029, 32 of 256
+# 937 / 829 / 759 / 687, 512 of 16 4,341 / 2,949 / 2,274 / 1,601 (1.6 GB).
+SCAN_STATES_BYTES = 256 << 20
+
+
+def scan_room(chunks: int, state_bytes: int) -> int:
+    """How many chunks' states a chunked scan holds at a time: all of them, or what fits SCAN_STATES_BYTES together with the two that
+    pass from one window to the next, but at least 8 chunks (below that the launches would show)."""
+    return max(1, min(chunks, max(8, SCAN_STATES_BYTES // state_bytes - 2)))
 
 
 def _cols(t: torch.Tensor, name: str, n_rows: int, width: int):
@@ -1055,7 +1067,8 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
         qd = ws.get("scan_qd", (N, n_heads * dk), torch.float32) if by_channel else None
         kd = ws.get("scan_kd", (N, n_heads * dk), torch.float32) if by_channel else None
         ed = ws.get("scan_ed", (chunks, n_heads * dk), torch.float32) if by_channel else None
-        before = ws.get("scan_before", (chunks, n_heads, dv, (dk + 3) & ~3), torch.float32)
+        room = scan_room(chunks, n_heads * dv * ((dk + 3) & ~3) * 4)
+        before = ws.get("scan_before", (room + 2 * (room < chunks), n_heads, dv, (dk + 3) & ~3), torch.float32)
         factors = None if by_channel else ws.get("scan_factors", (chunks, int(_fn("core", "mv_decay_factor_floats")(n_heads))),
                                                  torch.float32)
         pm = ws.get("scan_p", (chunks, n_heads, DECAY_CHUNK, DECAY_CHUNK), torch.float32)
@@ -1064,8 +1077,8 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
             float(inv_tau), float(q_scale), int(act), state.data_ptr(), _need(slots, "slots", torch.int32),
             _need(cu, "cu", torch.int32), _need(out, "decay_scan out", torch.float32, (N, n_heads * dv)),
             *(t.data_ptr() if t is not None else None for t in (copies, qd, kd, ed)), pm.data_ptr(), before.data_ptr(),
-            factors.data_ptr() if factors is not None else None, chunks, N, int(n_seqs), int(max_len), n_heads, dk, dv, _stream()), "mv_decay_scan_chunked")
-        add_launches(int(bool(act)) + int(not by_channel))
+            factors.data_ptr() if factors is not None else None, room, chunks, N, int(n_seqs), int(max_len), n_heads, dk, dv, _stream()), "mv_decay_scan_chunked")
+        add_launches(int(bool(act)) + int(not by_channel) + 2 * (-(-chunks // room) - 1))
         account(N * n_heads * (6 * dk + 2 * dv) * 4 + 2 * (n_seqs + chunks) * n_heads * dk * dv * 4, 5 * N * n_heads * dk * dv)
         return out
     _check(_fn("core", "mv_decay_scan")(
