@@ -276,7 +276,18 @@ MV_API int mv_qk_prepare(const float* qkv, const float* wq, const float* wk, flo
 // scores one key (its row of hd elements is contiguous), the warp agrees on the
 // running maximum, then the lanes split the head's elements for the weighted
 // sum of the values.  Works for every hd that is a multiple of 8 up to 256.
-template <typename T>
+//
+// SHORT: only the rows that attention_f32_tile_kernel leaves (ft_long_run).
+constexpr int FT_Q = 32, FT_LONG = 16;
+
+// Whether the rows r0 .. r1 - 1 of the tile that starts at row n0, which read sequence b, belong to a long run of rows of that
+// sequence: FT_LONG of them in the tile, or a run that goes on in the tile before or behind.
+__device__ __forceinline__ bool ft_long_run(const int* __restrict__ seq_of, int N, int n0, int r0, int r1, int b) {
+    return r1 - r0 >= FT_LONG || (r0 == 0 && n0 > 0 && seq_of[n0 - 1] == b) ||
+           (r1 == FT_Q && n0 + FT_Q < N && seq_of[n0 + FT_Q] == b);
+}
+
+template <typename T, bool SHORT = false>
 __global__ void __launch_bounds__(128)
 attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ pool, long long page_stride,
                          const int* __restrict__ page_table, int table_stride, int page_shift,
@@ -288,6 +299,12 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ pool, lo
     const long long warp = (long long)blockIdx.x * 4 + wib;
     if (warp >= (long long)N * nh) return;
     const int n = (int)(warp / nh), h = (int)(warp - (long long)n * nh);
+    if (SHORT) {
+        const int at = n & (FT_Q - 1), n0 = n - at, b = seq_of[n];
+        const unsigned same = __ballot_sync(0xffffffffu, n0 + lane < N && seq_of[min(n0 + lane, N - 1)] == b);
+        const unsigned below = ~same & ((1u << at) - 1), above = ~same >> at;       // the nearest other rows on either side
+        if (ft_long_run(seq_of, N, n0, 32 - __clz(below), above ? at + __ffs(above) - 1 : FT_Q, b)) return;
+    }
     const int g = h / (nh / nkv);
     const int pos = positions[n];
     const int page_size = 1 << page_shift;
@@ -349,19 +366,26 @@ attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ pool, lo
     }
 }
 
-// The same in float32 for steps of many tokens: a block is 32 packed query rows of one head; keys and values come in blocks of 64
-// into shared memory, once for all of the rows that read their sequence, where a warp a row reads every key for itself.  The
-// rows' sequences are taken one after the other (most tiles have one); scores, weights and sums are float32 throughout.  A
+// The same in float32 for long runs of rows of one sequence: a block is 32 packed query rows of one head; keys and values come in
+// blocks of 64 into shared memory, once for all of the rows that read their sequence, where a warp a row reads every key for
+// itself.  The rows' sequences are taken one after the other; scores, weights and sums are float32 throughout.  A
 // thread has 4 x 4 scores and 4 x (4 NB) of the output, four threads a row do the softmax.  Bound by the latency of its few
 // steps a tile: 1,165 rows of four prompts, 16 heads of 64: 680 us with a warp a row, 129 so.
-constexpr int FT_Q = 32, FT_K = 64, FT_SLD = FT_K + 4;
+//
+// A block pays for every sequence in its tile as if all rows were that one's: about 0.15 us a key, and 2 a sequence, where the kernel above takes
+// 0.8 us a key for any number of rows that fill the device.  So it takes the runs of FT_LONG rows and what long runs leave at the tile's
+// edges - three sequences a tile at most - and leaves the others to the kernel above (`all`: it takes every run).  Sequences of
+// 3 rows behind 2,000 keys (64 of them): 1,583 us above, 3,488 here; of 8 rows (32) 1,562 and 1,208; of 16 2,651 and 700; without keys before
+// them 21 and 55, 26 and 40, 43 and 38.  A 512-token prompt beside 31 rows behind 2,000 keys: 1,764 above, 9,242 with every run here, 1,693 so.
+// With a window the blocks of keys start where the tile's first row sees, so a row's sums may be cut elsewhere beside other rows.
+constexpr int FT_K = 64, FT_SLD = FT_K + 4;
 
 template <int NB>
 __global__ void __launch_bounds__(128)
 attention_f32_tile_kernel(const float* __restrict__ q, const float* __restrict__ pool, long long page_stride,
                           const int* __restrict__ page_table, int table_stride, int page_shift,
                           const int* __restrict__ positions, const int* __restrict__ seq_of, float* __restrict__ o, int N,
-                          int nh, int nkv, int hd, float scale, int window) {
+                          int nh, int nkv, int hd, float scale, int window, int all) {
     constexpr int W = 64 * NB, LD = W + 4;
     extern __shared__ __align__(16) float ft_smem[];
     float* qs = ft_smem;                        // [FT_Q][LD]
@@ -384,6 +408,7 @@ attention_f32_tile_kernel(const float* __restrict__ q, const float* __restrict__
 #pragma unroll
         for (int x = 0; x < 4 * NB; ++x) acc[y][x] = 0.f;
     const int my_pos = row < rows ? positions[n0 + row] : -1;
+    unsigned taken = 0;                         // the rows that are worked out here
     for (int r0 = 0; r0 < rows;) {
         // the rows r0 .. r1 - 1 read one sequence; the keys that any of them sees
         const int b = seq_of[n0 + r0];
@@ -393,6 +418,11 @@ attention_f32_tile_kernel(const float* __restrict__ q, const float* __restrict__
             last = max(last, p);
             first = min(first, window > 0 ? max(0, p - window + 1) : 0);
         }
+        if (!all && !ft_long_run(seq_of, N, n0, r0, r1, b)) {
+            r0 = r1;
+            continue;
+        }
+        taken |= (r1 - r0 == 32 ? 0xffffffffu : (1u << (r1 - r0)) - 1) << r0;
         const int* table = page_table + (size_t)b * table_stride;
         const bool mine = row >= r0 && row < r1;
         for (int t0 = first; t0 <= last; t0 += FT_K) {
@@ -496,7 +526,7 @@ attention_f32_tile_kernel(const float* __restrict__ q, const float* __restrict__
 #pragma unroll
     for (int y = 0; y < 4; ++y) {
         const int r = tq + 8 * y;
-        if (r >= rows) continue;
+        if (!(taken >> r & 1)) continue;
         const float inv = cs[r];
         float* to = o + (size_t)(n0 + r) * nh * hd + (size_t)h * hd;
 #pragma unroll
@@ -510,35 +540,40 @@ attention_f32_tile_kernel(const float* __restrict__ q, const float* __restrict__
 template <int NB>
 static int attention_f32_tile_launch(const float* q, const float* pool, long long page_stride, const int* page_table, int table_stride,
                                      int page_shift, const int* positions, const int* seq_of, float* o, int N, int nh, int nkv, int hd,
-                                     float scale, int window, cudaStream_t stream) {
+                                     float scale, int window, int all, cudaStream_t stream) {
     constexpr size_t smem = sizeof(float) * ((FT_Q + FT_K) * (64 * NB + 4) + FT_K * 64 * NB + FT_Q * FT_SLD + FT_Q);
     static const cudaError_t attr = cudaFuncSetAttribute(attention_f32_tile_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (attr != cudaSuccess) return (int)attr;
     mv_launch(attention_f32_tile_kernel<NB>, dim3((N + FT_Q - 1) / FT_Q, nh), 128, smem, stream, q, pool, page_stride, page_table,
-              table_stride, page_shift, positions, seq_of, o, N, nh, nkv, hd, scale, window);
+              table_stride, page_shift, positions, seq_of, o, N, nh, nkv, hd, scale, window, all);
     return mv_launch_status();
 }
 
+// runs, for float32: 0 the rows' sequences come in runs of any length, 1 of FT_LONG rows or more, 2 of fewer
 MV_API int mv_attention_generic(const void* q, const void* pool, long long page_stride,
                                 const int* page_table, int table_stride, int page_size,
                                 const int* positions, const int* seq_of, void* o, int dtype, int N,
-                                int nh, int nkv, int hd, float scale, int window, cudaStream_t stream) {
+                                int nh, int nkv, int hd, float scale, int window, int runs, cudaStream_t stream) {
     if (N <= 0) return 0;
     if (hd % 8 || hd > MV_MAX_HEAD_DIM || nh % nkv || (page_size & (page_size - 1)))
         return (int)cudaErrorInvalidValue;
     int page_shift = 0;
     while ((1 << page_shift) < page_size) ++page_shift;
     const unsigned blocks = (unsigned)(((long long)N * nh + 3) / 4);
+    const bool tiles = runs != 2 && N >= FT_Q && hd <= 128 && page_stride % 4 == 0 && ((uintptr_t)pool & 15) == 0;
     if (dtype == MV_DT_BF16)
         mv_launch(attention_generic_kernel<__nv_bfloat16>, blocks, 128, 0, stream, 
             (const __nv_bfloat16*)q, (const __nv_bfloat16*)pool, page_stride, page_table, table_stride,
             page_shift, positions, seq_of, (__nv_bfloat16*)o, N, nh, nkv, hd, scale, window);
-    else if (N >= FT_Q && hd <= 128 && hd % 4 == 0 && page_stride % 4 == 0 && ((uintptr_t)pool & 15) == 0)
-        // (a tile of one or two rows repays nothing)
-        return hd <= 64 ? attention_f32_tile_launch<1>((const float*)q, (const float*)pool, page_stride, page_table, table_stride, page_shift,
-                                                       positions, seq_of, (float*)o, N, nh, nkv, hd, scale, window, stream)
-                        : attention_f32_tile_launch<2>((const float*)q, (const float*)pool, page_stride, page_table, table_stride, page_shift,
-                                                       positions, seq_of, (float*)o, N, nh, nkv, hd, scale, window, stream);
+    else if (tiles) {
+        const auto go = hd <= 64 ? attention_f32_tile_launch<1> : attention_f32_tile_launch<2>;
+        const int code = go((const float*)q, (const float*)pool, page_stride, page_table, table_stride, page_shift, positions, seq_of,
+                            (float*)o, N, nh, nkv, hd, scale, window, runs == 1, stream);
+        if (code || runs == 1) return code;
+        mv_launch(attention_generic_kernel<float, true>, blocks, 128, 0, stream,
+            (const float*)q, (const float*)pool, page_stride, page_table, table_stride, page_shift,
+            positions, seq_of, (float*)o, N, nh, nkv, hd, scale, window);
+    }
     else
         mv_launch(attention_generic_kernel<float>, blocks, 128, 0, stream, 
             (const float*)q, (const float*)pool, page_stride, page_table, table_stride, page_shift,

@@ -42,7 +42,7 @@ _SIGNATURES = {
         "mv_shortconv": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
         "mv_shortconv_decode": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],
         "mv_qk_prepare": [_P, _P, _P, _F, _P, _I, _P, _P, _P, _I, _I, _P, _Q, _I, _P, _I, _I, _I, _I, _I, _P],
-        "mv_attention_generic": [_P, _P, _Q, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P],
+        "mv_attention_generic": [_P, _P, _Q, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P],
         "mv_attention_decode": [_P, _P, _Q, _P, _I, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I,
                                 _I, _I, _P],
         "mv_layernorm": [_P, _P, _P, _P, _I, _P, _I, _I, _F, _P],
@@ -2256,9 +2256,11 @@ def qk_prepare_q_only(qkv: torch.Tensor, wq: Optional[torch.Tensor], eps: float,
 
 
 def attention_generic(q: torch.Tensor, pool: torch.Tensor, page_table, positions, seq_of,
-                      out: torch.Tensor, nh: int, nkv: int, hd: int, scale: float, window: int = 0):
+                      out: torch.Tensor, nh: int, nkv: int, hd: int, scale: float, window: int = 0, lens=None):
     """Causal attention of every token of the step over its sequence's cache
-    (which already holds the step's own keys), optional sliding window."""
+    (which already holds the step's own keys), optional sliding window.  ``lens``: how many tokens each sequence of the step
+    brings, its rows together, if the caller knows; in float32 long runs of rows and short ones take different kernels, and one
+    launch is left out where there are none of a kind."""
     N = q.shape[0]
     if hd % 8 or hd > MAX_HEAD_DIM:
         raise KernelError(f"attention: head size {hd} must be a multiple of 8 and at most {MAX_HEAD_DIM}")
@@ -2269,13 +2271,26 @@ def attention_generic(q: torch.Tensor, pool: torch.Tensor, page_table, positions
     if q.dtype != pool.dtype or out.dtype != q.dtype:
         raise KernelError(f"attention: q {q.dtype}, cache {pool.dtype}, out {out.dtype} must agree")
     _guard("core", "attention", q.device, n_pages=pool.shape[0])
+    runs = attention_runs(lens)
+    tiles = q.dtype == torch.float32 and N >= 32 and hd <= 128 and runs == 0
     _check(_fn("core", "mv_attention_generic")(
         _need(q, "q", None, (N, nh * hd)), _need(pool, "cache pool"), pool.stride(0),
         _need(page_table, "page table", torch.int32), page_table.shape[1], page_size,
         _need(positions, "positions", torch.int32), _need(seq_of, "seq_of", torch.int32),
-        _need(out, "attention out", None, (N, nh * hd)), _dt(q), N, nh, nkv, hd, float(scale), int(window),
+        _need(out, "attention out", None, (N, nh * hd)), _dt(q), N, nh, nkv, hd, float(scale), int(window), runs,
         _stream()), "mv_attention_generic")
+    add_launches(int(tiles))                      # both kernels
     return out
+
+
+LONG_RUN = 16                   # rows of one sequence in a tile of 32 from which float32 attention works in tiles (attention.cu)
+
+
+def attention_runs(lens) -> int:
+    """What the runs of rows of these lengths are for the float32 attention: 1 all long, 2 all short, 0 of both kinds or unknown."""
+    if lens is None or not len(lens):
+        return 0
+    return 1 if min(lens) >= LONG_RUN else 2 if max(lens) < LONG_RUN else 0
 
 
 _n_sms = {}

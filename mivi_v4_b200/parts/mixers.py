@@ -178,7 +178,7 @@ class GroupedQueryAttention(Part):
                                 self.scale, self.window)
         else:
             K.attention_generic(q, view.pool, view.page_table, step.positions, step.seq_of, o, nh, nkv, hd,
-                                self.scale, self.window)
+                                self.scale, self.window, step.host_lens)
         if K.profiling_on():
             # keys that the step's queries read (each query its own context), for the attention launch
             pairs = sum(n * s + n * (n + 1) // 2 for s, n in zip(step.host_starts, step.host_lens))
