@@ -95,17 +95,31 @@ layernorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ w, 
         }
 }
 
+// The kernel for a width that its warps divide evenly, up to 4,096 (a lane then holds 128 values); false: none for this one.
+template <typename TO>
+static bool layernorm_warp_launch(const float* x, const float* w, const float* b, TO* y, const int* rows, int n_rows, int H, float eps,
+                                  cudaStream_t stream) {
+#define GN_CASE(WP, PER)                                                                                                       \
+    case 32 * WP * PER:                                                                                                        \
+        mv_launch(layernorm_warp_kernel<TO, WP, PER>, (n_rows + 3) / 4, 128, 0, stream, x, w, b, y, rows, n_rows, eps);         \
+        return true;
+    switch (H) {
+        GN_CASE(4, 1) GN_CASE(4, 2) GN_CASE(4, 3)
+        GN_CASE(8, 2) GN_CASE(8, 3) GN_CASE(8, 4) GN_CASE(8, 5) GN_CASE(8, 6) GN_CASE(8, 7)
+        GN_CASE(16, 4) GN_CASE(16, 5) GN_CASE(16, 6) GN_CASE(16, 7) GN_CASE(16, 8)
+    }
+#undef GN_CASE
+    return false;
+}
+
 // b: the bias [H], or null for none
 MV_API int mv_layernorm(const float* x, const float* w, const float* b, void* y, int y_dtype, const int* rows, int n_rows,
                         int H, float eps, cudaStream_t stream) {
     if (n_rows <= 0) return 0;
     // (from about four rows a multiprocessor on; fewer are done sooner with a block each)
-    if (n_rows >= 592 && y_dtype == MV_DT_BF16 && (H == 2048 || H == 1024)) {
-        const int blocks = (n_rows + 3) / 4;
-        if (H == 2048) mv_launch(layernorm_warp_kernel<__nv_bfloat16, 16, 4>, blocks, 128, 0, stream, x, w, b, (__nv_bfloat16*)y, rows, n_rows, eps);
-        else mv_launch(layernorm_warp_kernel<__nv_bfloat16, 8, 4>, blocks, 128, 0, stream, x, w, b, (__nv_bfloat16*)y, rows, n_rows, eps);
+    if (n_rows >= 592 && (y_dtype == MV_DT_BF16 ? layernorm_warp_launch(x, w, b, (__nv_bfloat16*)y, rows, n_rows, H, eps, stream)
+                                                : layernorm_warp_launch(x, w, b, (float*)y, rows, n_rows, H, eps, stream)))
         return mv_launch_status();
-    }
     const int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
     if (y_dtype == MV_DT_BF16)
         mv_launch(layernorm_kernel<__nv_bfloat16>, n_rows, threads, 0, stream, x, w, b, (__nv_bfloat16*)y, rows, H, eps);
