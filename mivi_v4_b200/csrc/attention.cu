@@ -542,7 +542,7 @@ static int attention_f32_tile_launch(const float* q, const float* pool, long lon
                                      int page_shift, const int* positions, const int* seq_of, float* o, int N, int nh, int nkv, int hd,
                                      float scale, int window, int all, cudaStream_t stream) {
     constexpr size_t smem = sizeof(float) * ((FT_Q + FT_K) * (64 * NB + 4) + FT_K * 64 * NB + FT_Q * FT_SLD + FT_Q);
-    static const cudaError_t attr = cudaFuncSetAttribute(attention_f32_tile_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t attr = mv_allow_smem<attention_f32_tile_kernel<NB>>(smem);
     if (attr != cudaSuccess) return (int)attr;
     mv_launch(attention_f32_tile_kernel<NB>, dim3((N + FT_Q - 1) / FT_Q, nh), 128, smem, stream, q, pool, page_stride, page_table,
               table_stride, page_shift, positions, seq_of, o, N, nh, nkv, hd, scale, window, all);

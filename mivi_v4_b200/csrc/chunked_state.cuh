@@ -474,8 +474,7 @@ inline bool cs_aligned(const float* p, int ld, int cols) { return ((uintptr_t)p 
 template <int TJ, int GROUPS, bool CHANNEL>
 int cs_walk_launch(const CsArgs& a, int tiles, int n_seqs, cudaStream_t stream) {
     constexpr size_t smem = sizeof(float) * (2 * CS_CHUNK * (64 + 8 * TJ + 1) + (GROUPS - 1) * TJ * CS_THREADS * 4);
-    static const cudaError_t attr = cudaFuncSetAttribute(cs_walk_kernel<TJ, GROUPS, CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)smem);
+    const cudaError_t attr = mv_allow_smem<cs_walk_kernel<TJ, GROUPS, CHANNEL>>(smem);
     if (attr != cudaSuccess) return (int)attr;
     mv_launch(cs_walk_kernel<TJ, GROUPS, CHANNEL>, dim3(tiles, a.n_heads, n_seqs), CS_THREADS * GROUPS, smem, stream, a);
     return mv_launch_status();
@@ -506,7 +505,7 @@ int cs_launch(CsArgs a, float* G, float* factors, int chunks, int n_seqs, int ma
     }
     const int tiles_i = (a.dk + 63) / 64;
     const long tiles = (long)((a.dv + 63) / 64) * tiles_i * a.n_heads * n_seqs;
-    static const cudaError_t attr = cudaFuncSetAttribute(cs_output_kernel<CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CO_SMEM);
+    const cudaError_t attr = mv_allow_smem<cs_output_kernel<CHANNEL>>(CO_SMEM);
     if (attr != cudaSuccess) return (int)attr;
     const int per_seq = min((max_len + CS_CHUNK - 1) / CS_CHUNK, a.room);       // the most chunks a sequence has in a window
     for (a.w0 = 0; a.w0 < chunks; a.w0 += a.room) {

@@ -159,6 +159,24 @@ static inline void mv_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 }
 #endif
 
+#ifndef __CUDACC_RTC__
+#include <atomic>
+// Allows a kernel more dynamic shared memory than the default.  The permission belongs to a device, so it is asked for once on each
+// that the process uses (a bit a device; two threads that both find it unset ask for the same).
+template <auto KERNEL>
+static inline cudaError_t mv_allow_smem(size_t bytes) {
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
+}
+#endif
+
 // A cluster barrier that orders nothing in memory: for "nobody leaves before everybody is here".
 __device__ __forceinline__ void mv_cluster_sync_relaxed() {
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");

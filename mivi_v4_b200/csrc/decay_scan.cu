@@ -307,8 +307,7 @@ static int decay_prepare_launch(const float* q, int ldq, const float* k, int ldk
                                 float q_scale, const int* cu, float* qd, float* kd, float* ed, float* P, int n_seqs, int max_len,
                                 int n_heads, int dk, cudaStream_t stream) {
     constexpr size_t smem = sizeof(float) * 3 * CS_CHUNK * 32 * NC;
-    static const cudaError_t attr = cudaFuncSetAttribute(decay_chunk_prepare_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)smem);
+    const cudaError_t attr = mv_allow_smem<decay_chunk_prepare_kernel<NC>>(smem);
     if (attr != cudaSuccess) return (int)attr;
     mv_launch(decay_chunk_prepare_kernel<NC>, dim3((max_len + CS_CHUNK - 1) / CS_CHUNK, n_heads, n_seqs), DC_THREADS, smem, stream,
               q, ldq, k, ldk, z, ldz, inv_tau, q_scale, cu, qd, kd, ed, P, n_heads, dk);
@@ -575,7 +574,7 @@ static int decay_few_scan_launch(dim3 grid, cudaStream_t stream, const float* qd
                                    const int* cu, float* o, int n_heads, int dk, int dv) {
     const size_t smem = sizeof(float) * ((size_t)2 * DF_CHUNK * DF_GROUPS * RH + DF_CHUNK * DF_COLS + DF_CHUNK * DF_CHUNK +
                                          DF_GROUPS * RH + DF_GROUPS * DF_RED_STRIDE);
-    const cudaError_t attr = cudaFuncSetAttribute(decay_few_scan_kernel<RH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t attr = mv_allow_smem<decay_few_scan_kernel<RH>>(smem);
     if (attr != cudaSuccess) return (int)attr;
     mv_launch(decay_few_scan_kernel<RH>, grid, DF_SCAN_THREADS, smem, stream, qd, kd, ed, P, v, ldv, act, state, slots, cu, o,
               n_heads, dk, dv);
@@ -593,8 +592,7 @@ MV_API int mv_decay_scan_few(const float* q, int ldq, const float* k, int ldk, c
     if (n_seqs <= 0 || max_len <= 0) return 0;
     if (dk < 1 || dk > 256 || dv < 1 || (!z && !head_decay)) return (int)cudaErrorInvalidValue;
     const size_t smem_a = sizeof(float) * (size_t)3 * DF_CHUNK * (dk + 1);
-    const cudaError_t attr = cudaFuncSetAttribute(decay_few_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)sizeof(float) * 3 * DF_CHUNK * 257);      // what the largest dk needs
+    const cudaError_t attr = mv_allow_smem<decay_few_prepare_kernel>(sizeof(float) * 3 * DF_CHUNK * 257);     // what the largest dk needs
     if (attr != cudaSuccess) return (int)attr;
     mv_launch(decay_few_prepare_kernel, dim3((max_len + DF_CHUNK - 1) / DF_CHUNK, n_heads, n_seqs), DF_THREADS, smem_a,
               stream, q, ldq, k, ldk, z, ldz, head_decay, inv_tau, q_scale, act, cu, qd, kd, ed, P, n_heads, dk);

@@ -166,8 +166,7 @@ int gemm_f32_tile_launch(const float* X, const float* W, const float* bias, void
     constexpr int BM = TM * 8;
     constexpr size_t smem = sizeof(float) * FT_STAGES * (BM + FT_BN) * FT_LD;
     static_assert(sizeof(float) * BM * FT_BN <= smem, "the tile takes the stages' place");
-    static const cudaError_t attr = cudaFuncSetAttribute(gemm_f32_tile_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)smem);
+    const cudaError_t attr = mv_allow_smem<gemm_f32_tile_kernel<TM>>(smem);
     if (attr != cudaSuccess) return (int)attr;
     const int gx = (N + FT_BN - 1) / FT_BN, gy = (M + BM - 1) / BM, kb = (K + FT_BK - 1) / FT_BK;
     int ranks = 1;

@@ -407,8 +407,7 @@ int launch(const void* q, const void* kx, int ld_kx, int v0, const void* rk, con
            float scale, int window, cudaStream_t stream) {
     constexpr int QT = NWARPS * 16 * MT;
     const size_t smem = (size_t)3 * KB * (dim + rot + 8 + dv + 8) * sizeof(__nv_bfloat16);
-    static const cudaError_t attr = cudaFuncSetAttribute(latent_attention_prefill_kernel<DKM, DVM, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)((size_t)3 * KB * (DKM + 8 + DVM + 8) * sizeof(__nv_bfloat16)));
+    const cudaError_t attr = mv_allow_smem<latent_attention_prefill_kernel<DKM, DVM, MT>>((size_t)3 * KB * (DKM + 8 + DVM + 8) * sizeof(__nv_bfloat16));
     if (attr != cudaSuccess) return (int)attr;
     const dim3 grid((N + QT - 1) / QT + B, nh);       // an upper bound of the tiles; spare blocks return at once
     mv_launch(latent_attention_prefill_kernel<DKM, DVM, MT>, grid, NWARPS * 32, smem, stream, (const __nv_bfloat16*)q,

@@ -653,12 +653,9 @@ MV_API int mv_scalar_scan_chunked(const float* q, int ldq, const float* k, int l
     a.n_heads = n_heads; a.heads_per_group = heads_per_group; a.dk = dk; a.dv = dv; a.lds = (dk + 3) & ~3;
     a.normalizer = normalizer ? 1 : 0; a.room = room;
     a.wide = cs_aligned(q, ldq, dk) && cs_aligned(k, ldk, dk) && cs_aligned(v, ldv, dv);
-    static const cudaError_t attr[3] = {
-        cudaFuncSetAttribute(ss_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SW_SMEM),
-        cudaFuncSetAttribute(ss_output_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SO_SMEM),
-        cudaFuncSetAttribute(ss_output_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SO_SMEM)};
-    for (const cudaError_t e : attr)
-        if (e != cudaSuccess) return (int)e;
+    cudaError_t attr = mv_allow_smem<ss_walk_kernel>(SW_SMEM);
+    if (attr == cudaSuccess) attr = dk <= 128 ? mv_allow_smem<ss_output_kernel<4>>(SO_SMEM) : mv_allow_smem<ss_output_kernel<8>>(SO_SMEM);
+    if (attr != cudaSuccess) return (int)attr;
     const int n_chunks = (max_len + SC_CHUNK - 1) / SC_CHUNK;
     mv_launch(ss_factors_kernel, dim3(n_chunks, (n_heads + 3) / 4, n_seqs), 128, 0, stream, a);
     int code = mv_launch_status();
@@ -882,7 +879,7 @@ static int scalar_few_scan_launch(dim3 grid, cudaStream_t stream, const float* q
                                     const int* cu, float* o, int n_heads, int hpg, int dk, int dv, int ones_col) {
     const size_t smem = sizeof(float) * ((size_t)2 * SC_CHUNK * SF_GROUPS * RH + SC_CHUNK * SF_COLS + SC_CHUNK * SC_CHUNK +
                                          4 * SC_CHUNK + 16 + SF_GROUPS * SF_RED_STRIDE);
-    const cudaError_t attr = cudaFuncSetAttribute(scalar_few_scan_kernel<RH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t attr = mv_allow_smem<scalar_few_scan_kernel<RH>>(smem);
     if (attr != cudaSuccess) return (int)attr;
     mv_launch(scalar_few_scan_kernel<RH>, grid, SF_SCAN_THREADS, smem, stream, q, ldq, k, ldk, v, ldv, log_a, ld_a, b, ld_b,
               skip, q_scale, G, state, slots, cu, o, n_heads, hpg, dk, dv, ones_col);
@@ -915,8 +912,7 @@ MV_API int mv_scalar_scan_few(const float* q, int ldq, const float* k, int ldk, 
         return (int)cudaErrorInvalidValue;
     const int n_groups = n_heads / heads_per_group;
     const size_t smem_a = sizeof(float) * (size_t)2 * SC_CHUNK * (dk + 1);
-    const cudaError_t attr = cudaFuncSetAttribute(scalar_few_products_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)sizeof(float) * 2 * SC_CHUNK * 257);      // what the largest dk needs
+    const cudaError_t attr = mv_allow_smem<scalar_few_products_kernel>(sizeof(float) * 2 * SC_CHUNK * 257);   // what the largest dk needs
     if (attr != cudaSuccess) return (int)attr;
     mv_launch(scalar_few_products_kernel, dim3((max_len + SC_CHUNK - 1) / SC_CHUNK, n_groups, n_seqs), SF_THREADS, smem_a,
               stream, q, ldq, k, ldk, cu, G, n_groups, dk);

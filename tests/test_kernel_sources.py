@@ -18,3 +18,10 @@ def test_instructions_of_a_whole_warp_are_volatile():
     found = [f"{name}: {m.group(1)[:60]}" for name, text in sources()
              for m in re.finditer(r'asm\s*\(\s*"([^"]*)"', text) if ".sync" in m.group(1) or ".aligned" in m.group(1)]
     assert not found, found
+
+
+def test_shared_memory_is_allowed_on_every_device():
+    """A kernel's permission for more shared memory belongs to a device: asked for once in a process, its launches on another device fail.
+    (float32 models ran on any device of a process before their kernels needed the permission.)"""
+    once = [name for name, text in sources() if re.search(r"static\s+(const\s+)?cudaError_t[^;]*cudaFuncSetAttribute", text)]
+    assert not once, once
