@@ -340,6 +340,13 @@ gemm_simt_kernel(const T* __restrict__ X, const T* __restrict__ W, const float* 
 
 }  // namespace
 
+// The tile's rows (32 or 64) that a float32 product of more than 8 rows is cut into, plus the number of blocks that share K.
+MV_API int mv_gemm_f32_plan(int M, int N, int K) {
+    int r32 = 1, r64 = 1;
+    const bool small = gemm_f32_tile_cost(32, M, N, K, &r32) < gemm_f32_tile_cost(64, M, N, K, &r64);
+    return small ? 32 + r32 : 64 + r64;
+}
+
 MV_API int mv_gemm_simt(const void* X, const void* W, int in_dtype, const float* bias, void* out,
                         int mode, int M, int N, int K, int ldo, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
@@ -351,8 +358,7 @@ MV_API int mv_gemm_simt(const void* X, const void* W, int in_dtype, const float*
         if (M <= 8) return gemm_f32_stream_launch<8, 4>(x, w, bias, out, mode, M, N, K, ldo, stream);
         // 1,165 rows against 1,024 x 4,608: 152 tiles of 64 rows leave one block on a multiprocessor (305 us with K cut in four), 296
         // of 32 rows fill them (273; against 1,024 x 1,024: 109 and 63)
-        int r;
-        if (gemm_f32_tile_cost(32, M, N, K, &r) < gemm_f32_tile_cost(64, M, N, K, &r))
+        if (mv_gemm_f32_plan(M, N, K) < 64)
             return gemm_f32_tile_launch<4>(x, w, bias, out, mode, M, N, K, ldo, stream);
         return gemm_f32_tile_launch<8>(x, w, bias, out, mode, M, N, K, ldo, stream);
     }

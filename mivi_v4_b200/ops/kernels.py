@@ -38,6 +38,7 @@ _SIGNATURES = {
         "mv_swiglu": [_P, _P, _I, _I, _I, _I, _I, _P],
         "mv_copy_to_host": [_P, _P, _Q, _P],
         "mv_delay": [_Q, _P],
+        "mv_gemm_f32_plan": [_I, _I, _I],
         "mv_gemm_simt": [_P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P],
         "mv_shortconv": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
         "mv_shortconv_decode": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],

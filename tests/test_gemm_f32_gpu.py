@@ -47,6 +47,20 @@ def test_gemm_f32(M, N, Kd):
     close(narrow, x, w, bias.double(), step=2.0 ** -8)
 
 
+@pytest.mark.parametrize("rows,cut,M,N,Kd", [(32, 1, 9, 65, 36), (32, 2, 1200, 129, 260), (32, 4, 600, 129, 132), (32, 8, 9, 65, 132),
+                                             (64, 1, 257, 4100, 36), (64, 1, 1165, 9216, 1024), (64, 2, 257, 2049, 1024),
+                                             (64, 4, 1200, 129, 2052), (64, 8, 1010, 129, 9000)])
+def test_every_tile_and_cut(rows, cut, M, N, Kd):
+    """Both tiles with K whole and cut in 2, 4 and 8, none of them filled; the rule that chooses them still chooses each."""
+    assert K()._fn("core", "mv_gemm_f32_plan")(M, N, Kd) == rows + cut
+    x, w, bias, base = rnd(M, Kd), rnd(N, Kd, seed=1), rnd(N, seed=2), rnd(M, N, seed=3)
+    acc, again = base.clone(), base.clone()
+    K().gemm_simt(x, w, acc, bias=bias, accumulate=True)
+    close(acc, x, w, base.double() + bias.double())
+    K().gemm_simt(x, w, again, bias=bias, accumulate=True)
+    assert torch.equal(acc, again)
+
+
 @pytest.mark.parametrize("M", [3, 40])
 def test_rows_off_16_bytes(M):
     """Operands that begin 4 bytes past a 16-byte boundary take the kernel without wide loads."""
