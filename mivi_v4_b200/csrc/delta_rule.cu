@@ -163,7 +163,7 @@ MV_API int mv_delta_scan(const float* q, int ldq, const float* k, int ldk, const
 // Two kernels.  delta_prepare does, once per token, what does not depend on the state: q and k as unit vectors
 // (q also times q_scale), k . q of each q/k head, the decays g, and beta; one row of `prep` a token:
 //     [q: kv_heads W | k: kv_heads W | g: heads W | beta: heads | k.q: kv_heads]      (row stride ldp, 32-bit)
-// W is dk, or from 64 key channels on what delta_scan_wide_kernel reads: dk rounded up to 32 R = 64, 128 or 256 (zeros beyond dk)
+// W is dk, or from 64 key channels on what delta_scan_wide_kernel reads: dk rounded up to 32 R = 64, 128, 192 or 256 (zeros beyond dk)
 // in the order in which its lanes own them.
 // delta_scan_long then walks a sequence with nothing but the recurrence in its loop.  The tokens come through
 // shared memory sixteen at a time, the next sixteen on their way (cp.async) while these are worked on.  In the
@@ -270,10 +270,9 @@ __device__ __forceinline__ void dl_stage(float* buf, const float* __restrict__ p
     }
 
 // One buffer of shared memory: [q: CHUNK dk | k: CHUNK dk | g: CHUNK dk | v: CHUNK DR_COLS | beta: CHUNK | k.q: CHUNK]
-// PART lanes share a column of the state (element i of it with lane i % PART).  Keys under 64 channels run here with 8
-// lanes a column; from 64 channels on delta_scan_wide_kernel below takes over.
-template <int R, int PART>
-__global__ void __launch_bounds__(DR_COLS * PART)
+// DR_PART lanes share a column of the state (element i of it with lane i % DR_PART).  Keys under 64 channels run here; from 64 channels on delta_scan_wide_kernel below takes over.
+template <int R>
+__global__ void __launch_bounds__(DR_COLS * DR_PART)
 delta_scan_long_kernel(const float* __restrict__ prep, int ldp, const float* __restrict__ v, int ldv,
                        float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ cu,
                        float* __restrict__ o, int n_heads, int kv_heads, int dk, int dv, int wide) {
@@ -281,7 +280,7 @@ delta_scan_long_kernel(const float* __restrict__ prep, int ldp, const float* __r
     extern __shared__ __align__(16) float dl_smem[];
     const int per = DL_CHUNK * (3 * dk + DR_COLS + 2);
     const int tile = blockIdx.x, h = blockIdx.y, sq = blockIdx.z;
-    const int tid = threadIdx.x, p = tid & (PART - 1), jl = tid / PART;
+    const int tid = threadIdx.x, p = tid & (DR_PART - 1), jl = tid / DR_PART;
     const int j = tile * DR_COLS + jl;
     const int row0 = cu[sq], len = cu[sq + 1] - row0;
     if (len <= 0) return;
@@ -292,13 +291,13 @@ delta_scan_long_kernel(const float* __restrict__ prep, int ldp, const float* __r
     float S[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        const int i = p + PART * r;
+        const int i = p + DR_PART * r;
         S[r] = (j < dv && i < dk) ? srow[i] : 0.f;
     }
     const int col0 = tile * DR_COLS;
 
     auto stage = [&](int c0, float* buf) {
-        dl_stage(buf, prep, ldp, v, ldv, row0, c0, len, h, hk, qk, n_heads, dk, dv, col0, wide, tid, DR_COLS * PART);
+        dl_stage(buf, prep, ldp, v, ldv, row0, c0, len, h, hk, qk, n_heads, dk, dv, col0, wide, tid, DR_COLS * DR_PART);
     };
 
     stage(0, dl_smem);
@@ -328,7 +327,7 @@ delta_scan_long_kernel(const float* __restrict__ prep, int ldp, const float* __r
             float a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
 #pragma unroll
             for (int r = 0; r < R; r += 2) {
-                const int i0 = p + PART * r, i1 = i0 + PART;
+                const int i0 = p + DR_PART * r, i1 = i0 + DR_PART;
                 if (i0 < dk) {
                     S[r] *= gt[i0];
                     a0 = fmaf(S[r], kt[i0], a0);
@@ -342,14 +341,14 @@ delta_scan_long_kernel(const float* __restrict__ prep, int ldp, const float* __r
             }
             float said = a0 + a1, read = b0 + b1;
 #pragma unroll
-            for (int d = 1; d < PART; d <<= 1) {
+            for (int d = 1; d < DR_PART; d <<= 1) {
                 said += __shfl_xor_sync(0xffffffffu, said, d);
                 read += __shfl_xor_sync(0xffffffffu, read, d);
             }
             const float u = bs[t] * ((j < dv ? vs[t * DR_COLS + jl] : 0.f) - said);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                const int i = p + PART * r;
+                const int i = p + DR_PART * r;
                 if (i < dk) S[r] = fmaf(kt[i], u, S[r]);
             }
             if (p == 0 && j < dv) o[(size_t)(row0 + c0 + t) * n_heads * dv + (size_t)h * dv + j] = fmaf(u, ds[t], read);
@@ -360,7 +359,7 @@ delta_scan_long_kernel(const float* __restrict__ prep, int ldp, const float* __r
     if (j < dv && mv_slot_ok(slots[sq])) {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const int i = p + PART * r;
+            const int i = p + DR_PART * r;
             if (i < dk) srow[i] = S[r];
         }
     }
@@ -375,22 +374,26 @@ delta_scan_long_kernel(const float* __restrict__ prep, int ldp, const float* __r
 // 690 us for 2,048 tokens of 16 heads of 128 x 128; without the two further warps 540.  The order in which a sum's parts are
 // added is the same in all of them, and so is every bit.)  2,048 tokens of 16 heads of
 // 128 x 128: 690 -> 395 us (four sequences of 130 to 1,500 tokens, 8 heads: 572 -> 345).
+// `bufs`: two buffers, or one where no sequence brings more than a chunk, so that more blocks fit a multiprocessor (32 sequences of
+// 16 tokens, 8 heads of 128 x 128: 63 us with two buffers, 57 with one, 55 with two columns a warp; of 160 x 128, with R 8 127, now 78
+// and 70).
 constexpr int DW_THREADS = DR_COLS * 8, DW_ALL = DW_THREADS + 64;
-constexpr size_t dw_smem(int R) {
-    return sizeof(float) * 2 * (DL_CHUNK * (3 * 8 * (4 * R + 4) + DR_COLS + 1 + 3) + DL_CHUNK * (DW_THREADS + DR_COLS));
+constexpr size_t dw_smem(int R, int bufs) {
+    return sizeof(float) * bufs * (DL_CHUNK * (3 * 8 * (4 * R + 4) + DR_COLS + 1 + 3) + DL_CHUNK * (DW_THREADS + DR_COLS));
 }
 
 template <int R>
 __global__ void __launch_bounds__(DW_ALL)
 delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __restrict__ v, int ldv,
                        float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ cu,
-                       float* __restrict__ o, int n_heads, int kv_heads, int dk, int dv) {
+                       float* __restrict__ o, int n_heads, int kv_heads, int dk, int dv, int bufs) {
     constexpr int E = 4 * R, LANE = E + 4, ROW = 8 * LANE;
     constexpr int BUF = DL_CHUNK * (3 * ROW + DR_COLS + 4), PART = DL_CHUNK * DW_THREADS;
     mv_pdl_wait();                          // the successor is let go when the last token is done
-    extern __shared__ __align__(16) float dl_smem[];    // 2 x [q | k | g: 16 x ROW; v: 16 x 16; beta: 16 (64)], 2 x parts, 2 x u
-    float* parts = dl_smem + 2 * BUF;       // [16 tokens][16 columns][8 lanes]
-    float* us = parts + 2 * PART;           // [16 tokens][16 columns]
+    extern __shared__ __align__(16) float dl_smem[];    // bufs x [q | k | g: 16 x ROW; v: 16 x 16; beta: 16 (64)], as many parts and u
+    float* parts = dl_smem + bufs * BUF;    // [16 tokens][16 columns][8 lanes]
+    float* us = parts + bufs * PART;        // [16 tokens][16 columns]
+    const int odd = bufs - 1;               // (one buffer: no sequence has a second chunk)
     const int tile = blockIdx.x, h = blockIdx.y, sq = blockIdx.z;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int col0 = tile * DR_COLS;
@@ -404,7 +407,7 @@ delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __r
         const size_t to_g = 2 * (size_t)qk + (size_t)(h - hk) * ROW;
         auto load = [&](int c) {
             const int nt = min(DL_CHUNK, len - c * DL_CHUNK);
-            float* buf = dl_smem + (c & 1) * BUF;
+            float* buf = dl_smem + (c & odd) * BUF;
             for (int t = 0; t < nt; ++t) {
                 const float* src = qp + (size_t)(c * DL_CHUNK + t) * ldp;
                 float* to = buf + t * ROW + lane * 4;
@@ -437,7 +440,7 @@ delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __r
     if (warp > DW_THREADS / 32) {           // outputs of the chunk before
         auto write = [&](int c) {
             const int nt = min(DL_CHUNK, len - c * DL_CHUNK);
-            const float *p = parts + (c & 1) * PART, *u = us + (c & 1) * DL_CHUNK * DR_COLS;
+            const float *p = parts + (c & odd) * PART, *u = us + (c & odd) * DL_CHUNK * DR_COLS;
 #pragma unroll 4
             for (int e = 0; e < DL_CHUNK * DR_COLS / 32; ++e) {
                 const int idx = lane + 32 * e, t = idx / DR_COLS, x = idx % DR_COLS;
@@ -480,14 +483,14 @@ delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __r
     __syncthreads();
     for (int chunk = 0; chunk < n_chunks; ++chunk) {
         const int nt = min(DL_CHUNK, len - chunk * DL_CHUNK);
-        const float* buf = dl_smem + (chunk & 1) * BUF;
+        const float* buf = dl_smem + (chunk & odd) * BUF;
         const float* qs = buf + l * LANE;
         const float* ks = qs + DL_CHUNK * ROW;
         const float* gs = ks + DL_CHUNK * ROW;
         const float* vs = buf + 3 * DL_CHUNK * ROW + jl;
         const float* bs = buf + 3 * DL_CHUNK * ROW + DL_CHUNK * DR_COLS;
-        float* p = parts + (chunk & 1) * PART + tid;
-        float* up = us + (chunk & 1) * DL_CHUNK * DR_COLS + jl;
+        float* p = parts + (chunk & odd) * PART + tid;
+        float* up = us + (chunk & odd) * DL_CHUNK * DR_COLS + jl;
         auto token = [&](int t, const Token& x, Token& next) {
             float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -546,7 +549,7 @@ delta_scan_wide_kernel(const float* __restrict__ prep, int ldp, const float* __r
 }
 
 // Row width of `prep` for these sizes (a multiple of 4 floats, so that rows start on 16 bytes).
-static inline int dl_rounds(int dk) { return dk < 64 ? 0 : dk == 64 ? 2 : dk <= 128 ? 4 : 8; }
+static inline int dl_rounds(int dk) { return dk < 64 ? 0 : dk == 64 ? 2 : dk <= 128 ? 4 : dk <= 192 ? 6 : 8; }
 static inline int dl_width(int dk) { return dk < 64 ? dk : 8 * (4 * dl_rounds(dk) + 4); }
 MV_API int mv_delta_prep_width(int n_heads, int kv_heads, int dk) {
     const int w = (2 * kv_heads + n_heads) * dl_width(dk) + n_heads + kv_heads;
@@ -557,7 +560,7 @@ MV_API int mv_delta_prep_width(int n_heads, int kv_heads, int dk) {
 MV_API int mv_delta_scan_long(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* b,
                               int ldb, const float* a, int lda, const float* dt_bias, const float* a_log, float q_scale,
                               float norm_eps, float* prep, float* state, const int* slots, const int* cu, float* o, int N,
-                              int n_seqs, int n_heads, int kv_heads, int dk, int dv, int head_decay, cudaStream_t stream) {
+                              int n_seqs, int max_len, int n_heads, int kv_heads, int dk, int dv, int head_decay, cudaStream_t stream) {
     if (n_seqs <= 0 || N <= 0) return 0;
     if (dk < 1 || dk > 256 || dv < 1 || kv_heads < 1 || n_heads % kv_heads) return (int)cudaErrorInvalidValue;
     const int ldp = mv_delta_prep_width(n_heads, kv_heads, dk), W = dl_width(dk), R = dl_rounds(dk);
@@ -569,34 +572,25 @@ MV_API int mv_delta_scan_long(const float* q, int ldq, const float* k, int ldk, 
     // long as when they are dealt out over an idle device (measured: 1.26 ms against 0.72 for 2,048 tokens).
     const dim3 grid((dv + DR_COLS - 1) / DR_COLS, n_heads, n_seqs);
     if (R && ((uintptr_t)prep & 15)) return (int)cudaErrorInvalidValue;
-    const size_t smem = R ? dw_smem(R) : 2 * (size_t)DL_CHUNK * (3 * dk + DR_COLS + 2) * sizeof(float);
+    const int bufs = max_len > DL_CHUNK ? 2 : 1;
+    const size_t smem = R ? dw_smem(R, bufs) : 2 * (size_t)DL_CHUNK * (3 * dk + DR_COLS + 2) * sizeof(float);      // below 48 KB with R 0
     // 16-byte copies: every row of q, k and g of a head starts on 16 bytes (ldp is a multiple of 4 floats)
     const int wide = dk % 4 == 0 && (((uintptr_t)prep) & 15) == 0;
-#define DL_LAUNCH(R, PART)                                                                                                   \
-    do {                                                                                                                 \
-        if (smem > 48 * 1024) {                                                                                          \
-            const cudaError_t e = cudaFuncSetAttribute(delta_scan_long_kernel<R, PART>,                                  \
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
-            if (e != cudaSuccess) return (int)e;                                                                         \
-        }                                                                                                                \
-        delta_scan_long_kernel<R, PART><<<grid, DR_COLS * PART, smem, stream>>>((const float*)prep, ldp, v, ldv, state,  \
-                                                                                slots, cu, o, n_heads, kv_heads, dk, dv, \
-                                                                                wide);                                   \
-    } while (0)
+#define DL_LAUNCH(R)                                                                                                     \
+    delta_scan_long_kernel<R><<<grid, DR_COLS * DR_PART, smem, stream>>>((const float*)prep, ldp, v, ldv, state, slots, cu, o,  \
+                                                                         n_heads, kv_heads, dk, dv, wide)
 #define DW_LAUNCH(R)                                                                                                     \
     do {                                                                                                                 \
-        if (smem > 48 * 1024) {                                                                                          \
-            const cudaError_t e = cudaFuncSetAttribute(delta_scan_wide_kernel<R>,                                        \
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
-            if (e != cudaSuccess) return (int)e;                                                                         \
-        }                                                                                                                \
-        delta_scan_wide_kernel<R><<<grid, DW_ALL, smem, stream>>>((const float*)prep, ldp, v, ldv, state, slots,  \
-                                                                        cu, o, n_heads, kv_heads, dk, dv);               \
+        const cudaError_t e = mv_allow_smem<delta_scan_wide_kernel<R>>(dw_smem(R, 2));                                  \
+        if (e != cudaSuccess) return (int)e;                                                                             \
+        delta_scan_wide_kernel<R><<<grid, DW_ALL, smem, stream>>>((const float*)prep, ldp, v, ldv, state, slots, cu, o,  \
+                                                                  n_heads, kv_heads, dk, dv, bufs);                      \
     } while (0)
-    if (dk <= 32) DL_LAUNCH(4, 8);
-    else if (dk < 64) DL_LAUNCH(8, 8);
-    else if (dk == 64) DW_LAUNCH(2);
-    else if (dk <= 128) DW_LAUNCH(4);
+    if (dk <= 32) DL_LAUNCH(4);
+    else if (dk < 64) DL_LAUNCH(8);
+    else if (R == 2) DW_LAUNCH(2);
+    else if (R == 4) DW_LAUNCH(4);
+    else if (R == 6) DW_LAUNCH(6);
     else DW_LAUNCH(8);
 #undef DW_LAUNCH
 #undef DL_LAUNCH

@@ -83,7 +83,8 @@ def test_scalar_scan(monkeypatch, heads, group, dk, dv, pad, lens, normalizer, c
     assert torch.equal(got[0].cpu(), state[0])
 
 
-@pytest.mark.parametrize("heads,kv,dk,dv", [(2, 1, 128, 16), (2, 2, 64, 17), (3, 1, 65, 40), (2, 1, 130, 33), (1, 1, 256, 8), (2, 1, 63, 20)])
+@pytest.mark.parametrize("heads,kv,dk,dv", [(2, 1, 128, 16), (2, 2, 64, 17), (3, 1, 65, 40), (2, 1, 130, 33), (1, 1, 192, 16), (2, 1, 193, 9),
+                                            (1, 1, 256, 8), (2, 1, 63, 20)])
 @pytest.mark.parametrize("lens", [[16], [8, 17], [47, 1, 32]])
 @pytest.mark.parametrize("head_decay", [False, True])
 def test_delta_scan(heads, kv, dk, dv, lens, head_decay):
