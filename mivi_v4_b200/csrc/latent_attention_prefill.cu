@@ -2,8 +2,8 @@
 // tensor cores.  Where a few query tokens fold W_uk into the query and read the cached rows as they are, many query
 // tokens pay for building every head's keys and values once: the cached rows a step can see are copied out of their
 // pages side by side, one product with [W_uk; W_uv] turns them into keys and values for all heads, and the attention
-// itself is attention_sink_prefill.cu's plan: a block is 64 or 128 consecutive query tokens of one sequence for one head, 4
-// warps of 16 or 32 queries; keys and values stream through shared memory in blocks of 64 (cp.async, three buffers); both
+// itself is attention_sink_prefill.cu's plan: a block is 64 consecutive query tokens of one sequence for one head, 4
+// warps of 16 queries; keys and values stream through shared memory in blocks of 64 (cp.async, two or three buffers); both
 // products are mma.sync m16n8k16 with float32 accumulation and the running-maximum softmax in float32 registers
 // between them.  A head's key is [its unrotated part | the rotated part that all heads share]; the sink starts every
 // row's maximum and denominator; the output is multiplied element by element by the sigmoid of a gate.
@@ -17,6 +17,7 @@
 
 namespace {
 
+constexpr int QT = 64;          // queries per block
 constexpr int KB = 64;          // keys per block of the stream
 constexpr int NWARPS = 4;
 constexpr float LOG2E = 1.4426950408889634f;
@@ -125,21 +126,21 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, long long page_stri
 // second product as two bfloat16 numbers each (the rounded weight and what the rounding left), so the sum over the
 // values carries the weights to 16 bits of mantissa although the tensor cores read bfloat16.
 //
-// A warp has MT tiles of 16 queries.  Bound by mma.sync (8 cycles an instruction and scheduler): with MT 2 a key or value
-// fragment that is read from shared memory serves two of them, the reads are ldmatrix, and the softmax of one warp runs under the
-// products of the scheduler's other one.  A row's sums are added in the same order whatever MT is: blocks of 64 keys from multiples
+// Bound by mma.sync and by the softmax between its two products, which runs under the products of a scheduler's other warps: what
+// counts is how many blocks a multiprocessor holds.  So the keys have two buffers, or three where the registers allow two blocks anyway (values
+// above 64, keys up to 128): 4,000 tokens of 32 heads with two / three buffers 527 / 548 us for 64 + 32 / 64, 558 / 661 for 64 + 64 / 64, 725 /
+// 908 for 128 + 64 / 64, 905 / 789 for 64 + 32 / 128, 1,024 / 1,427 for 128 + 64 / 128; 64 prompts of 16 tokens 44 / 44, 44 / 57, 49 / 65, 66 /
+// 60, 68 / 113.  (Two tiles of 16 queries a warp, so that a fragment read serves both, 607 for the first and 64 for its short prompts.)
+// A row's sums are added in the same order wherever it lies: blocks of 64 keys from multiples
 // of 64, 16 channels and 16 keys at a time, and key blocks that a warp's queries cannot see change nothing and are passed over.
-// Longest blocks first, so that no long one is left for the end.  A third of what was issued used to be the copies' addresses and
-// branches, and every score had a branch for the mask.  32 heads of 64 + 32 / 64: 6,000 tokens 2,050 -> 1,205 us (0.37 of what
-// mma.sync gives), three prompts of 333 to 2,048 tokens 355 -> 235 us.
-template <int DKM, int DVM, int MT>
+// Longest blocks first, so that no long one is left for the end.
+template <int DKM, int DVM, int STAGES>
 __global__ void __launch_bounds__(NWARPS * 32)
 latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kx, int ld_kx,
                                 int v0, const __nv_bfloat16* __restrict__ rk, const int* __restrict__ cu,
                                 const int* __restrict__ starts, const float* __restrict__ sinks,
                                 const float* __restrict__ gate, int ld_gate, int gate_heads, __nv_bfloat16* __restrict__ o, int B, int nh,
                                 int dim, int rot, int dv, float scale, int window) {
-    constexpr int QT = NWARPS * 16 * MT, STAGES = 3;
     mv_pdl_begin();
     const int dk = dim + rot;
     const int ldk = dk + 8, ldv = dv + 8;             // padded rows: conflict-free fragment loads
@@ -163,31 +164,28 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
     const int pos0 = starts[b] + tile * QT;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gq = lane >> 2, t4 = lane & 3;
-    const int w0 = warp * 16 * MT;                    // the warp's first query
+    const int w0 = warp * 16;                         // the warp's first query
 
-    unsigned qf[MT][DKM / 16][4];
+    unsigned qf[DKM / 16][4];
+    const int qi = w0 + gq;
+    const __nv_bfloat16* r0 = q + ((size_t)(row0 + min(qi, nq - 1)) * nh + h) * dk;
+    const __nv_bfloat16* r1 = q + ((size_t)(row0 + min(qi + 8, nq - 1)) * nh + h) * dk;
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-        const int qi = w0 + mt * 16 + gq;
-        const __nv_bfloat16* r0 = q + ((size_t)(row0 + min(qi, nq - 1)) * nh + h) * dk;
-        const __nv_bfloat16* r1 = q + ((size_t)(row0 + min(qi + 8, nq - 1)) * nh + h) * dk;
-#pragma unroll
-        for (int kk = 0; kk < DKM / 16; ++kk) {
-            if (kk * 16 < dk) {
-                qf[mt][kk][0] = *reinterpret_cast<const unsigned*>(r0 + kk * 16 + 2 * t4);
-                qf[mt][kk][1] = *reinterpret_cast<const unsigned*>(r1 + kk * 16 + 2 * t4);
-                qf[mt][kk][2] = *reinterpret_cast<const unsigned*>(r0 + kk * 16 + 2 * t4 + 8);
-                qf[mt][kk][3] = *reinterpret_cast<const unsigned*>(r1 + kk * 16 + 2 * t4 + 8);
-            }
+    for (int kk = 0; kk < DKM / 16; ++kk) {
+        if (kk * 16 < dk) {
+            qf[kk][0] = *reinterpret_cast<const unsigned*>(r0 + kk * 16 + 2 * t4);
+            qf[kk][1] = *reinterpret_cast<const unsigned*>(r1 + kk * 16 + 2 * t4);
+            qf[kk][2] = *reinterpret_cast<const unsigned*>(r0 + kk * 16 + 2 * t4 + 8);
+            qf[kk][3] = *reinterpret_cast<const unsigned*>(r1 + kk * 16 + 2 * t4 + 8);
         }
     }
 
-    float oacc[MT][DVM / 8][4], m[MT][2], l[MT][2];
+    float oacc[DVM / 8][4], m[2], l[2];
     const int last_pos = pos0 + nq - 1;
     const int first_key = window > 0 ? max(0, pos0 - window + 1) : 0;
     const int kb_begin = first_key / KB, n_iter = last_pos / KB + 1 - kb_begin;
     // the key blocks that the warp's queries see
-    const int w_last = min(pos0 + w0 + 16 * MT - 1, last_pos), w_first = window > 0 ? max(0, pos0 + w0 - window + 1) : 0;
+    const int w_last = min(pos0 + w0 + 15, last_pos), w_first = window > 0 ? max(0, pos0 + w0 - window + 1) : 0;
     const bool live = w0 < nq;
 
     // eight lanes a row, 16 rows a round: no lane takes another branch than its neighbours (dealt out chunk by chunk, a third of
@@ -210,21 +208,18 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
 
     // One walk over the keys.  ex2 gives 0 for a weight below 2^-126, which is nothing beside the row's other weights as long as its
     // largest is a key's; where that is the sink, far above them all, the block walks once more with an exponential that keeps them
-    // (with exp2f in every walk 6,000 tokens of 32 heads of 64 + 32 / 64 take 1,280 us and not 1,190; 800 of 16 heads of 128 + 64 / 128,
+    // (with exp2f in every walk 6,000 tokens of 32 heads of 64 + 32 / 64 took 1,280 us and not 1,190, two tiles of queries a warp; 800 of 16 heads of 128 + 64 / 128,
     // where it is in the only walk, 45 and with two walks 69).
     auto walk = [&](auto keep_small) {
     auto weight = [&](float x) { return decltype(keep_small)::value ? exp2f(x) : ex2(x); };
     // the sink starts the running maximum and the denominator (its own term, exp(sink - max), is 1 now); a row's
     // denominator is summed over the four lanes of its quad at the end, so one of them holds the sink's 1
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
+    for (int j = 0; j < DVM / 8; ++j)
 #pragma unroll
-        for (int j = 0; j < DVM / 8; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) oacc[mt][j][e] = 0.f;
-        m[mt][0] = m[mt][1] = sinks ? sinks[h] : -INFINITY;
-        l[mt][0] = l[mt][1] = (sinks && t4 == 0) ? 1.f : 0.f;
-    }
+        for (int e = 0; e < 4; ++e) oacc[j][e] = 0.f;
+    m[0] = m[1] = sinks ? sinks[h] : -INFINITY;
+    l[0] = l[1] = (sinks && t4 == 0) ? 1.f : 0.f;
 #pragma unroll
     for (int i = 0; i < STAGES - 1; ++i) {
         if (i < n_iter) load_block(kb_begin + i, i);
@@ -242,15 +237,13 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
 
         const __nv_bfloat16* kt = ks + (size_t)buf * KB * ldk;
         const __nv_bfloat16* vt = vs + (size_t)buf * KB * ldv;
-        float s[MT][KB / 8][4];
+        float s[KB / 8][4];
         const int mi = lane >> 3, r8 = lane & 7;
 #pragma unroll
         for (int j = 0; j < KB / 8; ++j)
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) s[mt][j][e] = 0.f;
-        // channels outside, keys inside: 8 MT sums take turns, no product waits for the one before it
+            for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
+        // channels outside, keys inside: 8 sums take turns, no product waits for the one before it
 #pragma unroll
         for (int kk = 0; kk < DKM / 16; ++kk) {
             if (kk * 16 < dk) {
@@ -258,108 +251,92 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
                 for (int j = 0; j < KB / 8; j += 2) {
                     unsigned kf[4];                                      // 16 keys x 16 elements
                     ldmatrix_x4(kf, kt + (size_t)(j * 8 + (mi >> 1) * 8 + r8) * ldk + kk * 16 + (mi & 1) * 8);
-#pragma unroll
-                    for (int mt = 0; mt < MT; ++mt) {
-                        mma_bf16(s[mt][j], qf[mt][kk][0], qf[mt][kk][1], qf[mt][kk][2], qf[mt][kk][3], kf[0], kf[1]);
-                        mma_bf16(s[mt][j + 1], qf[mt][kk][0], qf[mt][kk][1], qf[mt][kk][2], qf[mt][kk][3], kf[2], kf[3]);
-                    }
+                    mma_bf16(s[j], qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3], kf[0], kf[1]);
+                    mma_bf16(s[j + 1], qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3], kf[2], kf[3]);
                 }
             }
         }
+        const int q0 = pos0 + w0, p0 = q0 + gq, p1 = p0 + 8;
+        const bool need_mask = key0 + KB - 1 > q0 || (window > 0 && key0 <= q0 + 15 - window);
+        float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-            const int q0 = pos0 + w0 + mt * 16, p0 = q0 + gq, p1 = p0 + 8;
-            const bool need_mask = key0 + KB - 1 > q0 || (window > 0 && key0 <= q0 + 15 - window);
-            float mx0 = -INFINITY, mx1 = -INFINITY;
+        for (int j = 0; j < KB / 8; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[j][e] *= scale;
+        if (need_mask) {                          // (one branch a tile; inside the loop it was one a score)
+            const int from0 = window > 0 ? p0 - window : -1, from1 = window > 0 ? p1 - window : -1;
 #pragma unroll
             for (int j = 0; j < KB / 8; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) s[mt][j][e] *= scale;
-            if (need_mask) {                          // (one branch a tile; inside the loop it was one a score)
-                const int from0 = window > 0 ? p0 - window : -1, from1 = window > 0 ? p1 - window : -1;
-#pragma unroll
-                for (int j = 0; j < KB / 8; ++j)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int t = key0 + j * 8 + 2 * t4 + (e & 1);
-                        if (t > (e < 2 ? p0 : p1) || t <= (e < 2 ? from0 : from1)) s[mt][j][e] = -INFINITY;
-                    }
-            }
-#pragma unroll
-            for (int j = 0; j < KB / 8; ++j) {
-                mx0 = fmaxf(mx0, fmaxf(s[mt][j][0], s[mt][j][1]));
-                mx1 = fmaxf(mx1, fmaxf(s[mt][j][2], s[mt][j][3]));
-            }
-            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-            const float mn0 = fmaxf(m[mt][0], mx0), mn1 = fmaxf(m[mt][1], mx1);
-            // a row whose keys are all masked so far (and that has no sink) keeps m = -inf; use 0 as its reference
-            const float ref0 = mn0 == -INFINITY ? 0.f : mn0, ref1 = mn1 == -INFINITY ? 0.f : mn1;
-            const float c0 = m[mt][0] == -INFINITY ? 0.f : weight((m[mt][0] - ref0) * LOG2E);
-            const float c1 = m[mt][1] == -INFINITY ? 0.f : weight((m[mt][1] - ref1) * LOG2E);
-            m[mt][0] = mn0; m[mt][1] = mn1;
-            float sum0 = 0.f, sum1 = 0.f;
-#pragma unroll
-            for (int j = 0; j < KB / 8; ++j) {
-                s[mt][j][0] = weight((s[mt][j][0] - ref0) * LOG2E);
-                s[mt][j][1] = weight((s[mt][j][1] - ref0) * LOG2E);
-                s[mt][j][2] = weight((s[mt][j][2] - ref1) * LOG2E);
-                s[mt][j][3] = weight((s[mt][j][3] - ref1) * LOG2E);
-                sum0 += s[mt][j][0] + s[mt][j][1];
-                sum1 += s[mt][j][2] + s[mt][j][3];
-            }
-            l[mt][0] = l[mt][0] * c0 + sum0;
-            l[mt][1] = l[mt][1] * c1 + sum1;
-            if (__any_sync(0xffffffffu, c0 != 1.f || c1 != 1.f)) {
-#pragma unroll
-                for (int j = 0; j < DVM / 8; ++j) {
-                    oacc[mt][j][0] *= c0; oacc[mt][j][1] *= c0;
-                    oacc[mt][j][2] *= c1; oacc[mt][j][3] *= c1;
+                for (int e = 0; e < 4; ++e) {
+                    const int t = key0 + j * 8 + 2 * t4 + (e & 1);
+                    if (t > (e < 2 ? p0 : p1) || t <= (e < 2 ? from0 : from1)) s[j][e] = -INFINITY;
                 }
+        }
+#pragma unroll
+        for (int j = 0; j < KB / 8; ++j) {
+            mx0 = fmaxf(mx0, fmaxf(s[j][0], s[j][1]));
+            mx1 = fmaxf(mx1, fmaxf(s[j][2], s[j][3]));
+        }
+        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+        const float mn0 = fmaxf(m[0], mx0), mn1 = fmaxf(m[1], mx1);
+        // a row whose keys are all masked so far (and that has no sink) keeps m = -inf; use 0 as its reference
+        const float ref0 = mn0 == -INFINITY ? 0.f : mn0, ref1 = mn1 == -INFINITY ? 0.f : mn1;
+        const float c0 = m[0] == -INFINITY ? 0.f : weight((m[0] - ref0) * LOG2E);
+        const float c1 = m[1] == -INFINITY ? 0.f : weight((m[1] - ref1) * LOG2E);
+        m[0] = mn0; m[1] = mn1;
+        float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+        for (int j = 0; j < KB / 8; ++j) {
+            s[j][0] = weight((s[j][0] - ref0) * LOG2E);
+            s[j][1] = weight((s[j][1] - ref0) * LOG2E);
+            s[j][2] = weight((s[j][2] - ref1) * LOG2E);
+            s[j][3] = weight((s[j][3] - ref1) * LOG2E);
+            sum0 += s[j][0] + s[j][1];
+            sum1 += s[j][2] + s[j][3];
+        }
+        l[0] = l[0] * c0 + sum0;
+        l[1] = l[1] * c1 + sum1;
+        if (__any_sync(0xffffffffu, c0 != 1.f || c1 != 1.f)) {
+#pragma unroll
+            for (int j = 0; j < DVM / 8; ++j) {
+                oacc[j][0] *= c0; oacc[j][1] *= c0;
+                oacc[j][2] *= c1; oacc[j][3] *= c1;
             }
         }
         // O += P V, 16 keys at a time; P = hi + lo
 #pragma unroll
         for (int kk = 0; kk < KB / 16; ++kk) {
-            unsigned hi[MT][4], lw[MT][4];
+            unsigned hi[4], lw[4];
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                for (int f = 0; f < 4; ++f) {
-                    const float x = s[mt][2 * kk + (f >> 1)][(f & 1) * 2], y = s[mt][2 * kk + (f >> 1)][(f & 1) * 2 + 1];
-                    const __nv_bfloat162 hv = __floats2bfloat162_rn(x, y);
-                    hi[mt][f] = *reinterpret_cast<const unsigned*>(&hv);
-                    lw[mt][f] = pack_bf16(x - __uint_as_float(hi[mt][f] << 16), y - __uint_as_float(hi[mt][f] & 0xffff0000u));
-                }
+            for (int f = 0; f < 4; ++f) {
+                const float x = s[2 * kk + (f >> 1)][(f & 1) * 2], y = s[2 * kk + (f >> 1)][(f & 1) * 2 + 1];
+                const __nv_bfloat162 hv = __floats2bfloat162_rn(x, y);
+                hi[f] = *reinterpret_cast<const unsigned*>(&hv);
+                lw[f] = pack_bf16(x - __uint_as_float(hi[f] << 16), y - __uint_as_float(hi[f] & 0xffff0000u));
+            }
 #pragma unroll
             for (int dj = 0; dj < DVM / 16; ++dj) {
                 if (dj * 16 < dv) {
                     unsigned vb[4];
                     ldmatrix_x4_trans(vb, vt + (size_t)(kk * 16 + (mi & 1) * 8 + r8) * ldv + dj * 16 + (mi >> 1) * 8);
-#pragma unroll
-                    for (int mt = 0; mt < MT; ++mt) {
-                        mma_bf16(oacc[mt][2 * dj], hi[mt][0], hi[mt][1], hi[mt][2], hi[mt][3], vb[0], vb[1]);
-                        mma_bf16(oacc[mt][2 * dj + 1], hi[mt][0], hi[mt][1], hi[mt][2], hi[mt][3], vb[2], vb[3]);
-                    }
-#pragma unroll
-                    for (int mt = 0; mt < MT; ++mt) {
-                        mma_bf16(oacc[mt][2 * dj], lw[mt][0], lw[mt][1], lw[mt][2], lw[mt][3], vb[0], vb[1]);
-                        mma_bf16(oacc[mt][2 * dj + 1], lw[mt][0], lw[mt][1], lw[mt][2], lw[mt][3], vb[2], vb[3]);
-                    }
+                    mma_bf16(oacc[2 * dj], hi[0], hi[1], hi[2], hi[3], vb[0], vb[1]);
+                    mma_bf16(oacc[2 * dj + 1], hi[0], hi[1], hi[2], hi[3], vb[2], vb[3]);
+                    mma_bf16(oacc[2 * dj], lw[0], lw[1], lw[2], lw[3], vb[0], vb[1]);
+                    mma_bf16(oacc[2 * dj + 1], lw[0], lw[1], lw[2], lw[3], vb[2], vb[3]);
                 }
             }
         }
     }
     // a row's denominator, in all four lanes of its quad
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            l[mt][half] += __shfl_xor_sync(0xffffffffu, l[mt][half], 1);
-            l[mt][half] += __shfl_xor_sync(0xffffffffu, l[mt][half], 2);
-        }
+    for (int half = 0; half < 2; ++half) {
+        l[half] += __shfl_xor_sync(0xffffffffu, l[half], 1);
+        l[half] += __shfl_xor_sync(0xffffffffu, l[half], 2);
+    }
     };  // walk
 
     constexpr bool TWICE = DKM <= 128 && DVM <= 64;   // (with more sums a second walk's code costs the first its registers)
@@ -367,50 +344,44 @@ latent_attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, const __nv_
     if (TWICE && sinks) {
         bool alone = false;                           // the sink is a row's maximum and all that its denominator shows
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-            for (int half = 0; half < 2; ++half) alone = alone || (live && m[mt][half] == sinks[h] && l[mt][half] == 1.f);
+        for (int half = 0; half < 2; ++half) alone = alone || (live && m[half] == sinks[h] && l[half] == 1.f);
         if (__syncthreads_or(alone)) walk(Flag<true>());
     }
     if (!live) return;
 
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
+    for (int half = 0; half < 2; ++half) {
+        const float den = l[half];
+        const float inv = den > 0.f ? 1.f / den : 0.f;
+        const int qi = w0 + gq + 8 * half;
+        if (qi >= nq) continue;
+        const size_t n = (size_t)(row0 + qi);
+        const float* g = gate && !gate_heads ? gate + n * ld_gate + (size_t)h * dv + 2 * t4 : nullptr;
+        const float gh = (gate && gate_heads ? 1.0f / (1.0f + expf(-gate[n * ld_gate + h])) : 1.f) * inv;
+        __nv_bfloat16* dst = o + (n * nh + h) * dv + 2 * t4;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const float den = l[mt][half];
-            const float inv = den > 0.f ? 1.f / den : 0.f;
-            const int qi = w0 + mt * 16 + gq + 8 * half;
-            if (qi >= nq) continue;
-            const size_t n = (size_t)(row0 + qi);
-            const float* g = gate && !gate_heads ? gate + n * ld_gate + (size_t)h * dv + 2 * t4 : nullptr;
-            const float gh = (gate && gate_heads ? 1.0f / (1.0f + expf(-gate[n * ld_gate + h])) : 1.f) * inv;
-            __nv_bfloat16* dst = o + (n * nh + h) * dv + 2 * t4;
-#pragma unroll
-            for (int j = 0; j < DVM / 8; ++j) {
-                if (j * 8 < dv) {
-                    float x = oacc[mt][j][2 * half] * gh, y = oacc[mt][j][2 * half + 1] * gh;
-                    if (g) {
-                        x *= 1.0f / (1.0f + expf(-g[j * 8]));
-                        y *= 1.0f / (1.0f + expf(-g[j * 8 + 1]));
-                    }
-                    *reinterpret_cast<unsigned*>(dst + j * 8) = pack_bf16(x, y);
+        for (int j = 0; j < DVM / 8; ++j) {
+            if (j * 8 < dv) {
+                float x = oacc[j][2 * half] * gh, y = oacc[j][2 * half + 1] * gh;
+                if (g) {
+                    x *= 1.0f / (1.0f + expf(-g[j * 8]));
+                    y *= 1.0f / (1.0f + expf(-g[j * 8 + 1]));
                 }
+                *reinterpret_cast<unsigned*>(dst + j * 8) = pack_bf16(x, y);
             }
         }
     }
 }
 
-template <int DKM, int DVM, int MT>
+template <int DKM, int DVM, int STAGES>
 int launch(const void* q, const void* kx, int ld_kx, int v0, const void* rk, const int* cu, const int* starts,
            const float* sinks, const float* gate, int ld_gate, int gate_heads, void* o, int N, int B, int nh, int dim, int rot, int dv,
            float scale, int window, cudaStream_t stream) {
-    constexpr int QT = NWARPS * 16 * MT;
-    const size_t smem = (size_t)3 * KB * (dim + rot + 8 + dv + 8) * sizeof(__nv_bfloat16);
-    const cudaError_t attr = mv_allow_smem<latent_attention_prefill_kernel<DKM, DVM, MT>>((size_t)3 * KB * (DKM + 8 + DVM + 8) * sizeof(__nv_bfloat16));
+    const size_t smem = (size_t)STAGES * KB * (dim + rot + 8 + dv + 8) * sizeof(__nv_bfloat16);
+    const cudaError_t attr = mv_allow_smem<latent_attention_prefill_kernel<DKM, DVM, STAGES>>((size_t)STAGES * KB * (DKM + 8 + DVM + 8) * sizeof(__nv_bfloat16));
     if (attr != cudaSuccess) return (int)attr;
     const dim3 grid((N + QT - 1) / QT + B, nh);       // an upper bound of the tiles; spare blocks return at once
-    mv_launch(latent_attention_prefill_kernel<DKM, DVM, MT>, grid, NWARPS * 32, smem, stream, (const __nv_bfloat16*)q,
+    mv_launch(latent_attention_prefill_kernel<DKM, DVM, STAGES>, grid, NWARPS * 32, smem, stream, (const __nv_bfloat16*)q,
               (const __nv_bfloat16*)kx, ld_kx, v0, (const __nv_bfloat16*)rk, cu, starts, sinks, gate, ld_gate,
               gate_heads, (__nv_bfloat16*)o, B, nh, dim, rot, dv, scale, window);
     return mv_launch_status();
@@ -456,14 +427,13 @@ MV_API int mv_latent_attention_prefill(const void* q, const void* kx, int ld_kx,
     if (dim % 8 || rot % 8 || dk % 16 || dv % 16 || dk < 16 || dv < 16 || dk > 192 || dv > 128 || ld_kx % 8 || v0 % 8 ||
         window < 0)
         return (int)cudaErrorInvalidValue;
-#define LP_GO(A, C, M)                                                                                                     \
-    return launch<A, C, M>(q, kx, ld_kx, v0, r, cu, starts, sinks, gate, ld_gate, gate_heads, o, N, B, nh, dim, rot, dv, scale, window, \
+#define LP_GO(A, C, S)                                                                                                     \
+    return launch<A, C, S>(q, kx, ld_kx, v0, r, cu, starts, sinks, gate, ld_gate, gate_heads, o, N, B, nh, dim, rot, dv, scale, window, \
                            stream)
-    // two tiles of queries a warp where their fragments fit the registers and the blocks of 128 queries still go round
-    if (dk <= 96 && dv <= 64 && (long long)N * nh >= 148 * 2 * 64) LP_GO(96, 64, 2);
-    if (dk <= 128 && dv <= 64) LP_GO(128, 64, 1);
-    if (dk <= 128) LP_GO(128, 128, 1);
-    if (dv <= 64) LP_GO(192, 64, 1);
-    LP_GO(192, 128, 1);
+    if (dk <= 96 && dv <= 64) LP_GO(96, 64, 2);
+    if (dk <= 128 && dv <= 64) LP_GO(128, 64, 2);
+    if (dk <= 128) LP_GO(128, 128, 3);
+    if (dv <= 64) LP_GO(192, 64, 2);
+    LP_GO(192, 128, 2);
 #undef LP_GO
 }
