@@ -146,7 +146,7 @@ MV_API int mv_decay_scan(const float* q, int ldq, const float* k, int ldk, const
 // on it is held as a - 1 to full relative precision and the row becomes fma(p, a - 1, p), rounded once a step and nowhere else
 // (64 tokens with decays about 1 - 2^-13: 4.2e-7 off the 64-bit outputs with plain factors, 1.9e-7 so; with an exponential for every
 // difference of sums, as in the kernels for few tokens, 2.1e-7).
-// 2,048 tokens of 8 heads of 128 x 256 with a decay a channel: 43 us this kernel, 59 the walk, 48 the outputs, where preparing
+// 2,048 tokens of 8 heads of 128 x 256 with a decay a channel: 52 us this kernel (43 with plain factors), 59 the walk, 48 the outputs, where preparing
 // with an exponential for every t, s and channel and walking 32 tokens and 16 columns at a time took 64 and 243; of 16 heads
 // of 128 x 128 with a constant decay and the activation: 20 + 3 + 23 + 65 + 55 us against 64 and 243.
 
@@ -356,7 +356,7 @@ MV_API int mv_decay_scan_chunked(const float* q, int ldq, const float* k, int ld
 }
 
 // ---------------------------------------------------------------------------------------------
-// Chunks for steps of few tokens (below 400, the wrapper's DECAY_CHUNKS_FROM): the same sums with 32 tokens a chunk in two launches.
+// Chunks for steps of few tokens (the wrapper's scan_takes_few): the same sums with 32 tokens a chunk in two launches.
 // The first kernel prepares, per (sequence, head, chunk), the decayed q and k, the chunk's total decay and P; the second walks a
 // sequence's chunks with the state in registers and works the outputs out on the way.  Such a step is bound by its launches and by
 // a handful of chunks one after the other: one sequence of 16 tokens 41 us (8 heads of 128 x 256, a decay a channel) and 35 (16 heads

@@ -675,7 +675,7 @@ MV_API int mv_scalar_scan_chunked(const float* q, int ldq, const float* k, int l
 }
 
 // ------------------------------------------------------------------------------------------------
-// Chunks for steps of few tokens (below 128, the wrapper's SCALAR_CHUNKS_FROM): the same sums in the same order in two launches (three
+// Chunks for steps of few tokens (the wrapper's scan_takes_few): the same sums in the same order in two launches (three
 // with a normalizer).  The second kernel walks a sequence's chunks with the state in registers and works the outputs out on the way: a block is
 // 16 value columns of one head of one sequence, its 32 half-warps each hold RH key channels of every column.  Such a step is bound by its
 // launches: 16 tokens of 64 heads of 128 x 64 in one group 36 us against 46 with the four kernels above, 64 tokens 46 against 51, 128 57

@@ -671,7 +671,7 @@ def scalar_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_a: torch.
     norm = m_tok is not None
     _need(state, "scalar_scan state", torch.float32, (None, n_heads, dv + (1 if norm else 0), dk))
     _guard("core", "scalar_scan", out.device, n_slots=state.shape[0])
-    if ws is not None and max_len >= SCAN_CHUNKED_FROM and N < SCALAR_CHUNKS_FROM:
+    if ws is not None and max_len >= SCAN_CHUNKED_FROM and scan_takes_few("token", N, n_seqs, max_len, n_heads, dk, dv):
         chunks = int(_fn("core", "mv_scalar_chunks")(N, int(n_seqs)))
         G = ws.get("scalar_scan_products", (chunks, groups, SCAN_CHUNK, SCAN_CHUNK), torch.float32)
         o_aug = ws.get("scalar_scan_o_aug", (N, n_heads * (dv + 1)), torch.float32) if norm else None
@@ -998,10 +998,24 @@ SCAN_ACT_NONE, SCAN_ACT_SILU = 0, 1
 SCAN_CHUNKED_FROM = 16          # a step whose longest sequence brings this many tokens walks them in chunks
 SCAN_CHUNK = 32                 # of scalar_scan, and of decay_scan's steps of few tokens
 DECAY_CHUNK = 64                # of decay_scan
-# Chunked steps of fewer tokens in all are bound by launches and take kernels that do more in each (the figures where both are equal
-# stand beside those kernels in decay_scan.cu and scalar_scan.cu)
-DECAY_CHUNKS_FROM = 400
-SCALAR_CHUNKS_FROM = 128
+# Chunked steps that are short are bound by launches and take kernels that do more in each.  What they cost grows with the chunks of 32 tokens
+# one after the other: a sequence's own, or those of all heads and 16 value columns where they do not fit the device side by side.
+# Up to so many of them they are the faster ones (13 shapes x 25 batches: at most 1.1 times the other kernels' time where they are
+# left, and a launch or three fewer): a decay a channel, a decay a head, a decay a token.
+FEW_CHUNKS = {"channel": 10, "head": 8, "token": 5}
+
+
+def scan_takes_few(kind: str, N: int, n_seqs: int, max_len: int, n_heads: int, dk: int, dv: int) -> bool:
+    """Whether a chunked scan of this step takes the kernels for few tokens."""
+    chain = max_len / SCAN_CHUNK
+    if kind == "channel" and dk <= 32:
+        # the other kernels pad such keys to 128: 16 sequences of 128 tokens, 32 heads of 32 x 32, 238 us against 139
+        return chain <= FEW_CHUNKS[kind]
+    side_by_side = -(-dv // 16) * n_heads * (N / SCAN_CHUNK + n_seqs / 2) / n_sms()
+    longer = 1.3 if kind == "token" and dk > 128 else 1.0       # (twice the key channels a thread)
+    return max(chain, side_by_side) * longer <= FEW_CHUNKS[kind]
+
+
 # The states before a step's chunks are scratch that an engine keeps: so many bytes of them at a time.  64 heads of 128 x 64 with one decay a
 # token, at 64 / 128 / 256 MB / all at once: one sequence of 2,048 tokens (134 MB) 254 / 251 / 233 / 235 us, of 8,192 890 / 961 / 940 / 1,029, 32 of 256
 # 937 / 829 / 759 / 687, 512 of 16 4,341 / 2,949 / 2,274 / 1,601 (1.6 GB).
@@ -1035,7 +1049,7 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
     float32 and may be column slices of one wider matrix; ``act`` is applied to all three as they are read
     and ``q_scale`` multiplies q.  Everything is computed in float32.  ``max_len``: the most tokens that a
     sequence brings; with ``ws`` (a Workspace, for scratch) steps of ``SCAN_CHUNKED_FROM`` tokens a sequence and
-    more take kernels that work in chunks of 32 or, from ``DECAY_CHUNKS_FROM`` tokens in the step on, of 64 tokens, whose sums
+    more take kernels that work in chunks of 32 or, in steps of many tokens (:func:`scan_takes_few`), of 64 tokens, whose sums
     come in another order (the results differ from the token-by-token kernel's, and from each other, by rounding)."""
     N = out.shape[0]
     if not 1 <= dk <= MAX_SCAN_KEY_DIM:
@@ -1048,7 +1062,8 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
     zp, ldz = _cols(decay_logits, "decay_scan decay logits", N, n_heads * dk) if decay_logits is not None else (None, 0)
     _need(state, "decay_scan state", torch.float32, (None, n_heads, dv, dk))
     _guard("core", "decay_scan", out.device, n_slots=state.shape[0])
-    if ws is not None and max_len >= SCAN_CHUNKED_FROM and N < DECAY_CHUNKS_FROM:
+    if ws is not None and max_len >= SCAN_CHUNKED_FROM and scan_takes_few(
+            "head" if decay_logits is None else "channel", N, n_seqs, max_len, n_heads, dk, dv):
         chunks = int(_fn("core", "mv_decay_few_chunks")(N, int(n_seqs)))
         qd = ws.get("scan_qd", (N, n_heads * dk), torch.float32)
         kd = ws.get("scan_kd", (N, n_heads * dk), torch.float32)

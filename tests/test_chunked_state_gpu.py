@@ -16,7 +16,7 @@ F64 = torch.float64
 def kernels_for(request, monkeypatch):
     """Every case with the kernels for steps of few tokens and with those for many, whatever the step's size would choose."""
     from mivi_v4_b200.ops import kernels as K
-    monkeypatch.setattr(K, "DECAY_CHUNKS_FROM", 0 if request.param == "many" else 1 << 30)
+    monkeypatch.setattr(K, "scan_takes_few", lambda *a: request.param == "few")
     return request.param
 
 
@@ -118,9 +118,9 @@ def test_decay_near_one(kernels_for, tokens, shift, inv_tau):
     assert (out.double().cpu() - want).norm() / want.norm() <= 2.2e-7
 
 
-@pytest.mark.parametrize("tokens,few", [(16, True), (399, True), (400, False)])
+@pytest.mark.parametrize("tokens,few", [(16, True), (320, True), (321, False)])
 def test_which_kernels(monkeypatch, tokens, few):
-    """A step's tokens in all choose: below DECAY_CHUNKS_FROM the two launches that suit a short prompt."""
+    """Up to ten chunks of 32 tokens one after the other a step takes the two launches that suit a short prompt."""
     from mivi_v4_b200.ops import kernels as K
     monkeypatch.undo()
     x, before = torch.randn(tokens, 32, device=DEV), K.launch_count()

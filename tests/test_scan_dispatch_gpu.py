@@ -36,10 +36,10 @@ def close(got, want, tol, what):
 @pytest.mark.parametrize("heads,group,dk,dv,pad", [(1, 1, 128, 64, 0), (2, 2, 33, 65, 0), (3, 1, 4, 7, 1), (6, 3, 64, 64, 3), (2, 1, 200, 66, 0)])
 @pytest.mark.parametrize("lens", [[32], [16, 1, 33], [95, 64]])
 @pytest.mark.parametrize("normalizer", [False, True])
-@pytest.mark.parametrize("chunks_from", [0, 1 << 30])        # the kernels for many tokens, and those for few
-def test_scalar_scan(monkeypatch, heads, group, dk, dv, pad, lens, normalizer, chunks_from):
+@pytest.mark.parametrize("few", [False, True])               # the kernels for many tokens, and those for few
+def test_scalar_scan(monkeypatch, heads, group, dk, dv, pad, lens, normalizer, few):
     from mivi_v4_b200.ops import kernels as K
-    monkeypatch.setattr(K, "SCALAR_CHUNKS_FROM", chunks_from)
+    monkeypatch.setattr(K, "scan_takes_few", lambda *a: few)
     g = torch.Generator().manual_seed(heads * 1000 + dk + sum(lens))
     N, groups, B, cu = sum(lens), heads // group, len(lens), starts_of(lens)
     q, k = (torch.randn(N, groups * dk, generator=g) for _ in "qk")
@@ -126,8 +126,8 @@ def test_scalar_scan_few_and_many_agree(monkeypatch):
         q, k, v, m = r(N, heads // group * dk), r(N, heads // group * dk), r(N, heads * dv), r(N, heads)
         log_a, b, state = -r(N, heads).abs(), r(N, heads).abs(), r(B, heads, dv + norm, dk)
         got = []
-        for chunks_from in (0, 1 << 30):
-            monkeypatch.setattr(K, "SCALAR_CHUNKS_FROM", chunks_from)
+        for few in (False, True):
+            monkeypatch.setattr(K, "scan_takes_few", lambda *a: few)
             s, out = state.clone(), torch.full((N, heads * dv), float("nan"), device=DEV)
             K.scalar_scan(q, k, v, log_a, b, s, i32(list(range(B))), i32(starts_of(lens)), out, B, heads, dk, dv, heads_per_group=group,
                           m_tok=m if norm else None, q_scale=0.1, max_len=max(lens), ws=Scratch())
@@ -135,7 +135,7 @@ def test_scalar_scan_few_and_many_agree(monkeypatch):
         assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
-@pytest.mark.parametrize("tokens,few", [(16, True), (127, True), (128, False)])
+@pytest.mark.parametrize("tokens,few", [(16, True), (160, True), (161, False)])
 def test_which_kernels(tokens, few):
     from mivi_v4_b200.ops import kernels as K
     x, ones, before = torch.randn(tokens, 32, device=DEV), torch.ones(tokens, 1, device=DEV), K.launch_count()

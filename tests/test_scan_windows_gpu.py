@@ -27,6 +27,20 @@ def test_room_is_bounded(state_bytes):
         assert held <= max(K.SCAN_STATES_BYTES, 10 * state_bytes)
 
 
+def test_which_steps_are_short():
+    """By the chunks one after the other: a sequence's own or, where they do not fit side by side, all heads' and columns'."""
+    n = 148 if not torch.cuda.is_available() else K.n_sms()
+    few = K.scan_takes_few
+    assert few("channel", 320, 1, 320, 8, 128, 256) and not few("channel", 321, 1, 321, 8, 128, 256)
+    assert few("head", 256, 1, 256, 1, 128, 16) and not few("head", 257, 1, 257, 1, 128, 16)
+    assert few("token", 160, 1, 160, 1, 128, 16) and not few("token", 161, 1, 161, 1, 128, 16)
+    assert few("token", 123, 1, 123, 1, 200, 16) and not few("token", 124, 1, 124, 1, 200, 16)
+    # 64 sequences of 16 tokens are 64 chunks for each head and 16 columns
+    heads = 10 * n // 64
+    assert few("channel", 1024, 64, 16, heads, 128, 16) and not few("channel", 1024, 64, 16, heads + 2, 128, 16)
+    assert few("channel", 1024, 64, 16, heads + 2, 32, 16)
+
+
 def i32(v):
     return torch.tensor(v, dtype=torch.int32, device=DEV)
 
@@ -53,7 +67,7 @@ def test_same_bits_in_windows(monkeypatch, lens, kind, heads, dk, dv):
     for room in (1 << 30, 1, 2, 3, 10):
         monkeypatch.setattr(K, "scan_room", lambda chunks, state_bytes: min(room, chunks))
         s, out, ws = state.clone(), torch.full((N, heads * dv), float("nan"), device=DEV), Scratch()
-        monkeypatch.setattr(K, "DECAY_CHUNKS_FROM", 0)
+        monkeypatch.setattr(K, "scan_takes_few", lambda *a: False)
         if kind.startswith("scalar"):
             K.scalar_scan(q, k, v, log_a, b, s, slots, i32(cu), out, B, heads, dk, dv, m_tok=m if norm else None, q_scale=0.1,
                           max_len=max(lens), ws=ws)
