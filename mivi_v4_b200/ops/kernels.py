@@ -1000,20 +1000,22 @@ SCAN_CHUNK = 32                 # of scalar_scan, and of decay_scan's steps of f
 DECAY_CHUNK = 64                # of decay_scan
 # Chunked steps that are short are bound by launches and take kernels that do more in each.  What they cost grows with the chunks of 32 tokens
 # one after the other: a sequence's own, or those of all heads and 16 value columns where they do not fit the device side by side.
-# Up to so many of them they are the faster ones (13 shapes x 25 batches: at most 1.1 times the other kernels' time where they are
-# left, and a launch or three fewer): a decay a channel, a decay a head, a decay a token.
-FEW_CHUNKS = {"channel": 10, "head": 8, "token": 5}
+# Up to so many of the former and of the latter they are taken, for a decay a channel, a decay a head, a decay a token.  The lines lie where
+# both take as long with 5 us for the other kernels' further launches (13 shapes x 25 batches; on the device alone a step is at most 1.35 times as
+# long as with the other kernels where they are left, in all but 10 of 1,325 at most 1.05 times, and 1.6 times where they are taken).
+FEW_CHUNKS = {"channel": (10, 10), "head": (6, 10), "token": (5, 5)}
 
 
 def scan_takes_few(kind: str, N: int, n_seqs: int, max_len: int, n_heads: int, dk: int, dv: int) -> bool:
     """Whether a chunked scan of this step takes the kernels for few tokens."""
-    chain = max_len / SCAN_CHUNK
+    own, all_heads = FEW_CHUNKS[kind]
+    longer = 1.3 if kind == "token" and dk > 128 else 1.0       # (twice the key channels a thread)
+    if max_len / SCAN_CHUNK * longer > own:
+        return False
     if kind == "channel" and dk <= 32:
         # the other kernels pad such keys to 128: 16 sequences of 128 tokens, 32 heads of 32 x 32, 238 us against 139
-        return chain <= FEW_CHUNKS[kind]
-    side_by_side = -(-dv // 16) * n_heads * (N / SCAN_CHUNK + n_seqs / 2) / n_sms()
-    longer = 1.3 if kind == "token" and dk > 128 else 1.0       # (twice the key channels a thread)
-    return max(chain, side_by_side) * longer <= FEW_CHUNKS[kind]
+        return True
+    return -(-dv // 16) * n_heads * (N / SCAN_CHUNK + n_seqs / 2) / n_sms() * longer <= all_heads
 
 
 # The states before a step's chunks are scratch that an engine keeps: so many bytes of them at a time.  64 heads of 128 x 64 with one decay a

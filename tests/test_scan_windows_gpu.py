@@ -32,7 +32,7 @@ def test_which_steps_are_short():
     n = 148 if not torch.cuda.is_available() else K.n_sms()
     few = K.scan_takes_few
     assert few("channel", 320, 1, 320, 8, 128, 256) and not few("channel", 321, 1, 321, 8, 128, 256)
-    assert few("head", 256, 1, 256, 1, 128, 16) and not few("head", 257, 1, 257, 1, 128, 16)
+    assert few("head", 192, 1, 192, 1, 128, 16) and not few("head", 193, 1, 193, 1, 128, 16)
     assert few("token", 160, 1, 160, 1, 128, 16) and not few("token", 161, 1, 161, 1, 128, 16)
     assert few("token", 123, 1, 123, 1, 200, 16) and not few("token", 124, 1, 124, 1, 200, 16)
     # 64 sequences of 16 tokens are 64 chunks for each head and 16 columns
