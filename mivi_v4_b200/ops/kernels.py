@@ -129,6 +129,7 @@ _SIGNATURES = {
         "mv_latent_attention_decode": [_P, _P, _Q, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _P, _P, _P, _P],
         "mv_latent_query": [_P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _P],
         "mv_latent_gather": [_P, _Q, _P, _I, _I, _P, _P, _I, _I, _I, _I, _P, _P, _I, _P],
+        "mv_latent_attention_tc": [_P, _P, _I, _I, _I, _P, _P, _P, _P, _P, _I, _I, _P, _I, _I, _I, _I, _F, _I, _P, _P],
         "mv_latent_attention_prefill": [_P, _P, _I, _I, _P, _P, _P, _P, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P],
     },
 }
@@ -1543,6 +1544,19 @@ def latent_prefill_fits(dim: int, rot: int, dv: int, rank: int) -> bool:
         and 16 <= dv <= 128 and rank % 8 == 0
 
 
+# The tcgen05 kernel's blocks are 256 query tokens of one sequence: it takes steps whose sequences fill such a block or have many keys (its bits are the
+# other kernel's).  32 heads of 64 + 32 / 64 with a gate, this kernel / the other: 32 prompts of 64 tokens 109 / 56 us, 32 of 128 123 / 96, 16 of 200
+# 82 / 95, 8 of 300 74 / 76, 4 of 256 27 / 44, one of 1,024 39 / 74, one of 6,000 363 / 1,132; behind 190 earlier tokens 16 times 64 tokens 72 / 51,
+# behind 300 8 times 128 tokens 45 / 66, behind 800 3 times 32 tokens 33 / 53.
+LATENT_TC_TOKENS, LATENT_TC_ROWS = 200, 400
+
+
+def latent_tc_takes(N: int, rows: int, n_seqs: int, dim: int, rot: int, dv: int, scale: float) -> bool:
+    """Whether the tcgen05 kernel takes a step of ``N`` tokens of ``n_seqs`` sequences that see ``rows`` cached rows."""
+    return (dim == 64 and rot in (32, 64) and dv == 64 and scale > 0 and (N + 255) // 256 + n_seqs <= 65535 and rows < 2 ** 31
+            and (N >= LATENT_TC_TOKENS * n_seqs or rows >= LATENT_TC_ROWS * n_seqs))
+
+
 def latent_query(proj: torch.Tensor, q0: int, inv_freq: Optional[torch.Tensor], positions, q: torch.Tensor, nh: int,
                  dim: int, rot: int, rot_dims: int, amplitude: float = 1.0) -> torch.Tensor:
     """``q`` [N, nh, dim + rot] (bfloat16) from float32 rows of a projection (the queries from column ``q0``), the first
@@ -1594,6 +1608,15 @@ def latent_attention_prefill(q: torch.Tensor, kx: torch.Tensor, v0: int, r: torc
         raise KernelError(f"latent_attention_prefill: keys and values {kx.dtype} {tuple(kx.shape)}, values from {v0}")
     per_head = gate is not None and gate.shape[1] == nh
     gp, ldg = _cols(gate, "latent_attention_prefill gate", N, nh if per_head else nh * dv) if gate is not None else (None, 0)
+    if latent_tc_takes(N, rows, n_seqs, dim, rot, dv, scale) and kx.stride(0) % 8 == 0 and v0 % 8 == 0 and not any(
+            t.data_ptr() % 16 for t in (q, kx, r, out)):
+        _check(_fn("bf16", "mv_latent_attention_tc")(
+            _need(q, "q", torch.bfloat16, (N, nh, dim + rot)), kx.data_ptr(), rows, kx.stride(0), int(v0),
+            _need(r, "rotated keys", torch.bfloat16, (rows, rot)), _need(cu, "cu", torch.int32),
+            _need(starts, "starts", torch.int32), _need(sinks, "sinks", torch.float32, (nh,), True), gp, ldg, int(per_head),
+            _need(out, "attention out", torch.bfloat16, (N, nh * dv)), N, int(n_seqs), nh, rot, float(scale), int(window),
+            _error_flag(q.device).data_ptr(), _stream()), "mv_latent_attention_tc")
+        return out
     _check(_fn("bf16", "mv_latent_attention_prefill")(
         _need(q, "q", torch.bfloat16, (N, nh, dim + rot)), kx.data_ptr(), kx.stride(0), int(v0),
         _need(r, "rotated keys", torch.bfloat16, (rows, rot)), _need(cu, "cu", torch.int32),
