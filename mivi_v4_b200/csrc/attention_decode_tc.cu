@@ -125,7 +125,7 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     const int per = (blocks_all + splits - 1) / splits;
     const int j0 = split * per, n_blocks = max(0, min(blocks_all, j0 + per) - j0);
     const int* table = page_table + (size_t)seq_of[n] * table_stride;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         mbar_init(bar(B_Q), 1);
@@ -156,21 +156,25 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         // registers move from this warpgroup to the softmax warps (128 each at launch)
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         if (warp == 0) {
-            if (lane == 0 && n_blocks > 0) {
-                // head i of the group: one row of 128 bytes, row i of the Q tile (the MMA's N side)
+            // head i of the group: one row of 128 bytes, row i of the Q tile (the MMA's N side)
+            if (n_blocks > 0 && elect_one()) {
                 mbar_expect_tx(bar(B_Q), (unsigned)G * HD * 2);
                 for (int i = 0; i < G; ++i) tma_load_2d(q_s + (unsigned)(i * 128), &map_q, 0, n * nh + g * G + i, bar(B_Q));
-                for (int j = 0; j < n_blocks; ++j) {
-                    const int s = j % STAGES_KV;
-                    const unsigned ph = (unsigned)(j / STAGES_KV) & 1u;
-                    const int jb = j0 + j;
-                    const int pg0 = table[min(2 * jb, table_stride - 1)], pg1 = table[min(2 * jb + 1, table_stride - 1)];
-                    if (!mbar_wait(bar(B_KEMPTY + s), ph ^ 1u, err, 31)) break;
+            }
+            for (int j = 0; j < n_blocks; ++j) {
+                const int s = j % STAGES_KV;
+                const unsigned ph = (unsigned)(j / STAGES_KV) & 1u;
+                const int jb = j0 + j;
+                const int pg0 = table[min(2 * jb, table_stride - 1)], pg1 = table[min(2 * jb + 1, table_stride - 1)];
+                if (!mbar_wait_warp(bar(B_KEMPTY + s), ph ^ 1u, err, 31)) break;
+                if (elect_one()) {
                     mbar_expect_tx(bar(B_KFULL + s), KV_BYTES);
                     tma_load_2d(k_s + s * KV_BYTES, &map_kv, 0, ((pg0 * 2 + 0) * nkv + g) * PAGE, bar(B_KFULL + s));
                     tma_load_2d(k_s + s * KV_BYTES + KV_BYTES / 2, &map_kv, 0, ((pg1 * 2 + 0) * nkv + g) * PAGE,
                                 bar(B_KFULL + s));
-                    if (!mbar_wait(bar(B_VEMPTY + s), ph ^ 1u, err, 32)) break;
+                }
+                if (!mbar_wait_warp(bar(B_VEMPTY + s), ph ^ 1u, err, 32)) break;
+                if (elect_one()) {
                     mbar_expect_tx(bar(B_VFULL + s), KV_BYTES);
                     tma_load_2d(v_s + s * KV_BYTES, &map_kv, 0, ((pg0 * 2 + 1) * nkv + g) * PAGE, bar(B_VFULL + s));
                     tma_load_2d(v_s + s * KV_BYTES + KV_BYTES / 2, &map_kv, 0, ((pg1 * 2 + 1) * nkv + g) * PAGE,
@@ -178,20 +182,21 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 }
             }
         } else if (warp == 1) {
-            if (lane == 0 && n_blocks > 0) {
+            if (n_blocks > 0) {
                 const unsigned idesc_qk = instr_desc(BKV, NQ);                      // keys x heads
                 const unsigned idesc_pv = instr_desc(BQ, HD) | (1u << 16);          // B operand MN-major
-                bool ok = mbar_wait(bar(B_Q), 0, err, 33);
+                bool ok = mbar_wait_warp(bar(B_Q), 0, err, 33);
                 auto issue_qk = [&](int j) {
                     const int s = j % STAGES_KV;
-                    if (!mbar_wait(bar(B_KFULL + s), (unsigned)(j / STAGES_KV) & 1u, err, 34)) return false;
+                    if (!mbar_wait_warp(bar(B_KFULL + s), (unsigned)(j / STAGES_KV) & 1u, err, 34)) return false;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const unsigned long long kd = smem_desc(k_s + s * KV_BYTES), qd = smem_desc(q_s);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < HD / 16; ++k)
-                        mma_f16(tmem_base + S_COL0, smem_desc(k_s + s * KV_BYTES + k * 32), smem_desc(q_s + k * 32),
-                                idesc_qk, k > 0 ? 1u : 0u);
-                    mma_commit(bar(B_SFULL));
-                    mma_commit(bar(B_KEMPTY + s));
+                        for (int k = 0; k < HD / 16; ++k) mma_f16(tmem_base + S_COL0, kd + 2 * k, qd + 2 * k, idesc_qk, k > 0 ? 1u : 0u);
+                        mma_commit(bar(B_SFULL));
+                        mma_commit(bar(B_KEMPTY + s));
+                    }
                     return true;
                 };
                 if (ok) ok = issue_qk(0);
@@ -199,21 +204,20 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                     const int s = j % STAGES_KV;
                     if (j + 1 < n_blocks) {
                         // S^T of block j is in the softmax warps' registers: its columns are free for block j + 1
-                        if (!(ok = mbar_wait(bar(B_SEMPTY), (unsigned)j & 1u, err, 35))) break;
+                        if (!(ok = mbar_wait_warp(bar(B_SEMPTY), (unsigned)j & 1u, err, 35))) break;
                         if (!(ok = issue_qk(j + 1))) break;
                     }
-                    if (!(ok = mbar_wait(bar(B_PFULL), (unsigned)j & 1u, err, 36))) break;
-                    if (!(ok = mbar_wait(bar(B_VFULL + s), (unsigned)(j / STAGES_KV) & 1u, err, 37))) break;
+                    if (!(ok = mbar_wait_warp(bar(B_PFULL), (unsigned)j & 1u, err, 36))) break;
+                    if (!(ok = mbar_wait_warp(bar(B_VFULL + s), (unsigned)(j / STAGES_KV) & 1u, err, 37))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const unsigned long long pd = smem_desc(p_s), vd = smem_desc_mn(v_s + s * KV_BYTES);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BKV / 16; ++k) {
-                        const unsigned a_addr = p_s + (k >> 2) * (BQ * 128) + (k & 3) * 32;
-                        const unsigned b_addr = v_s + s * KV_BYTES + k * 16 * 128;
-                        mma_f16(tmem_base + O_COL0, smem_desc(a_addr), smem_desc_mn(b_addr), idesc_pv,
-                                (j > 0 || k > 0) ? 1u : 0u);
+                        for (int k = 0; k < BKV / 16; ++k)
+                            mma_f16(tmem_base + O_COL0, pd + (k >> 2) * (BQ * 128 / 16) + (k & 3) * 2, vd + k * 128, idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
+                        mma_commit(bar(B_PVDONE));
+                        mma_commit(bar(B_VEMPTY + s));
                     }
-                    mma_commit(bar(B_PVDONE));
-                    mma_commit(bar(B_VEMPTY + s));
                 }
             }
         }

@@ -166,7 +166,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     for (int t = 0; t < TILES; ++t) nb[t] = nq > t * BQ ? (pos0 + min(nq, (t + 1) * BQ) - 1) / BKV + 1 : 0;
     const int nb_max = max(nb[0], nb[1]);
     const int* table = page_table + (size_t)b * table_stride;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         mbar_init(bar(B_Q), 1);
@@ -200,19 +200,23 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         // registers move from this warpgroup to the softmax warps (168 each at launch)
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         if (warp == 0) {
-            if (lane == 0) {
+            if (elect_one()) {
                 mbar_expect_tx(bar(B_Q), TILES * Q_BYTES);
                 for (int t = 0; t < TILES; ++t) tma_load_2d(q_s + t * Q_BYTES, &map_q, h * HD, row0 + t * BQ, bar(B_Q));
-                for (int j = 0; j < nb_max; ++j) {
-                    const int s = j % STAGES_KV;
-                    const unsigned ph = (unsigned)(j / STAGES_KV) & 1u;
-                    const int pg0 = table[min(2 * j, table_stride - 1)], pg1 = table[min(2 * j + 1, table_stride - 1)];
-                    if (!mbar_wait(bar(B_KEMPTY + s), ph ^ 1u, err, 11)) break;
+            }
+            for (int j = 0; j < nb_max; ++j) {
+                const int s = j % STAGES_KV;
+                const unsigned ph = (unsigned)(j / STAGES_KV) & 1u;
+                const int pg0 = table[min(2 * j, table_stride - 1)], pg1 = table[min(2 * j + 1, table_stride - 1)];
+                if (!mbar_wait_warp(bar(B_KEMPTY + s), ph ^ 1u, err, 11)) break;
+                if (elect_one()) {
                     mbar_expect_tx(bar(B_KFULL + s), KV_BYTES);
                     tma_load_2d(k_s + s * KV_BYTES, &map_kv, 0, ((pg0 * 2 + 0) * nkv + g) * PAGE, bar(B_KFULL + s));
                     tma_load_2d(k_s + s * KV_BYTES + KV_BYTES / 2, &map_kv, 0, ((pg1 * 2 + 0) * nkv + g) * PAGE,
                                 bar(B_KFULL + s));
-                    if (!mbar_wait(bar(B_VEMPTY + s), ph ^ 1u, err, 12)) break;
+                }
+                if (!mbar_wait_warp(bar(B_VEMPTY + s), ph ^ 1u, err, 12)) break;
+                if (elect_one()) {
                     mbar_expect_tx(bar(B_VFULL + s), KV_BYTES);
                     tma_load_2d(v_s + s * KV_BYTES, &map_kv, 0, ((pg0 * 2 + 1) * nkv + g) * PAGE, bar(B_VFULL + s));
                     tma_load_2d(v_s + s * KV_BYTES + KV_BYTES / 2, &map_kv, 0, ((pg1 * 2 + 1) * nkv + g) * PAGE,
@@ -220,62 +224,61 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 }
             }
         } else if (warp == 1) {
-            if (lane == 0) {
-                const unsigned idesc_qk = instr_desc(BQ, BKV);
-                const unsigned idesc_pv = instr_desc(BQ, HD) | (1u << 16);          // B operand MN-major
-                bool ok = mbar_wait(bar(B_Q), 0, err, 13);
-                // S(t, j) = Q_t K_j^T; the caller has waited for K_j
-                auto issue_qk = [&](int t, int j) {
-                    const int s = j % STAGES_KV;
-    #pragma unroll
-                    for (int k = 0; k < HD / 16; ++k)
-                        mma_f16(tmem_base + S_COL0 + (unsigned)t * BKV, smem_desc(q_s + t * Q_BYTES + k * 32),
-                                smem_desc(k_s + s * KV_BYTES + k * 32), idesc_qk, k > 0 ? 1u : 0u);
-                    mma_commit(bar(B_SFULL + t));
-                };
-                if (ok) ok = mbar_wait(bar(B_KFULL), 0, err, 14);
-                if (ok) {
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    #pragma unroll
-                    for (int t = 0; t < TILES; ++t)
-                        if (nb[t] > 0) issue_qk(t, 0);
-                    mma_commit(bar(B_KEMPTY));
-                }
-                for (int j = 0; j < nb_max && ok; ++j) {
-                    const int s = j % STAGES_KV, s1 = (j + 1) % STAGES_KV;
-                    const unsigned ph = (unsigned)(j / STAGES_KV) & 1u, ph1 = (unsigned)((j + 1) / STAGES_KV) & 1u;
-                    // S(t, j + 1) as soon as the tile's softmax warps hold S(t, j) in registers
-                    if (j + 1 < nb_max) {
-                        if (!(ok = mbar_wait(bar(B_KFULL + s1), ph1, err, 14))) break;
+            const unsigned idesc_qk = instr_desc(BQ, BKV);
+            const unsigned idesc_pv = instr_desc(BQ, HD) | (1u << 16);              // B operand MN-major
+            bool ok = mbar_wait_warp(bar(B_Q), 0, err, 13);
+            // S(t, j) = Q_t K_j^T; the caller has waited for K_j
+            auto issue_qk = [&](int t, int j) {
+                const unsigned long long qd = smem_desc(q_s + t * Q_BYTES), kd = smem_desc(k_s + (j % STAGES_KV) * KV_BYTES);
+                if (elect_one()) {
 #pragma unroll
-                        for (int t = 0; t < TILES; ++t) {
-                            if (!ok || j + 1 >= nb[t]) continue;
-                            if (!(ok = mbar_wait(bar(B_SFREE + t), (unsigned)j & 1u, err, 15))) break;
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            issue_qk(t, j + 1);
-                        }
-                        if (!ok) break;
-                        mma_commit(bar(B_KEMPTY + s1));
-                    }
-                    if (!(ok = mbar_wait(bar(B_VFULL + s), ph, err, 17))) break;
+                    for (int k = 0; k < HD / 16; ++k)
+                        mma_f16(tmem_base + S_COL0 + (unsigned)t * BKV, qd + 2 * k, kd + 2 * k, idesc_qk, k > 0 ? 1u : 0u);
+                    mma_commit(bar(B_SFULL + t));
+                }
+            };
+            if (ok) ok = mbar_wait_warp(bar(B_KFULL), 0, err, 14);
+            if (ok) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int t = 0; t < TILES; ++t)
+                    if (nb[t] > 0) issue_qk(t, 0);
+                if (elect_one()) mma_commit(bar(B_KEMPTY));
+            }
+            for (int j = 0; j < nb_max && ok; ++j) {
+                const int s = j % STAGES_KV, s1 = (j + 1) % STAGES_KV;
+                const unsigned ph = (unsigned)(j / STAGES_KV) & 1u, ph1 = (unsigned)((j + 1) / STAGES_KV) & 1u;
+                // S(t, j + 1) as soon as the tile's softmax warps hold S(t, j) in registers
+                if (j + 1 < nb_max) {
+                    if (!(ok = mbar_wait_warp(bar(B_KFULL + s1), ph1, err, 14))) break;
 #pragma unroll
                     for (int t = 0; t < TILES; ++t) {
-                        if (!ok || j >= nb[t]) continue;
-                        if (!(ok = mbar_wait(bar(B_PFULL + t), (unsigned)j & 1u, err, 16))) break;
+                        if (!ok || j + 1 >= nb[t]) continue;
+                        if (!(ok = mbar_wait_warp(bar(B_SFREE + t), (unsigned)j & 1u, err, 15))) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-                        for (int k = 0; k < BKV / 16; ++k) {
-                            // A: P, K-major, sub-tile k / 4 (64 keys), 32 bytes per 16 keys within it
-                            const unsigned a_addr = p_s + t * P_BYTES + (k >> 2) * (BQ * 128) + (k & 3) * 32;
-                            // B: V, MN-major: 16 keys are 16 rows of 128 bytes
-                            const unsigned b_addr = v_s + s * KV_BYTES + k * 16 * 128;
-                            mma_f16(tmem_base + O_COL0 + (unsigned)t * HD, smem_desc(a_addr), smem_desc_mn(b_addr),
-                                    idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
-                        }
-                        mma_commit(bar(B_PVDONE + t));         // P and O of this tile are free again once it is done
+                        issue_qk(t, j + 1);
                     }
-                    mma_commit(bar(B_VEMPTY + s));
+                    if (!ok) break;
+                    if (elect_one()) mma_commit(bar(B_KEMPTY + s1));
                 }
+                if (!(ok = mbar_wait_warp(bar(B_VFULL + s), ph, err, 17))) break;
+#pragma unroll
+                for (int t = 0; t < TILES; ++t) {
+                    if (!ok || j >= nb[t]) continue;
+                    if (!(ok = mbar_wait_warp(bar(B_PFULL + t), (unsigned)j & 1u, err, 16))) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const unsigned long long pd = smem_desc(p_s + t * P_BYTES), vd = smem_desc_mn(v_s + s * KV_BYTES);
+                    if (elect_one()) {
+                        // A: P, K-major, sub-tile k / 4 (64 keys), 32 bytes per 16 keys within it; B: V, MN-major: 16 keys are 16 rows of
+                        // 128 bytes (a descriptor's address counts 16 bytes)
+#pragma unroll
+                        for (int k = 0; k < BKV / 16; ++k)
+                            mma_f16(tmem_base + O_COL0 + (unsigned)t * HD, pd + (k >> 2) * (BQ * 128 / 16) + (k & 3) * 2, vd + k * 128, idesc_pv,
+                                    (j > 0 || k > 0) ? 1u : 0u);
+                        mma_commit(bar(B_PVDONE + t));             // P and O of this tile are free again once it is done
+                    }
+                }
+                if (elect_one()) mma_commit(bar(B_VEMPTY + s));
             }
         }
     } else {

@@ -88,7 +88,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const unsigned full0 = smem_u32(bars), empty0 = full0 + 8 * STAGES, acc_bar = full0 + 16 * STAGES;
     const unsigned tiles0 = smem_u32(smem);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int kblocks = (K + BK - 1) / BK;
 
@@ -111,39 +111,34 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const unsigned tmem_base = *tmem_holder;
 
     if (warp == 0) {
-        if (lane == 0) {
-            for (int kb = 0; kb < kblocks; ++kb) {
-                const int s = kb % STAGES;
-                const unsigned phase = (unsigned)(kb / STAGES) & 1u;
-                if (!mbar_wait(empty0 + 8 * s, phase ^ 1u, err, 1)) break;
+        for (int kb = 0; kb < kblocks; ++kb) {
+            const int s = kb % STAGES;
+            const unsigned phase = (unsigned)(kb / STAGES) & 1u;
+            if (!mbar_wait_warp(empty0 + 8 * s, phase ^ 1u, err, 1)) break;
+            const unsigned a_dst = tiles0 + s * L::STAGE_BYTES;
+            if (elect_one()) {
                 mbar_expect_tx(full0 + 8 * s, L::STAGE_BYTES);
-                const unsigned a_dst = tiles0 + s * L::STAGE_BYTES;
                 tma_load_2d(a_dst, &map_a, kb * BK, m0, full0 + 8 * s);
                 tma_load_2d(a_dst + L::A_BYTES, &map_b, kb * BK + b_k0, n0 + b_row0, full0 + 8 * s);
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const unsigned idesc = instr_desc(BM, BN);
-            bool ok = true;
-            for (int kb = 0; kb < kblocks && ok; ++kb) {
-                const int s = kb % STAGES;
-                const unsigned phase = (unsigned)(kb / STAGES) & 1u;
-                ok = mbar_wait(full0 + 8 * s, phase, err, 2);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const unsigned a_addr = tiles0 + s * L::STAGE_BYTES;
-                const unsigned b_addr = a_addr + L::A_BYTES;
+        const unsigned idesc = instr_desc(BM, BN);
+        for (int kb = 0; kb < kblocks; ++kb) {
+            const int s = kb % STAGES;
+            const unsigned phase = (unsigned)(kb / STAGES) & 1u;
+            if (!mbar_wait_warp(full0 + 8 * s, phase, err, 2)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const unsigned a_addr = tiles0 + s * L::STAGE_BYTES;
+            const unsigned long long a = smem_desc(a_addr), b = smem_desc(a_addr + L::A_BYTES);
+            if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k) {
-                    // 16 elements of K are 32 bytes further along the swizzled row
-                    mma_f16(tmem_base, smem_desc(a_addr + k * 32), smem_desc(b_addr + k * 32), idesc,
-                            (kb > 0 || k > 0) ? 1u : 0u);
-                }
+                for (int k = 0; k < BK / 16; ++k)         // 16 elements of K: 32 bytes, two units of a descriptor's address
+                    mma_f16(tmem_base, a + 2 * k, b + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                 mma_commit(empty0 + 8 * s);               // the stage is free once these MMAs have read it
             }
-            mma_commit(acc_bar);                          // the accumulator is complete
         }
+        if (elect_one()) mma_commit(acc_bar);             // the accumulator is complete
     } else {
         // epilogue: warp w reads tensor-memory lanes 32 * (w % 4) .. + 31
         const int quarter = warp & 3;
@@ -208,7 +203,7 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const unsigned acc_full0 = full0 + 16 * STAGES, acc_empty0 = acc_full0 + 16;
     const unsigned tiles0 = smem_u32(smem);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int m_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
     const int tiles = m_tiles * n_tiles;
     const int kblocks = (K + BK - 1) / BK;
@@ -235,51 +230,49 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const unsigned tmem_base = *tmem_holder;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int it = 0;                                   // K blocks issued so far, over all tiles
-            bool ok = true;
-            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-                const int m0 = (t % m_tiles) * BM, n0 = (t / m_tiles) * BN;
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    const unsigned phase = (unsigned)(it / STAGES) & 1u;
-                    ok = mbar_wait(empty0 + 8 * s, phase ^ 1u, err, 1);
-                    if (!ok) break;
+        int it = 0;                                       // K blocks issued so far, over all tiles
+        bool ok = true;
+        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+            const int m0 = (t % m_tiles) * BM, n0 = (t / m_tiles) * BN;
+            for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                const int s = it % STAGES;
+                const unsigned phase = (unsigned)(it / STAGES) & 1u;
+                ok = mbar_wait_warp(empty0 + 8 * s, phase ^ 1u, err, 1);
+                if (!ok) break;
+                const unsigned a_dst = tiles0 + s * L::STAGE_BYTES;
+                if (elect_one()) {
                     mbar_expect_tx(full0 + 8 * s, L::STAGE_BYTES);
-                    const unsigned a_dst = tiles0 + s * L::STAGE_BYTES;
                     tma_load_2d(a_dst, &map_a, kb * BK, m0, full0 + 8 * s);
                     tma_load_2d(a_dst + L::A_BYTES, &map_b, kb * BK, n0, full0 + 8 * s);
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const unsigned idesc = instr_desc(BM, BN);
-            int it = 0, local = 0;
-            bool ok = true;
-            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++local) {
-                const int acc = local & 1;
-                const unsigned acc_phase = (unsigned)(local >> 1) & 1u;
-                ok = mbar_wait(acc_empty0 + 8 * acc, acc_phase ^ 1u, err, 4);   // the epilogue has drained it
+        const unsigned idesc = instr_desc(BM, BN);
+        int it = 0, local = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++local) {
+            const int acc = local & 1;
+            const unsigned acc_phase = (unsigned)(local >> 1) & 1u;
+            ok = mbar_wait_warp(acc_empty0 + 8 * acc, acc_phase ^ 1u, err, 4);   // the epilogue has drained it
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const unsigned tmem_acc = tmem_base + (unsigned)(acc * BN);
+            for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                const int s = it % STAGES;
+                const unsigned phase = (unsigned)(it / STAGES) & 1u;
+                ok = mbar_wait_warp(full0 + 8 * s, phase, err, 2);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const unsigned tmem_acc = tmem_base + (unsigned)(acc * BN);
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    const unsigned phase = (unsigned)(it / STAGES) & 1u;
-                    ok = mbar_wait(full0 + 8 * s, phase, err, 2);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const unsigned a_addr = tiles0 + s * L::STAGE_BYTES;
-                    const unsigned b_addr = a_addr + L::A_BYTES;
+                const unsigned a_addr = tiles0 + s * L::STAGE_BYTES;
+                const unsigned long long a = smem_desc(a_addr), b = smem_desc(a_addr + L::A_BYTES);
+                if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k)
-                        mma_f16(tmem_acc, smem_desc(a_addr + k * 32), smem_desc(b_addr + k * 32), idesc,
-                                (kb > 0 || k > 0) ? 1u : 0u);
+                    for (int k = 0; k < BK / 16; ++k) mma_f16(tmem_acc, a + 2 * k, b + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     mma_commit(empty0 + 8 * s);
                 }
-                mma_commit(acc_full0 + 8 * acc);
             }
+            if (elect_one()) mma_commit(acc_full0 + 8 * acc);
         }
     } else {
         const int quarter = warp & 3;

@@ -114,7 +114,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const unsigned acc_full0 = full0 + 16 * STAGES, acc_empty0 = acc_full0 + 16;
     const unsigned tiles0 = smem_u32(smem);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const unsigned rank = cluster_rank();
     const bool leader = rank == 0;
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
@@ -145,52 +145,53 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     mv_pdl_begin();                                       // X and Y belong to the kernel before until here
 
     if (warp == 0) {
-        if (lane == 0) {
-            int it = 0;                                   // K blocks issued so far, over all tiles
-            bool ok = true;
-            for (int t = pair; t < tiles && ok; t += n_pairs) {
-                const int m0 = (t % m_tiles) * 2 * BM + (int)rank * BM;
-                const int n0 = (t / m_tiles) * BN + (int)rank * (BN / 2);
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    const unsigned phase = (unsigned)(it / STAGES) & 1u;
-                    ok = mbar_wait(empty0 + 8 * s, phase ^ 1u, err, 1);
-                    if (!ok) break;
+        int it = 0;                                       // K blocks issued so far, over all tiles
+        bool ok = true;
+        for (int t = pair; t < tiles && ok; t += n_pairs) {
+            const int m0 = (t % m_tiles) * 2 * BM + (int)rank * BM;
+            const int n0 = (t / m_tiles) * BN + (int)rank * (BN / 2);
+            for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                const int s = it % STAGES;
+                const unsigned phase = (unsigned)(it / STAGES) & 1u;
+                ok = mbar_wait_warp(empty0 + 8 * s, phase ^ 1u, err, 1);
+                if (!ok) break;
+                const unsigned bar = in_block(full0 + 8 * s, 0);
+                const unsigned a_dst = tiles0 + s * L::STAGE_BYTES;
+                if (elect_one()) {
                     if (leader) mbar_expect_tx(full0 + 8 * s, 2 * L::STAGE_BYTES);
-                    const unsigned bar = in_block(full0 + 8 * s, 0);
-                    const unsigned a_dst = tiles0 + s * L::STAGE_BYTES;
                     tma_load_2d_pair(a_dst, &map_a, kb * BK, m0, bar);
                     tma_load_2d_pair(a_dst + L::A_BYTES, &map_b, kb * BK, n0, bar);
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && leader) {
+        if (leader) {
             const unsigned idesc = instr_desc(2 * BM, BN);
             int it = 0, local = 0;
             bool ok = true;
             for (int t = pair; t < tiles && ok; t += n_pairs, ++local) {
                 const int acc = local & 1;
                 const unsigned acc_phase = (unsigned)(local >> 1) & 1u;
-                ok = mbar_wait(acc_empty0 + 8 * acc, acc_phase ^ 1u, err, 4);   // both blocks have drained it
+                ok = mbar_wait_warp(acc_empty0 + 8 * acc, acc_phase ^ 1u, err, 4);   // both blocks have drained it
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned tmem_acc = tmem_base + (unsigned)(acc * BN);
                 for (int kb = 0; kb < kblocks; ++kb, ++it) {
                     const int s = it % STAGES;
                     const unsigned phase = (unsigned)(it / STAGES) & 1u;
-                    ok = mbar_wait(full0 + 8 * s, phase, err, 2);
+                    ok = mbar_wait_warp(full0 + 8 * s, phase, err, 2);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned a_addr = tiles0 + s * L::STAGE_BYTES;
-                    const unsigned b_addr = a_addr + L::A_BYTES;
+                    const unsigned long long a = smem_desc(a_addr), b = smem_desc(a_addr + L::A_BYTES);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k)
-                        mma_f16_pair(tmem_acc, smem_desc(a_addr + k * 32), smem_desc(b_addr + k * 32), idesc,
-                                     (kb > 0 || k > 0) ? 1u : 0u);
-                    mma_commit_pair(empty0 + 8 * s);
+                        for (int k = 0; k < BK / 16; ++k)     // 16 elements of K: 32 bytes, two units of a descriptor's address
+                            mma_f16_pair(tmem_acc, a + 2 * k, b + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        mma_commit_pair(empty0 + 8 * s);
+                    }
                 }
-                mma_commit_pair(acc_full0 + 8 * acc);
+                if (elect_one()) mma_commit_pair(acc_full0 + 8 * acc);
             }
         }
     } else {

@@ -107,7 +107,7 @@ gemm_tc_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const unsigned full0 = smem_u32(bars), empty0 = full0 + 8 * STAGES, acc_bar = full0 + 16 * STAGES;
     const unsigned tiles0 = smem_u32(smem);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int slices = gridDim.x, slice = blockIdx.x;
     const int n0 = blockIdx.y * L::W_ROWS;
     const int mt0 = blockIdx.z * BN;                    // this block's first token (TAIL 1 and 2: always 0)
@@ -141,21 +141,25 @@ gemm_tc_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     // requested at once; X, and everything the epilogue reads, only after the wait.
     mv_pdl_launch_dependents();
     if (warp == 0) {
-        if (lane == 0) {
-            const int first = nkb < STAGES ? nkb : STAGES;
+        const int first = nkb < STAGES ? nkb : STAGES;
+        if (elect_one()) {
             for (int i = 0; i < first; ++i) {
                 mbar_expect_tx(full0 + 8 * i, L::TX_BYTES);
                 tma_load_2d(tiles0 + i * L::STAGE_BYTES, &map_w, (kb0 + i) * BK, n0, full0 + 8 * i);
             }
-            mv_pdl_wait();
+        }
+        mv_pdl_wait();
+        if (elect_one()) {
             for (int i = 0; i < first; ++i)
                 tma_load_2d(tiles0 + i * L::STAGE_BYTES + L::A_BYTES, &map_x, (kb0 + i) * BK, mt0, full0 + 8 * i);
-            for (int i = first; i < nkb; ++i) {
-                const int s = i % STAGES;
-                const unsigned phase = (unsigned)(i / STAGES) & 1u;
-                if (!mbar_wait(empty0 + 8 * s, phase ^ 1u, err, 1)) break;
+        }
+        for (int i = first; i < nkb; ++i) {
+            const int s = i % STAGES;
+            const unsigned phase = (unsigned)(i / STAGES) & 1u;
+            if (!mbar_wait_warp(empty0 + 8 * s, phase ^ 1u, err, 1)) break;
+            const unsigned a_dst = tiles0 + s * L::STAGE_BYTES;
+            if (elect_one()) {
                 mbar_expect_tx(full0 + 8 * s, L::TX_BYTES);
-                const unsigned a_dst = tiles0 + s * L::STAGE_BYTES;
                 tma_load_2d(a_dst, &map_w, (kb0 + i) * BK, n0, full0 + 8 * s);
                 tma_load_2d(a_dst + L::A_BYTES, &map_x, (kb0 + i) * BK, mt0, full0 + 8 * s);
             }
@@ -169,22 +173,23 @@ gemm_tc_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)ahead.w + (l << 7)));
         }
     } else if (warp == 1) {
-        if (lane == 0 && nkb > 0) {
+        if (nkb > 0) {
             const unsigned idesc = instr_desc(BM, BN);
             for (int i = 0; i < nkb; ++i) {
                 const int s = i % STAGES;
                 const unsigned phase = (unsigned)(i / STAGES) & 1u;
-                if (!mbar_wait(full0 + 8 * s, phase, err, 2)) break;
+                if (!mbar_wait_warp(full0 + 8 * s, phase, err, 2)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned a_addr = tiles0 + s * L::STAGE_BYTES;
-                const unsigned b_addr = a_addr + L::A_BYTES;
+                const unsigned long long a = smem_desc(a_addr), b = smem_desc(a_addr + L::A_BYTES);
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k)
-                    mma_f16(tmem_base, smem_desc(a_addr + k * 32), smem_desc(b_addr + k * 32), idesc,
-                            (i > 0 || k > 0) ? 1u : 0u);
-                mma_commit(empty0 + 8 * s);
+                    for (int k = 0; k < BK / 16; ++k)      // 16 elements of K: 32 bytes, two units of a descriptor's address
+                        mma_f16(tmem_base, a + 2 * k, b + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+                    mma_commit(empty0 + 8 * s);
+                }
             }
-            mma_commit(acc_bar);
+            if (elect_one()) mma_commit(acc_bar);
         }
     } else {
         // this block's accumulator: tensor memory -> shared memory, rows = rows of W, columns = tokens

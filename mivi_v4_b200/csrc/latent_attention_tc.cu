@@ -25,8 +25,8 @@
 //
 // Bound by the softmax (a block of 64 keys of both tiles needs 1,024 clocks of the exponential unit and some 1,000 instructions of each
 // scheduler, and its products 1,100 clocks beside it).  32 heads of 64 + 32 / 64 with a gate, this kernel / latent_attention_prefill.cu: one prompt of 6,000 tokens
-// 363 / 1,132 us, of 2,048 72 / 190, three of 333 to 2,048 103 / 226.  What it took: an elected lane of a whole warp issues the products (a lane
-// by itself in a diverged warp takes some 120 clocks a product to bring its operands into uniform registers; a first form of the kernel with it 495), one warp for
+// 363 / 1,132 us, of 2,048 72 / 190, three of 333 to 2,048 103 / 226.  What it took: an elected lane of a whole warp issues the products (see
+// tc_common.cuh; a first form of the kernel with a lane by itself 495 us), one warp for
 // either product (one for both: the waits of one hold up the other, 296 against 273 for a form of other sums), gates read 32 bytes at a time (a block's gates element by
 // element took longer than its softmax: 344 against 317).
 #include "tc_common.cuh"
@@ -64,11 +64,6 @@ __device__ __forceinline__ unsigned long long smem_desc_64(unsigned addr) {
     d |= (unsigned long long)4 << 61;
     return d;
 }
-__device__ __forceinline__ bool elect_one() {
-    unsigned p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
-}
 __device__ __forceinline__ void mbar_arrive(unsigned bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -103,12 +98,6 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
     unsigned long long r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(*reinterpret_cast<unsigned long long*>(&a)),
         "l"(*reinterpret_cast<unsigned long long*>(&b)));
-    return *reinterpret_cast<float2*>(&r);
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(*reinterpret_cast<unsigned long long*>(&a)),
-        "l"(*reinterpret_cast<unsigned long long*>(&b)), "l"(*reinterpret_cast<unsigned long long*>(&c)));
     return *reinterpret_cast<float2*>(&r);
 }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) {
@@ -194,7 +183,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     // rows of the first and the last block that are not this sequence's, or come after the pair's last query
     const int rows_before = max(0, lo - key_first), last_rows = pos0 + nq - key_first - (nb_max - 1) * BKV;
     const bool fix_first = rows_before > 0, fix_last = last_rows < BKV;
-    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < B_COUNT; ++i) mbar_init(bar(i), i >= B_PFULL && i < B_PFULL + 2 * TILES ? 4 : 1);
@@ -214,22 +203,26 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         // registers move from this warpgroup to the softmax warps (168 each at launch)
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         if (warp == 0) {
-            if (lane == 0) {
+            if (elect_one()) {
                 mbar_expect_tx(bar(B_Q), TILES * L::Q_BYTES);
                 for (int t = 0; t < TILES; ++t) {
                     tma_load_2d(q_s + t * L::Q_BYTES, &map_q, h * (DIM + ROT), row0 + t * BQ, bar(B_Q));
                     tma_load_2d(q_s + t * L::Q_BYTES + L::Q_PART, &map_qr, h * (DIM + ROT) + DIM, row0 + t * BQ, bar(B_Q));
                 }
-                for (int j = 0; j < nb_max; ++j) {
-                    const int s = j % KSTAGES, row = key_row + j * BKV;
-                    const unsigned ph = (unsigned)(j / KSTAGES) & 1u;
-                    if (!mbar_wait(bar(B_KEMPTY + s), ph ^ 1u, err, 51)) break;
+            }
+            for (int j = 0; j < nb_max; ++j) {
+                const int s = j % KSTAGES, row = key_row + j * BKV;
+                const unsigned ph = (unsigned)(j / KSTAGES) & 1u;
+                if (!mbar_wait_warp(bar(B_KEMPTY + s), ph ^ 1u, err, 51)) break;
+                if (elect_one()) {
                     mbar_expect_tx(bar(B_KFULL + s), L::K_BYTES);
                     tma_load_2d(k_s + s * L::K_BYTES, &map_kx, h * DIM, row, bar(B_KFULL + s));
                     tma_load_2d(k_s + s * L::K_BYTES + L::K_PART, &map_r, 0, row, bar(B_KFULL + s));
-                    if (!mbar_wait(bar(B_VEMPTY + s), ph ^ 1u, err, 52)) break;
-                    // blocks with rows of others go by way of warp 2, which then says that they are there
-                    const unsigned full = j == 0 && fix_first ? bar(B_VFIX) : j == nb_max - 1 && fix_last ? bar(B_VFIX + 1) : bar(B_VFULL + s);
+                }
+                if (!mbar_wait_warp(bar(B_VEMPTY + s), ph ^ 1u, err, 52)) break;
+                // blocks with rows of others go by way of warp 2, which then says that they are there
+                const unsigned full = j == 0 && fix_first ? bar(B_VFIX) : j == nb_max - 1 && fix_last ? bar(B_VFIX + 1) : bar(B_VFULL + s);
+                if (elect_one()) {
                     mbar_expect_tx(full, V_BYTES);
                     tma_load_2d(v_s + s * V_BYTES, &map_kx, v0 + h * DV, row, full);
                 }
@@ -237,14 +230,14 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         } else if (warp == 1) {
             // S(t, j) = Q_t K_j^T as soon as the keys are there and the buffer's weights, those of the tile's block before the last, are used
             const unsigned idesc = instr_desc(BQ, BKV);
-            bool ok = mbar_wait(bar(B_Q), 0, err, 53);
+            bool ok = mbar_wait_warp(bar(B_Q), 0, err, 53);
             for (int j = 0; j < nb_max && ok; ++j) {
                 const int s = j % KSTAGES;
-                if (!(ok = mbar_wait(bar(B_KFULL + s), (unsigned)(j / KSTAGES) & 1u, err, 54))) break;
+                if (!(ok = mbar_wait_warp(bar(B_KFULL + s), (unsigned)(j / KSTAGES) & 1u, err, 54))) break;
 #pragma unroll
                 for (int t = 0; t < TILES; ++t) {
                     if (!ok || j >= nb[t]) continue;
-                    if (j > 1 && !(ok = mbar_wait(bar(B_PVDONE + 2 * t + (j & 1)), (unsigned)((j - 2) >> 1) & 1u, err, 55))) break;
+                    if (j > 1 && !(ok = mbar_wait_warp(bar(B_PVDONE + 2 * t + (j & 1)), (unsigned)((j - 2) >> 1) & 1u, err, 55))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned d = tmem_base + (unsigned)(2 * t + (j & 1)) * BKV;
                     const unsigned qa = q_s + t * L::Q_BYTES, ka = k_s + s * L::K_BYTES;
@@ -267,12 +260,12 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             bool ok = true;
             for (int j = 0; j < nb_max && ok; ++j) {
                 const int s = j % KSTAGES;
-                if (!(ok = mbar_wait(bar(B_VFULL + s), (unsigned)(j / KSTAGES) & 1u, err, 56))) break;
+                if (!(ok = mbar_wait_warp(bar(B_VFULL + s), (unsigned)(j / KSTAGES) & 1u, err, 56))) break;
                 const unsigned long long v0d = smem_desc(v_s + s * V_BYTES);
 #pragma unroll
                 for (int t = 0; t < TILES; ++t) {
                     if (!ok || j >= nb[t]) continue;
-                    if (!(ok = mbar_wait(bar(B_PFULL + 2 * t + (j & 1)), (unsigned)(j >> 1) & 1u, err, 58))) break;
+                    if (!(ok = mbar_wait_warp(bar(B_PFULL + 2 * t + (j & 1)), (unsigned)(j >> 1) & 1u, err, 58))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned p = tmem_base + (unsigned)(2 * t + (j & 1)) * BKV, d = tmem_base + O_COL0 + (unsigned)t * DV;
                     if (elect_one()) {
@@ -292,7 +285,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 // (one block that is the first and the last comes by the first way)
                 const int j = f ? nb_max - 1 : 0, s = j % KSTAGES;
                 if (f ? !fix_last || (fix_first && j == 0) : !fix_first) continue;
-                if (!mbar_wait(bar(B_VFIX + f), 0, err, 59)) break;
+                if (!mbar_wait_warp(bar(B_VFIX + f), 0, err, 59)) break;
                 const int head = j == 0 ? rows_before : 0, tail = j == nb_max - 1 ? last_rows : BKV;
                 for (int i = lane; i < BKV * 8; i += 32)
                     if (i < head * 8 || i >= tail * 8) *reinterpret_cast<uint4*>(smem + L::V_AT + s * V_BYTES + i * 16) = make_uint4(0u, 0u, 0u, 0u);
@@ -314,7 +307,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         float m = -INFINITY, l[4] = {0.f, 0.f, 0.f, 0.f};                // m: the reference of the row's exponentials
         bool ok = true;
         for (int j = 0; j < my_nb; ++j) {
-            if (!(ok = mbar_wait(bar(B_SFULL + 2 * t + (j & 1)), (unsigned)(j >> 1) & 1u, err, 60))) break;
+            if (!(ok = mbar_wait_warp(bar(B_SFULL + 2 * t + (j & 1)), (unsigned)(j >> 1) & 1u, err, 60))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned s_addr = lane_addr + (unsigned)(2 * t + (j & 1)) * BKV;
             unsigned s0[32], s1[32];
@@ -350,7 +343,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             for (int i = 0; i < 4; ++i) l[i] = fmaf(l[i], c, sum[i]);
             if (j > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {
                 // O is the block before's until its product is done
-                if (!(ok = mbar_wait(bar(B_PVDONE + 2 * t + ((j - 1) & 1)), (unsigned)((j - 1) >> 1) & 1u, err, 61))) break;
+                if (!(ok = mbar_wait_warp(bar(B_PVDONE + 2 * t + ((j - 1) & 1)), (unsigned)((j - 1) >> 1) & 1u, err, 61))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                 for (int d = 0; d < DV; d += 32) {
@@ -372,7 +365,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(B_PFULL + 2 * t + (j & 1)));
         }
-        if (ok && my_nb > 0) ok = mbar_wait(bar(B_PVDONE + 2 * t + ((my_nb - 1) & 1)), (unsigned)((my_nb - 1) >> 1) & 1u, err, 62);
+        if (ok && my_nb > 0) ok = mbar_wait_warp(bar(B_PVDONE + 2 * t + ((my_nb - 1) & 1)), (unsigned)((my_nb - 1) >> 1) & 1u, err, 62);
         if (ok && my_nb > 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float den = __fadd_rn(__fadd_rn(l[0], l[1]), __fadd_rn(l[2], l[3])), by;     // the row is O by

@@ -50,6 +50,27 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, int* er
         }
     }
 }
+// A warp that issues copies or products runs its loop as a whole and lets one elected lane issue: their operands then live in uniform registers.
+// (A lane by itself in a diverged branch takes some 120 clocks a product to bring them there, several times what the product takes.)
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_one() {
+    unsigned p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// mbar_wait by a whole warp, with one answer for all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(unsigned bar, unsigned parity, int* err, int code) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const unsigned long long t0 = globaltimer();
+    for (;;) {
+        for (int i = 0; i < 256; ++i)
+            if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if (__any_sync(0xffffffffu, globaltimer() - t0 > WAIT_NS)) {
+            if (elect_one()) atomicExch(err, code);
+            return false;
+        }
+    }
+}
 __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
