@@ -62,9 +62,6 @@ __device__ __forceinline__ unsigned long long smem_desc_mn(unsigned addr) {
     d |= (unsigned long long)2 << 61;
     return d;
 }
-__device__ __forceinline__ void mbar_arrive(unsigned bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

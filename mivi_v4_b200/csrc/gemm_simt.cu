@@ -2,7 +2,7 @@
 // float32 or bfloat16, accumulation in float32 with fused multiply-add.
 //
 // This is the matrix product of the true 32-bit path (no tensor-core mode is
-// involved, so no reduced-precision matrix mode can slip in), and the product
+// involved, so no reduced-precision matrix mode can slip in; large ones go to gemm_f32_tc.cu, which is no less exact), and the product
 // of last resort for shapes that the tensor-core kernels refuse.  It computes
 // what the reference's matvec / matmul rows do
 // (crates/mivi-quant/src/lib.rs:75-135, 143-245): out[b, n] = sum_d in[b, d] * W[n, d].

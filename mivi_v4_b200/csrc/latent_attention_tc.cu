@@ -54,19 +54,6 @@ enum { B_Q = 0, B_KFULL = 1, B_KEMPTY = B_KFULL + KSTAGES, B_VFULL = B_KEMPTY + 
        B_COUNT = B_VFIX + 2 };
 static_assert(B_COUNT * 8 + 8 <= 256, "barrier area");
 
-// K-major rows of 64 bytes, 64-byte swizzle: 8-row groups 512 bytes apart
-__device__ __forceinline__ unsigned long long smem_desc_64(unsigned addr) {
-    unsigned long long d = 0;
-    d |= (unsigned long long)((addr & 0x3ffffu) >> 4);
-    d |= (unsigned long long)1 << 16;
-    d |= (unsigned long long)(512 >> 4) << 32;
-    d |= (unsigned long long)1 << 46;
-    d |= (unsigned long long)4 << 61;
-    return d;
-}
-__device__ __forceinline__ void mbar_arrive(unsigned bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

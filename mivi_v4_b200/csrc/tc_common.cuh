@@ -28,6 +28,9 @@ __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
 __device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
     unsigned ok;
     asm volatile(
@@ -86,6 +89,16 @@ __device__ __forceinline__ unsigned long long smem_desc(unsigned addr) {
     d |= (unsigned long long)2 << 61;                            // SWIZZLE_128B
     return d;
 }
+// The same with rows of 64 bytes and the 64-byte swizzle: 8-row groups are 512 bytes apart.
+__device__ __forceinline__ unsigned long long smem_desc_64(unsigned addr) {
+    unsigned long long d = 0;
+    d |= (unsigned long long)((addr & 0x3ffffu) >> 4);
+    d |= (unsigned long long)1 << 16;
+    d |= (unsigned long long)(512 >> 4) << 32;
+    d |= (unsigned long long)1 << 46;
+    d |= (unsigned long long)4 << 61;                            // SWIZZLE_64B
+    return d;
+}
 // Instruction descriptor of kind::f16: bf16 x bf16 -> f32, both operands K-major.
 __device__ __forceinline__ unsigned instr_desc(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(m >> 4) << 24);
@@ -139,36 +152,36 @@ EncodeTiled encoder() {
 }
 
 struct MapKey {
-    const void* ptr; int rows, cols, box_rows, box_cols;
+    const void* ptr; int rows, cols, box_rows, box_cols, elem_bytes;
     bool operator==(const MapKey& o) const {
-        return ptr == o.ptr && rows == o.rows && cols == o.cols && box_rows == o.box_rows && box_cols == o.box_cols;
+        return ptr == o.ptr && rows == o.rows && cols == o.cols && box_rows == o.box_rows && box_cols == o.box_cols && elem_bytes == o.elem_bytes;
     }
 };
 struct MapKeyHash {
     size_t operator()(const MapKey& k) const {
         return std::hash<const void*>()(k.ptr) ^ ((size_t)k.rows * 1000003u) ^ ((size_t)k.cols * 7919u) ^
-               ((size_t)k.box_rows << 20) ^ ((size_t)k.box_cols << 32);
+               ((size_t)k.box_rows << 20) ^ ((size_t)k.box_cols << 32) ^ ((size_t)k.elem_bytes << 40);
     }
 };
 
-// A row-major [rows, cols] bfloat16 matrix read in boxes of box_rows x 64 with the 128-byte swizzle, or of box_rows x 32 with
-// the 64-byte one.
-bool tensor_map(const void* ptr, int rows, int cols, int box_rows, CUtensorMap* out, int box_cols = BK) {
+// A row-major [rows, cols] matrix of bfloat16 (or, with elem_bytes 4, of float32) read in boxes of box_rows x box_cols: boxes of 128 bytes a row
+// with the 128-byte swizzle, of 64 with the 64-byte one.
+bool tensor_map(const void* ptr, int rows, int cols, int box_rows, CUtensorMap* out, int box_cols = BK, int elem_bytes = 2) {
     static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
     static std::mutex mu;
     std::lock_guard<std::mutex> lock(mu);
-    const MapKey key{ptr, rows, cols, box_rows, box_cols};
+    const MapKey key{ptr, rows, cols, box_rows, box_cols, elem_bytes};
     auto it = cache.find(key);
     if (it != cache.end()) { *out = it->second; return true; }
     EncodeTiled enc = encoder();
     if (!enc) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    const cuuint64_t strides[1] = {(cuuint64_t)cols * elem_bytes};
     const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1, 1};
     CUtensorMap m;
-    if (enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, elem,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == BK ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    if (enc(&m, elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, elem,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols * elem_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return false;
     if (cache.size() > 4096) cache.clear();

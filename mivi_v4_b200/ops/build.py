@@ -24,9 +24,9 @@ from typing import Dict, List
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "csrc")
 
 # library name -> sources.  ``core`` holds what every model and both dtypes
-# need; the tensor-core libraries serve bfloat16 only.
+# need; the tensor-core library serves bfloat16 only.
 LIBRARIES: Dict[str, List[str]] = {
-    "core": ["elementwise.cu", "gemm_simt.cu", "shortconv.cu", "attention.cu", "attention_decode.cu",
+    "core": ["elementwise.cu", "gemm_simt.cu", "gemm_f32_tc.cu", "shortconv.cu", "attention.cu", "attention_decode.cu",
              "sampling.cu", "gated_norms.cu", "decay_scan.cu", "attention_sink.cu", "scalar_scan.cu", "state_space.cu",
              "routed_experts.cu", "latent_attention.cu", "delta_rule.cu", "gated_recurrence.cu"],
     "bf16": ["gemm_small_m.cu", "gemm_tc.cu", "gemm_tc_pair.cu", "gemm_tc_swap.cu", "attention_prefill.cu",

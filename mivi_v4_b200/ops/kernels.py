@@ -39,6 +39,7 @@ _SIGNATURES = {
         "mv_copy_to_host": [_P, _P, _Q, _P],
         "mv_delay": [_Q, _P],
         "mv_gemm_f32_plan": [_I, _I, _I],
+        "mv_gemm_f32_tc": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
         "mv_gemm_simt": [_P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P],
         "mv_shortconv": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
         "mv_shortconv_decode": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],
@@ -1713,10 +1714,26 @@ def _account_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulat
                 2 * x.shape[0] * w.shape[0] * w.shape[1])
 
 
+F32_TC_ROWS, F32_TC_K = 9, 1024
+
+
+def gemm_f32_tc_takes(M: int, N: int, K: int, sms: int) -> bool:
+    """Whether a float32 product goes to the tensor cores (``gemm_f32_tc.cu``) or to the CUDA cores: by what either is expected to take, in us.  The
+    tensor cores work in rounds of tiles of 128 x 128 or 128 x 96, 26.4 or 21.9 us for 1,024 of K whatever a tile's rows; the CUDA cores add
+    up some 40e6 products a us, and lose about 32 rows to their tiles.  Measured (tensor / CUDA cores) on nine shapes at 9 to 1,165 rows, never the
+    slower one by more than a tenth: 9,216 x 1,024 at 16 rows 29 / 37, at 1,165 133 / 516; 1,024 x 4,608 at 128 rows 80 / 45, at 600 80 / 172; 6,144 x
+    2,048 at 32 rows 45 / 43, at 48 45 / 68.  From K = 1,024 on: below, sums are so short that float32 multiply-adds are as exact."""
+    if M < F32_TC_ROWS or K < F32_TC_K or K % 4 or M > 65535 * 128:
+        return False
+    rows = -(-M // 128)
+    tensor = 4.0 + K / 1024.0 * min(26.4 * -(-rows * -(-N // 128) // sms), 21.9 * -(-rows * -(-N // 96) // sms))
+    return tensor < 5.0 + 2.0 * (M + 32) * N * K / 40e6
+
+
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, bias: Optional[torch.Tensor] = None,
               accumulate: bool = False) -> torch.Tensor:
     """out = x @ w.T (+ bias), or out += ... when ``accumulate`` (out float32).
-    CUDA-core kernel, float32 accumulation, any sizes."""
+    CUDA-core kernels, float32 accumulation, any sizes; large float32 products on the tensor cores, no less exact."""
     M, K = x.shape
     N, K2 = w.shape
     if K != K2:
@@ -1730,6 +1747,12 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, bias: Opti
         mode = 0 if out.dtype == torch.float32 else 1
         _need(out, "gemm out", None, (M, N))
         _dt(out)
+    if x.dtype == torch.float32 and gemm_f32_tc_takes(M, N, K, n_sms(x.device)) and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
+        _check(_fn("core", "mv_gemm_f32_tc")(
+            _need(x, "gemm x"), _need(w, "gemm w"), _need(bias, "gemm bias", torch.float32, (N,), True), out.data_ptr(), mode, M, N, K, N, n_sms(x.device),
+            _error_flag(x.device).data_ptr(), _stream()), "mv_gemm_f32_tc")
+        _account_gemm(x, w, out, accumulate)
+        return out
     _check(_fn("core", "mv_gemm_simt")(
         _need(x, "gemm x"), _need(w, "gemm w"), _dt(x), _need(bias, "gemm bias", torch.float32, (N,), True),
         out.data_ptr(), mode, M, N, K, N, _stream()), "mv_gemm_simt")
