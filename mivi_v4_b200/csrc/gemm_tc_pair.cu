@@ -103,7 +103,7 @@ template <int STAGES, int ACT>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const float* __restrict__ bias, void* __restrict__ out, int mode, int M, int N, int K, int ldo,
-                    const PairLink link, const RowWeights rw, int* __restrict__ err) {
+                    const PairLink link, const RowWeights rw, int* __restrict__ err, const int* __restrict__ tile_group, int b_row_step, int b_k_step) {
     using L = PairLayout<STAGES>;
     constexpr int BN = PAIR_BN;
     extern __shared__ unsigned char smem_raw[];
@@ -149,7 +149,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         bool ok = true;
         for (int t = pair; t < tiles && ok; t += n_pairs) {
             const int m0 = (t % m_tiles) * 2 * BM + (int)rank * BM;
-            const int n0 = (t / m_tiles) * BN + (int)rank * (BN / 2);
+            const int group = tile_group ? tile_group[t % m_tiles] : 0;
+            if (group < 0) continue;                      // a spare tile
+            const int n0 = (t / m_tiles) * BN + (int)rank * (BN / 2) + group * b_row_step, k0 = group * b_k_step;
             for (int kb = 0; kb < kblocks; ++kb, ++it) {
                 const int s = it % STAGES;
                 const unsigned phase = (unsigned)(it / STAGES) & 1u;
@@ -160,7 +162,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 if (elect_one()) {
                     if (leader) mbar_expect_tx(full0 + 8 * s, 2 * L::STAGE_BYTES);
                     tma_load_2d_pair(a_dst, &map_a, kb * BK, m0, bar);
-                    tma_load_2d_pair(a_dst + L::A_BYTES, &map_b, kb * BK, n0, bar);
+                    tma_load_2d_pair(a_dst + L::A_BYTES, &map_b, kb * BK + k0, n0, bar);
                 }
             }
         }
@@ -169,9 +171,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const unsigned idesc = instr_desc(2 * BM, BN);
             int it = 0, local = 0;
             bool ok = true;
-            for (int t = pair; t < tiles && ok; t += n_pairs, ++local) {
+            for (int t = pair; t < tiles && ok; t += n_pairs) {
+                if (tile_group && tile_group[t % m_tiles] < 0) continue;
                 const int acc = local & 1;
                 const unsigned acc_phase = (unsigned)(local >> 1) & 1u;
+                ++local;
                 ok = mbar_wait_warp(acc_empty0 + 8 * acc, acc_phase ^ 1u, err, 4);   // both blocks have drained it
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -200,10 +204,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         const bool by_rows = link.by_rows != 0;
         int local = 0;
         bool ok = true;
-        for (int t = pair; t < tiles && ok; t += n_pairs, ++local) {
+        for (int t = pair; t < tiles && ok; t += n_pairs) {
+            if (tile_group && tile_group[t % m_tiles] < 0) continue;
             const int m0 = (t % m_tiles) * 2 * BM + (int)rank * BM, n0 = (t / m_tiles) * BN;
             const int acc = local & 1;
             const unsigned acc_phase = (unsigned)(local >> 1) & 1u;
+            ++local;
             const int row = m0 + quarter * 32 + lane;
             // What the epilogue needs from memory is asked for before the wait for the accumulator, while
             // the tile's products still run: a carried norm's partial sums of this row, and the first old
@@ -326,12 +332,19 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
 }
 
+// A grouped product (see gemm_tc.cu): which group every tile of 256 rows of X belongs to (negative: none), and where a group's part of W lies.
+struct Groups {
+    const int* tile_group;
+    int w_rows, w_cols, b_row_step, b_k_step;
+};
+
 template <int STAGES, int ACT>
 int launch_pair(const void* X, const void* W, const float* bias, void* out, int mode, int M, int N, int K, int ldo,
-                const PairLink& link, const RowWeights& rw, int* err, cudaStream_t stream) {
+                const PairLink& link, const RowWeights& rw, int* err, cudaStream_t stream, const Groups& groups = Groups{}) {
     using L = PairLayout<STAGES>;
     CUtensorMap ma, mb;
-    if (!tensor_map(X, M, K, BM, &ma) || !tensor_map(W, N, K, PAIR_BN / 2, &mb)) return (int)cudaErrorInvalidValue;
+    if (!tensor_map(X, M, K, BM, &ma) || !tensor_map(W, groups.tile_group ? groups.w_rows : N, groups.tile_group ? groups.w_cols : K, PAIR_BN / 2, &mb))
+        return (int)cudaErrorInvalidValue;
     static int max_pairs = 0;
     if (max_pairs == 0) {
         cudaFuncSetAttribute(gemm_tc_pair_kernel<STAGES, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
@@ -367,7 +380,8 @@ int launch_pair(const void* X, const void* W, const float* bias, void* out, int 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = mv_pdl_enabled() ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<STAGES, ACT>, ma, mb, bias, out, mode, M, N, K, ldo, link, rw, err);
+    cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<STAGES, ACT>, ma, mb, bias, out, mode, M, N, K, ldo, link, rw, err,
+                       groups.tile_group, groups.b_row_step, groups.b_k_step);
     return mv_launch_status();
 }
 
@@ -412,4 +426,18 @@ MV_API int mv_gemm_tc_pair(const void* X, const void* W, const float* bias, void
     if (mode == 6) PAIR_GO(ACT_WEIGHTED);
     PAIR_GO(ACT_PLAIN);
 #undef PAIR_GO
+}
+
+// The grouped product of mv_gemm_tc_grouped (gemm_tc.cu) for runs of rows padded to tiles of 256: tile_group [M / 256].
+MV_API int mv_gemm_tc_pair_grouped(const void* X, const void* W, const float* bias, void* out, int mode, int M, int N, int K, int ldo,
+                                   int w_rows, int w_cols, const int* tile_group, int b_row_step, int b_k_step, int* err,
+                                   cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (K <= 0 || K % 8 || M % (2 * BM) || b_k_step % 8 || !tile_group || ((uintptr_t)X & 15) || ((uintptr_t)W & 15)) return (int)cudaErrorInvalidValue;
+    if (mode < 0 || mode > 4 || (mode >= 3 && (N % 32 || ldo % 2 || (mode == 4 && !bias)))) return (int)cudaErrorInvalidValue;
+    PairLink link = {};
+    link.by_rows = mode == 0 && N % 32 == 0 && ldo % 4 == 0 && !(((uintptr_t)out | (uintptr_t)bias) & 15);
+    const Groups groups = {tile_group, w_rows, w_cols, b_row_step, b_k_step};
+    if (mode == 4) return launch_pair<6, ACT_CLAMPED>(X, W, bias, out, mode, M, N, K, ldo, link, RowWeights{}, err, stream, groups);
+    return launch_pair<6, ACT_PLAIN>(X, W, bias, out, mode, M, N, K, ldo, link, RowWeights{}, err, stream, groups);
 }

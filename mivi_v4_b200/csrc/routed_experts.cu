@@ -135,32 +135,54 @@ MV_API int mv_route(const float* z, int ld, float* dense, int* pick, float* pick
     return mv_launch_status();
 }
 
-// resid[n, :] += (sum of dense[n, col0 .. col0 + n_cols)) * h[n, :]: experts whose output is their input.
-template <typename T>
+// resid[n, :] += (sum of dense[n, col0 .. col0 + n_cols)) * h[n, :]: experts whose output is their input; V columns a thread (4 where H is a
+// multiple: 2,048 tokens of 2,048 28.6 -> 13.6 us).
+template <typename T, int V>
 __global__ void __launch_bounds__(256)
 identity_experts_kernel(const T* __restrict__ h, const float* __restrict__ dense, int ld, int col0, int n_cols,
                         float* __restrict__ resid, long long total, int H, int accumulate) {
     mv_pdl_begin();
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * V;
     if (idx >= total) return;
     const long long n = idx / H;
+    float x[V], old[V];
+    if constexpr (V == 4) {
+        if constexpr (sizeof(T) == 2) {
+            const uint2 r = *reinterpret_cast<const uint2*>(h + idx);
+            x[0] = __uint_as_float(r.x << 16); x[1] = __uint_as_float(r.x & 0xffff0000u);
+            x[2] = __uint_as_float(r.y << 16); x[3] = __uint_as_float(r.y & 0xffff0000u);
+        } else {
+            const float4 r = *reinterpret_cast<const float4*>(h + idx);
+            x[0] = r.x; x[1] = r.y; x[2] = r.z; x[3] = r.w;
+        }
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (accumulate) o = *reinterpret_cast<const float4*>(resid + idx);
+        old[0] = o.x; old[1] = o.y; old[2] = o.z; old[3] = o.w;
+    } else {
+        x[0] = mv_to_f32(h[idx]);
+        old[0] = accumulate ? resid[idx] : 0.f;
+    }
     float w = 0.f;
     for (int c = 0; c < n_cols; ++c) w += dense[n * ld + col0 + c];
-    const float v = w * mv_to_f32(h[idx]);
-    resid[idx] = accumulate ? resid[idx] + v : v;
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+        const float v = __fmul_rn(w, x[j]);
+        x[j] = accumulate ? __fadd_rn(old[j], v) : v;
+    }
+    if constexpr (V == 4) *reinterpret_cast<float4*>(resid + idx) = make_float4(x[0], x[1], x[2], x[3]);
+    else resid[idx] = x[0];
 }
 
 MV_API int mv_identity_experts(const void* h, int dtype, const float* dense, int ld, int col0, int n_cols, float* resid,
                                int N, int H, int accumulate, cudaStream_t stream) {
     if (N <= 0 || n_cols <= 0) return 0;
     const long long total = (long long)N * H;
-    const unsigned blocks = (unsigned)((total + 255) / 256);
-    if (dtype == MV_DT_BF16)
-        mv_launch(identity_experts_kernel<__nv_bfloat16>, blocks, 256, 0, stream, (const __nv_bfloat16*)h, dense, ld, col0,
-                  n_cols, resid, total, H, accumulate);
-    else
-        mv_launch(identity_experts_kernel<float>, blocks, 256, 0, stream, (const float*)h, dense, ld, col0, n_cols, resid,
-                  total, H, accumulate);
+    const bool vec = H % 4 == 0 && (((uintptr_t)h | (uintptr_t)resid) & 15) == 0;
+    const unsigned blocks = (unsigned)((total / (vec ? 4 : 1) + 255) / 256);
+#define ID_LAUNCH(T, V) mv_launch(identity_experts_kernel<T, V>, blocks, 256, 0, stream, (const T*)h, dense, ld, col0, n_cols, resid, total, H, accumulate)
+    if (dtype == MV_DT_BF16) { if (vec) ID_LAUNCH(__nv_bfloat16, 4); else ID_LAUNCH(__nv_bfloat16, 1); }
+    else { if (vec) ID_LAUNCH(float, 4); else ID_LAUNCH(float, 1); }
+#undef ID_LAUNCH
     return mv_launch_status();
 }
 
@@ -219,27 +241,55 @@ MV_API int mv_routed_glu(const float* gu, const float* dense, void* hid, int hid
 // For steps of many tokens: the (token, choice) entries sorted by expert, so that every expert multiplies its own
 // tokens' rows only.  The sort is a stable counting sort: a block an expert walks the entries in order and ranks
 // its own; the ranks depend on the entries alone, not on which block ran first.
-__global__ void __launch_bounds__(256)
+// 1,024 threads take 4 entries each a round, the loads of a round ahead of its barrier (24,000 entries are 6 rounds and were 94 of 256: ranks, tiles and
+// rows of 6,000 tokens together 140 -> 36 us).
+constexpr int RANK_THREADS = 1024;
+__global__ void __launch_bounds__(RANK_THREADS)
 expert_rank_kernel(const int* __restrict__ pick, int total, int* __restrict__ rank, int* __restrict__ counts) {
     mv_pdl_begin();
-    __shared__ int warp_sum[8];
+    __shared__ int warp_sum[2][RANK_THREADS / 32];
     const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int base = 0;
-    for (int t0 = 0; t0 < total; t0 += 256) {
-        const int idx = t0 + tid;
-        const bool mine = idx < total && pick[idx] == e;
-        const unsigned votes = __ballot_sync(0xffffffffu, mine);
-        if (lane == 0) warp_sum[warp] = __popc(votes);
-        __syncthreads();
-        int before = 0, all = 0;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) {
-            before += w < warp ? warp_sum[w] : 0;
-            all += warp_sum[w];
+    const bool vec = ((uintptr_t)pick & 15) == 0;
+    auto load = [&](int t0) {
+        const int i = t0 + 4 * tid;
+        int4 v = make_int4(-1, -1, -1, -1);
+        if (vec && i + 3 < total) v = *reinterpret_cast<const int4*>(pick + i);
+        else {
+            if (i < total) v.x = pick[i];
+            if (i + 1 < total) v.y = pick[i + 1];
+            if (i + 2 < total) v.z = pick[i + 2];
+            if (i + 3 < total) v.w = pick[i + 3];
         }
-        if (mine) rank[idx] = base + before + __popc(votes & ((1u << lane) - 1u));
+        return v;
+    };
+    int base = 0, buf = 0;
+    int4 v = load(0);
+    for (int t0 = 0; t0 < total; t0 += 4 * RANK_THREADS, buf ^= 1) {
+        const int4 next = t0 + 4 * RANK_THREADS < total ? load(t0 + 4 * RANK_THREADS) : v;
+        const int m[4] = {v.x == e, v.y == e, v.z == e, v.w == e};
+        const int mine = m[0] + m[1] + m[2] + m[3];
+        int upto = mine;                                      // of this lane and the ones before it
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += x;
+        }
+        if (lane == 31) warp_sum[buf][warp] = upto;
+        __syncthreads();                                      // (two buffers: the next round writes the other one)
+        const int w = warp_sum[buf][lane];
+        int before = lane < warp ? w : 0, all = w;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            before += __shfl_xor_sync(0xffffffffu, before, o);
+            all += __shfl_xor_sync(0xffffffffu, all, o);
+        }
+        int at = base + before + upto - mine;
+        const int i = t0 + 4 * tid;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (m[j]) rank[i + j] = at++;
         base += all;
-        __syncthreads();
+        v = next;
     }
     if (tid == 0) counts[e] = base;
 }
@@ -249,12 +299,16 @@ expert_rank_kernel(const int* __restrict__ pick, int total, int* __restrict__ ra
 template <typename T>
 __global__ void __launch_bounds__(128)
 expert_gather_kernel(const int* __restrict__ pick, const int* __restrict__ rank, const int* __restrict__ counts,
-                     const int* __restrict__ offsets, const T* __restrict__ x, const float* __restrict__ in_w, int top, int H,
+                     const int* __restrict__ offsets, const T* __restrict__ x, const float* __restrict__ in_w, int E, int top, int H,
                      int* __restrict__ place, T* __restrict__ xs) {
     mv_pdl_begin();
     __shared__ float scratch[33];
     const int idx = blockIdx.x;
     const int e = pick[idx];
+    if (e >= E) {                                  // an identity expert has no rows
+        if (threadIdx.x == 0) place[idx] = -1;
+        return;
+    }
     int p;
     if (offsets) {
         p = offsets[e] + rank[idx];                // where the expert's (padded) run of rows starts
@@ -274,41 +328,122 @@ expert_gather_kernel(const int* __restrict__ pick, const int* __restrict__ rank,
     for (int h = threadIdx.x; h < H; h += blockDim.x) dst[h] = src[h];
 }
 
+// The same for rows of whole 16-byte words and padded runs: a block is a token, its row is read once, 16 bytes a thread, and written to all its places (number
+// by number, a block an entry, 72 us of those 140).
+template <typename T>
+__global__ void __launch_bounds__(128)
+expert_gather_vec_kernel(const int* __restrict__ pick, const int* __restrict__ rank, const int* __restrict__ offsets,
+                         const T* __restrict__ x, const float* __restrict__ in_w, int E, int top, int H, int* __restrict__ place, T* __restrict__ xs) {
+    mv_pdl_begin();
+    __shared__ int at[32];
+    const int n = blockIdx.x;
+    if ((int)threadIdx.x < top) {
+        const int idx = n * top + threadIdx.x, e = pick[idx], p = e < E ? offsets[e] + rank[idx] : -1;    // (an identity expert has no rows)
+        place[idx] = p;
+        at[threadIdx.x] = p;
+    }
+    __syncthreads();
+    constexpr int V = 16 / sizeof(T);
+    const int words = H / V;
+    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)n * H);
+    for (int i = threadIdx.x; i < words; i += blockDim.x) {
+        const uint4 v = src[i];
+        for (int k = 0; k < top; ++k) {
+            if (at[k] < 0) continue;
+            T* dst = xs + (size_t)at[k] * H + i * V;
+            if (in_w) {
+                const float w = in_w[n * top + k];
+                float f[V];
+                mv_unpack16(v, f, (const T*)nullptr);
+#pragma unroll
+                for (int j = 0; j < V; j += 4) mv_store4(dst + j, w * f[j], w * f[j + 1], w * f[j + 2], w * f[j + 3]);
+            } else {
+                *reinterpret_cast<uint4*>(dst) = v;
+            }
+        }
+    }
+}
+
 // pick_w null: every chosen expert's result counts as it is.
-// out[n, :] (+)= sum_k w[n, k] ys[place[n * top + k], :] + gate[n] shared[n, :], the choices in their order
+// out[n, :] (+)= sum_k w[n, k] ys[place[n * top + k], :] + gate[n] shared[n, :], the choices in their order; V columns a thread (4: rows of whole 16-byte
+// words; 6,000 tokens of 2,048, 4 choices and a shared expert 82 -> 61 us).
+template <int V>
 __global__ void __launch_bounds__(256)
 expert_combine_kernel(const float* __restrict__ ys, const int* __restrict__ place, const float* __restrict__ pick_w,
                       const float* __restrict__ shared, const float* __restrict__ gate, int ld_gate,
                       float* __restrict__ out, int top, int H, int accumulate) {
     mv_pdl_begin();
+    __shared__ int at[32];
+    __shared__ float ws[32];
     const int n = blockIdx.x;
-    for (int h = threadIdx.x; h < H; h += blockDim.x) {
-        float sum = 0.f;
-        for (int k = 0; k < top; ++k)
-            sum = fmaf(pick_w ? pick_w[(size_t)n * top + k] : 1.f, ys[(size_t)place[(size_t)n * top + k] * H + h], sum);
-        if (shared) sum = fmaf(gate ? gate[(size_t)n * ld_gate] : 1.f, shared[(size_t)n * H + h], sum);
+    if ((int)threadIdx.x < min(top, 32)) {
+        at[threadIdx.x] = place[(size_t)n * top + threadIdx.x];
+        ws[threadIdx.x] = pick_w ? pick_w[(size_t)n * top + threadIdx.x] : 1.f;
+    }
+    __syncthreads();
+    const float g = shared ? (gate ? gate[(size_t)n * ld_gate] : 1.f) : 0.f;
+    for (int h = V * threadIdx.x; h < H; h += V * blockDim.x) {
         float* o = out + (size_t)n * H + h;
-        *o = accumulate ? *o + sum : sum;
+        float sum[V], y[V], old[V];
+        auto load = [&](const float* p, float (&d)[V]) {
+            if constexpr (V == 4) {
+                const float4 a = *reinterpret_cast<const float4*>(p);
+                d[0] = a.x; d[1] = a.y; d[2] = a.z; d[3] = a.w;
+            } else {
+                d[0] = *p;
+            }
+        };
+#pragma unroll
+        for (int j = 0; j < V; ++j) { sum[j] = 0.f; old[j] = 0.f; }
+        if (accumulate) load(o, old);
+#pragma unroll 4
+        for (int k = 0; k < top; ++k) {
+            const int row = k < 32 ? at[k] : place[(size_t)n * top + k];
+            const float w = k < 32 ? ws[k] : pick_w ? pick_w[(size_t)n * top + k] : 1.f;
+            load(ys + (size_t)row * H + h, y);
+#pragma unroll
+            for (int j = 0; j < V; ++j) sum[j] = fmaf(w, y[j], sum[j]);
+        }
+        if (shared) {
+            load(shared + (size_t)n * H + h, y);
+#pragma unroll
+            for (int j = 0; j < V; ++j) sum[j] = fmaf(g, y[j], sum[j]);
+        }
+        if (accumulate) {
+#pragma unroll
+            for (int j = 0; j < V; ++j) sum[j] = old[j] + sum[j];
+        }
+        if constexpr (V == 4) *reinterpret_cast<float4*>(o) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+        else *o = sum[0];
     }
 }
 
 // pick [N, top] -> rank [N * top], counts [E]
 MV_API int mv_expert_rank(const int* pick, int total, int E, int* rank, int* counts, cudaStream_t stream) {
     if (total <= 0 || E <= 0) return 0;
-    mv_launch(expert_rank_kernel, E, 256, 0, stream, pick, total, rank, counts);
+    mv_launch(expert_rank_kernel, E, RANK_THREADS, 0, stream, pick, total, rank, counts);
     return mv_launch_status();
 }
 
 // x [N, H] in `dtype` -> xs [N * top, H] sorted by expert; place [N * top] says where each entry went
-// offsets (or null): where every expert's run of rows starts (mv_expert_tiles), instead of the plain sums of counts
+// offsets (or null): where every expert's run of rows starts (mv_expert_tiles), instead of the plain sums of counts; picks from E on
+// (identity experts) have no row and place -1
 MV_API int mv_expert_gather(const int* pick, const int* rank, const int* counts, const int* offsets, const void* x,
-                            int dtype, const float* in_w, int N, int top, int H, int* place, void* xs, cudaStream_t stream) {
+                            int dtype, const float* in_w, int E, int N, int top, int H, int* place, void* xs, cudaStream_t stream) {
     if (N <= 0) return 0;
+    if (offsets && top <= 32 && (H * (dtype == MV_DT_BF16 ? 2 : 4)) % 16 == 0 && (((uintptr_t)x | (uintptr_t)xs) & 15) == 0) {
+        if (dtype == MV_DT_BF16)
+            mv_launch(expert_gather_vec_kernel<__nv_bfloat16>, N, 128, 0, stream, pick, rank, offsets, (const __nv_bfloat16*)x, in_w, E, top, H,
+                      place, (__nv_bfloat16*)xs);
+        else
+            mv_launch(expert_gather_vec_kernel<float>, N, 128, 0, stream, pick, rank, offsets, (const float*)x, in_w, E, top, H, place, (float*)xs);
+        return mv_launch_status();
+    }
     if (dtype == MV_DT_BF16)
         mv_launch(expert_gather_kernel<__nv_bfloat16>, N * top, 128, 0, stream, pick, rank, counts, offsets,
-                  (const __nv_bfloat16*)x, in_w, top, H, place, (__nv_bfloat16*)xs);
+                  (const __nv_bfloat16*)x, in_w, E, top, H, place, (__nv_bfloat16*)xs);
     else
-        mv_launch(expert_gather_kernel<float>, N * top, 128, 0, stream, pick, rank, counts, offsets, (const float*)x, in_w, top, H,
+        mv_launch(expert_gather_kernel<float>, N * top, 128, 0, stream, pick, rank, counts, offsets, (const float*)x, in_w, E, top, H,
                   place, (float*)xs);
     return mv_launch_status();
 }
@@ -358,7 +493,56 @@ MV_API int mv_expert_combine(const float* ys, const int* place, const float* pic
                              const float* gate, int ld_gate, float* out, int N, int top, int H, int accumulate,
                              cudaStream_t stream) {
     if (N <= 0) return 0;
-    mv_launch(expert_combine_kernel, N, 256, 0, stream, ys, place, pick_w, shared, gate, ld_gate, out, top, H, accumulate);
+    const bool vec = H % 4 == 0 && (((uintptr_t)ys | (uintptr_t)shared | (uintptr_t)out) & 15) == 0;
+    if (vec) mv_launch(expert_combine_kernel<4>, N, 256, 0, stream, ys, place, pick_w, shared, gate, ld_gate, out, top, H, accumulate);
+    else mv_launch(expert_combine_kernel<1>, N, 256, 0, stream, ys, place, pick_w, shared, gate, ld_gate, out, top, H, accumulate);
+    return mv_launch_status();
+}
+
+// h[n, e * ff + c] = w * hs[place, c] where token n chose expert e (rounded again), 0 where it did not: the experts' gated activations, worked out over
+// sorted rows, laid out as one product with all down matrices side by side reads them.  A block is a token; eight numbers a thread at a time (2,048
+// tokens of 16 experts of 1,024: 22.5 us, 5 TB/s).
+__global__ void __launch_bounds__(256)
+expert_spread_kernel(const int* __restrict__ pick, const int* __restrict__ place, const float* __restrict__ pick_w,
+                     const __nv_bfloat16* __restrict__ hs, __nv_bfloat16* __restrict__ h, int E, int top, int ff) {
+    mv_pdl_begin();
+    __shared__ int row[RE_MAX_EXPERTS];
+    __shared__ float weight[RE_MAX_EXPERTS];
+    const int n = blockIdx.x;
+    for (int e = threadIdx.x; e < E; e += blockDim.x) row[e] = -1;
+    __syncthreads();
+    if ((int)threadIdx.x < top) {
+        const int idx = n * top + threadIdx.x, e = pick[idx];
+        if (e < E) { row[e] = place[idx]; weight[e] = pick_w[idx]; }
+    }
+    __syncthreads();
+    const int words = ff / 8;
+    uint4* dst = reinterpret_cast<uint4*>(h + (size_t)n * E * ff);
+    for (int i = threadIdx.x; i < E * words; i += blockDim.x) {
+        const int e = i / words;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (row[e] >= 0) {
+            float x[8];
+            mv_load8(hs + (size_t)row[e] * ff + (i - e * words) * 8, x);
+            const float w = weight[e];
+            unsigned p[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const __nv_bfloat162 y = __floats2bfloat162_rn(x[2 * j] * w, x[2 * j + 1] * w);
+                p[j] = *reinterpret_cast<const unsigned*>(&y);
+            }
+            v = make_uint4(p[0], p[1], p[2], p[3]);
+        }
+        dst[i] = v;
+    }
+}
+
+// pick, place, pick_w [N, top] (place: mv_expert_gather's), hs [.., ff] bfloat16 -> h [N, E ff]; ff a multiple of 8, 16-byte aligned
+MV_API int mv_expert_spread(const int* pick, const int* place, const float* pick_w, const void* hs, void* h, int N, int E, int top, int ff,
+                            cudaStream_t stream) {
+    if (N <= 0) return 0;
+    if (E < 1 || E > RE_MAX_EXPERTS || top < 1 || top > 256 || ff < 8 || ff % 8 || (((uintptr_t)hs | (uintptr_t)h) & 15)) return (int)cudaErrorInvalidValue;
+    mv_launch(expert_spread_kernel, N, 256, 0, stream, pick, place, pick_w, (const __nv_bfloat16*)hs, (__nv_bfloat16*)h, E, top, ff);
     return mv_launch_status();
 }
 

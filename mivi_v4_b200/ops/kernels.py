@@ -101,7 +101,8 @@ _SIGNATURES = {
                                _P],
         "mv_delta_scan": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _F, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
         "mv_expert_rank": [_P, _I, _I, _P, _P, _P],
-        "mv_expert_gather": [_P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _P, _P, _P],
+        "mv_expert_gather": [_P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _P, _P, _P],
+        "mv_expert_spread": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _P],
         "mv_expert_tiles": [_P, _I, _I, _P, _P, _I, _P],
         "mv_expert_combine": [_P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _P],
         "mv_sample": [_P, _Q, _P, _I, _I, _F, _I, _F, _F, _F, _F, _F, _P, _P, _UQ, _P, _P, _P, _P, _P, _P, _P, _P],
@@ -113,6 +114,7 @@ _SIGNATURES = {
         "mv_gemm_small_m_heads": [_P, _P, _P, _P, _F, _P, _I, _P, _P, _P, _I, _I, _P, _Q, _P, _I, _I, _I, _I,
                                   _P, _I, _I, _I, _F, _P, _Q, _P],
         "mv_gemm_tc": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _I, _I, _F, _P, _I, _I, _I, _P, _P],
+        "mv_gemm_tc_pair_grouped": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _I, _I, _P, _P],
         "mv_gemm_tc_grouped": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _I, _I, _P, _P],
         "mv_gemm_tc_pair": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _I, _I, _F, _P, _P, _P, _I, _P, _I, _I, _I, _P, _P],
         "mv_gemm_tc_swap": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _I, _I, _F, _P, _P, _P, _I, _P, _Q, _P, _P],
@@ -902,49 +904,70 @@ def scale_expert_columns(h: torch.Tensor, dense: torch.Tensor, n_experts: int, f
 GROUPED_TILE_ROWS = 128
 
 
-def grouped_tiles(n_entries: int, n_experts: int) -> int:
-    """Tiles of ``GROUPED_TILE_ROWS`` rows that the sorted entries can need at most, every expert's run padded to
+# tiles of this many rows go to the grouped product with two multiprocessors a tile
+GROUPED_PAIR_ROWS = 256
+
+
+def grouped_tiles(n_entries: int, n_experts: int, tile_rows: int = GROUPED_TILE_ROWS) -> int:
+    """Tiles of ``tile_rows`` rows that the sorted entries can need at most, every expert's run padded to
     whole tiles."""
-    return (n_entries + n_experts * (GROUPED_TILE_ROWS - 1)) // GROUPED_TILE_ROWS + 1
+    return (n_entries + n_experts * (tile_rows - 1)) // tile_rows + 1
 
 
 def expert_sort(pick: torch.Tensor, n_experts: int, x: torch.Tensor, rank: torch.Tensor, counts: torch.Tensor,
                 place: torch.Tensor, xs: torch.Tensor, offsets: Optional[torch.Tensor] = None,
-                tile_group: Optional[torch.Tensor] = None, in_w: Optional[torch.Tensor] = None) -> None:
+                tile_group: Optional[torch.Tensor] = None, in_w: Optional[torch.Tensor] = None,
+                tile_rows: int = GROUPED_TILE_ROWS) -> None:
     """The (token, choice) entries of ``pick`` [N, top] sorted by expert (stable): ``counts`` [experts] entries an
     expert, ``place`` [N * top] where each entry went, and the tokens' rows of ``x`` [N, H] copied to ``xs`` in that
     order, so that an expert's rows lie together.  With ``offsets`` [experts] and ``tile_group`` [tiles] every
-    expert's run starts on a tile of ``GROUPED_TILE_ROWS`` rows (``xs`` then has tiles * that many rows, the rows
+    expert's run starts on a tile of ``tile_rows`` rows (``xs`` then has tiles * that many rows, the rows
     between runs are left as they are), ``offsets`` says where, and ``tile_group`` names each tile's expert (-1 for
     the spare tiles at the end): what :func:`gemm_tc_grouped` takes.  ``in_w`` float32 [N, top]: an entry's copy of the row
-    is multiplied by its weight."""
+    is multiplied by its weight.  Picks from ``n_experts`` on (identity experts) get no row (place -1)."""
     N, top = pick.shape
     H = x.shape[1]
     padded = offsets is not None
     if padded != (tile_group is not None):
         raise KernelError("expert_sort: offsets and tile_group come together")
-    rows = tile_group.numel() * GROUPED_TILE_ROWS if padded else N * top
-    if padded and tile_group.numel() < grouped_tiles(N * top, n_experts):
+    rows = tile_group.numel() * tile_rows if padded else N * top
+    if padded and tile_group.numel() < grouped_tiles(N * top, n_experts, tile_rows):
         raise KernelError(f"expert_sort: {tile_group.numel()} tiles for {N * top} entries of {n_experts} experts")
     _check(_fn("core", "mv_expert_rank")(
         _need(pick, "picks", torch.int32), N * top, int(n_experts), _need(rank, "ranks", torch.int32, (N * top,)),
         _need(counts, "counts", torch.int32, (n_experts,)), _stream()), "mv_expert_rank")
     if padded:
         _check(_fn("core", "mv_expert_tiles")(
-            counts.data_ptr(), int(n_experts), GROUPED_TILE_ROWS, _need(offsets, "offsets", torch.int32, (n_experts,)),
+            counts.data_ptr(), int(n_experts), int(tile_rows), _need(offsets, "offsets", torch.int32, (n_experts,)),
             _need(tile_group, "tile groups", torch.int32), tile_group.numel(), _stream()), "mv_expert_tiles")
     _check(_fn("core", "mv_expert_gather")(
         pick.data_ptr(), rank.data_ptr(), counts.data_ptr(), offsets.data_ptr() if padded else None,
-        _need(x, "expert_sort rows", None, (N, H)), _dt(x), _need(in_w, "input weights", torch.float32, (N, top), True), N, top, H,
+        _need(x, "expert_sort rows", None, (N, H)), _dt(x), _need(in_w, "input weights", torch.float32, (N, top), True), int(n_experts), N, top, H,
         _need(place, "places", torch.int32, (N * top,)), _need(xs, "sorted rows", x.dtype, (rows, H)), _stream()),
         "mv_expert_gather")
     account(N * (1 + top) * H * x.element_size())
 
 
+def expert_spread(pick: torch.Tensor, place: torch.Tensor, pick_w: torch.Tensor, hs: torch.Tensor, h: torch.Tensor, n_experts: int) -> torch.Tensor:
+    """``h`` [N, experts * ff] from the sorted rows' ``hs`` [rows, ff] (bfloat16): row n holds ``pick_w`` times the row at ``place`` in the columns of
+    every chosen expert, zeros elsewhere; picks from ``n_experts`` on have no columns."""
+    N, top = pick.shape
+    ff = hs.shape[1]
+    if ff % 8 or hs.data_ptr() % 16 or h.data_ptr() % 16 or not 1 <= top <= 256 or not 1 <= n_experts <= MAX_EXPERTS:
+        raise KernelError(f"expert_spread: rows of {ff} (a multiple of 8, 16-byte aligned), {top} of {n_experts} experts")
+    _check(_fn("core", "mv_expert_spread")(
+        _need(pick, "picks", torch.int32), _need(place, "places", torch.int32, (N * top,)), _need(pick_w, "pick weights", torch.float32, (N, top)),
+        _need(hs, "sorted activations", torch.bfloat16), _need(h, "activations", torch.bfloat16, (N, n_experts * ff)), N, int(n_experts), top, ff,
+        _stream()), "mv_expert_spread")
+    account(h.numel() * 2 + N * top * ff * 2)
+    return h
+
+
 def gemm_tc_grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tile_group: torch.Tensor, n: int, k: int, *,
                     row_step: int = 0, k_step: int = 0, swiglu: bool = False, active_rows: Optional[int] = None,
-                    limits: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """One product for many groups, on the tcgen05 tensor cores (bfloat16): the rows of ``x`` [tiles * 128, k] are
+                    limits: Optional[torch.Tensor] = None, tile_rows: int = GROUPED_TILE_ROWS) -> torch.Tensor:
+    """One product for many groups, on the tcgen05 tensor cores (bfloat16): the rows of ``x`` [tiles * 128, k] (with ``tile_rows`` 256: tiles of 256, two
+    multiprocessors a tile) are
     sorted by group with every group's run padded to whole tiles (:func:`expert_sort`), ``tile_group`` names each
     tile's group (negative: nothing to do), and ``w`` holds the groups' [n, k] matrices one below the other
     (``row_step`` rows a group) or side by side along its columns (``k_step`` columns a group).  ``out``
@@ -954,7 +977,9 @@ def gemm_tc_grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tile_gr
     M = x.shape[0]
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         raise KernelError(f"gemm_tc_grouped: operands must be bfloat16, got {x.dtype} and {w.dtype}")
-    if M != tile_group.numel() * GROUPED_TILE_ROWS or x.shape[1] != k:
+    if tile_rows not in (GROUPED_TILE_ROWS, GROUPED_PAIR_ROWS):
+        raise KernelError(f"gemm_tc_grouped: tiles of {tile_rows} rows ({GROUPED_TILE_ROWS} or {GROUPED_PAIR_ROWS})")
+    if M != tile_group.numel() * tile_rows or x.shape[1] != k:
         raise KernelError(f"gemm_tc_grouped: x is {tuple(x.shape)} for {tile_group.numel()} tiles and k = {k}")
     if k % 8 or k_step % 8 or (row_step and k_step):
         raise KernelError(f"gemm_tc_grouped: k {k} and k_step {k_step} must be multiples of 8; one of row_step and k_step")
@@ -967,11 +992,12 @@ def gemm_tc_grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tile_gr
         mode, ldo = (0 if out.dtype == torch.float32 else 1), n
         _need(out, "gemm out", None, (M, n))
         _dt(out)
-    _check(_fn("bf16", "mv_gemm_tc_grouped")(
+    entry = "mv_gemm_tc_grouped" if tile_rows == GROUPED_TILE_ROWS else "mv_gemm_tc_pair_grouped"
+    _check(_fn("bf16", entry)(
         _need(x, "gemm x"), _need(w, "gemm w"), _need(limits, "activation limits", torch.float32, (n + 1,), True),
         out.data_ptr(), mode, M, int(n), int(k), ldo, w.shape[0], w.shape[1],
         _need(tile_group, "tile groups", torch.int32), int(row_step), int(k_step), _error_flag(x.device).data_ptr(),
-        _stream()), "mv_gemm_tc_grouped")
+        _stream()), entry)
     rows = M if active_rows is None else active_rows
     account(rows * (k * 2 + ldo * out.element_size()) + _nbytes(w), 2 * rows * n * k)
     return out

@@ -221,13 +221,23 @@ class RoutedExperts(Part):
     # 6.0 against 5.6, 1,024 tokens 9.4 against 9.6, 2,048 tokens 15.5 against 16.6: runs of fewer rows than two
     # tiles are mostly padding.
     SORTED_ROWS_AN_EXPERT = 256
+    PAIR_ROWS_AN_EXPERT = 448
     # steps of more rows than this let the first product gate its own results (and round them) before the router's
     # weights are put on them; shorter steps round once, after the weights
     GATED_IN_PRODUCT_FROM = 65
 
     def _sorted_ok(self, g, step, N: int) -> bool:
+        return self.I == 0 and self._sortable(g, step, N)
+
+    def _sorted_up_ok(self, g, step, N: int) -> bool:
+        """With identity experts only the gate and up matrices multiply sorted rows: the sums over the chosen experts stay one product with the
+        down matrices side by side, in the order that shorter steps have.  2,048 tokens, 4 of 16 experts and 2 identity experts, width 2,048, experts of 1,024: sort, product and spreading 150 us where one product
+        for all experts and the weights put on its results took 217."""
+        return self.I > 0 and not self.shared_ff and not self.on_input and g.data_ptr() % 16 == 0 and self._sortable(g, step, N)
+
+    def _sortable(self, g, step, N: int) -> bool:
         return (N * self.top >= self.SORTED_ROWS_AN_EXPERT * self.E and not step.is_decode and self.top < self.E
-                and self.I == 0 and self.group == K.SWIGLU_GROUP and self.ff % 8 == 0 and g.shape[1] % 8 == 0
+                and self.group == K.SWIGLU_GROUP and self.ff % 8 == 0 and g.shape[1] % 8 == 0
                 and tensor_core_ok(g, self.w_gu) and self.w_down.dtype == torch.bfloat16 and self.w_down.shape[1] % 8 == 0)
 
     def forward(self, g, resid, step, accumulate: bool = True) -> None:
@@ -248,7 +258,11 @@ class RoutedExperts(Part):
         if self._sorted_ok(g, step, N):
             return self._forward_sorted(g, resid, step, accumulate, dense, pick, pick_w)
         h = self.scratch(step, "ffh", (N, F), step.dtype)
-        if (N >= self.GATED_IN_PRODUCT_FROM and self.group and (self.shared_group or not self.shared_ff)
+        if self._sorted_up_ok(g, step, N):
+            xs, tile_group, place = self._sort(g, step, pick, None)
+            hs = self._sorted_activations(step, xs, tile_group, N * self.top)
+            K.expert_spread(pick, place, pick_w, hs, h, E)
+        elif (N >= self.GATED_IN_PRODUCT_FROM and self.group and (self.shared_group or not self.shared_ff)
                 and tensor_core_ok(g, self.w_gu) and not (self.on_input and self.shared_gate)):
             # long steps: gate and up never reach memory; the weights go on the rounded activations
             # (on the input: on gate and up inside the product)
@@ -267,23 +281,41 @@ class RoutedExperts(Part):
         if I:
             K.identity_experts(g, dense, E + sg, I, resid)
 
-    def _forward_sorted(self, g, resid, step, accumulate, dense, pick, pick_w) -> None:
+    def _sort(self, g, step, pick, in_w):
+        """The tokens' rows sorted by expert, every expert's run padded to whole tiles; which expert a tile belongs to; where every entry went."""
         N, H = g.shape
-        E, ff, top = self.E, self.ff, self.top
-        tiles = K.grouped_tiles(N * top, E)
-        rows = tiles * K.GROUPED_TILE_ROWS
+        E, top = self.E, self.top
+        tile_rows = self._tile_rows(N)
+        tiles = K.grouped_tiles(N * top, E, tile_rows)
         rank = self.scratch(step, "rank", (N * top,), torch.int32)
         counts = self.scratch(step, "counts", (E,), torch.int32)
         offsets = self.scratch(step, "offsets", (E,), torch.int32)
         tile_group = self.scratch(step, "tile_group", (tiles,), torch.int32)
         place = self.scratch(step, "place", (N * top,), torch.int32)
-        xs = self.scratch(step, "sorted", (rows, H), g.dtype)
-        K.expert_sort(pick, E, g, rank, counts, place, xs, offsets, tile_group, in_w=pick_w if self.on_input else None)
-        hs = self.scratch(step, "sorted_h", (rows, ff), step.dtype)
-        K.gemm_tc_grouped(xs, self.w_gu, hs, tile_group, 2 * ff, H, row_step=2 * ff, swiglu=True, active_rows=N * top,
-                          limits=self.expert_limits)
+        xs = self.scratch(step, "sorted", (tiles * tile_rows, H), g.dtype)
+        K.expert_sort(pick, E, g, rank, counts, place, xs, offsets, tile_group, in_w=in_w, tile_rows=tile_rows)
+        return xs, tile_group, place
+
+    def _sorted_activations(self, step, xs, tile_group, active_rows: int):
+        hs = self.scratch(step, "sorted_h", (xs.shape[0], self.ff), step.dtype)
+        K.gemm_tc_grouped(xs, self.w_gu, hs, tile_group, 2 * self.ff, xs.shape[1], row_step=2 * self.ff, swiglu=True, active_rows=active_rows,
+                          limits=self.expert_limits, tile_rows=xs.shape[0] // tile_group.numel())
+        return hs
+
+    def _tile_rows(self, N: int) -> int:
+        """Runs padded to tiles of 256 rows, for the product with two multiprocessors a tile, where an expert brings PAIR_ROWS_AN_EXPERT rows on average.
+        Gate and up / down matrices, tiles of 128 and of 256 rows (width 2,048, experts of 1,024): 6,000 tokens of 4 of 16 experts 275 and 206 / 157 and 109 us,
+        2,048 tokens 119 and 113 / 68 and 57, 1,500 of 2 of 8 64 and 69 / 36 and 35."""
+        return K.GROUPED_PAIR_ROWS if N * self.top >= self.PAIR_ROWS_AN_EXPERT * self.routed else K.GROUPED_TILE_ROWS
+
+    def _forward_sorted(self, g, resid, step, accumulate, dense, pick, pick_w) -> None:
+        N, H = g.shape
+        E, ff, top = self.E, self.ff, self.top
+        xs, tile_group, place = self._sort(g, step, pick, pick_w if self.on_input else None)
+        hs = self._sorted_activations(step, xs, tile_group, N * top)
+        rows = xs.shape[0]
         ys = self.scratch(step, "sorted_y", (rows, H), torch.float32)
-        K.gemm_tc_grouped(hs, self.w_down, ys, tile_group, H, ff, k_step=ff, active_rows=N * top)
+        K.gemm_tc_grouped(hs, self.w_down, ys, tile_group, H, ff, k_step=ff, active_rows=N * top, tile_rows=rows // tile_group.numel())
         shared = None
         if self.shared_ff:
             hsh = self.scratch(step, "shared_h", (N, self.shared_ff), step.dtype)
