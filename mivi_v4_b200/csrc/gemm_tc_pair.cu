@@ -20,10 +20,12 @@
 //            in the leader one lane issues four 256 x 256 x 16 MMAs per K block and
 //            commits them to the stage's "empty" barrier of BOTH blocks, at a tile's
 //            end to the "accumulator full" barrier of both;
-//   warps 2-5 in both blocks drain their block's 128 rows of the accumulator (two
+//   warps 2-9 in both blocks drain their block's 128 rows of the accumulator, two warps 32
+//            rows, 128 columns each (two
 //            accumulators of 256 columns alternate, so the drain of one tile runs
 //            under the MMAs of the next) and arrive on the leader's "accumulator
-//            empty" barrier.
+//            empty" barrier.  (With four warps a drain that works out a gated activation took longer than the
+//            products of the next tile: 7,407 x 20,480 x 1,536 with silu 377 -> 305 us, with the clamped activation 451 -> 331, 6,000 x 8,192 x 2,048 152 -> 129.)
 // Every wait is bounded as in gemm_tc.cu; a block that gives up still reaches the
 // pair's final barrier, so its peer is never left waiting for it.
 //
@@ -33,7 +35,8 @@
 
 namespace {
 
-constexpr int PAIR_THREADS = 192;
+constexpr int PAIR_THREADS = 320;
+constexpr int DRAIN_WARPS = 8;          // a block's warps that drain accumulators: two for each quarter of its rows
 constexpr int PAIR_BN = 256;          // columns of Y a pair's tile has; each block holds 128 rows of W for them
 
 #include "gemm_tc_store.cuh"
@@ -58,7 +61,7 @@ struct PairLayout {
     static constexpr int A_BYTES = BM * BK * 2, B_BYTES = (PAIR_BN / 2) * BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;                 // of one block
     static constexpr int TILE_BYTES = STAGES * STAGE_BYTES;
-    static constexpr int TURN_BYTES = 4 * 32 * 32 * 4;                    // each epilogue warp turns 32 x 32 floats
+    static constexpr int TURN_BYTES = DRAIN_WARPS * 32 * 32 * 4;                    // each epilogue warp turns 32 x 32 floats
     static constexpr int BAR_BYTES = (2 * STAGES + 4) * 8 + 8;
     static constexpr int TOTAL = TILE_BYTES + TURN_BYTES + BAR_BYTES + 1024;
 };
@@ -129,7 +132,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(acc_full0 + 8 * a, 1);              // each block's own
-            mbar_init(acc_empty0 + 8 * a, 8);             // the leader's: four epilogue warps of each block
+            mbar_init(acc_empty0 + 8 * a, 2 * DRAIN_WARPS);   // the leader's: the epilogue warps of both blocks
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -199,8 +202,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
         }
     } else {
-        const int quarter = warp & 3;
-        float* turn = (float*)(smem + L::TILE_BYTES) + quarter * (32 * 32);
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        // this warp's chunks of 32 columns (a product that emits a norm sums a row's squares over the whole tile: one warp for all)
+        const int c_first = link.emit_x ? 0 : half * (BN / 64), c_last = link.emit_x ? (half ? 0 : BN / 32) : c_first + BN / 64;
+        float* turn = (float*)(smem + L::TILE_BYTES) + (half * 4 + quarter) * (32 * 32);
         const bool by_rows = link.by_rows != 0;
         int local = 0;
         bool ok = true;
@@ -233,9 +238,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         if (row0 + 4 * i < M) dst[i] = *reinterpret_cast<const float4*>(op + (size_t)(4 * i) * ldo + 32 * c);
                 }
             };
-            if (link.emit_x) request(0, old);
+            if (link.emit_x && half == 0) request(0, old);
             WeightCursor wc;
-            if (ACT == ACT_WEIGHTED) wc.move(rw, row, M, n0 >> 5);
+            if (ACT == ACT_WEIGHTED) wc.move(rw, row, M, (n0 >> 5) + c_first);
             ok = mbar_wait(acc_full0 + 8 * acc, acc_phase, err, 3);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -245,7 +250,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll
                 for (int i = 0; i < 8; ++i) sq[i] = 0.f;
 #pragma unroll 1
-                for (int c = 0; c < BN / 32; ++c) {
+                for (int c = c_first; c < c_last; ++c) {
                     if (n0 + 32 * c >= N) break;
                     unsigned r[32];
                     tmem_ld32(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(acc * BN + 32 * c), r);
@@ -292,7 +297,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         for (int i = 0; i < 8; ++i) old[i] = nxt[i];
                     }
                 }
-                if (link.emit_x) {
+                if (link.emit_x && half == 0) {
                     // a row's sum of squares over the tile: its eight lanes' sums together
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
@@ -305,7 +310,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
             } else {
 #pragma unroll 1
-                for (int c0 = 0; c0 < BN; c0 += 32) {
+                for (int c0 = 32 * c_first; c0 < 32 * c_last; c0 += 32) {
                     if (n0 + c0 >= N) break;
                     unsigned r[32];
                     tmem_ld32(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(acc * BN + c0), r);
