@@ -9,6 +9,7 @@ is an error, and so is a library that cannot be built.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from dataclasses import dataclass
 from typing import Optional, Tuple
@@ -1743,6 +1744,7 @@ def _account_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulat
 F32_TC_ROWS, F32_TC_K = 9, 1024
 
 
+@functools.lru_cache(maxsize=4096)
 def gemm_f32_tc_takes(M: int, N: int, K: int, sms: int) -> bool:
     """Whether a float32 product goes to the tensor cores (``gemm_f32_tc.cu``) or to the CUDA cores: by what either is expected to take, in us.  The
     tensor cores work in rounds of tiles of 128 x 128 or 128 x 96, 26.4 or 21.9 us for 1,024 of K whatever a tile's rows; the CUDA cores add
@@ -1773,9 +1775,9 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, bias: Opti
         mode = 0 if out.dtype == torch.float32 else 1
         _need(out, "gemm out", None, (M, N))
         _dt(out)
-    if x.dtype == torch.float32 and gemm_f32_tc_takes(M, N, K, n_sms(x.device)) and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
+    if x.dtype == torch.float32 and gemm_f32_tc_takes(M, N, K, n_sms()) and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
         _check(_fn("core", "mv_gemm_f32_tc")(
-            _need(x, "gemm x"), _need(w, "gemm w"), _need(bias, "gemm bias", torch.float32, (N,), True), out.data_ptr(), mode, M, N, K, N, n_sms(x.device),
+            _need(x, "gemm x"), _need(w, "gemm w"), _need(bias, "gemm bias", torch.float32, (N,), True), out.data_ptr(), mode, M, N, K, N, n_sms(),
             _error_flag(x.device).data_ptr(), _stream()), "mv_gemm_f32_tc")
         _account_gemm(x, w, out, accumulate)
         return out
