@@ -140,6 +140,7 @@ class SequenceCache:
         self._nblk = np.zeros(max(n_slots, 1), dtype=np.int64)
         self._table: Dict[int, np.ndarray] = {g: np.zeros((max(n_slots, 1), 8), dtype=np.int32) for g in self.kv_groups}
         self.storage: Dict[int, torch.Tensor] = {}
+        self._state_views: Dict[int, List[torch.Tensor]] = {}      # slot -> its state in every layer
         for gi, g in enumerate(plan.groups):
             if isinstance(g.need, KVNeed):
                 if g.need.uneven:
@@ -168,6 +169,7 @@ class SequenceCache:
             new = torch.zeros((old.shape[0], n_slots) + tuple(old.shape[2:]), dtype=old.dtype, device=old.device)
             new[:, :old.shape[1]] = old
             self.storage[gi] = new
+        self._state_views.clear()
         add = n_slots - self._len.shape[0]
         if add > 0:
             self._len = np.concatenate([self._len, np.zeros(add, dtype=np.int64)])
@@ -185,8 +187,12 @@ class SequenceCache:
         self._len[s], self._nblk[s], self._assigned[s] = 0, 0, True
         for t in self._table.values():
             t[s] = 0
-        for gi in self.state_groups:
-            self.storage[gi][:, s].zero_()
+        if self.state_groups:
+            # one launch for the states of all layers (a launch a group took 5 us of the host each)
+            views = self._state_views.get(s)
+            if views is None:
+                views = self._state_views[s] = [layer for gi in self.state_groups for layer in self.storage[gi][:, s].unbind(0)]
+            torch._foreach_zero_(views)
         return s
 
     def release(self, slot: int) -> None:

@@ -116,7 +116,7 @@ class StepContext:
     """
 
     def __init__(self, *, slots: List[int], starts: List[int], token_lists: List[List[int]],
-                 out_rows: List[int], page_rows: Dict[int, List[List[int]]], dtype: torch.dtype,
+                 out_rows: Sequence[int], page_rows: Dict[int, List[List[int]]], dtype: torch.dtype,
                  ws: Workspace, upload: bool = True):
         device = ws.device
         self.ws, self.dtype, self.device = ws, dtype, device
@@ -124,8 +124,9 @@ class StepContext:
         self.host_lens = [len(t) for t in token_lists]
         self.n_seqs = len(slots)
         self.n_tokens = sum(self.host_lens)
-        self.n_out = len(out_rows)
-        self.out_rows_all = list(out_rows) == list(range(self.n_tokens))     # every row's logits, in order
+        out_rows = np.asarray(out_rows, dtype=np.int64).ravel()
+        self.n_out = int(out_rows.size)
+        self.out_rows_all = self.n_out == self.n_tokens and bool((out_rows == np.arange(self.n_tokens)).all())   # every row's logits, in order
         self.is_decode = all(n == 1 for n in self.host_lens)
         self.max_len = max(self.host_lens, default=0)
         self.max_context = max((s + n for s, n in zip(starts, self.host_lens)), default=0)
@@ -165,7 +166,7 @@ class StepContext:
         put("slots", list(slots))
         put("starts", starts_a)
         put("lens", lens)
-        put("out_rows", list(out_rows))
+        put("out_rows", out_rows)
         widths: Dict[int, int] = {}
         for g, rows in page_rows.items():
             widths[g] = len(rows[0]) if rows else 1
