@@ -195,6 +195,50 @@ gated_rmsnorm_block_kernel(const float* __restrict__ x, const float* __restrict_
     }
 }
 
+// The same with a row's values and gates in registers, at most PER a thread: they are read once, and a gate before the norm is worked out once
+// (2,048 tokens of 4,096 with the gate first 44 -> 32 us; of 2,048 with it last 22 -> 16).
+template <typename TO, int PER>
+__global__ void __launch_bounds__(1024)
+gated_rmsnorm_held_kernel(const float* __restrict__ x, const float* __restrict__ gate, int ld_gate,
+                          const float* __restrict__ w, int w_len, TO* __restrict__ y, int C, int group, float eps,
+                          int act) {
+    mv_pdl_begin();
+    __shared__ float scratch[33];
+    const int per_row = C / group;
+    const long long n = blockIdx.x / per_row;
+    const int c0 = (int)(blockIdx.x - n * per_row) * group;
+    const float* xr = x + (size_t)n * C + c0;
+    const float* gr = gate + (size_t)n * ld_gate + c0;
+    float v[PER], g[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int d = threadIdx.x + i * blockDim.x;
+        v[i] = d < group ? xr[d] : 0.f;
+        g[i] = d < group ? gr[d] : 0.f;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        if (act == 2) v[i] = gn_gated_first(v[i], g[i]);
+        if ((int)(threadIdx.x + i * blockDim.x) < group) ss = fmaf(v[i], v[i], ss);
+    }
+    const float scale = 1.0f / sqrtf(mv_block_sum(ss, scratch) / (float)group + eps);
+    TO* yr = y + (size_t)n * C + c0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int d = threadIdx.x + i * blockDim.x;
+        if (d < group) {
+            const float wv = w[w_len == C ? c0 + d : (c0 + d) % w_len];
+            float out = v[i] * scale * wv;
+            if (act != 2) {
+                const float sg = 1.0f / (1.0f + expf(-g[i]));
+                out *= act == 0 ? g[i] * sg : sg;
+            }
+            yr[d] = mv_from_f32<TO>(out);
+        }
+    }
+}
+
 MV_API int mv_gated_rmsnorm(const float* x, const float* gate, int ld_gate, const float* w, int w_len, void* y,
                             int y_dtype, int N, int C, int group, float eps, int act, cudaStream_t stream) {
     if (N <= 0) return 0;
@@ -203,6 +247,13 @@ MV_API int mv_gated_rmsnorm(const float* x, const float* gate, int ld_gate, cons
     if (group >= 512) {
         // few (row, group) pairs of many values each (a decode step of a wide layer): more threads a block
         const int threads = (n_groups < 1024 && group >= 4096) ? 1024 : ((n_groups < 2048 && group >= 2048) ? 512 : 256);
+        if (group <= 16 * threads) {
+#define GR_HELD(TO, PER) mv_launch(gated_rmsnorm_held_kernel<TO, PER>, (unsigned)n_groups, threads, 0, stream, x, gate, ld_gate, w, w_len, (TO*)y, C, group, eps, act)
+            if (y_dtype == MV_DT_BF16) { if (group <= 8 * threads) GR_HELD(__nv_bfloat16, 8); else GR_HELD(__nv_bfloat16, 16); }
+            else { if (group <= 8 * threads) GR_HELD(float, 8); else GR_HELD(float, 16); }
+#undef GR_HELD
+            return mv_launch_status();
+        }
         if (y_dtype == MV_DT_BF16)
             mv_launch(gated_rmsnorm_block_kernel<__nv_bfloat16>, (unsigned)n_groups, threads, 0, stream, x, gate, ld_gate, w,
                       w_len, (__nv_bfloat16*)y, C, group, eps, act);
@@ -472,10 +523,65 @@ __global__ void rmsnorm_add_layernorm_kernel(const float* __restrict__ y, const 
     for (int h = threadIdx.x; h < H; h += blockDim.x) orow[h] = mv_from_f32<TO>((rr[h] - mean) * rstd * ln_w[h]);
 }
 
+// The same with the row in registers, at most PER values a thread (2,048 rows of 2,048: 22 -> 14 us; with room for 8 the block
+// needs twice the registers: 26).
+template <typename TO, int PER>
+__global__ void __launch_bounds__(512)
+rmsnorm_add_layernorm_held_kernel(const float* __restrict__ y, const float* __restrict__ w, float eps,
+                                  float* __restrict__ resid, const float* __restrict__ ln_w, float ln_eps,
+                                  TO* __restrict__ out, int H) {
+    mv_pdl_begin();
+    __shared__ float scratch[33];
+    const float* yr = y + (size_t)blockIdx.x * H;
+    float* rr = resid + (size_t)blockIdx.x * H;
+    float v[PER], r[PER];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int h = threadIdx.x + i * blockDim.x;
+        v[i] = h < H ? yr[h] : 0.f;
+        r[i] = h < H ? rr[h] : 0.f;
+        ss = fmaf(v[i], v[i], ss);
+    }
+    const float scale = 1.0f / sqrtf(mv_block_sum(ss, scratch) / (float)H + eps);
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int h = threadIdx.x + i * blockDim.x;
+        if (h < H) {
+            r[i] = r[i] + v[i] * scale * w[h];
+            rr[h] = r[i];
+            sum += r[i];
+        }
+    }
+    const float mean = mv_block_sum(sum, scratch) / (float)H;
+    float dev = 0.f;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const float d = r[i] - mean;
+        if ((int)(threadIdx.x + i * blockDim.x) < H) dev = fmaf(d, d, dev);
+    }
+    const float rstd = 1.0f / sqrtf(mv_block_sum(dev, scratch) / (float)H + ln_eps);
+    TO* orow = out + (size_t)blockIdx.x * H;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int h = threadIdx.x + i * blockDim.x;
+        if (h < H) orow[h] = mv_from_f32<TO>((r[i] - mean) * rstd * ln_w[h]);
+    }
+}
+
 MV_API int mv_rmsnorm_add_layernorm(const float* y, const float* w, float eps, float* resid, const float* ln_w,
                                     float ln_eps, void* out, int out_dtype, int N, int H, cudaStream_t stream) {
     if (N <= 0) return 0;
     const int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
+    if (H <= 4 * threads) {
+        if (out_dtype == MV_DT_BF16)
+            mv_launch(rmsnorm_add_layernorm_held_kernel<__nv_bfloat16, 4>, N, threads, 0, stream, y, w, eps, resid, ln_w, ln_eps,
+                      (__nv_bfloat16*)out, H);
+        else
+            mv_launch(rmsnorm_add_layernorm_held_kernel<float, 4>, N, threads, 0, stream, y, w, eps, resid, ln_w, ln_eps, (float*)out, H);
+        return mv_launch_status();
+    }
     if (out_dtype == MV_DT_BF16)
         mv_launch(rmsnorm_add_layernorm_kernel<__nv_bfloat16>, N, threads, 0, stream, y, w, eps, resid, ln_w, ln_eps,
                   (__nv_bfloat16*)out, H);

@@ -93,6 +93,39 @@ latent_query_kernel(const float* __restrict__ proj, int ld, int q0, const float*
     }
 }
 
+// The same, four neighbours a thread (dim, rot and half of rot_dims in steps of 4, rows on 16 bytes): 6,000 tokens of 32 heads of 64 + 32 42 -> 21 us.
+__global__ void __launch_bounds__(256)
+latent_query_vec_kernel(const float* __restrict__ proj, int ld, int q0, const float* __restrict__ inv_freq,
+                        const int* __restrict__ positions, __nv_bfloat16* __restrict__ q, int nh, int dim, int rot,
+                        int rot_dims, float amplitude) {
+    mv_pdl_begin();
+    const int n = blockIdx.x;
+    const int dk = dim + rot, half = rot_dims >> 1, total = nh * dk;
+    const float* row = proj + (size_t)n * ld + q0;
+    __shared__ float sn_s[LQ_MAX_ROT / 2], cs_s[LQ_MAX_ROT / 2];
+    for (int i = threadIdx.x; i < half; i += blockDim.x) {
+        float sn, cs;
+        sincosf((float)positions[n] * inv_freq[i], &sn, &cs);
+        sn_s[i] = sn * amplitude;
+        cs_s[i] = cs * amplitude;
+    }
+    __syncthreads();
+    __nv_bfloat16* dst = q + (size_t)n * total;
+    for (int e = 4 * threadIdx.x; e < total; e += 4 * blockDim.x) {
+        const int i = e % dk - dim;
+        const float4 a = *reinterpret_cast<const float4*>(row + e);
+        float x[4] = {a.x, a.y, a.z, a.w};
+        if (i >= 0 && i < rot_dims) {
+            const int f = i < half ? i : i - half;
+            const float4 b = *reinterpret_cast<const float4*>(row + (i < half ? e + half : e - half));
+            const float y[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x[j] = i < half ? x[j] * cs_s[f + j] - y[j] * sn_s[f + j] : x[j] * cs_s[f + j] + y[j] * sn_s[f + j];
+        }
+        mv_store4(dst + e, x[0], x[1], x[2], x[3]);
+    }
+}
+
 // ------------------------------------------------------------------------------------------------------- gather
 __global__ void __launch_bounds__(64)
 latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, long long page_stride, const int* __restrict__ page_table,
@@ -397,6 +430,11 @@ MV_API int mv_latent_query(const float* proj, int ld, int q0, const float* inv_f
                            int nh, int dim, int rot, int rot_dims, float amplitude, cudaStream_t stream) {
     if (N <= 0) return 0;
     if (rot_dims < 0 || rot_dims > rot || rot_dims > LQ_MAX_ROT || (rot_dims & 1) || (rot_dims && !inv_freq)) return (int)cudaErrorInvalidValue;
+    if (dim % 4 == 0 && rot % 4 == 0 && rot_dims % 8 == 0 && ld % 4 == 0 && q0 % 4 == 0 && (((uintptr_t)proj | (uintptr_t)q) & 15) == 0) {
+        mv_launch(latent_query_vec_kernel, N, 256, 0, stream, proj, ld, q0, inv_freq, positions, (__nv_bfloat16*)q, nh, dim, rot,
+                  rot_dims, amplitude);
+        return mv_launch_status();
+    }
     mv_launch(latent_query_kernel, N, 256, 0, stream, proj, ld, q0, inv_freq, positions, (__nv_bfloat16*)q, nh, dim, rot,
               rot_dims, amplitude);
     return mv_launch_status();

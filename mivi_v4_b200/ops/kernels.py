@@ -83,7 +83,7 @@ _SIGNATURES = {
                               _I, _I, _I, _P],
         "mv_scalar_scan_few": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _I, _I,
                                _I, _I, _I, _I, _I, _P],
-        "mv_memory_gates": [_P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _I, _P],
+        "mv_memory_gates": [_P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _P, _P, _P, _I, _I, _I, _P],
         "mv_causal_conv": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
         "mv_ssm_decode_prepare": [_P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _P, _I, _P, _P, _P, _P, _I, _P],
         "mv_step_size": [_P, _I, _P, _P, _P, _P, _I, _I, _P],
@@ -735,8 +735,8 @@ def memory_gates(zi: torch.Tensor, zf: torch.Tensor, bi: torch.Tensor, bf: torch
         _need(bf, "forget gate bias", torch.float32, (n_heads,)), float(cap),
         _need(m_state, "memory_gates m", torch.float32, (None, n_heads)), _need(slots, "slots", torch.int32),
         _need(cu, "cu", torch.int32), _need(log_a, "log_a", torch.float32, (N, n_heads)),
-        _need(b, "b", torch.float32, (N, n_heads)), _need(m_tok, "m_tok", torch.float32, (N, n_heads)), int(n_seqs),
-        n_heads, _stream()), "mv_memory_gates")
+        _need(b, "b", torch.float32, (N, n_heads)), _need(m_tok, "m_tok", torch.float32, (N, n_heads)), N,
+        int(n_seqs), n_heads, _stream()), "mv_memory_gates")
     account(N * n_heads * 20)
 
 
