@@ -15,7 +15,7 @@
 // elements; a gate per element instead of per head; every head's weights applied to every kv head's values (32-bit
 // results, for weights that are mixed between the heads afterwards).  SPLIT: a softmax weight enters the value
 // product as two bfloat16 numbers, the rounded weight and the rounding's remainder (two mma a tile), which
-// carries 16 bits of its mantissa.
+// carries 16 bits of its mantissa.  Steps whose sequences bring many tokens take attention_sink_tc.cu where it serves the sizes.
 #include "common.cuh"
 
 namespace {

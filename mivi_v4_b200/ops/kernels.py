@@ -126,6 +126,8 @@ _SIGNATURES = {
         "mv_attention_prefill": [_P, _P, _Q, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P],
         "mv_attention_sink_prefill": [_P, _P, _Q, _P, _I, _I, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _F, _I,
                                       _I, _I, _P, _P, _P, _I, _I, _I, _P, _I, _P],
+        "mv_attention_sink_tc": [_P, _P, _I, _Q, _P, _I, _I, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _F, _I,
+                                 _I, _I, _P, _P, _P, _I, _I, _I, _P, _I, _P, _P],
         "mv_attention_sink_decode": [_P, _P, _Q, _P, _I, _I, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _F, _F, _I, _I, _I, _P,
                                      _P, _P],
         "mv_attention_decode_tc": [_P, _P, _Q, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P, _P],
@@ -1330,6 +1332,20 @@ def attention_sink_prefill_supported(dtype: torch.dtype, dk: int, dv: int) -> bo
             and 16 <= dv <= PREFILL_ATTENTION_MAX_HEAD_DIM)
 
 
+# The tcgen05 kernel's blocks are 128 query tokens of one sequence and two heads: it takes steps whose sequences fill most of a tile and that have enough
+# of them for the device (its bits are the other kernel's).  This kernel / the other, us, 32 heads of 64 with chunks of 1,024, of 80 / 64 with a cap and a
+# window of 1,024, and of 64 with a cap and a table by distance and split weights: one prompt of 512 tokens 16 / 21, 24 / 25, 35 / 29; four of 300
+# 20 / 25, 27 / 28, 40 / 34; 16 of 96 20 / 25, 24 / 29, 32 / 33; 32 of 64 32 / 28, 36 / 30, 44 / 32; 32 of 128 44 / 50, 53 / 55, 67 / 64; behind 1,000
+# earlier tokens 8 times 128 38 / 60, 48 / 103, 63 / 118.
+SINK_TC_TOKENS, SINK_TC_ALL = 96, 1280
+
+
+def sink_tc_takes(N: int, n_seqs: int, nh: int, nkv: int, dk: int, dv: int, page_size: int) -> bool:
+    """Whether the tcgen05 kernel takes a step of ``N`` tokens of ``n_seqs`` sequences."""
+    return (N >= max(SINK_TC_TOKENS * n_seqs, SINK_TC_ALL) and nh % (2 * nkv) == 0 and dk <= 128 and dv <= 64 and page_size % 64 == 0
+            and (N + 127) // 128 + n_seqs <= 65535)
+
+
 def attention_sink_prefill(q: torch.Tensor, pool: torch.Tensor, page_size: int, page_table, cu, starts,
                            out: torch.Tensor, n_seqs: int, nh: int, nkv: int, dk: int, dv: int, scale: float, *,
                            softcap: float = 0.0, window: int = 0, keep_first: int = 0,
@@ -1354,17 +1370,22 @@ def attention_sink_prefill(q: torch.Tensor, pool: torch.Tensor, page_size: int, 
     gp, ldg = _cols(gate, "attention gate", N, nh * dv if gate_wide else nh) if gate is not None else (None, 0)
     r1, r2 = _bias_pair(distance_bias, nh, values_in_keys, dk, dv)
     dist, dist_len = _distance_table(distance_table, distance_bias, nh)
-    _guard("bf16", "attention_sink_prefill", q.device, n_pages=pool.shape[0])
-    _check(_fn("bf16", "mv_attention_sink_prefill")(
-        _need(q, "q", None, (N, nh * dk)), _need(pool, "cache pool"), pool.stride(0),
-        _need(page_table, "page table", torch.int32), page_table.shape[1], page_size,
-        _need(cu, "cu", torch.int32), _need(starts, "starts", torch.int32),
-        _need(sinks, "sinks", torch.float32, (nh,), True), gp, ldg,
-        _need(out, "attention out", None, (N, nh * dv), out_all is not None),
-        N, n_seqs, nh, nkv, dk, dv, float(scale), float(softcap), int(window), int(keep_first), int(chunk), r1, r2,
-        dist, dist_len, int(bool(values_in_keys)), int(bool(gate_wide)),
-        _need(out_all, "attention out of all kv heads", torch.float32, (N, nh, nkv, dv), True), int(bool(split_weights)),
-        _stream()), "mv_attention_sink_prefill")
+    shape = (_need(page_table, "page table", torch.int32), page_table.shape[1], page_size,
+             _need(cu, "cu", torch.int32), _need(starts, "starts", torch.int32),
+             _need(sinks, "sinks", torch.float32, (nh,), True), gp, ldg,
+             _need(out, "attention out", None, (N, nh * dv), out_all is not None),
+             N, n_seqs, nh, nkv, dk, dv, float(scale), float(softcap), int(window), int(keep_first), int(chunk), r1, r2,
+             dist, dist_len, int(bool(values_in_keys)), int(bool(gate_wide)),
+             _need(out_all, "attention out of all kv heads", torch.float32, (N, nh, nkv, dv), True), int(bool(split_weights)))
+    qp, pp = _need(q, "q", None, (N, nh * dk)), _need(pool, "cache pool")
+    if sink_tc_takes(N, n_seqs, nh, nkv, dk, dv, page_size) and pool.stride(0) % 8 == 0 and not any(
+            t is not None and t.data_ptr() % 16 for t in (q, pool, out, out_all)):
+        _guard("bf16", "attention_sink_tc", q.device, n_pages=pool.shape[0])
+        _check(_fn("bf16", "mv_attention_sink_tc")(qp, pp, pool.shape[0], pool.stride(0), *shape, _error_flag(q.device).data_ptr(), _stream()),
+               "mv_attention_sink_tc")
+    else:
+        _guard("bf16", "attention_sink_prefill", q.device, n_pages=pool.shape[0])
+        _check(_fn("bf16", "mv_attention_sink_prefill")(qp, pp, pool.stride(0), *shape, _stream()), "mv_attention_sink_prefill")
     return out if out_all is None else out_all
 
 
