@@ -61,6 +61,7 @@ __device__ __forceinline__ void tma_load_3d(unsigned dst, const CUtensorMap* map
         ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_st16(unsigned taddr, const unsigned (&r)[16]) {
+    __syncwarp();
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
         "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
@@ -69,6 +70,7 @@ __device__ __forceinline__ void tmem_st16(unsigned taddr, const unsigned (&r)[16
         : "memory");
 }
 __device__ __forceinline__ void tmem_st32(unsigned taddr, const unsigned (&r)[32]) {
+    __syncwarp();
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
         "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
@@ -378,7 +380,6 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             const float c = m == -INFINITY ? 0.f : ex2(__fsub_rn(m, ref));
             m = mn;
             float sum[4] = {0.f, 0.f, 0.f, 0.f};
-            __syncwarp();                                                // (16 rows of a warp may take another way than the others above)
             chunk_weights<SPLIT>(s0, ref, s_addr, sum);
             chunk_weights<SPLIT>(s1, ref, s_addr + 16, sum);
 #pragma unroll
@@ -462,6 +463,7 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) {
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
 }

@@ -65,6 +65,7 @@ __device__ __forceinline__ void split2(float a, float b, unsigned& h, unsigned& 
     l = bits(__floats2bfloat162_rn(y.x, y.y));
 }
 __device__ __forceinline__ void tmem_st8(unsigned taddr, const unsigned (&r)[8]) {
+    __syncwarp();
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
@@ -280,6 +281,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         }
     }
     if (warp == 1) {
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
 }

@@ -429,6 +429,7 @@ gemm_tc_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     if (slices > 1) mv_cluster_sync_relaxed();
     else __syncthreads();
     if (warp == 1) {
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                      "r"((unsigned)L::TMEM_COLS) : "memory");
     }

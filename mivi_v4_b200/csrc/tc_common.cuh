@@ -121,7 +121,10 @@ __device__ __forceinline__ void mma_f16_ts(unsigned tmem_d, unsigned tmem_a, uns
 __device__ __forceinline__ void mma_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// Loads and stores of tensor memory are for a whole warp at once, and so is giving it back: each is preceded by a __syncwarp, whatever
+// branches by row the lanes have come from.
 __device__ __forceinline__ void tmem_ld32(unsigned taddr, unsigned (&r)[32]) {
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "

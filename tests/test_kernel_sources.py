@@ -25,3 +25,15 @@ def test_shared_memory_is_allowed_on_every_device():
     (float32 models ran on any device of a process before their kernels needed the permission.)"""
     once = [name for name, text in sources() if re.search(r"static\s+(const\s+)?cudaError_t[^;]*cudaFuncSetAttribute", text)]
     assert not once, once
+
+
+def test_tensor_memory_is_accessed_by_whole_warps():
+    """Loads, stores and the return of tensor memory are .sync.aligned: lanes that come from a branch by row (a row's sink, a row beyond the last) have to
+    be together again, which only a __syncwarp right before the instruction assures."""
+    found, seen = [], 0
+    for name, text in sources():
+        for m in re.finditer(r'asm volatile\(\s*"(tcgen05\.(?:ld|st|dealloc)[^"]*)"', text):
+            seen += 1
+            if not text[:m.start()].rstrip().endswith("__syncwarp();"):
+                found.append(f"{name}: {m.group(1)[:60]}")
+    assert not found and seen > 10, found
