@@ -46,8 +46,6 @@ enum { B_RAWFULL = 0, B_RAWEMPTY = B_RAWFULL + RAW, B_PLFULL = B_RAWEMPTY + RAW,
        B_ACCEMPTY = B_ACCFULL + 2, B_COUNT = B_ACCEMPTY + 2 };
 static_assert(B_COUNT * 8 + 8 <= 256, "barrier area");
 
-__device__ __forceinline__ unsigned bits(__nv_bfloat162 v) { return *reinterpret_cast<const unsigned*>(&v); }
-
 // a packed pair's bfloat16 numbers as floats, and what they leave of (a, b)
 __device__ __forceinline__ float2 rest(float2 x, unsigned h) {
     float2 y = make_float2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), minus = make_float2(-1.f, -1.f);
@@ -63,11 +61,6 @@ __device__ __forceinline__ void split2(float a, float b, unsigned& h, unsigned& 
     m = bits(__floats2bfloat162_rn(x.x, x.y));
     const float2 y = rest(x, m);
     l = bits(__floats2bfloat162_rn(y.x, y.y));
-}
-__device__ __forceinline__ void tmem_st8(unsigned taddr, const unsigned (&r)[8]) {
-    __syncwarp();
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
 __device__ __noinline__ float plain_product(const float* x, const float* w, int K) {

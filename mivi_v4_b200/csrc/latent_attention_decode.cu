@@ -39,7 +39,6 @@ __device__ __forceinline__ void ldmatrix_x4_trans(unsigned (&r)[4], const void* 
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(s) : "memory");
 }
-__device__ __forceinline__ unsigned bits(const __nv_bfloat162& v) { return *reinterpret_cast<const unsigned*>(&v); }
 
 // row pitch of the tiles in elements: whole steps of 16, and 16 bytes more so that ldmatrix meets no bank twice
 __host__ __device__ __forceinline__ int row_pitch(int w) { return (w + 15) / 16 * 16 + 8; }
