@@ -12,13 +12,15 @@
 //   warps 4-7    add the finished 128 of K of h h (two accumulators take turns) to their registers, TN columns of a row a thread;
 //   warps 8-15   split X, a row a thread, out of a stage of the ring into tensor memory, from where the products read it;
 //   warps 16-23  split W, a row a thread, into shared memory, in the layout that the products read.
-// At the end the tile goes through shared memory, and all warps store it by rows.  A result that is not finite, or below 2^-80, is worked out again
-// by float32 multiply-adds: infinities and numbers that bfloat16 rounds to infinity split into NaNs, and what is left of numbers below
-// 2^-110 after their first eight bits falls out of bfloat16's range.
+// At the end the tile goes through shared memory, and all warps store it by rows.  Where the parts do not hold the operands, results are worked out again
+// by float32 multiply-adds.  Infinities and numbers that bfloat16 rounds to infinity split into NaNs: results that are not finite.  What is
+// left of a number below 2^-110 after its first eight bits falls out of bfloat16's range, so up to 2^-134 of every operand is lost, times the other one: results
+// whose row of X or of W has a number above 2^32 (the warps that split keep the largest), and results below 2^-60 unless X's or W's row is all
+// zeros.  For the others that is at most K 2^-134 2^33, less than 2^-24 of the result up to K = 65,536.
 //
 // Bound by the splitting (some 560 instructions of every scheduler a stage, and waits: 0.58 us for 128 x 96, 0.8 for 128 x 128), then by shared memory (a stage of
 // 128 columns writes and reads 32 KB of float32 tiles, writes 24 KB and has the products read 48 KB of W's planes: 1,060 clocks beside the products'
-// 780).  1,165 rows against 9,216 x 1,024 516 -> 133 us (165 TFLOP/s), against 1,024 x 4,608 280 -> 84; error against 64 bits 1.3e-7 where the
+// 780).  1,165 rows against 9,216 x 1,024 516 -> 133 us (165 TFLOP/s), against 1,024 x 4,608 280 -> 88; error against 64 bits 1.3e-7 where the
 // multiply-adds have 4.1e-7 (K = 1,024), 1.8e-7 where they have 8.6e-7 (K = 4,608).  With X's planes in shared memory too, which the products then read at all
 // its bandwidth, 174 us; with the two groups of splitting warps on the same stage 145.
 #include "tc_common.cuh"
@@ -35,11 +37,12 @@ template <int TN> struct F3Layout {
     // tensor memory: two accumulators of h h, one of the others, and X's planes in two stages or four
     static constexpr unsigned LOW_COL = 2 * TN, X_COL = 3 * TN;
     static constexpr int PLANES = 512 - 3 * TN >= 4 * 3 * (int)X_PLANE ? 4 : 2;
-    static constexpr int PLANES_AT = RAW * RAW_STAGE, BARS_AT = PLANES_AT + PLANES * PLANE_STAGE, TOTAL = BARS_AT + 256 + 1024;
+    static constexpr int PLANES_AT = RAW * RAW_STAGE, BARS_AT = PLANES_AT + PLANES * PLANE_STAGE, LARGEST_AT = BARS_AT + 256;
+    static constexpr int TOTAL = LARGEST_AT + 2 * (TM + TN) * 4 + 1024;
     static constexpr int OUT_LD = TN + 4;                            // the tile at the end: 16-byte words of 8 rows in 8 bank groups
     static_assert(TN % 16 == 0 && TN <= 128 && TM * OUT_LD * 4 <= BARS_AT, "the tile fits the rings");
 };
-constexpr float TINY = 8.271806125530277e-25f;                                 // 2^-80
+constexpr float TINY = 8.673617379884035e-19f, LARGE = 4294967296.0f;         // 2^-60, 2^32
 
 constexpr int MAX_PLANES = 4;
 enum { B_RAWFULL = 0, B_RAWEMPTY = B_RAWFULL + RAW, B_PLFULL = B_RAWEMPTY + RAW, B_PLEMPTY = B_PLFULL + MAX_PLANES, B_ACCFULL = B_PLEMPTY + MAX_PLANES,
@@ -63,34 +66,69 @@ __device__ __forceinline__ void split2(float a, float b, unsigned& h, unsigned& 
     l = bits(__floats2bfloat162_rn(y.x, y.y));
 }
 
-__device__ __noinline__ float plain_product(const float* x, const float* w, int K) {
-    float s = 0.f;
-    for (int k = 0; k < K; ++k) s = fmaf(x[k], w[k], s);
-    return s;
+struct F3Args {
+    const float *X, *W, *bias;
+    void* out;
+    int mode, M, N, K, ldo;
+    __device__ __forceinline__ void put(size_t o, int n, float v) const {
+        if (bias) v += bias[n];
+        if (mode == 1) ((__nv_bfloat16*)out)[o] = __float2bfloat16_rn(v);
+        else ((float*)out)[o] = mode == 2 ? ((float*)out)[o] + v : v;
+    }
+};
+// whether any of four results may have to be worked out again
+__device__ __forceinline__ bool doubtful(float4 v) {
+    const float a = fabsf(v.x), b = fabsf(v.y), c = fabsf(v.z), d = fabsf(v.w);
+    return fminf(fminf(a, b), fminf(c, d)) < TINY || !(a + b + c + d < INFINITY);
+}
+// A thread's doubtful results: which of them the parts do not give, and these by multiply-adds, K in its order.
+template <int TN>
+__device__ __noinline__ void finish_doubtful(const F3Args& g, const float* tile, const float* largest, bool all, int m0, int n0) {
+    const int lane = threadIdx.x & 31, n = n0 + 4 * lane;
+    for (int r = threadIdx.x >> 5; r < TM && m0 + r < g.M; r += F3_THREADS / 32) {
+        const float* at = tile + r * F3Layout<TN>::OUT_LD + 4 * lane;
+        if (!all && !doubtful(*reinterpret_cast<const float4*>(at))) continue;
+        const float x_top = fmaxf(largest[r], largest[TM + r]);
+        for (int e = 0; e < 4 && n + e < g.N; ++e) {
+            const float w_top = fmaxf(largest[2 * TM + 4 * lane + e], largest[2 * TM + TN + 4 * lane + e]);
+            float v = at[e];
+            if (!(fabsf(v) < INFINITY) || x_top > LARGE || w_top > LARGE || (fabsf(v) < TINY && x_top > 0.f && w_top > 0.f)) {
+                const float *x = g.X + (size_t)(m0 + r) * g.K, *w = g.W + (size_t)(n + e) * g.K;
+                v = 0.f;
+                for (int k = 0; k < g.K; k += 4) {
+                    const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
+                    v = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, v))));
+                }
+            }
+            g.put((size_t)(m0 + r) * g.ldo + n + e, n + e, v);
+        }
+    }
 }
 
 template <int TN>
 __global__ void __launch_bounds__(F3_THREADS, 1)
-gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const float* __restrict__ X,
-                   const float* __restrict__ W, const float* __restrict__ bias, void* __restrict__ out, int mode, int M, int N, int K,
-                   int ldo, int* __restrict__ err) {
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ F3Args g,
+                   int* __restrict__ err) {
     using L = F3Layout<TN>;
     constexpr int PLANES = L::PLANES;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned long long* bars = (unsigned long long*)(smem + L::BARS_AT);
     unsigned* tmem_holder = (unsigned*)(bars + B_COUNT);
+    float* largest = reinterpret_cast<float*>(smem + L::LARGEST_AT);     // [2][TM] of X's rows, [2][TN] of W's: the largest magnitude in either group's stages
+    volatile int* too_large = reinterpret_cast<int*>(tmem_holder + 1);    // one of them is above LARGE
     const unsigned base = smem_u32(smem), bar0 = smem_u32(bars);
     auto bar = [&](int i) { return bar0 + 8u * (unsigned)i; };
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    const int nkb = (K + KB - 1) / KB, chunks = (nkb + CHUNK - 1) / CHUNK;
+    const int nkb = (g.K + KB - 1) / KB, chunks = (nkb + CHUNK - 1) / CHUNK;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < B_COUNT; ++i) {
             const bool split = (i >= B_RAWEMPTY && i < B_RAWEMPTY + RAW) || (i >= B_PLFULL && i < B_PLFULL + MAX_PLANES);
             mbar_init(bar(i), split ? 8 : i >= B_ACCEMPTY ? 4 : 1);
         }
+        *too_large = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -106,7 +144,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     bool ok = true;
 
     if (warp < 4) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
         if (warp == 0) {
             for (int kb = 0; kb < nkb; ++kb) {
                 const int s = kb % RAW;
@@ -186,6 +224,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         const bool is_x = warp < 16;
         const int r = (warp & 3) * 32 + lane, group = (warp >> 2) & 1;     // this thread's row of the tile of X or W
         const bool live = is_x || r < TN;
+        float top = 0.f;
         const unsigned at0 = tmem_base + ((unsigned)((warp & 3) * 32) << 16) + L::X_COL;
         for (int kb = group; kb < nkb; kb += 2) {
             const int s = kb % RAW, d = kb % PLANES;
@@ -202,6 +241,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll
                     for (int w = 0; w < 4; ++w) {
                         const float4 a = *reinterpret_cast<const float4*>(src + (((4 * half + w) ^ (r & 7)) << 4));
+                        top = fmaxf(top, fmaxf(fabsf(a.x), fabsf(a.y)));
+                        top = fmaxf(top, fmaxf(fabsf(a.z), fabsf(a.w)));
                         split2(a.x, a.y, h[2 * w], m[2 * w], l[2 * w]);
                         split2(a.z, a.w, h[2 * w + 1], m[2 * w + 1], l[2 * w + 1]);
                     }
@@ -238,28 +279,32 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 mbar_arrive(bar(B_RAWEMPTY + s));
             }
         }
+        if (live) largest[is_x ? group * TM + r : 2 * TM + group * TN + r] = top;
+        if (top > LARGE) *too_large = 1;
     }
     mv_pdl_launch_dependents();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     // a row's TN columns by a warp, four neighbours a lane
-    const int n = 4 * lane < TN ? n0 + 4 * lane : N;
-    const bool vec = n + 3 < N && (ldo & 3) == 0 && ((uintptr_t)out & 15) == 0 && mode != 1;
-    for (int r = warp; r < TM && m0 + r < M; r += F3_THREADS / 32) {
-        if (n >= N) continue;
+    const int n = 4 * lane < TN ? n0 + 4 * lane : g.N;
+    const bool vec = n + 3 < g.N && (g.ldo & 3) == 0 && ((uintptr_t)g.out & 15) == 0 && g.mode != 1, all = *too_large != 0;
+    bool left = all;
+    for (int r = warp; r < TM && m0 + r < g.M && !all; r += F3_THREADS / 32) {
+        if (n >= g.N) continue;
         const float4 got = *reinterpret_cast<const float4*>(tile + r * L::OUT_LD + 4 * lane);
-        float v[4] = {got.x, got.y, got.z, got.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float a = fabsf(v[e]);
-            if (n + e < N && (!(a < INFINITY) || (a < TINY && a > 0.f)))
-                v[e] = plain_product(X + (size_t)(m0 + r) * K, W + (size_t)(n + e) * K, K);
-            if (bias && n + e < N) v[e] += bias[n + e];
+        if (doubtful(got)) {
+            left = true;
+            continue;
         }
-        const size_t o = (size_t)(m0 + r) * ldo + n;
+        float v[4] = {got.x, got.y, got.z, got.w};
+        const size_t o = (size_t)(m0 + r) * g.ldo + n;
         if (vec) {
-            float4* p = reinterpret_cast<float4*>((float*)out + o);
-            if (mode == 2) {
+            if (g.bias) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] += g.bias[n + e];
+            }
+            float4* p = reinterpret_cast<float4*>((float*)g.out + o);
+            if (g.mode == 2) {
                 const float4 old = *p;
                 v[0] += old.x; v[1] += old.y; v[2] += old.z; v[3] += old.w;
             }
@@ -267,12 +312,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         } else {
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-                if (n + e < N) {
-                    if (mode == 1) ((__nv_bfloat16*)out)[o + e] = __float2bfloat16_rn(v[e]);
-                    else ((float*)out)[o + e] = mode == 2 ? ((float*)out)[o + e] + v[e] : v[e];
-                }
+                if (n + e < g.N) g.put(o + e, n + e, v[e]);
         }
     }
+    if (left && n < g.N) finish_doubtful<TN>(g, tile, largest, all, m0, n0);
     if (warp == 1) {
         __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
@@ -286,7 +329,7 @@ int launch(const float* X, const float* W, const float* bias, void* out, int mod
     const cudaError_t attr = mv_allow_smem<gemm_f32_tc_kernel<TN>>(F3Layout<TN>::TOTAL);
     if (attr != cudaSuccess) return (int)attr;
     gemm_f32_tc_kernel<TN><<<dim3((N + TN - 1) / TN, (M + TM - 1) / TM), F3_THREADS, F3Layout<TN>::TOTAL, stream>>>(
-        mx, mw, X, W, bias, out, mode, M, N, K, ldo, err);
+        mx, mw, F3Args{X, W, bias, out, mode, M, N, K, ldo}, err);
     return mv_launch_status();
 }
 
@@ -299,11 +342,11 @@ int tile_width(int M, int N, int sms) {
 
 }  // namespace
 
-// float32 X, W and sums; modes and bias as mv_gemm_simt's.  K a multiple of 4, X and W on 16 bytes, rows without gaps; `sms`: the device's multiprocessors.
+// float32 X, W and sums; modes and bias as mv_gemm_simt's.  K a multiple of 4 up to 65,536, X and W on 16 bytes, rows without gaps; `sms`: the device's multiprocessors.
 MV_API int mv_gemm_f32_tc(const float* X, const float* W, const float* bias, void* out, int mode, int M, int N, int K, int ldo, int sms, int* err,
                           cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (K < 4 || K % 4 || mode < 0 || mode > 2 || (((uintptr_t)X | (uintptr_t)W) & 15) || (M + TM - 1) / TM > 65535 || sms < 1) return (int)cudaErrorInvalidValue;
+    if (K < 4 || K % 4 || K > 65536 || mode < 0 || mode > 2 || (((uintptr_t)X | (uintptr_t)W) & 15) || (M + TM - 1) / TM > 65535 || sms < 1) return (int)cudaErrorInvalidValue;
     return tile_width(M, N, sms) == 128 ? launch<128>(X, W, bias, out, mode, M, N, K, ldo, err, stream)
                                         : launch<96>(X, W, bias, out, mode, M, N, K, ldo, err, stream);
 }

@@ -16,6 +16,7 @@ def test_which_products_go_there():
     takes = K().gemm_f32_tc_takes
     assert takes(1165, 1024, 4608, 148) and takes(16, 9216, 1024, 148) and not takes(8, 9216, 1024, 148)
     assert not takes(128, 1024, 4608, 148) and not takes(1165, 1024, 1020, 148) and not takes(1165, 1024, 1026, 148)
+    assert takes(1165, 1024, 65536, 148) and not takes(1165, 1024, 65540, 148)
 
 
 @pytest.fixture
@@ -63,6 +64,28 @@ def test_no_less_exact_than_multiply_adds(Kd, monkeypatch):
         K().gemm_simt(x, w, out)
         off.append(float((out - want).norm() / want.norm()))
     assert off[0] <= off[1], off
+
+
+@gpu
+@pytest.mark.parametrize("e", [100, 112, 118, 122, 126, 134, 137, 145])
+@pytest.mark.parametrize("small", ["x", "w"])
+@pytest.mark.parametrize("large", [0, 20, 31, 33, 120])
+def test_operands_far_apart(e, small, large, everything):
+    """Numbers whose lower parts, or all of them, fall out of bfloat16's range, against ordinary and against large ones."""
+    Kd = 1024
+    g = torch.Generator(device=DEV).manual_seed(e)
+    a, b = torch.randn(140, Kd, generator=g, device=DEV), torch.randn(130, Kd, generator=g, device=DEV)
+    a, b = (a.double() * 2.0 ** -e).float(), b * 2.0 ** large
+    b[7] = torch.randn(Kd, generator=g, device=DEV)
+    a[5, ::2], a[6] = 0.0, 0.0
+    x, w = (a, b) if small == "x" else (b, a)
+    got, want = torch.empty(x.shape[0], w.shape[0], device=DEV), x.double() @ w.double().T
+    K().gemm_simt(x, w, got)
+    # K roundings of half a unit in the last place of what there is so far, of any sign; float32's steps below its smallest exponent
+    row = (x.double() ** 2).sum(1)[:, None].sqrt() * (w.double() ** 2).sum(1)[None].sqrt()
+    bound = 4 * 2.0 ** -24 * row + Kd * 2.0 ** -150
+    assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() / bound).max())
+    K().check_device_errors()
 
 
 @gpu
