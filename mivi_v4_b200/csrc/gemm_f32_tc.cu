@@ -1,7 +1,7 @@
 // Y[M, N] = X[M, K] . W[N, K]^T of float32 operands on the tensor cores, with an error against 64 bits no larger than that of float32
 // multiply-adds (gemm_simt.cu), for products of many rows.
 //
-// Every operand is split into three bfloat16 numbers, x = h + m + l (each what rounding left of the one before; together its 24 bits), and
+// Every operand is split into three bfloat16 numbers, 2^39 x = h + m + l (each what rounding left of the one before; together its 24 bits), and
 // six of the nine products are added up: h h, then h m + m h, m m, h l + l h; what is left out is below 2^-25 of |x w|.  The tensor cores cut the
 // sums that they add to off, so a long chain of them loses places (K = 1,024 in one chain: 1e-6): h h is added over 128 of K in tensor memory and then in
 // float32 registers; the five others, 2^-8 of it, have an accumulator of their own over all of K.
@@ -12,15 +12,14 @@
 //   warps 4-7    add the finished 128 of K of h h (two accumulators take turns) to their registers, TN columns of a row a thread;
 //   warps 8-15   split X, a row a thread, out of a stage of the ring into tensor memory, from where the products read it;
 //   warps 16-23  split W, a row a thread, into shared memory, in the layout that the products read.
-// At the end the tile goes through shared memory, and all warps store it by rows.  Where the parts do not hold the operands, results are worked out again
-// by float32 multiply-adds.  Infinities and numbers that bfloat16 rounds to infinity split into NaNs: results that are not finite.  What is
-// left of a number below 2^-110 after its first eight bits falls out of bfloat16's range, so up to 2^-134 of every operand is lost, times the other one: results
-// whose row of X or of W has a number above 2^32 (the warps that split keep the largest), and results below 2^-60 unless X's or W's row is all
-// zeros.  For the others that is at most K 2^-134 2^33, less than 2^-24 of the result up to K = 65,536.
+// At the end the tile goes through shared memory, is multiplied by 2^-78, and all warps store it by rows.  The scale keeps all parts of all float32 numbers in bfloat16's range, down
+// to the smallest subnormal one (without it what is left of a number below 2^-110 after its first eight bits falls out, which shows beside large numbers in the other operand).  Infinities,
+// NaNs, operands from 2^88 on and sums from 2^50 on end as results that are not finite: these, and no others, are worked out again by float32
+// multiply-adds, in a function of its own that leaves the others' way its registers.
 //
 // Bound by the splitting (some 560 instructions of every scheduler a stage, and waits: 0.58 us for 128 x 96, 0.8 for 128 x 128), then by shared memory (a stage of
 // 128 columns writes and reads 32 KB of float32 tiles, writes 24 KB and has the products read 48 KB of W's planes: 1,060 clocks beside the products'
-// 780).  1,165 rows against 9,216 x 1,024 516 -> 133 us (165 TFLOP/s), against 1,024 x 4,608 280 -> 88; error against 64 bits 1.3e-7 where the
+// 780).  1,165 rows against 9,216 x 1,024 516 -> 133 us (165 TFLOP/s), against 1,024 x 4,608 280 -> 85; error against 64 bits 1.3e-7 where the
 // multiply-adds have 4.1e-7 (K = 1,024), 1.8e-7 where they have 8.6e-7 (K = 4,608).  With X's planes in shared memory too, which the products then read at all
 // its bandwidth, 174 us; with the two groups of splitting warps on the same stage 145.
 #include "tc_common.cuh"
@@ -37,12 +36,11 @@ template <int TN> struct F3Layout {
     // tensor memory: two accumulators of h h, one of the others, and X's planes in two stages or four
     static constexpr unsigned LOW_COL = 2 * TN, X_COL = 3 * TN;
     static constexpr int PLANES = 512 - 3 * TN >= 4 * 3 * (int)X_PLANE ? 4 : 2;
-    static constexpr int PLANES_AT = RAW * RAW_STAGE, BARS_AT = PLANES_AT + PLANES * PLANE_STAGE, LARGEST_AT = BARS_AT + 256;
-    static constexpr int TOTAL = LARGEST_AT + 2 * (TM + TN) * 4 + 1024;
+    static constexpr int PLANES_AT = RAW * RAW_STAGE, BARS_AT = PLANES_AT + PLANES * PLANE_STAGE, TOTAL = BARS_AT + 256 + 1024;
     static constexpr int OUT_LD = TN + 4;                            // the tile at the end: 16-byte words of 8 rows in 8 bank groups
     static_assert(TN % 16 == 0 && TN <= 128 && TM * OUT_LD * 4 <= BARS_AT, "the tile fits the rings");
 };
-constexpr float TINY = 8.673617379884035e-19f, LARGE = 4294967296.0f;         // 2^-60, 2^32
+constexpr float SCALE = 549755813888.0f, UNSCALE = 3.3087224502121107e-24f;      // 2^39, 2^-78
 
 constexpr int MAX_PLANES = 4;
 enum { B_RAWFULL = 0, B_RAWEMPTY = B_RAWFULL + RAW, B_PLFULL = B_RAWEMPTY + RAW, B_PLEMPTY = B_PLFULL + MAX_PLANES, B_ACCFULL = B_PLEMPTY + MAX_PLANES,
@@ -57,13 +55,14 @@ __device__ __forceinline__ float2 rest(float2 x, unsigned h) {
         "l"(*reinterpret_cast<unsigned long long*>(&x)));
     return *reinterpret_cast<float2*>(&r);
 }
-// two floats -> their three bfloat16 numbers, packed by plane
-__device__ __forceinline__ void split2(float a, float b, unsigned& h, unsigned& m, unsigned& l) {
-    h = bits(__floats2bfloat162_rn(a, b));
-    const float2 x = rest(make_float2(a, b), h);
-    m = bits(__floats2bfloat162_rn(x.x, x.y));
-    const float2 y = rest(x, m);
-    l = bits(__floats2bfloat162_rn(y.x, y.y));
+// two floats times SCALE -> their three bfloat16 numbers, packed by plane
+__device__ __forceinline__ void split2(float2 a, unsigned& h, unsigned& m, unsigned& l) {
+    const float2 x = mul2(a, make_float2(SCALE, SCALE));
+    h = bits(__floats2bfloat162_rn(x.x, x.y));
+    const float2 y = rest(x, h);
+    m = bits(__floats2bfloat162_rn(y.x, y.y));
+    const float2 z = rest(y, m);
+    l = bits(__floats2bfloat162_rn(z.x, z.y));
 }
 
 struct F3Args {
@@ -76,23 +75,17 @@ struct F3Args {
         else ((float*)out)[o] = mode == 2 ? ((float*)out)[o] + v : v;
     }
 };
-// whether any of four results may have to be worked out again
-__device__ __forceinline__ bool doubtful(float4 v) {
-    const float a = fabsf(v.x), b = fabsf(v.y), c = fabsf(v.z), d = fabsf(v.w);
-    return fminf(fminf(a, b), fminf(c, d)) < TINY || !(a + b + c + d < INFINITY);
-}
-// A thread's doubtful results: which of them the parts do not give, and these by multiply-adds, K in its order.
+__device__ __forceinline__ bool finite4(float4 v) { return fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) < INFINITY; }
+// A thread's results that are not finite, by multiply-adds, K in its order.
 template <int TN>
-__device__ __noinline__ void finish_doubtful(const F3Args& g, const float* tile, const float* largest, bool all, int m0, int n0) {
+__device__ __noinline__ void multiply_again(const F3Args& g, const float* tile, int m0, int n0) {
     const int lane = threadIdx.x & 31, n = n0 + 4 * lane;
     for (int r = threadIdx.x >> 5; r < TM && m0 + r < g.M; r += F3_THREADS / 32) {
         const float* at = tile + r * F3Layout<TN>::OUT_LD + 4 * lane;
-        if (!all && !doubtful(*reinterpret_cast<const float4*>(at))) continue;
-        const float x_top = fmaxf(largest[r], largest[TM + r]);
+        if (finite4(*reinterpret_cast<const float4*>(at))) continue;
         for (int e = 0; e < 4 && n + e < g.N; ++e) {
-            const float w_top = fmaxf(largest[2 * TM + 4 * lane + e], largest[2 * TM + TN + 4 * lane + e]);
             float v = at[e];
-            if (!(fabsf(v) < INFINITY) || x_top > LARGE || w_top > LARGE || (fabsf(v) < TINY && x_top > 0.f && w_top > 0.f)) {
+            if (!(fabsf(v) < INFINITY)) {
                 const float *x = g.X + (size_t)(m0 + r) * g.K, *w = g.W + (size_t)(n + e) * g.K;
                 v = 0.f;
                 for (int k = 0; k < g.K; k += 4) {
@@ -115,8 +108,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned long long* bars = (unsigned long long*)(smem + L::BARS_AT);
     unsigned* tmem_holder = (unsigned*)(bars + B_COUNT);
-    float* largest = reinterpret_cast<float*>(smem + L::LARGEST_AT);     // [2][TM] of X's rows, [2][TN] of W's: the largest magnitude in either group's stages
-    volatile int* too_large = reinterpret_cast<int*>(tmem_holder + 1);    // one of them is above LARGE
     const unsigned base = smem_u32(smem), bar0 = smem_u32(bars);
     auto bar = [&](int i) { return bar0 + 8u * (unsigned)i; };
     const int warp = warp_index(), lane = threadIdx.x & 31;
@@ -128,7 +119,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             const bool split = (i >= B_RAWEMPTY && i < B_RAWEMPTY + RAW) || (i >= B_PLFULL && i < B_PLFULL + MAX_PLANES);
             mbar_init(bar(i), split ? 8 : i >= B_ACCEMPTY ? 4 : 1);
         }
-        *too_large = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -215,7 +205,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             add(L::LOW_COL);
 #pragma unroll
             for (int j = 0; j < TN; j += 4)
-                *reinterpret_cast<float4*>(tile + r * L::OUT_LD + j) = make_float4(sum[j], sum[j + 1], sum[j + 2], sum[j + 3]);
+                *reinterpret_cast<float4*>(tile + r * L::OUT_LD + j) = make_float4(sum[j] * UNSCALE, sum[j + 1] * UNSCALE, sum[j + 2] * UNSCALE, sum[j + 3] * UNSCALE);
         }
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
@@ -224,7 +214,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         const bool is_x = warp < 16;
         const int r = (warp & 3) * 32 + lane, group = (warp >> 2) & 1;     // this thread's row of the tile of X or W
         const bool live = is_x || r < TN;
-        float top = 0.f;
         const unsigned at0 = tmem_base + ((unsigned)((warp & 3) * 32) << 16) + L::X_COL;
         for (int kb = group; kb < nkb; kb += 2) {
             const int s = kb % RAW, d = kb % PLANES;
@@ -241,10 +230,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll
                     for (int w = 0; w < 4; ++w) {
                         const float4 a = *reinterpret_cast<const float4*>(src + (((4 * half + w) ^ (r & 7)) << 4));
-                        top = fmaxf(top, fmaxf(fabsf(a.x), fabsf(a.y)));
-                        top = fmaxf(top, fmaxf(fabsf(a.z), fabsf(a.w)));
-                        split2(a.x, a.y, h[2 * w], m[2 * w], l[2 * w]);
-                        split2(a.z, a.w, h[2 * w + 1], m[2 * w + 1], l[2 * w + 1]);
+                        split2(make_float2(a.x, a.y), h[2 * w], m[2 * w], l[2 * w]);
+                        split2(make_float2(a.z, a.w), h[2 * w + 1], m[2 * w + 1], l[2 * w + 1]);
                     }
                 }
                 if (half == 0) {
@@ -279,20 +266,18 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 mbar_arrive(bar(B_RAWEMPTY + s));
             }
         }
-        if (live) largest[is_x ? group * TM + r : 2 * TM + group * TN + r] = top;
-        if (top > LARGE) *too_large = 1;
     }
     mv_pdl_launch_dependents();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     // a row's TN columns by a warp, four neighbours a lane
     const int n = 4 * lane < TN ? n0 + 4 * lane : g.N;
-    const bool vec = n + 3 < g.N && (g.ldo & 3) == 0 && ((uintptr_t)g.out & 15) == 0 && g.mode != 1, all = *too_large != 0;
-    bool left = all;
-    for (int r = warp; r < TM && m0 + r < g.M && !all; r += F3_THREADS / 32) {
+    const bool vec = n + 3 < g.N && (g.ldo & 3) == 0 && ((uintptr_t)g.out & 15) == 0 && g.mode != 1;
+    bool left = false;
+    for (int r = warp; r < TM && m0 + r < g.M; r += F3_THREADS / 32) {
         if (n >= g.N) continue;
         const float4 got = *reinterpret_cast<const float4*>(tile + r * L::OUT_LD + 4 * lane);
-        if (doubtful(got)) {
+        if (!finite4(got)) {
             left = true;
             continue;
         }
@@ -315,7 +300,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 if (n + e < g.N) g.put(o + e, n + e, v[e]);
         }
     }
-    if (left && n < g.N) finish_doubtful<TN>(g, tile, largest, all, m0, n0);
+    if (left) multiply_again<TN>(g, tile, m0, n0);
     if (warp == 1) {
         __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
@@ -342,11 +327,11 @@ int tile_width(int M, int N, int sms) {
 
 }  // namespace
 
-// float32 X, W and sums; modes and bias as mv_gemm_simt's.  K a multiple of 4 up to 65,536, X and W on 16 bytes, rows without gaps; `sms`: the device's multiprocessors.
+// float32 X, W and sums; modes and bias as mv_gemm_simt's.  K a multiple of 4, X and W on 16 bytes, rows without gaps; `sms`: the device's multiprocessors.
 MV_API int mv_gemm_f32_tc(const float* X, const float* W, const float* bias, void* out, int mode, int M, int N, int K, int ldo, int sms, int* err,
                           cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (K < 4 || K % 4 || K > 65536 || mode < 0 || mode > 2 || (((uintptr_t)X | (uintptr_t)W) & 15) || (M + TM - 1) / TM > 65535 || sms < 1) return (int)cudaErrorInvalidValue;
+    if (K < 4 || K % 4 || mode < 0 || mode > 2 || (((uintptr_t)X | (uintptr_t)W) & 15) || (M + TM - 1) / TM > 65535 || sms < 1) return (int)cudaErrorInvalidValue;
     return tile_width(M, N, sms) == 128 ? launch<128>(X, W, bias, out, mode, M, N, K, ldo, err, stream)
                                         : launch<96>(X, W, bias, out, mode, M, N, K, ldo, err, stream);
 }

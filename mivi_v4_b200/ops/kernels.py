@@ -1772,7 +1772,7 @@ def gemm_f32_tc_takes(M: int, N: int, K: int, sms: int) -> bool:
     up some 40e6 products a us, and lose about 32 rows to their tiles.  Measured (tensor / CUDA cores) on nine shapes at 9 to 1,165 rows, never the
     slower one by more than a tenth: 9,216 x 1,024 at 16 rows 29 / 37, at 1,165 133 / 516; 1,024 x 4,608 at 128 rows 80 / 45, at 600 80 / 172; 6,144 x
     2,048 at 32 rows 45 / 43, at 48 45 / 68.  From K = 1,024 on: below, sums are so short that float32 multiply-adds are as exact."""
-    if M < F32_TC_ROWS or K < F32_TC_K or K > 65536 or K % 4 or M > 65535 * 128:
+    if M < F32_TC_ROWS or K < F32_TC_K or K % 4 or M > 65535 * 128:
         return False
     rows = -(-M // 128)
     tensor = 4.0 + K / 1024.0 * min(26.4 * -(-rows * -(-N // 128) // sms), 21.9 * -(-rows * -(-N // 96) // sms))
