@@ -1,15 +1,20 @@
-// Y[M, N] = X[M, K] . W[N, K]^T of float32 operands on the tensor cores, with an error against 64 bits no larger than that of float32
-// multiply-adds (gemm_simt.cu), for products of many rows.
+// Y[M, N] = X[M, K] . W[N, K]^T of float32 operands on the tensor cores, for products of many rows.
 //
-// Every operand is split into three bfloat16 numbers, 2^39 x = h + m + l (each what rounding left of the one before; together its 24 bits), and
-// six of the nine products are added up: h h, then h m + m h, m m, h l + l h; what is left out is below 2^-25 of |x w|.  The tensor cores cut the
-// sums that they add to off, so a long chain of them loses places (K = 1,024 in one chain: 1e-6): h h is added over 128 of K in tensor memory and then in
-// float32 registers; the five others, 2^-8 of it, have an accumulator of their own over all of K.
+// Every operand, times 2^39, is split into three bfloat16 numbers, h + m + l (each what rounding left of the one before; together its 24 bits), and
+// six of the nine products are added up: h h, then h m + m h, m m, h l + l h; what is left out is below 2^-25 of |x w|.  The tensor cores cut
+// off what they add, to the last place of the largest number there is: a long chain of it loses places (K = 1,024 in one: 1e-6), and where all terms have one sign the loss adds up.  So h h
+// is added over 64 of K in tensor memory and then in float32 registers; the five others, 2^-8 of it, have an accumulator of their own over all of K.
+//
+// Error against 64 bits in the 2-norm, 256 x 512, this kernel / float32 multiply-adds (gemm_simt.cu), 1e-7, at K = 1,024 | 2,048 | 4,608: terms of both signs 1.1 / 1.6 | 1.3 / 2.1 | 1.8 / 3.1;
+// of one sign 1.1 / 0.6 | 1.2 / 0.7 | 1.5 / 0.8; X with magnitudes spread over e^9 (sigma of the logarithm 3) 1.5 / 1.3 | 1.2 / 1.4 | 2.2 / 3.1, and with W of one
+// sign 3.5 / 1.1 | 4.0 / 2.5 | 3.6 / 3.2.  Model weights have both signs: there it is the more exact of the two, where all terms have one sign the less exact, by half of float32's
+// last place.  (Runs of 128 of K: both signs 1.3 | 1.5 | 1.8, one sign 1.8 | 1.8 | 1.9, the last form 7.0 | 9.7 | 8.2, in the same time.  Runs that begin at minus half of what they will add, with what the
+// sum's rounding left, 0.9 and 0.5 | 0.5 | 0.5: the products take 16 to 23 % longer.)
 //
 // Block = a tile of 128 rows of X by TN of W, 32 of K at a time:
 //   warp 0       TMA: the float32 tiles of X and W into a ring of four stages;
 //   warp 1       the products, twelve 128 x TN x 16 a stage;
-//   warps 4-7    add the finished 128 of K of h h (two accumulators take turns) to their registers, TN columns of a row a thread;
+//   warps 4-7    add the finished 64 of K of h h (two accumulators take turns) to their registers, TN columns of a row a thread;
 //   warps 8-15   split X, a row a thread, out of a stage of the ring into tensor memory, from where the products read it;
 //   warps 16-23  split W, a row a thread, into shared memory, in the layout that the products read.
 // At the end the tile goes through shared memory, is multiplied by 2^-78, and all warps store it by rows.  The scale keeps all parts of all float32 numbers in bfloat16's range, down
@@ -19,15 +24,14 @@
 //
 // Bound by the splitting (some 560 instructions of every scheduler a stage, and waits: 0.58 us for 128 x 96, 0.8 for 128 x 128), then by shared memory (a stage of
 // 128 columns writes and reads 32 KB of float32 tiles, writes 24 KB and has the products read 48 KB of W's planes: 1,060 clocks beside the products'
-// 780).  1,165 rows against 9,216 x 1,024 516 -> 133 us (165 TFLOP/s), against 1,024 x 4,608 280 -> 85; error against 64 bits 1.3e-7 where the
-// multiply-adds have 4.1e-7 (K = 1,024), 1.8e-7 where they have 8.6e-7 (K = 4,608).  With X's planes in shared memory too, which the products then read at all
+// 780).  1,165 rows against 9,216 x 1,024 516 -> 129 us (170 TFLOP/s), against 1,024 x 4,608 280 -> 86.  With X's planes in shared memory too, which the products then read at all
 // its bandwidth, 174 us; with the two groups of splitting warps on the same stage 145.
 #include "tc_common.cuh"
 
 namespace {
 
 constexpr int F3_THREADS = 768;
-constexpr int TM = 128, KB = 32, RAW = 4, CHUNK = 4;     // CHUNK stages of KB: how long h h is added up in tensor memory
+constexpr int TM = 128, KB = 32, RAW = 4, CHUNK = 2;     // CHUNK stages of KB: how long h h is added up in tensor memory
 constexpr int X_BYTES = TM * KB * 4;
 constexpr unsigned X_PLANE = KB / 2;                                 // columns of tensor memory
 
@@ -177,18 +181,17 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
         const int quarter = warp & 3, r = quarter * 32 + lane;
         const unsigned lane_addr = tmem_base + ((unsigned)(quarter * 32) << 16);
-        float sum[TN];
+        float2 sum[TN / 2];
 #pragma unroll
-        for (int j = 0; j < TN; ++j) sum[j] = 0.f;
+        for (int j = 0; j < TN / 2; ++j) sum[j] = make_float2(0.f, 0.f);
         auto add = [&](unsigned col) {
 #pragma unroll
-            for (int c = 0; c < TN; c += 32) {                    // (columns past TN are there and not looked at)
-                unsigned v[32];
-                tmem_ld32(lane_addr + col + (unsigned)c, v);
+            for (int c = 0; c < TN; c += 16) {
+                unsigned v[16];
+                tmem_ld16(lane_addr + col + (unsigned)c, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    if (c + j < TN) sum[c + j] += __uint_as_float(v[j]);
+                for (int j = 0; j < 8; ++j) sum[c / 2 + j] = add2(sum[c / 2 + j], make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])));
             }
         };
         for (int chunk = 0; chunk < chunks; ++chunk) {
@@ -205,7 +208,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             add(L::LOW_COL);
 #pragma unroll
             for (int j = 0; j < TN; j += 4)
-                *reinterpret_cast<float4*>(tile + r * L::OUT_LD + j) = make_float4(sum[j] * UNSCALE, sum[j + 1] * UNSCALE, sum[j + 2] * UNSCALE, sum[j + 3] * UNSCALE);
+                *reinterpret_cast<float4*>(tile + r * L::OUT_LD + j) =
+                    make_float4(sum[j / 2].x * UNSCALE, sum[j / 2].y * UNSCALE, sum[j / 2 + 1].x * UNSCALE, sum[j / 2 + 1].y * UNSCALE);
         }
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
