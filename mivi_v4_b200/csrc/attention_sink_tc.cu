@@ -10,18 +10,19 @@
 //   warp 0      TMA: the Q tiles once, then keys and values into rings of four stages each;
 //   warp 1      S = Q K^T (128 x 64 x dk);
 //   warp 3      O += P V (128 x 64 x 64; with SPLIT twice, P being two bfloat16 numbers), P read from tensor memory;
-//   warp 2      zeroes the value rows of the last block that come after the last query: whatever lies there would pass through a weight of 0;
+//   warp 2      looks through the values of the blocks that some row of the tile does not see whole (attention_tc.cuh): rows after the last query become
+//               zeros, and so do infinities and NaNs, which would pass through a weight of 0;
 //   warps 4-11  softmax, four warps a tile, one query row a thread.
 //
 // Every sum is added and every score rounded as attention_sink_prefill.cu does it, so that a row's result does not hang on which of the two kernels its
 // step took: both kinds of tensor-core instruction add alike; key blocks lie at multiples of 64, and a block that shows a row nothing changes nothing; a
 // row's reference is its running maximum after every block; its denominator is four sums, of every eighth key and its neighbour; whether a block lies wholly
-// beyond the distance table is decided for the same 16 queries.
+// beyond the distance table is decided for the same 16 queries.  (Of values that are not finite the other kernel lets a tile's 64 queries see all that one of them sees.)
 //
 // Bound by the exponential unit where scores are capped (three of its results a score), else by the softmax's instructions.  This kernel /
 // attention_sink_prefill.cu: one prompt of 2,048 tokens, 32 heads of 80 / 64 in groups of 4, capped, a window of 1,024 75 / 115 us; of 64 with chunks of
 // 1,024 32 / 63; capped, a table of 241 distances, split weights 100 / 153.
-#include "tc_common.cuh"
+#include "attention_tc.cuh"
 
 namespace {
 
@@ -35,15 +36,15 @@ constexpr float LOG2E = 1.4426950408889634f;
 // PARTS: parts of 64 channels that queries and keys lie in
 template <int PARTS> struct StLayout {
     static constexpr int Q_PART = BQ * BK * 2, Q_BYTES = PARTS * Q_PART, K_PART = BKV * BK * 2, K_BYTES = PARTS * K_PART;
-    static constexpr int K_AT = TILES * Q_BYTES, V_AT = K_AT + KSTAGES * K_BYTES, BAR_AT = V_AT + KSTAGES * V_BYTES, DIST_AT = BAR_AT + 256;
+    static constexpr int K_AT = TILES * Q_BYTES, V_AT = K_AT + KSTAGES * K_BYTES, BAR_AT = V_AT + KSTAGES * V_BYTES, DIST_AT = BAR_AT + 512;
     static constexpr int TOTAL = DIST_AT + 1024;   // (with the alignment of the start; two heads' distance tables come on top)
 };
 
 // barriers, 8 bytes each.  Scores, weights and products have two a tile, by the key block's parity.
 enum { B_Q = 0, B_KFULL = 1, B_KEMPTY = B_KFULL + KSTAGES, B_VFULL = B_KEMPTY + KSTAGES, B_VEMPTY = B_VFULL + KSTAGES,
        B_SFULL = B_VEMPTY + KSTAGES, B_PFULL = B_SFULL + 2 * TILES, B_PVDONE = B_PFULL + 2 * TILES, B_VFIX = B_PVDONE + 2 * TILES,
-       B_COUNT = B_VFIX + 1 };
-static_assert(B_COUNT * 8 + 8 <= 256, "barrier area");
+       B_LOOKED = B_VFIX + KSTAGES, B_COUNT };
+static_assert(B_COUNT * 8 + 8 <= 512, "barrier area");
 
 __device__ __forceinline__ float rcp(float x) {
     float y;
@@ -125,10 +126,12 @@ __device__ __forceinline__ void chunk_weights(const unsigned (&s)[32], float ref
 struct StArgs {
     const int *page_table, *cu, *starts;
     const float *sinks, *gate, *r1, *r2, *dist;
+    const __nv_bfloat16* values;                       // the first page's; ld_v a row
+    long long page_stride;
     __nv_bfloat16* o;
     float* o_all;
     int* err;
-    int table_stride, page_shift, B, nh, nkv, dk, dv, ld_gate, window, keep_first, chunk, dist_len, gate_wide;
+    int table_stride, page_shift, B, nh, nkv, dk, dv, ld_gate, window, keep_first, chunk, dist_len, gate_wide, ld_v;
     float scale, cap;
 };
 
@@ -142,6 +145,7 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const unsigned q_s = smem_u32(smem), k_s = q_s + L::K_AT, v_s = q_s + L::V_AT;
     unsigned long long* bars = (unsigned long long*)(smem + L::BAR_AT);
     unsigned* tmem_holder = (unsigned*)(bars + B_COUNT);
+    volatile int* found = (volatile int*)(tmem_holder + 1);               // warp 2 has met a value that is not finite
     float* dist_s = (float*)(smem + L::DIST_AT);
     const unsigned bar0 = smem_u32(bars);
     auto bar = [&](int i) { return bar0 + 8u * (unsigned)i; };
@@ -166,11 +170,20 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const int n_iter = n_kept + kb_end - kb_begin;
     auto block_of = [&](int j) { return j < n_kept ? j : kb_begin + (j - n_kept); };
     const int last_rows = last_pos + 1 - (kb_end - 1) * BKV;             // rows of the last block up to the last query's
-    const bool fix_last = last_rows < BKV;
+    const int keep = a.chunk == 0 && a.window > 0 ? a.keep_first : 0;
+    // some row of the tile does not see all of block j: from the block on that reaches past the first query, from the last kept block on to where the last
+    // query's window or chunk starts (a block with rows after the last query is one of these)
+    const int last_from = a.chunk > 0 ? last_pos - last_pos % a.chunk : a.window > 0 ? max(0, last_pos - a.window + 1) : 0;
+    const int seen_to = n_kept + (pos0 + 1) / BKV - kb_begin, kept_to = min(keep / BKV, n_kept);
+    const int seen_from = n_kept + max(0, (last_from + BKV - 1) / BKV - kb_begin);
+    auto partly_seen = [&](int j) { return j >= seen_to || (j >= kept_to && j < seen_from); };
+    const int* table = a.page_table + (size_t)b * a.table_stride;
+    const int page_size = 1 << a.page_shift;
     const int warp = warp_index(), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < B_COUNT; ++i) mbar_init(bar(i), i >= B_PFULL && i < B_PFULL + 2 * TILES ? 4 : 1);
+        *found = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (a.dist && a.dist_len <= DIST_SMEM)
@@ -187,15 +200,13 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 
     if (warp < 4) {
         // registers move from this warpgroup to the softmax warps (168 each at launch)
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
         if (warp == 0) {
             if (elect_one()) {
                 mbar_expect_tx(bar(B_Q), TILES * L::Q_BYTES);
                 for (int t = 0; t < TILES; ++t)
                     for (int p = 0; p < PARTS; ++p) tma_load_3d(q_s + t * L::Q_BYTES + p * L::Q_PART, &map_q, p * BK, h0 + t, row0, bar(B_Q));
             }
-            const int* table = a.page_table + (size_t)b * a.table_stride;
-            const int page_size = 1 << a.page_shift;
             for (int j = 0; j < n_iter; ++j) {
                 const int s = j % KSTAGES, t0 = block_of(j) * BKV;
                 const unsigned ph = (unsigned)(j / KSTAGES) & 1u;
@@ -207,8 +218,8 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                         tma_load_3d(k_s + s * L::K_BYTES + p * L::K_PART, &map_k, p * BK, g * page_size + in_page, page, bar(B_KFULL + s));
                 }
                 if (!mbar_wait_warp(bar(B_VEMPTY + s), ph ^ 1u, a.err, 72)) break;
-                // a last block with rows of nobody's goes by way of warp 2, which then says that it is there
-                const unsigned full = j == n_iter - 1 && fix_last ? bar(B_VFIX) : bar(B_VFULL + s);
+                // blocks that are partly seen go by way of warp 2, which then says that they are there
+                const unsigned full = bar((partly_seen(j) ? B_VFIX : B_VFULL) + s);
                 if (elect_one()) {
                     mbar_expect_tx(full, V_BYTES);
                     tma_load_3d(v_s + s * V_BYTES, &map_v, 0, vg * page_size + in_page, page, full);
@@ -267,18 +278,22 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     }
                 }
             }
-        } else if (warp == 2 && fix_last) {
-            const int s = (n_iter - 1) % KSTAGES;
-            if (mbar_wait_warp(bar(B_VFIX), 0, a.err, 79)) {
-                for (int i = last_rows * 8 + lane; i < BKV * 8; i += 32)
-                    *reinterpret_cast<uint4*>(smem + L::V_AT + s * V_BYTES + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+        } else if (warp == 2) {
+            unsigned phases = 0;                                         // a bit a stage
+            for (int j = 0; j < n_iter; ++j) {
+                if (!partly_seen(j)) continue;
+                const int s = j % KSTAGES;
+                if (!mbar_wait_warp(bar(B_VFIX + s), (phases >> s) & 1u, a.err, 79)) break;
+                phases ^= 1u << s;
+                if (clean_values(smem + L::V_AT + s * V_BYTES, 0, j == n_iter - 1 ? last_rows : BKV, lane) && lane == 0) *found = 1;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(B_VFULL + s));
             }
+            if (lane == 0) mbar_arrive(bar(B_LOOKED));
         }
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
         const int t = (warp - 4) >> 2, quarter = warp & 3, h = h0 + t;
         const int r = quarter * 32 + lane;                               // this thread's query row within the tile
         const int pos = pos0 + r, tile_last = pos0 + BQ - 1;
@@ -293,8 +308,7 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         const float dist_unit = a.dist_len <= DIST_SMEM ? 1.0f : LOG2E;
         const int pos16 = pos0 + (r & ~15);                              // the first of the 16 queries that share the choice of the far end
         const int from_pos = a.chunk > 0 ? pos - pos % a.chunk : (a.window > 0 ? pos - a.window + 1 : 0);
-        const int keep = a.chunk == 0 && a.window > 0 ? a.keep_first : 0;
-        const int last_from = a.chunk > 0 ? tile_last - tile_last % a.chunk : (a.window > 0 ? tile_last - a.window + 1 : 0);
+        const int masked_to = a.chunk > 0 ? tile_last - tile_last % a.chunk : (a.window > 0 ? tile_last - a.window + 1 : 0);
         float m = a.sinks ? a.sinks[h] * LOG2E : -INFINITY;              // the reference of the row's exponentials; a sink starts it
         float l[4] = {a.sinks ? 1.f : 0.f, 0.f, 0.f, 0.f};
         bool ok = true;
@@ -326,7 +340,7 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 log_chunk(s1, db1, db2, n - 32);
             }
             // the same for all rows of the tile: the block reaches past its first query, or before what its last one sees
-            if (j < n_kept || key0 + BKV - 1 > pos0 || key0 < last_from) {
+            if (j < n_kept || key0 + BKV - 1 > pos0 || key0 < masked_to) {
                 mask_chunk(s0, 0, from_pos - key0, keep - key0, n + 1);
                 mask_chunk(s1, 32, from_pos - key0, keep - key0, n + 1);
             }
@@ -363,6 +377,7 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             if (lane == 0) mbar_arrive(bar(B_PFULL + 2 * t + (j & 1)));
         }
         if (ok) ok = mbar_wait_warp(bar(B_PVDONE + 2 * t + ((n_iter - 1) & 1)), (unsigned)((n_iter - 1) >> 1) & 1u, a.err, 82);
+        if (ok) ok = mbar_wait_warp(bar(B_LOOKED), 0, a.err, 83);
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const bool live = r < nq;
@@ -375,10 +390,24 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             float* dst_all = a.o_all ? a.o_all + ((row * a.nh + h) * a.nkv + vg) * a.dv : nullptr;
 #pragma unroll
             for (int c = 0; c < DV; c += 32) {
+                NotFinite seen;
+                if (*found && live && c < a.dv)
+                    for (int j = 0; j < n_iter; ++j) {
+                        if (!partly_seen(j)) continue;
+                        const int key0 = block_of(j) * BKV, upto = min(BKV, pos + 1 - key0), n = min(32, a.dv - c);
+                        const __nv_bfloat16* rows = a.values + (size_t)mv_read_page(table[key0 >> a.page_shift]) * a.page_stride +
+                                                    (size_t)(vg * page_size + (key0 & (page_size - 1))) * a.ld_v + c;
+                        seen = look_up(seen, rows, a.ld_v, 0, min(keep - key0, upto), n);
+                        seen = look_up(seen, rows, a.ld_v, max(0, from_pos - key0), upto, n);
+                    }
                 unsigned v[32];
                 tmem_ld32(o_addr + (unsigned)c, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (live) {
+                    if (seen.any()) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + seen.value(i));
+                    }
 #pragma unroll
                     for (int d = 0; d < 32; d += 8) {
                         if (c + d < a.dv) {
@@ -470,8 +499,8 @@ MV_API int mv_attention_sink_tc(const void* q, const void* pool, int n_pages, lo
     while ((1 << page_shift) < page_size) ++page_shift;
     const dim3 grid(nh / TILES * (o_all ? nkv : 1), (N + BQ - 1) / BQ + B);      // an upper bound of the tiles; spare blocks return at once
     if (grid.y > 65535u) return (int)cudaErrorInvalidValue;
-    const StArgs a = {page_table, cu, starts, sinks, gate, r1, r2, dist, (__nv_bfloat16*)o, o_all, err, table_stride, page_shift, B, nh, nkv, dk, dv,
-                      ld_gate, window, keep_first, chunk, dist_len, gate_wide, scale, cap};
+    const StArgs a = {page_table, cu, starts, sinks, gate, r1, r2, dist, values, page_stride, (__nv_bfloat16*)o, o_all, err, table_stride, page_shift,
+                      B, nh, nkv, dk, dv, ld_gate, window, keep_first, chunk, dist_len, gate_wide, v_in_k ? dk : dv, scale, cap};
     if (dk <= BK) return split ? launch<1, true>(mq, mk, mv, a, grid, stream) : launch<1, false>(mq, mk, mv, a, grid, stream);
     return split ? launch<2, true>(mq, mk, mv, a, grid, stream) : launch<2, false>(mq, mk, mv, a, grid, stream);
 }

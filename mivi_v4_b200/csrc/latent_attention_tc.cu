@@ -9,8 +9,8 @@
 //   warp 0      TMA: the two Q tiles once, then keys and values into rings of four stages each;
 //   warp 1      S = Q K^T (128 x 64 x 96 or 128);
 //   warp 3      O += P V (128 x 64 x 64, twice: P is two bfloat16 numbers), P read from tensor memory;
-//   warp 2      zeroes the value rows of the first and the last block that are another sequence's, whose infinities
-//               and NaNs would pass through a weight of 0;
+//   warp 2      looks through the values of the blocks that some row of the pair does not see whole (attention_tc.cuh): another sequence's rows
+//               become zeros, and so do infinities and NaNs, which would pass through a weight of 0;
 //   warps 4-11  softmax, four warps a tile, one query row a thread.
 //
 // Tensor memory: two buffers of 64 columns a tile for S, and O of 64 a tile.  A row's thread takes its 64 scores into registers and
@@ -25,11 +25,11 @@
 //
 // Bound by the softmax (a block of 64 keys of both tiles needs 1,024 clocks of the exponential unit and some 1,000 instructions of each
 // scheduler, and its products 1,100 clocks beside it).  32 heads of 64 + 32 / 64 with a gate, this kernel / latent_attention_prefill.cu: one prompt of 6,000 tokens
-// 363 / 1,132 us, of 2,048 72 / 190, three of 333 to 2,048 103 / 226.  What it took: an elected lane of a whole warp issues the products (see
+// 372 / 1,132 us, of 2,048 73 / 190, three of 333 to 2,048 108 / 226.  What it took: an elected lane of a whole warp issues the products (see
 // tc_common.cuh; a first form of the kernel with a lane by itself 495 us), one warp for
 // either product (one for both: the waits of one hold up the other, 296 against 273 for a form of other sums), gates read 32 bytes at a time (a block's gates element by
 // element took longer than its softmax: 344 against 317).
-#include "tc_common.cuh"
+#include "attention_tc.cuh"
 
 namespace {
 
@@ -44,15 +44,15 @@ template <int ROT> struct LtLayout {
     // queries and keys lie as two swizzled parts, the 64 unrotated channels and the rotated ones
     static constexpr int Q_PART = BQ * DIM * 2, Q_BYTES = Q_PART + BQ * ROT * 2, K_PART = BKV * DIM * 2, K_BYTES = K_PART + BKV * ROT * 2;
     static constexpr int K_AT = TILES * Q_BYTES, V_AT = K_AT + KSTAGES * K_BYTES, BAR_AT = V_AT + KSTAGES * V_BYTES;
-    static constexpr int TOTAL = BAR_AT + 256 + 1024;
+    static constexpr int TOTAL = BAR_AT + 512 + 1024;
 };
 
 // barriers, 8 bytes each.  Scores, weights and products have two a tile, by the key block's parity: the next block's may be complete before
 // whoever waits for this block's has looked, the one after that cannot.
 enum { B_Q = 0, B_KFULL = 1, B_KEMPTY = B_KFULL + KSTAGES, B_VFULL = B_KEMPTY + KSTAGES, B_VEMPTY = B_VFULL + KSTAGES,
        B_SFULL = B_VEMPTY + KSTAGES, B_PFULL = B_SFULL + 2 * TILES, B_PVDONE = B_PFULL + 2 * TILES, B_VFIX = B_PVDONE + 2 * TILES,
-       B_COUNT = B_VFIX + 2 };
-static_assert(B_COUNT * 8 + 8 <= 256, "barrier area");
+       B_LOOKED = B_VFIX + KSTAGES, B_COUNT };
+static_assert(B_COUNT * 8 + 8 <= 512, "barrier area");
 
 // scores of the keys outside [from, upto) become -inf; the chunk's first key is key c of the block
 __device__ __forceinline__ void mask_chunk(unsigned (&s)[32], int c, int from, int upto) {
@@ -92,7 +92,8 @@ __device__ __forceinline__ int first_seen(int start, int window) { return window
 template <int ROT>
 __global__ void __launch_bounds__(LT_THREADS, 1)
 latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_qr,
-                           const __grid_constant__ CUtensorMap map_kx, const __grid_constant__ CUtensorMap map_r, int v0,
+                           const __grid_constant__ CUtensorMap map_kx, const __grid_constant__ CUtensorMap map_r,
+                           const __nv_bfloat16* __restrict__ kx, int ld_kx, int v0,
                            const int* __restrict__ cu, const int* __restrict__ starts, const float* __restrict__ sinks,
                            const float* __restrict__ gate, int ld_gate, int gate_heads, __nv_bfloat16* __restrict__ o, int B,
                            int nh, float scale, int window, int* __restrict__ err) {
@@ -102,6 +103,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     const unsigned q_s = smem_u32(smem), k_s = q_s + L::K_AT, v_s = q_s + L::V_AT;
     unsigned long long* bars = (unsigned long long*)(smem + L::BAR_AT);
     unsigned* tmem_holder = (unsigned*)(bars + B_COUNT);
+    volatile int* found = (volatile int*)(tmem_holder + 1);               // warp 2 has met a value that is not finite
     const unsigned bar0 = smem_u32(bars);
     auto bar = [&](int i) { return bar0 + 8u * (unsigned)i; };
 
@@ -128,12 +130,16 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     for (int t = 0; t < TILES; ++t) nb[t] = nq > t * BQ ? (pos0 + min(nq, (t + 1) * BQ) - 1 - key_first) / BKV + 1 : 0;
     const int nb_max = max(nb[0], nb[1]);
     // rows of the first and the last block that are not this sequence's, or come after the pair's last query
-    const int rows_before = max(0, lo - key_first), last_rows = pos0 + nq - key_first - (nb_max - 1) * BKV;
-    const bool fix_first = rows_before > 0, fix_last = last_rows < BKV;
+    const int rows_before = max(0, lo - key_first), last_rows = min(BKV, pos0 + nq - key_first - (nb_max - 1) * BKV);
+    // some row of a tile that walks block j does not see all of it: from the block on that reaches past the first query (the second tile's own are among
+    // them), and before the last query's window (a block with rows of others is one of these)
+    const int seen_to = max(0, pos0 + 1 - key_first) / BKV, seen_from = window > 0 ? max(0, pos0 + nq - window - key_first + BKV - 1) / BKV : 0;
+    auto partly_seen = [&](int j) { return j >= seen_to || j < seen_from; };
     const int warp = warp_index(), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < B_COUNT; ++i) mbar_init(bar(i), i >= B_PFULL && i < B_PFULL + 2 * TILES ? 4 : 1);
+        *found = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -148,7 +154,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 
     if (warp < 4) {
         // registers move from this warpgroup to the softmax warps (168 each at launch)
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
         if (warp == 0) {
             if (elect_one()) {
                 mbar_expect_tx(bar(B_Q), TILES * L::Q_BYTES);
@@ -167,8 +173,8 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                     tma_load_2d(k_s + s * L::K_BYTES + L::K_PART, &map_r, 0, row, bar(B_KFULL + s));
                 }
                 if (!mbar_wait_warp(bar(B_VEMPTY + s), ph ^ 1u, err, 52)) break;
-                // blocks with rows of others go by way of warp 2, which then says that they are there
-                const unsigned full = j == 0 && fix_first ? bar(B_VFIX) : j == nb_max - 1 && fix_last ? bar(B_VFIX + 1) : bar(B_VFULL + s);
+                // blocks that are partly seen go by way of warp 2, which then says that they are there
+                const unsigned full = bar((partly_seen(j) ? B_VFIX : B_VFULL) + s);
                 if (elect_one()) {
                     mbar_expect_tx(full, V_BYTES);
                     tma_load_2d(v_s + s * V_BYTES, &map_kx, v0 + h * DV, row, full);
@@ -227,22 +233,21 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 }
             }
         } else if (warp == 2) {
-#pragma unroll
-            for (int f = 0; f < 2; ++f) {
-                // (one block that is the first and the last comes by the first way)
-                const int j = f ? nb_max - 1 : 0, s = j % KSTAGES;
-                if (f ? !fix_last || (fix_first && j == 0) : !fix_first) continue;
-                if (!mbar_wait_warp(bar(B_VFIX + f), 0, err, 59)) break;
-                const int head = j == 0 ? rows_before : 0, tail = j == nb_max - 1 ? last_rows : BKV;
-                for (int i = lane; i < BKV * 8; i += 32)
-                    if (i < head * 8 || i >= tail * 8) *reinterpret_cast<uint4*>(smem + L::V_AT + s * V_BYTES + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+            unsigned phases = 0;                                         // a bit a stage
+            for (int j = 0; j < nb_max; ++j) {
+                if (!partly_seen(j)) continue;
+                const int s = j % KSTAGES;
+                if (!mbar_wait_warp(bar(B_VFIX + s), (phases >> s) & 1u, err, 59)) break;
+                phases ^= 1u << s;
+                if (clean_values(smem + L::V_AT + s * V_BYTES, j == 0 ? rows_before : 0, j == nb_max - 1 ? last_rows : BKV, lane) && lane == 0) *found = 1;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(B_VFULL + s));
             }
+            if (lane == 0) mbar_arrive(bar(B_LOOKED));
         }
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
         const int t = (warp - 4) >> 2, quarter = warp & 3;
         const int r = quarter * 32 + lane;                               // this thread's query row within the tile
         const int pos = pos0 + t * BQ + r, tile_first = pos0 + t * BQ, tile_last = tile_first + BQ - 1;
@@ -313,6 +318,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             if (lane == 0) mbar_arrive(bar(B_PFULL + 2 * t + (j & 1)));
         }
         if (ok && my_nb > 0) ok = mbar_wait_warp(bar(B_PVDONE + 2 * t + ((my_nb - 1) & 1)), (unsigned)((my_nb - 1) >> 1) & 1u, err, 62);
+        if (ok && my_nb > 0) ok = mbar_wait_warp(bar(B_LOOKED), 0, err, 63);
         if (ok && my_nb > 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float den = __fadd_rn(__fadd_rn(l[0], l[1]), __fadd_rn(l[2], l[3])), by;     // the row is O by
@@ -330,10 +336,22 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             __nv_bfloat16* dst = o + (n * nh + h) * DV;
 #pragma unroll
             for (int c = 0; c < DV; c += 32) {
+                NotFinite seen;
+                if (*found && live)
+                    for (int j = 0; j < my_nb; ++j) {
+                        const int key0 = key_first + j * BKV;
+                        if (partly_seen(j))
+                            seen = look_up(seen, kx + (long long)(key_row + j * BKV) * ld_kx + v0 + h * DV + c, ld_kx,
+                                           window > 0 ? max(0, pos - window + 1 - key0) : 0, min(BKV, pos + 1 - key0), 32);
+                    }
                 unsigned v[32];
                 tmem_ld32(o_addr + (unsigned)c, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (live) {
+                    if (seen.any()) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + seen.value(i));
+                    }
 #pragma unroll
                     for (int d = 0; d < 32; d += 8) {
                         float x[8];
@@ -383,7 +401,7 @@ int launch(const void* q, const void* kx, int rows, int ld_kx, int v0, const voi
     const dim3 grid(nh, (N + TILES * BQ - 1) / (TILES * BQ) + B);      // an upper bound of the pairs; spare blocks return at once
     if (grid.y > 65535u) return (int)cudaErrorInvalidValue;
     latent_attention_tc_kernel<ROT><<<grid, LT_THREADS, LtLayout<ROT>::TOTAL, stream>>>(
-        mq, mqr, mkx, mr, v0, cu, starts, sinks, gate, ld_gate, gate_heads, (__nv_bfloat16*)o, B, nh, scale, window, err);
+        mq, mqr, mkx, mr, (const __nv_bfloat16*)kx, ld_kx, v0, cu, starts, sinks, gate, ld_gate, gate_heads, (__nv_bfloat16*)o, B, nh, scale, window, err);
     return mv_launch_status();
 }
 

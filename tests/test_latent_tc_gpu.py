@@ -79,3 +79,34 @@ def test_values_of_another_sequence_that_are_not_finite(bad):
         t[300:600] = bad                                       # all of the second sequence's rows
     got = attend(slice(0, 2), lens, starts, 0, q, k, v, r, sinks, None)
     assert torch.equal(got[:300], want[:300]) and torch.equal(got[590:], want[590:]) and not bool(got[300:590].isfinite().any())
+
+
+@gpu
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("lens,starts,window", [([700], [0], 0), ([300, 520], [70, 601], 0), ([700], [0], 100), ([190, 400], [300, 45], 37), ([1000], [77], 500)])
+@pytest.mark.parametrize("gate", [None, "element"])
+def test_values_that_are_not_finite_reach_the_rows_that_see_them(bad, lens, starts, window, gate, monkeypatch):
+    """Values of the sequence's own, each in a channel of its own: before and behind the edges of blocks, tiles and pairs of tiles, and of windows."""
+    from mivi_v4_b200.ops import kernels as K
+    monkeypatch.setattr(K, "LATENT_TC_TOKENS", 1)
+    nh = 2
+    q, k, v, r, sinks, gates = inputs(lens, starts, nh, 64, 32, 64, window, seed=5)
+    gates = gates if gate else None
+    dirty, clean = v.clone(), v.clone()
+    spots, base, row0 = [], 0, 0
+    for n, s in zip(lens, starts):
+        lo = max(0, s - window + 1) if window else 0
+        at = [s + p for p in (-60, -1, 0, 3, 62, 63, 64, 70, 126, 127, 128, 129, 190, 255, 256, 257, n - 70, n - 2, n - 1)]
+        spots += [(p, base + p - lo, s, row0, n) for p in sorted(set(at)) if lo <= p < s + n]
+        base, row0 = base + s + n - lo, row0 + n
+    assert len(spots) <= 64
+    for c, (_, row, *_) in enumerate(spots):
+        dirty[row, c % nh, c], clean[row, c % nh, c] = bad, 0.0
+    assert K.latent_tc_takes(sum(lens), rows_seen(lens, starts, window), len(lens), 64, 32, 64, 0.1)
+    got, want = (attend(slice(0, nh), lens, starts, window, q, k, x, r, sinks, gates) for x in (dirty, clean))
+    sees = torch.zeros(sum(lens), nh, 64, dtype=torch.bool, device=DEV)
+    for c, (p, _, s, first, n) in enumerate(spots):
+        pos = torch.arange(s, s + n, device=DEV)
+        sees[first:first + n, c % nh, c] = (pos >= p) & ((pos < p + window) if window else True)
+    assert torch.equal(got[~sees], want[~sees]) and bool(want.isfinite().all()) and not bool(got[sees].isfinite().any())
+    K.check_device_errors()

@@ -157,3 +157,49 @@ def test_sinks_of_any_size(monkeypatch):
         monkeypatch.setattr(K(), "SINK_TC_TOKENS", n)
         outs.append(run(q, pool, table, lens, starts, nh, nkv, dk, dv, page, sinks=sinks))
     assert torch.equal(*outs)
+
+
+@gpu
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("form", [dict(), dict(window=100, keep_first=70), dict(window=37), dict(window=300, keep_first=64, split_weights=True), dict(chunk=150),
+                                  dict(softcap=20.0, chunk=64, all_heads=True)])
+@pytest.mark.parametrize("lens,starts,dk,dv,page", [([700], [0], 64, 64, 64), ([130, 400], [301, 45], 80, 48, 128), ([520], [250], 128, 64, 64)])
+def test_values_that_are_not_finite_reach_the_rows_that_see_them(bad, form, lens, starts, dk, dv, page, monkeypatch):
+    """Values before and behind the edges of blocks, tiles, windows, kept tokens and chunks, each in a channel of its own of one kv head."""
+    monkeypatch.setattr(K(), "SINK_TC_TOKENS", 1)
+    monkeypatch.setattr(K(), "SINK_TC_ALL", 1)
+    nh, nkv, kw = 4, 2, dict(form)
+    q, _, _, pool, table = case(lens, starts, nh, nkv, dk, dv, page, 7)
+    window, keep, chunk = kw.get("window", 0), kw.get("keep_first", 0), kw.get("chunk", 0)
+    assert K().sink_tc_takes(sum(lens), len(lens), nh, nkv, dk, dv, page)
+    spots, row0 = [], 0
+    for b, (n, s) in enumerate(zip(lens, starts)):
+        at = [s + p for p in (-60, -1, 0, 3, 63, 64, 70, 127, 128, 129, 255, n - 70, n - 1)] + [5, 63, 64, 69, 70, 149, 150, 199]
+        spots += [(p, b, s, row0, n) for p in sorted(set(at)) if 0 <= p < s + n]
+        row0 += n
+    N = sum(lens)
+    for round0 in range(0, len(spots), dv):
+        some = spots[round0:round0 + dv]
+        pools = []
+        for value in (bad, 0.0):
+            pools.append(pool.clone())
+            for c, (p, b, *_) in enumerate(some):
+                pools[-1][int(table[b, p // page]), nkv * page * dk + ((c % nkv) * page + p % page) * dv + c] = value
+        got, want = (run(q, x, table, lens, starts, nh, nkv, dk, dv, page, **kw) for x in pools)
+        sees = torch.zeros(N, nh, nkv, dv, dtype=torch.bool)
+        for c, (p, b, s, r0, n) in enumerate(some):
+            pos = torch.arange(s, s + n)
+            see = pos >= p
+            if chunk:
+                see &= p >= pos - pos % chunk
+            elif window:
+                see &= (p > pos - window) | (p < keep)
+            for h in range(nh):
+                sees[r0:r0 + n, h, c % nkv, c] = see
+        if kw.get("all_heads"):
+            got, want = got.view(N, nh, nkv, dv), want.view(N, nh, nkv, dv)
+        else:
+            got, want = got.view(N, nh, dv), want.view(N, nh, dv)
+            sees = torch.stack([sees[:, h, h // (nh // nkv)] for h in range(nh)], 1)
+        assert torch.equal(got[~sees], want[~sees]) and bool(want.isfinite().all()) and not bool(got[sees].isfinite().any())
+    K().check_device_errors()
