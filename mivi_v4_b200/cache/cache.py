@@ -140,7 +140,7 @@ class SequenceCache:
         self._nblk = np.zeros(max(n_slots, 1), dtype=np.int64)
         self._table: Dict[int, np.ndarray] = {g: np.zeros((max(n_slots, 1), 8), dtype=np.int32) for g in self.kv_groups}
         self.storage: Dict[int, torch.Tensor] = {}
-        self._state_views: Dict[int, List[torch.Tensor]] = {}      # slot -> its state in every layer
+        self._state_views: Dict[int, List[List[torch.Tensor]]] = {}     # slot -> its state in every layer, a list a dtype
         for gi, g in enumerate(plan.groups):
             if isinstance(g.need, KVNeed):
                 if g.need.uneven:
@@ -188,11 +188,16 @@ class SequenceCache:
         for t in self._table.values():
             t[s] = 0
         if self.state_groups:
-            # one launch for the states of all layers (a launch a group took 5 us of the host each)
+            # one launch a dtype for the states of all layers (a launch a group took 5 us of the host each; tensors of different dtypes in one
+            # call are zeroed one by one, a launch a layer)
             views = self._state_views.get(s)
             if views is None:
-                views = self._state_views[s] = [layer for gi in self.state_groups for layer in self.storage[gi][:, s].unbind(0)]
-            torch._foreach_zero_(views)
+                by_dtype: Dict[torch.dtype, List[torch.Tensor]] = {}
+                for gi in self.state_groups:
+                    by_dtype.setdefault(self.storage[gi].dtype, []).extend(self.storage[gi][:, s].unbind(0))
+                views = self._state_views[s] = list(by_dtype.values())
+            for same in views:
+                torch._foreach_zero_(same)
         return s
 
     def release(self, slot: int) -> None:

@@ -48,6 +48,25 @@ def test_plan_shared_cache():
         plan_cache([KVNeed(2, 8), KVNeed(1, 8)], [None, 0])
 
 
+def test_a_new_sequences_states_are_zeroed_a_dtype_at_a_time(monkeypatch):
+    """States of several shapes and dtypes: zeros in the slot's and nowhere else, by one call for all tensors of a dtype (torch takes a call of mixed dtypes tensor by
+    tensor), before and after the slots' number grows."""
+    c = make(n_slots=2, needs=[StateNeed((1,), torch.int32), StateNeed((2, 8)), KVNeed(2, 8), StateNeed((2, 8)), StateNeed((3, 4)), StateNeed((1,), torch.int32)])
+    calls, zero = [], torch._foreach_zero_
+    monkeypatch.setattr(torch, "_foreach_zero_", lambda ts: (calls.append([t.dtype for t in ts]), zero(ts)))
+    for grow in (False, True):
+        if grow:
+            c.grow_slots(5)
+        for gi in c.state_groups:
+            c.storage[gi].fill_(7)
+        calls.clear()
+        s = c.assign()
+        assert sorted(len(d) for d in calls) == [2, 3] and all(len(set(d)) == 1 for d in calls)
+        for gi in c.state_groups:
+            st = c.storage[gi]
+            assert not st[:, s].any() and bool((st[:, [i for i in range(st.shape[1]) if i != s]] == 7).all())
+
+
 def test_slots_pages_and_lengths():
     c = make()
     s = c.assign()
