@@ -211,13 +211,13 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 const int s = j % KSTAGES, t0 = block_of(j) * BKV;
                 const unsigned ph = (unsigned)(j / KSTAGES) & 1u;
                 const int page = mv_read_page(table[t0 >> a.page_shift]), in_page = t0 & (page_size - 1);
-                if (!mbar_wait_warp(bar(B_KEMPTY + s), ph ^ 1u, a.err, 71)) break;
+                if (!mbar_wait_warp(bar(B_KEMPTY + s), ph ^ 1u, a.err, 81)) break;
                 if (elect_one()) {
                     mbar_expect_tx(bar(B_KFULL + s), L::K_BYTES);
                     for (int p = 0; p < PARTS; ++p)
                         tma_load_3d(k_s + s * L::K_BYTES + p * L::K_PART, &map_k, p * BK, g * page_size + in_page, page, bar(B_KFULL + s));
                 }
-                if (!mbar_wait_warp(bar(B_VEMPTY + s), ph ^ 1u, a.err, 72)) break;
+                if (!mbar_wait_warp(bar(B_VEMPTY + s), ph ^ 1u, a.err, 82)) break;
                 // blocks that are partly seen go by way of warp 2, which then says that they are there
                 const unsigned full = bar((partly_seen(j) ? B_VFIX : B_VFULL) + s);
                 if (elect_one()) {
@@ -229,14 +229,14 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             // S(t, j) = Q_t K_j^T as soon as the keys are there and the buffer's weights, those of the tile's block before the last, are used
             const unsigned idesc = instr_desc(BQ, BKV);
             const int steps = a.dk / 16;
-            bool ok = mbar_wait_warp(bar(B_Q), 0, a.err, 73);
+            bool ok = mbar_wait_warp(bar(B_Q), 0, a.err, 83);
             for (int j = 0; j < n_iter && ok; ++j) {
                 const int s = j % KSTAGES;
-                if (!(ok = mbar_wait_warp(bar(B_KFULL + s), (unsigned)(j / KSTAGES) & 1u, a.err, 74))) break;
+                if (!(ok = mbar_wait_warp(bar(B_KFULL + s), (unsigned)(j / KSTAGES) & 1u, a.err, 84))) break;
 #pragma unroll
                 for (int t = 0; t < TILES; ++t) {
                     if (!ok) continue;
-                    if (j > 1 && !(ok = mbar_wait_warp(bar(B_PVDONE + 2 * t + (j & 1)), (unsigned)((j - 2) >> 1) & 1u, a.err, 75))) continue;
+                    if (j > 1 && !(ok = mbar_wait_warp(bar(B_PVDONE + 2 * t + (j & 1)), (unsigned)((j - 2) >> 1) & 1u, a.err, 85))) continue;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned d = tmem_base + (unsigned)(2 * t + (j & 1)) * BKV;
                     const unsigned qa = q_s + t * L::Q_BYTES, ka = k_s + s * L::K_BYTES;
@@ -259,12 +259,12 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             bool ok = true;
             for (int j = 0; j < n_iter && ok; ++j) {
                 const int s = j % KSTAGES;
-                if (!(ok = mbar_wait_warp(bar(B_VFULL + s), (unsigned)(j / KSTAGES) & 1u, a.err, 76))) break;
+                if (!(ok = mbar_wait_warp(bar(B_VFULL + s), (unsigned)(j / KSTAGES) & 1u, a.err, 86))) break;
                 const unsigned long long v0d = smem_desc(v_s + s * V_BYTES);
 #pragma unroll
                 for (int t = 0; t < TILES; ++t) {
                     if (!ok) continue;
-                    if (!(ok = mbar_wait_warp(bar(B_PFULL + 2 * t + (j & 1)), (unsigned)(j >> 1) & 1u, a.err, 78))) continue;
+                    if (!(ok = mbar_wait_warp(bar(B_PFULL + 2 * t + (j & 1)), (unsigned)(j >> 1) & 1u, a.err, 88))) continue;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned p = tmem_base + (unsigned)(2 * t + (j & 1)) * BKV, d = tmem_base + O_COL0 + (unsigned)t * DV;
                     if (elect_one()) {
@@ -283,7 +283,7 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             for (int j = 0; j < n_iter; ++j) {
                 if (!partly_seen(j)) continue;
                 const int s = j % KSTAGES;
-                if (!mbar_wait_warp(bar(B_VFIX + s), (phases >> s) & 1u, a.err, 79)) break;
+                if (!mbar_wait_warp(bar(B_VFIX + s), (phases >> s) & 1u, a.err, 89)) break;
                 phases ^= 1u << s;
                 if (clean_values(smem + L::V_AT + s * V_BYTES, 0, j == n_iter - 1 ? last_rows : BKV, lane) && lane == 0) *found = 1;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -313,7 +313,7 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         float l[4] = {a.sinks ? 1.f : 0.f, 0.f, 0.f, 0.f};
         bool ok = true;
         for (int j = 0; j < n_iter; ++j) {
-            if (!(ok = mbar_wait_warp(bar(B_SFULL + 2 * t + (j & 1)), (unsigned)(j >> 1) & 1u, a.err, 80))) break;
+            if (!(ok = mbar_wait_warp(bar(B_SFULL + 2 * t + (j & 1)), (unsigned)(j >> 1) & 1u, a.err, 90))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned s_addr = lane_addr + (unsigned)(2 * t + (j & 1)) * BKV;
             unsigned s0[32], s1[32];
@@ -354,7 +354,7 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             for (int i = 0; i < 4; ++i) l[i] = fmaf(l[i], c, sum[i]);
             if (j > 0 && __any_sync(0xffffffffu, c != 1.0f)) {
                 // O is the block before's until its product is done
-                if (!(ok = mbar_wait_warp(bar(B_PVDONE + 2 * t + ((j - 1) & 1)), (unsigned)((j - 1) >> 1) & 1u, a.err, 81))) break;
+                if (!(ok = mbar_wait_warp(bar(B_PVDONE + 2 * t + ((j - 1) & 1)), (unsigned)((j - 1) >> 1) & 1u, a.err, 91))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                 for (int d = 0; d < DV; d += 32) {
@@ -376,8 +376,8 @@ attention_sink_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(B_PFULL + 2 * t + (j & 1)));
         }
-        if (ok) ok = mbar_wait_warp(bar(B_PVDONE + 2 * t + ((n_iter - 1) & 1)), (unsigned)((n_iter - 1) >> 1) & 1u, a.err, 82);
-        if (ok) ok = mbar_wait_warp(bar(B_LOOKED), 0, a.err, 83);
+        if (ok) ok = mbar_wait_warp(bar(B_PVDONE + 2 * t + ((n_iter - 1) & 1)), (unsigned)((n_iter - 1) >> 1) & 1u, a.err, 92);
+        if (ok) ok = mbar_wait_warp(bar(B_LOOKED), 0, a.err, 93);
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const bool live = r < nq;

@@ -255,7 +255,7 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++local) {
             const int acc = local & 1;
             const unsigned acc_phase = (unsigned)(local >> 1) & 1u;
-            ok = mbar_wait_warp(acc_empty0 + 8 * acc, acc_phase ^ 1u, err, 4);   // the epilogue has drained it
+            ok = mbar_wait_warp(acc_empty0 + 8 * acc, acc_phase ^ 1u, err, 5);   // the epilogue has drained it
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned tmem_acc = tmem_base + (unsigned)(acc * BN);

@@ -158,7 +158,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             for (int kb = 0; kb < kblocks; ++kb, ++it) {
                 const int s = it % STAGES;
                 const unsigned phase = (unsigned)(it / STAGES) & 1u;
-                ok = mbar_wait_warp(empty0 + 8 * s, phase ^ 1u, err, 1);
+                ok = mbar_wait_warp(empty0 + 8 * s, phase ^ 1u, err, 111);
                 if (!ok) break;
                 const unsigned bar = in_block(full0 + 8 * s, 0);
                 const unsigned a_dst = tiles0 + s * L::STAGE_BYTES;
@@ -179,14 +179,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 const int acc = local & 1;
                 const unsigned acc_phase = (unsigned)(local >> 1) & 1u;
                 ++local;
-                ok = mbar_wait_warp(acc_empty0 + 8 * acc, acc_phase ^ 1u, err, 4);   // both blocks have drained it
+                ok = mbar_wait_warp(acc_empty0 + 8 * acc, acc_phase ^ 1u, err, 115);   // both blocks have drained it
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned tmem_acc = tmem_base + (unsigned)(acc * BN);
                 for (int kb = 0; kb < kblocks; ++kb, ++it) {
                     const int s = it % STAGES;
                     const unsigned phase = (unsigned)(it / STAGES) & 1u;
-                    ok = mbar_wait_warp(full0 + 8 * s, phase, err, 2);
+                    ok = mbar_wait_warp(full0 + 8 * s, phase, err, 112);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned a_addr = tiles0 + s * L::STAGE_BYTES;
@@ -241,7 +241,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (link.emit_x && half == 0) request(0, old);
             WeightCursor wc;
             if (ACT == ACT_WEIGHTED) wc.move(rw, row, M, (n0 >> 5) + c_first);
-            ok = mbar_wait(acc_full0 + 8 * acc, acc_phase, err, 3);
+            ok = mbar_wait(acc_full0 + 8 * acc, acc_phase, err, 113);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const float sc = link.scale_part ? 1.0f / sqrtf(ss * link.inv_dim + link.eps) : 1.f;

@@ -156,7 +156,7 @@ gemm_tc_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         for (int i = first; i < nkb; ++i) {
             const int s = i % STAGES;
             const unsigned phase = (unsigned)(i / STAGES) & 1u;
-            if (!mbar_wait_warp(empty0 + 8 * s, phase ^ 1u, err, 1)) break;
+            if (!mbar_wait_warp(empty0 + 8 * s, phase ^ 1u, err, 101)) break;
             const unsigned a_dst = tiles0 + s * L::STAGE_BYTES;
             if (elect_one()) {
                 mbar_expect_tx(full0 + 8 * s, L::TX_BYTES);
@@ -178,7 +178,7 @@ gemm_tc_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             for (int i = 0; i < nkb; ++i) {
                 const int s = i % STAGES;
                 const unsigned phase = (unsigned)(i / STAGES) & 1u;
-                if (!mbar_wait_warp(full0 + 8 * s, phase, err, 2)) break;
+                if (!mbar_wait_warp(full0 + 8 * s, phase, err, 102)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned a_addr = tiles0 + s * L::STAGE_BYTES;
                 const unsigned long long a = smem_desc(a_addr), b = smem_desc(a_addr + L::A_BYTES);
@@ -195,7 +195,7 @@ gemm_tc_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         // this block's accumulator: tensor memory -> shared memory, rows = rows of W, columns = tokens
         const int quarter = warp & 3;
         const int r = quarter * 32 + lane;
-        if (acc_ok) acc_ok = mbar_wait(acc_bar, 0, err, 3);
+        if (acc_ok) acc_ok = mbar_wait(acc_bar, 0, err, 103);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
         for (int c0 = 0; c0 < BN; c0 += (BN < 32 ? BN : 32)) {

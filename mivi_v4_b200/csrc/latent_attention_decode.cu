@@ -152,9 +152,9 @@ latent_attention_decode_kernel(const float* __restrict__ qa, const __nv_bfloat16
     __syncthreads();                                                    // the queries are there
     for (int it = 0; it < n_iter; ++it) {
         const int j0 = first + it * LK, stage = it & 1;
-        const bool ok = mbar_wait(bar0 + 8 * stage, (unsigned)(it >> 1) & 1u, err, 51);
+        const bool ok = mbar_wait(bar0 + 8 * stage, (unsigned)(it >> 1) & 1u, err, 45);
         if (!__all_sync(0xffffffffu, ok)) {
-            if (it + 1 < n_iter) mbar_wait(bar0 + 8 * (stage ^ 1), (unsigned)((it + 1) >> 1) & 1u, err, 51);   // its other copies
+            if (it + 1 < n_iter) mbar_wait(bar0 + 8 * (stage ^ 1), (unsigned)((it + 1) >> 1) & 1u, err, 45);   // its other copies
             break;
         }
         const __nv_bfloat16* kt = mine + (size_t)stage * WK * pitch;

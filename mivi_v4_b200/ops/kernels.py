@@ -2017,7 +2017,12 @@ def _link_args(x, M: int, N: int, K: int, mode: int, scale: Optional[NormLink], 
 
 _error_flags = {}
 _error_mirrors = {}
-_ERROR_ROLES = {1: "the TMA producer", 2: "the MMA issuer", 3: "the epilogue", 4: "a guarded index"}
+# what a kernel's bounded waits put into the error flag when they run out: ranges of codes, a kernel each (4: a guarded index of any kernel)
+_ERROR_CODES = (((1, 3), "gemm_tc.cu"), ((5, 5), "gemm_tc.cu"), ((11, 21), "attention_prefill_tc.cu"), ((30, 40), "attention_decode_tc.cu"),
+                ((45, 45), "latent_attention_decode.cu"), ((51, 63), "latent_attention_tc.cu"), ((71, 76), "gemm_f32_tc.cu"),
+                ((81, 93), "attention_sink_tc.cu"), ((101, 103), "gemm_tc_swap.cu"), ((111, 115), "gemm_tc_pair.cu"))
+# the products' roles, by the last digit
+_ERROR_ROLES = {1: "the TMA producer", 2: "the MMA issuer", 3: "the epilogue", 5: "the MMA issuer (for the epilogue)"}
 
 
 def _error_flag(device) -> torch.Tensor:
@@ -2030,12 +2035,13 @@ def _error_flag(device) -> torch.Tensor:
 
 
 def _error_text(key: int, code: int) -> str:
-    role = _ERROR_ROLES.get(code, f"code {code}")
     if code == 4:
         return (f"a kernel on cuda:{key} was handed an index outside its bounds (a page or a slot); it skipped "
                 f"the access and its output is not valid")
-    return (f"a tensor-core kernel on cuda:{key} gave up waiting on a barrier in {role}; "
-            f"its output is not valid")
+    source = next((name for (low, high), name in _ERROR_CODES if low <= code <= high), None)
+    role = _ERROR_ROLES.get(code % 10) if source and source.startswith("gemm_tc") else None
+    return (f"a tensor-core kernel on cuda:{key} gave up waiting on a barrier in {role or 'one of its warps'} "
+            f"({source or 'unknown'}, code {code}); its output is not valid")
 
 
 def note_device_errors(device) -> None:

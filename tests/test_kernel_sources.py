@@ -37,3 +37,17 @@ def test_tensor_memory_is_accessed_by_whole_warps():
             if not text[:m.start()].rstrip().endswith("__syncwarp();"):
                 found.append(f"{name}: {m.group(1)[:60]}")
     assert not found and seen > 10, found
+
+
+def test_error_codes_name_their_kernel():
+    """Every bounded wait's code belongs to one kernel, and the error's text names it; 4 is a guarded index."""
+    from mivi_v4_b200.ops.kernels import _error_text
+    codes = {}
+    for name, text in sources():
+        for m in re.finditer(r"\berr, (\d+)\)", text):
+            codes.setdefault(int(m.group(1)), set()).add(name)
+    assert codes.pop(4) == {"common.cuh"} and len(codes) > 40
+    for code, files in codes.items():
+        assert len(files) == 1 and f"({min(files)}, code {code})" in _error_text(0, code), (code, files)
+        assert "outside its bounds" not in _error_text(0, code)
+    assert "outside its bounds" in _error_text(0, 4) and "unknown" in _error_text(0, 999)
