@@ -1332,18 +1332,27 @@ def attention_sink_prefill_supported(dtype: torch.dtype, dk: int, dv: int) -> bo
             and 16 <= dv <= PREFILL_ATTENTION_MAX_HEAD_DIM)
 
 
-# The tcgen05 kernel's blocks are 128 query tokens of one sequence and two heads: it takes steps whose sequences fill most of a tile and that have enough
-# of them for the device (its bits are the other kernel's).  This kernel / the other, us, 32 heads of 64 with chunks of 1,024, of 80 / 64 with a cap and a
-# window of 1,024, and of 64 with a cap and a table by distance and split weights: one prompt of 512 tokens 16 / 21, 24 / 25, 35 / 29; four of 300
-# 20 / 25, 27 / 28, 40 / 34; 16 of 96 20 / 25, 24 / 29, 32 / 33; 32 of 64 32 / 28, 36 / 30, 44 / 32; 32 of 128 44 / 50, 53 / 55, 67 / 64; behind 1,000
-# earlier tokens 8 times 128 38 / 60, 48 / 103, 63 / 118.
+# The tcgen05 kernel's blocks are 128 query tokens of one sequence and two heads, one a multiprocessor (its bits are the other kernel's).  This kernel / the other, us, cold
+# caches, heads of 64 with chunks of 1,024, of 80 / 64 with a cap and a window of 1,024, and of 64 with a cap, a table by distance and split weights:
+#   32 heads: one prompt of 512 tokens 23 / 25, 29 / 31, 39 / 33; of 2,048 39 / 69, 83 / 115, 103 / 161; 16 of 96 27 / 31, 31 / 33, 39 / 39; 32 of 64 42 / 35, 45 / 37,
+#   53 / 39; 32 of 128 54 / 56, 62 / 62, 76 / 70; 8 heads: one of 1,280 31 / 38, 51 / 49, 64 / 59; of 2,048 31 / 41, 51 / 53, 90 / 92; 32 of 128 18 / 23, 20 / 25, 25 / 27.
+# Sequences of less than 96 tokens leave most of a tile empty.  Steps of 1,280 tokens go there, but not where short sequences leave the device half empty: that is bound by the
+# length of one block, which is the longer one here (16 of 96 with 8 heads 14 / 14, 16 / 16, 20 / 18, with 2 heads 16 / 14, 16 / 14, 21 / 16; 32 of 128 with 2 heads 16 / 16,
+# 18 / 17, 21 / 18).  Below that, steps whose blocks are one round that fills most of the device (32 heads: 8 of 128 18 / 21, 19 / 24, 23 / 28, behind 1,000 earlier tokens
+# 45 / 64, 54 / 111, 66 / 125; one of 1,024 33 / 45, 48 / 54, 57 / 59; 4 of 256 18 / 23, 23 / 25, 30 / 30); with 48 heads 8 of 128 are a round and a third, 28 / 25, 31 / 27, 40 / 32.
 SINK_TC_TOKENS, SINK_TC_ALL = 96, 1280
 
 
-def sink_tc_takes(N: int, n_seqs: int, nh: int, nkv: int, dk: int, dv: int, page_size: int) -> bool:
+def sink_tc_takes(N: int, n_seqs: int, nh: int, nkv: int, dk: int, dv: int, page_size: int, sms: int = 148) -> bool:
     """Whether the tcgen05 kernel takes a step of ``N`` tokens of ``n_seqs`` sequences."""
-    return (N >= max(SINK_TC_TOKENS * n_seqs, SINK_TC_ALL) and nh % (2 * nkv) == 0 and dk <= 128 and dv <= 64 and page_size % 64 == 0
-            and (N + 127) // 128 + n_seqs <= 65535)
+    if not (nh % (2 * nkv) == 0 and dk <= 128 and dv <= 64 and page_size % 64 == 0 and (N + 127) // 128 + n_seqs <= 65535):
+        return False
+    if N < SINK_TC_TOKENS * n_seqs or 5 * N < 4 * SINK_TC_ALL:
+        return False
+    if N >= SINK_TC_ALL:
+        return N >= 512 * n_seqs or N * nh >= 19 * SINK_TC_ALL
+    blocks = n_seqs * -(-N // (128 * n_seqs)) * nh // 2
+    return 0.8 * sms <= blocks <= sms
 
 
 def attention_sink_prefill(q: torch.Tensor, pool: torch.Tensor, page_size: int, page_table, cu, starts,
@@ -1378,7 +1387,7 @@ def attention_sink_prefill(q: torch.Tensor, pool: torch.Tensor, page_size: int, 
              dist, dist_len, int(bool(values_in_keys)), int(bool(gate_wide)),
              _need(out_all, "attention out of all kv heads", torch.float32, (N, nh, nkv, dv), True), int(bool(split_weights)))
     qp, pp = _need(q, "q", None, (N, nh * dk)), _need(pool, "cache pool")
-    if sink_tc_takes(N, n_seqs, nh, nkv, dk, dv, page_size) and pool.stride(0) % 8 == 0 and not any(
+    if sink_tc_takes(N, n_seqs, nh, nkv, dk, dv, page_size, n_sms()) and pool.stride(0) % 8 == 0 and not any(
             t is not None and t.data_ptr() % 16 for t in (q, pool, out, out_all)):
         _guard("bf16", "attention_sink_tc", q.device, n_pages=pool.shape[0])
         _check(_fn("bf16", "mv_attention_sink_tc")(qp, pp, pool.shape[0], pool.stride(0), *shape, _error_flag(q.device).data_ptr(), _stream()),
@@ -1593,17 +1602,28 @@ def latent_prefill_fits(dim: int, rot: int, dv: int, rank: int) -> bool:
         and 16 <= dv <= 128 and rank % 8 == 0
 
 
-# The tcgen05 kernel's blocks are 256 query tokens of one sequence: it takes steps whose sequences fill such a block or have many keys (its bits are the
-# other kernel's).  32 heads of 64 + 32 / 64 with a gate, this kernel / the other: 32 prompts of 64 tokens 109 / 56 us, 32 of 128 123 / 96, 16 of 200
-# 82 / 95, 8 of 300 74 / 76, 4 of 256 27 / 44, one of 1,024 39 / 74, one of 6,000 363 / 1,132; behind 190 earlier tokens 16 times 64 tokens 72 / 51,
-# behind 300 8 times 128 tokens 45 / 66, behind 800 3 times 32 tokens 33 / 53.
+# The tcgen05 kernel's blocks are 256 query tokens of one sequence and a head, one a multiprocessor: it takes steps whose sequences fill such a block or have many keys (its
+# bits are the other kernel's).  64 + 32 / 64 with a gate, this kernel / the other, us, cold caches.  32 heads: 32 prompts of 64 tokens 111 / 55, 32 of 128 129 / 96, 16 of 200 82 / 94, 8 of
+# 300 76 / 76, one of 200 23 / 25, of 512 29 / 37, of 1,024 40 / 74, of 2,048 72 / 193; 8 heads: 32 of 128 41 / 39, 16 of 200 27 / 41, one of 200 23 / 23, of 2,048 56 / 92.  Behind earlier
+# tokens, 32 heads: 8 of 128 behind 300 47 / 64, 16 of 64 behind 190 76 / 51, 3 of 32 behind 800 31 / 47.  A sequence of at most 64 tokens is one short tile for the other kernel and a whole block
+# here: with many of them the rounds of blocks decide, each some 13 us and 15.5 us for 1,000 keys, against 0.15 (16 tokens) to 0.2 us for a tile and
+# 1,000 keys, and at least 14 us and 35 us for 1,000 keys: 32 of 16 behind 800 184 / 127, with 8 heads 57 / 47; 16 of 32 behind 800 107 / 92, with 8 heads 33 / 49; 8 of 32 behind 500 50 / 41; 16 of
+# 64 behind 800 113 / 104; 16 of 48 behind 2,000 172 / 197; 16 of 96 behind 800 113 / 158.
 LATENT_TC_TOKENS, LATENT_TC_ROWS = 200, 400
 
 
-def latent_tc_takes(N: int, rows: int, n_seqs: int, dim: int, rot: int, dv: int, scale: float) -> bool:
+def latent_tc_takes(N: int, rows: int, n_seqs: int, dim: int, rot: int, dv: int, scale: float, nh: int = 32, sms: int = 148) -> bool:
     """Whether the tcgen05 kernel takes a step of ``N`` tokens of ``n_seqs`` sequences that see ``rows`` cached rows."""
-    return (dim == 64 and rot in (32, 64) and dv == 64 and scale > 0 and (N + 255) // 256 + n_seqs <= 65535 and rows < 2 ** 31
-            and (N >= LATENT_TC_TOKENS * n_seqs or rows >= LATENT_TC_ROWS * n_seqs))
+    if not (dim == 64 and rot in (32, 64) and dv == 64 and scale > 0 and (N + 255) // 256 + n_seqs <= 65535 and rows < 2 ** 31):
+        return False
+    if N >= LATENT_TC_TOKENS * n_seqs:
+        return True
+    if rows < LATENT_TC_ROWS * n_seqs:
+        return False
+    if N > 64 * n_seqs:
+        return True
+    keys, blocks = rows / n_seqs / 1000.0, n_seqs * nh
+    return -(-blocks // sms) * (13.0 + 15.5 * keys) < max(14.0 + 35.0 * keys, blocks * keys * (0.15 if N <= 16 * n_seqs else 0.2))
 
 
 def latent_query(proj: torch.Tensor, q0: int, inv_freq: Optional[torch.Tensor], positions, q: torch.Tensor, nh: int,
@@ -1657,7 +1677,7 @@ def latent_attention_prefill(q: torch.Tensor, kx: torch.Tensor, v0: int, r: torc
         raise KernelError(f"latent_attention_prefill: keys and values {kx.dtype} {tuple(kx.shape)}, values from {v0}")
     per_head = gate is not None and gate.shape[1] == nh
     gp, ldg = _cols(gate, "latent_attention_prefill gate", N, nh if per_head else nh * dv) if gate is not None else (None, 0)
-    if latent_tc_takes(N, rows, n_seqs, dim, rot, dv, scale) and kx.stride(0) % 8 == 0 and v0 % 8 == 0 and not any(
+    if latent_tc_takes(N, rows, n_seqs, dim, rot, dv, scale, nh, n_sms()) and kx.stride(0) % 8 == 0 and v0 % 8 == 0 and not any(
             t.data_ptr() % 16 for t in (q, kx, r, out)):
         _check(_fn("bf16", "mv_latent_attention_tc")(
             _need(q, "q", torch.bfloat16, (N, nh, dim + rot)), kx.data_ptr(), rows, kx.stride(0), int(v0),

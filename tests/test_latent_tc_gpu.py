@@ -18,6 +18,16 @@ def test_which_steps_it_takes():
     assert not takes([199], [500], 100) and takes([200], [500], 100, rot=64) and not takes([200], [500], 100, rot=16)
 
 
+def test_steps_measured_on_both_sides_of_the_rule():
+    """(sequences, tokens of each, earlier ones, heads, whether it is the faster kernel)"""
+    from mivi_v4_b200.ops import kernels as K
+    for n, new, before, nh, there in [(1, 2048, 0, 8, True), (16, 200, 0, 32, True), (8, 128, 300, 32, True), (16, 96, 800, 32, True), (3, 32, 800, 32, True), (1, 64, 2000, 32, True),
+                                      (16, 32, 800, 8, True), (4, 16, 400, 32, True), (16, 48, 2000, 32, True), (16, 48, 2000, 16, True), (32, 64, 0, 32, False), (32, 128, 0, 32, False),
+                                      (16, 64, 190, 32, False), (32, 16, 800, 32, False), (32, 16, 800, 16, False), (32, 16, 800, 8, False), (16, 32, 800, 32, False), (16, 32, 800, 16, False),
+                                      (8, 32, 500, 32, False), (6, 32, 500, 32, False), (5, 16, 400, 32, False), (16, 64, 800, 32, False), (32, 64, 800, 32, False)]:
+        assert K.latent_tc_takes(n * new, n * (new + before), n, 64, 32, 64, 0.1, nh) == there, (n, new, before, nh)
+
+
 @gpu
 @pytest.mark.parametrize("lens,starts", [([1, 95, 96, 97, 300, 1000], [0, 5, 100, 0, 77, 3]), ([257, 640], [0, 0]), ([1, 31, 128], [700, 500, 383])])
 @pytest.mark.parametrize("window", [0, 37, 96, 500])

@@ -23,6 +23,14 @@ def test_which_steps_it_takes():
     assert not takes(n, 1, 4, 2, 64, 80, 64) and not takes(n, 1, 4, 2, 64, 64, 32) and not takes(n, 1, 4, 2, 144, 64, 64)
 
 
+def test_steps_measured_on_both_sides_of_the_rule():
+    """(tokens, sequences, heads, whether it is the faster kernel)"""
+    for N, n, nh, there in [(2048, 1, 32, True), (2048, 1, 8, True), (4096, 1, 2, True), (1024, 8, 32, True), (1024, 1, 32, True), (1024, 4, 32, True), (1536, 16, 32, True),
+                            (1536, 16, 16, True), (4096, 32, 8, True), (1024, 8, 48, False), (1200, 4, 32, False), (1024, 8, 16, False), (1536, 16, 8, False), (1536, 16, 2, False),
+                            (4096, 32, 2, False), (2048, 32, 32, False), (512, 1, 32, False), (256, 1, 128, False)]:
+        assert K().sink_tc_takes(N, n, nh, nh // 2, 64, 64, 64) == there, (N, n, nh)
+
+
 def case(lens, starts, nh, nkv, dk, dv, page, seed, v_in_k=False, tail=None):
     g = torch.Generator().manual_seed(seed)
     total = [a + n for a, n in zip(starts, lens)]
