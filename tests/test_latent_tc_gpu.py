@@ -34,13 +34,14 @@ def test_steps_measured_on_both_sides_of_the_rule():
 @pytest.mark.parametrize("rot,sink,gate", [(32, True, "element"), (64, False, None), (32, True, "head")])
 def test_against_64_bits_and_the_other_kernel(lens, starts, window, rot, sink, gate, monkeypatch):
     from mivi_v4_b200.ops import kernels as K
-    if not takes(lens, starts, window):
-        window = 0
     nh = 3
     q, k, v, r, sinks, gates = inputs(lens, starts, nh, 64, rot, 64, window, seed=window + rot)
     sinks = sinks if sink else None
     gates = {None: None, "element": gates, "head": gates[:, :, :1]}[gate]
-    got = attend(slice(0, nh), lens, starts, window, q, k, v, r, sinks, gates)
+    with monkeypatch.context() as m:                           # (short sequences behind a window would take the other kernel)
+        m.setattr(K, "LATENT_TC_TOKENS", 1)
+        assert takes(lens, starts, window, rot)
+        got = attend(slice(0, nh), lens, starts, window, q, k, v, r, sinks, gates)
     with monkeypatch.context() as m:                           # every sum in the other kernel's order: the same bits
         m.setattr(K, "LATENT_TC_TOKENS", 1 << 30)
         m.setattr(K, "LATENT_TC_ROWS", 1 << 30)
