@@ -22,9 +22,8 @@
 // NaNs, operands from 2^88 on and sums from 2^50 on end as results that are not finite: these, and no others, are worked out again by float32
 // multiply-adds, in a function of its own that leaves the others' way its registers.
 //
-// Bound by the splitting (some 560 instructions of every scheduler a stage, and waits: 0.58 us for 128 x 96, 0.8 for 128 x 128), then by shared memory (a stage of
-// 128 columns writes and reads 32 KB of float32 tiles, writes 24 KB and has the products read 48 KB of W's planes: 1,060 clocks beside the products'
-// 780).  1,165 rows against 9,216 x 1,024 516 -> 129 us (170 TFLOP/s), against 1,024 x 4,608 280 -> 86.  With X's planes in shared memory too, which the products then read at all
+// Bound by the splitting and its waits (720 instructions of every scheduler in a stage's 1,375 clocks for 128 x 128, 580 in 1,060 for 128 x 96; tensor cores busy 55 and 41 %), then by
+// shared memory (a stage of 128 columns writes and reads 32 KB of float32 tiles, writes 24 KB and has the products read 48 KB of W's planes: 1,060 clocks at 128 bytes a clock).  1,165 rows against 9,216 x 1,024 516 -> 129 us (170 TFLOP/s), against 1,024 x 4,608 280 -> 86.  With X's planes in shared memory too, which the products then read at all
 // its bandwidth, 174 us; with the two groups of splitting warps on the same stage 145.
 #include "tc_common.cuh"
 

@@ -23,8 +23,8 @@
 // reference is its running maximum after every block; its denominator is four sums, of every eighth key and its neighbour.  Only the sink of a row whose keys are all far
 // below it (e^-60 of it) is left out of the reference, and joins at the end: nothing is lost where it is all that the row shows.
 //
-// Bound by the softmax (a block of 64 keys of both tiles needs 1,024 clocks of the exponential unit and some 1,000 instructions of each
-// scheduler, and its products 1,100 clocks beside it).  32 heads of 64 + 32 / 64 with a gate, this kernel / latent_attention_prefill.cu: one prompt of 6,000 tokens
+// Bound by the softmax (a block of 64 keys of both tiles needs 1,024 clocks of the exponential unit at 16 a clock and some 1,000 instructions of each
+// scheduler; over one prompt of 2,048 tokens, whose tiles are two rounds of unequal length, schedulers 41 % busy, that unit 31 %, tensor cores 19 %).  32 heads of 64 + 32 / 64 with a gate, this kernel / latent_attention_prefill.cu: one prompt of 6,000 tokens
 // 372 / 1,132 us, of 2,048 73 / 190, three of 333 to 2,048 108 / 226.  What it took: an elected lane of a whole warp issues the products (see
 // tc_common.cuh; a first form of the kernel with a lane by itself 495 us), one warp for
 // either product (one for both: the waits of one hold up the other, 296 against 273 for a form of other sums), gates read 32 bytes at a time (a block's gates element by

@@ -1790,8 +1790,9 @@ def gemm_f32_tc_takes(M: int, N: int, K: int, sms: int) -> bool:
     """Whether a float32 product goes to the tensor cores (``gemm_f32_tc.cu``) or to the CUDA cores: by what either is expected to take, in us.  The
     tensor cores work in rounds of tiles of 128 x 128 or 128 x 96, 26.4 or 21.9 us for 1,024 of K whatever a tile's rows; the CUDA cores add
     up some 40e6 products a us, and lose about 32 rows to their tiles.  Measured (tensor / CUDA cores) on nine shapes at 9 to 1,165 rows, never the
-    slower one by more than a tenth: 9,216 x 1,024 at 16 rows 29 / 37, at 1,165 133 / 516; 1,024 x 4,608 at 128 rows 80 / 45, at 600 80 / 172; 6,144 x
-    2,048 at 32 rows 45 / 43, at 48 45 / 68.  From K = 1,024 on: below, sums are so short that float32 multiply-adds are as exact."""
+    slower one by more than a tenth: 9,216 x 1,024 at 16 rows 29 / 37, at 1,165 129 / 516; 1,024 x 4,608 at 128 rows 80 / 45, at 600 84 / 172; 6,144 x
+    2,048 at 32 rows 45 / 43, at 48 45 / 68.  From K = 1,024 on, where nearly all products of the float32 models lie.  (Shorter ones would gain too: 9,216 x 512 at
+    1,165 rows 81 / 265, 1,024 x 256 14 / 23, at 128 rows 9,216 x 256 15 / 25, error 0.8e-7 / 2.0e-7 at K = 256, 0.9e-7 / 2.9e-7 at 512; they were left as they are.)"""
     if M < F32_TC_ROWS or K < F32_TC_K or K % 4 or M > 65535 * 128:
         return False
     rows = -(-M // 128)
@@ -1802,7 +1803,8 @@ def gemm_f32_tc_takes(M: int, N: int, K: int, sms: int) -> bool:
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, bias: Optional[torch.Tensor] = None,
               accumulate: bool = False) -> torch.Tensor:
     """out = x @ w.T (+ bias), or out += ... when ``accumulate`` (out float32).
-    CUDA-core kernels, float32 accumulation, any sizes; large float32 products on the tensor cores, no less exact."""
+    CUDA-core kernels, float32 accumulation, any sizes; large float32 products on the tensor cores (``gemm_f32_tc.cu`` says how exact: more so where terms
+    have both signs, by half of float32's last place less where all have one)."""
     M, K = x.shape
     N, K2 = w.shape
     if K != K2:

@@ -3,7 +3,8 @@ dtype and shape.  All kernels are this library's own; none is a vendor library
 call.
 
 float32 operands take the CUDA-core kernel (true 32-bit products and
-sums) or, where they are large, the tensor cores with every operand as three bfloat16 numbers (no less exact).  bfloat16 operands take the tensor-core kernels where their shape
+sums) or, where they are large, the tensor cores with every operand as three bfloat16 numbers
+(the more exact of the two for terms of both signs).  bfloat16 operands take the tensor-core kernels where their shape
 rules hold and the CUDA-core kernel otherwise.  A weight that the checkpoint
 stores in 32-bit stays so; a bfloat16 activation is widened for it.
 """
